@@ -220,9 +220,11 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials,
  * psr_dedisperse_trials, searches and sessions treats samples stored in 8
  * bits (<= 8-bit data).  0: every channel added to every trial; 4 or 8:
  * channels in subbands of that width, each subband's partial sum formed once
- * per distinct intra-subband delay pattern of 8 consecutive trials and added
- * shifted to every trial that shares it (identical results); -1 (initial):
- * the library default.  Process-wide; affects searches prepared afterwards. */
+ * per distinct intra-subband delay pattern of a block of trials and added
+ * shifted to every trial that shares it (identical results; a plan whose
+ * patterns repeat too little falls back to 0); -1 (initial): the cheapest of
+ * the three for the plan.  Process-wide; affects searches prepared
+ * afterwards. */
 int psr_set_dedisp_subbands(int subbands);
 
 /* Test hook, no reference counterpart: one dedispersion launch (DM 0, up to

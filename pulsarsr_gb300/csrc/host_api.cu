@@ -771,8 +771,8 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
   PSR_TRY(err.ensure(8));
   PSR_CUDA(cudaMemsetAsync(err.p, 0, 8, st));
   SubbandPlan sbp;
-  const int G = o.kind == SAMPLE_U8 ? dedisp_subbands_default(o) : 0;
-  PSR_TRY(build_subband_plan(tab, o.nch, {0, ntrials}, G, sbp, st));
+  PSR_TRY(build_subband_plan(tab, o.nch, length, o.kind == SAMPLE_U8 ? o.max_value() : 0.0,
+                             {0, ntrials}, dedisp_subbands_default(o), sbp, st));
   PSR_TRY(launch_dedisperse_ex(o, dd.as<uint32_t>(), ntrials, length, ser.as<float>(), ldo,
                                parts.as<double>(), sums.as<double>(), means.as<float>(), spread,
                                err.as<unsigned>(), st, 0, 0, sums_out != nullptr, &sbp, 0));

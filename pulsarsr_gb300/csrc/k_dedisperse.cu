@@ -370,253 +370,342 @@ __global__ void __launch_bounds__(DD_NT, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Subband reuse (u8 samples, 16-bit lanes).  Channels are taken in subbands
-// of G adjacent channels.  For one block of SB_TB consecutive trials, the
-// delays of a subband's channels relative to its smallest delay form a
-// pattern; trials that share a pattern share the subband's partial series
-// up to a shift.  The plan (host, per block and subband) lists the distinct
-// patterns.  Stage A forms each pattern's partial sum over the tile (plus
-// the shift range) once in shared memory; stage B adds it, shifted, into
-// every trial that uses it.  A subband whose patterns do not repeat enough to
-// pay for stage A is added channel by channel (direct).  Every sum is an
-// integer below 2^16 in its lane, so the result is bit-identical to the
-// reference's channel-ordered f32 sum.
-constexpr int SB_TB = 8;    // trials per CTA
-constexpr int SB_PMAX = 4;  // patterns per subband held in shared memory
-constexpr int SB_GMAX = 8;
+// Two-level dedispersion of u8 samples.  Channels are taken in subbands of G
+// adjacent channels.  A trial's delays inside a subband, relative to the
+// subband's smallest delay, form a pattern; over a chunk of trials the same
+// patterns come back (DM plans of about one sample per trial have 4 to 30 of
+// them per subband and 256 trials), so
+//   k_sub_part  sums each pattern's G channels once per chunk, over the whole
+//               series (16-bit sums, rows of a scratch buffer), and
+//   k_sub_sum   adds, for every trial, one row per subband at the trial's
+//               shift.
+// Every sum is an integer (below 2^16 in its lane, below 2^24 in all), so
+// the result is bit-identical to the reference's channel-ordered f32 sum.
+constexpr int SUB_GMAX = 8;
+constexpr int SP_NT = 256;              // k_sub_part: threads
+constexpr int SP_TT = SP_NT * 16;       // and samples per tile (4 words of 4 per thread)
+constexpr int SS_TB = 16;               // k_sub_sum: trials per CTA, one warp each
+constexpr int SS_K = 16;                // 32-bit words (sample pairs) per lane
+constexpr int SS_TT = 32 * SS_K * 2;    // samples per tile (1024)
+constexpr int SS_NT = 32 * (SS_TB + 1); // and a warp that issues the copies
+constexpr int SS_MAXROWS = 64;          // rows of a stage (two per issuing lane)
+constexpr int SS_MAXBUF = 4;            // stage buffers
+constexpr int SS_MAXSTAGES = 1024;      // stages of a trial block
 
-struct SbEntry {
-  int32_t dref_min;               // smallest subband reference delay in the block
-  uint8_t npat, pad0, pad1, pad2;  // npat = 0: direct
-  uint8_t pid[SB_TB];             // pattern of each trial
-  uint16_t roff[SB_TB];           // reference delay - dref_min, per trial
-  uint16_t lo[SB_PMAX], hi[SB_PMAX];  // roff range of each pattern's trials
-  uint16_t rel[SB_PMAX][SB_GMAX];     // channel delay - reference delay
+// A subband of one chunk: its patterns are rows [row0, row0 + npat) of the
+// chunk's scratch; row sample i is series time i + seg0 of a trial whose
+// smallest subband delay is dmin.
+struct SubBand {
+  int32_t dmin, spread, row0, npat, relmax, pad;
 };
-static_assert(sizeof(SbEntry) == 112, "plan entry layout");
-
-// acc (16-bit lanes: acc[i] = samples 2i | 2i+1 << 16) += the 16 bytes of
-// `row` starting at byte `off` (thread's own 16 samples: off includes 16 tl).
-__device__ __forceinline__ void add_bytes16(const uint4 *row16, int off, uint32_t *acc) {
-  const int q = off >> 4, o = off & 15;
-  const uint4 lo = row16[q], hi = row16[q + 1];
-  uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x, w5 = hi.y, w6 = hi.z,
-           w7 = hi.w;
-  if (o & 8) {
-    w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = w6; w5 = w7;
-  }
-  if (o & 4) {
-    w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5;
-  }
-  const unsigned sh = (unsigned)(o & 3) * 8u;
-  const uint32_t x0 = __funnelshift_r(w0, w1, sh), x1 = __funnelshift_r(w1, w2, sh),
-                 x2 = __funnelshift_r(w2, w3, sh), x3 = __funnelshift_r(w3, w4, sh);
-  acc[0] += __byte_perm(x0, 0, 0x4140);
-  acc[1] += __byte_perm(x0, 0, 0x4342);
-  acc[2] += __byte_perm(x1, 0, 0x4140);
-  acc[3] += __byte_perm(x1, 0, 0x4342);
-  acc[4] += __byte_perm(x2, 0, 0x4140);
-  acc[5] += __byte_perm(x2, 0, 0x4342);
-  acc[6] += __byte_perm(x3, 0, 0x4140);
-  acc[7] += __byte_perm(x3, 0, 0x4342);
+// A stage of k_sub_sum, packed: the next nrows (bits 0-7) rows of the trial
+// block's row list, the next nsubs (bits 8-15) subbands, and a flush after it
+// (bit 16).
+constexpr uint32_t sub_stage(int nrows, int nsubs, int flush) {
+  return (uint32_t)nrows | (uint32_t)nsubs << 8 | (uint32_t)flush << 16;
 }
+// A staged row: a scratch row and the first sample copied.
+struct SubRow {
+  uint32_t row, start;  // start: a multiple of 8 samples (16 bytes)
+};
 
-// acc += 16 u16 samples of `pb` starting at sample j (any j >= 0).
-__device__ __forceinline__ void add_u16x16(const uint16_t *pb, int j, uint32_t *acc) {
-  const int w = j >> 1;  // first word
-  const uint4 *p4 = reinterpret_cast<const uint4 *>(pb) + (w >> 2);
-  const uint4 a = p4[0], b = p4[1], c = p4[2];
-  uint32_t x[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
-  const int e = w & 3;  // words x[e .. e+8] are needed
-  if (e & 2) {
-#pragma unroll
-    for (int i = 0; i < 10; ++i) x[i] = x[i + 2];
-  }
-  if (e & 1) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) x[i] = x[i + 1];
-  }
-  const unsigned sh = (unsigned)(j & 1) * 16u;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] += __funnelshift_r(x[i], x[i + 1], sh);
-}
-
-template <int G>
-__global__ void __launch_bounds__(DD_NT, 2)
-    k_dedisp_sb(const uint8_t *__restrict__ s, uint64_t ld, uint64_t ns, uint64_t nch,
-                uint64_t dstride, const uint32_t *__restrict__ delays, uint64_t ntrials,
-                uint64_t n, float *__restrict__ out, uint64_t ldo, double *__restrict__ part,
-                uint64_t ntiles, int cc, int rowcap, int accumulate, unsigned *err,
-                long long spin_limit, const SbEntry *__restrict__ plan, uint64_t nsub_total,
-                uint64_t sb0, uint64_t block0, int sbstride) {
-  static_assert(G <= SB_GMAX, "subband width");
+// Bound: shared memory and issue, about 22 instructions per 16 samples of a
+// pattern's channel (8 word loads, 4 funnel shifts, then 4 byte-lane adds or,
+// above 255, per word one full add and one add of the odd bytes: with
+// T = sum of the words mod 2^32 and O = sum of the odd bytes in 16-bit lanes,
+// the even bytes' sum is T - (O << 8)).
+// Measured on a GB300 with k_sub_sum below, against the channel-by-channel
+// kernel (and, at 4096 channels, the subband kernel that summed patterns per
+// 8 trials in shared memory): 96 4-bit channels, 2000 trials of 263,500
+// samples 0.60 + 1.58 ms against 3.22; 512 8-bit channels, 700 trials of
+// 523,500 samples 0.63 + 4.17 against 12.95; 4096 8-bit channels, 300 trials
+// of 1,045,000 samples 6.9 + 27.9 against 124 (118).
+template <int G, bool BYTE>
+__global__ void __launch_bounds__(SP_NT)
+    k_sub_part(const uint8_t *__restrict__ s, uint64_t ld, uint64_t ns, uint64_t nch,
+               const SubBand *__restrict__ subs, const uint16_t *__restrict__ rel,
+               uint64_t seg0, uint64_t seglen, uint16_t *__restrict__ scratch, uint64_t ldp,
+               int rowcap, unsigned *err, long long spin_limit) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const size_t bstride = (size_t)cc * rowcap;
-  uint16_t *pbuf = reinterpret_cast<uint16_t *>(smem + 2 * bstride);
-  __shared__ uint64_t bars[2];
-  __shared__ StageInfo info[2];
-  __shared__ unsigned long long wsum[DD_NT / 32][SB_TB];
-  // the plan entries of each staged chunk's subbands, copied with its rows
-  __shared__ __align__(16) SbEntry ents[2][DD_MAXCC / 4];
-
-  const uint64_t t0 = (uint64_t)blockIdx.x * DD_TT;
-  const uint64_t d0 = (uint64_t)blockIdx.y * SB_TB;
+  __shared__ uint64_t bar;
+  const SubBand sb = subs[blockIdx.y];
+  const uint64_t i0 = (uint64_t)blockIdx.x * SP_TT;
+  if (i0 >= seglen + (uint64_t)sb.spread + 2) return;  // (uniform) past every trial's last sample
   const int tl = threadIdx.x;
-  const int nchunks = (int)((nch + cc - 1) / cc);
-  const SbEntry *pl = plan + (block0 + blockIdx.y) * nsub_total + sb0;
-
+  const uint64_t c0 = (uint64_t)blockIdx.y * G;
+  const int gr = (int)min((uint64_t)G, nch - c0);
+  const uint64_t abs0 = seg0 + i0 + (uint64_t)sb.dmin;
+  const uint64_t a = abs0 & ~15ull;
   if (tl == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
+    mbar_init(&bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // Entries of chunk k: subbands [k cc / G, ...) of this block, contiguous in
-  // the plan; lane 0 copies them on the chunk's barrier before the rows'
-  // copies complete it.
-  auto stage_entries = [&](int k, int b) {
-    if (tl == 0) {
-      const uint64_t e0 = ((uint64_t)k * cc) / G;
-      const uint64_t ne = (min((uint64_t)cc, nch - (uint64_t)k * cc) + G - 1) / G;
-      const unsigned bytes = (unsigned)(ne * sizeof(SbEntry));
-      mbar_expect_tx(&bars[b], bytes);
-      bulk_g2s(&ents[b][0], pl + e0, bytes, &bars[b]);
+  if (tl < 32) {
+    const uint64_t rowend = (ns + 15) & ~15ull;
+    // + 4: the last word's funnel shift reads one word on
+    uint64_t b = (abs0 + SP_TT + (uint64_t)sb.relmax + 4 + 15) & ~15ull;
+    b = min(min(b, rowend), a + (uint64_t)rowcap);
+    if (tl < gr && b > a) mbar_expect_tx(&bar, (unsigned)(b - a));
+    __syncwarp();
+    if (tl < gr && b > a)
+      bulk_g2s(smem + (size_t)tl * rowcap, s + (c0 + tl) * ld + a, (unsigned)(b - a), &bar);
+    __syncwarp();
+    if (tl == 0) mbar_arrive(&bar);
+  }
+  const bool ok = mbar_wait_bounded(&bar, 0, err, spin_limit);
+  if (__syncthreads_or(!ok)) {
+    if (tl == 0) mbar_wait_bounded(&bar, 0, err, spin_limit);
+    return;
+  }
+  const uint16_t *rp = rel + (size_t)sb.row0 * G;
+  uint16_t *dst = scratch + (uint64_t)sb.row0 * ldp + i0 + 4 * tl;
+  const int base = (int)(abs0 - a);
+  uint16_t rn[G];
+  auto load_rel = [&](const uint16_t *q) {  // rows of the table are 2 G bytes, aligned
+    if constexpr (G == 8) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(q));
+      memcpy(rn, &v, 16);
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2 *>(q));
+      memcpy(rn, &v, 8);
     }
   };
-  if (tl < 32) {
-    stage_entries(0, 0);
-    issue_stage<SB_TB>(s, ld, ns, nch, dstride, delays, ntrials, d0, t0, 0, cc, smem, rowcap,
-                       &info[0], &bars[0], 0);
-    if (nchunks > 1) {
-      stage_entries(1, 1);
-      issue_stage<SB_TB>(s, ld, ns, nch, dstride, delays, ntrials, d0, t0, (uint64_t)cc, cc,
-                         smem + bstride, rowcap, &info[1], &bars[1], 0);
+  load_rel(rp);
+  for (int p = 0; p < sb.npat; ++p) {
+    int off[G];
+#pragma unroll
+    for (int r = 0; r < G; ++r) off[r] = base + (int)rn[r];
+    if (p + 1 < sb.npat) load_rel(rp + (size_t)(p + 1) * G);
+    uint32_t T[4] = {0, 0, 0, 0}, O[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      if (r < gr) {
+        const uint32_t *q =
+            reinterpret_cast<const uint32_t *>(smem + (size_t)r * rowcap) + tl + (off[r] >> 2);
+        const unsigned sh = (unsigned)(off[r] & 3) * 8u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t x = __funnelshift_r(q[256 * k], q[256 * k + 1], sh);
+          T[k] += x;
+          if constexpr (!BYTE) O[k] += __byte_perm(x, 0, 0x4341);
+        }
+      }
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint2 w;
+      if constexpr (BYTE) {
+        w.x = __byte_perm(T[k], 0, 0x4140);
+        w.y = __byte_perm(T[k], 0, 0x4342);
+      } else {
+        const uint32_t E = T[k] - (O[k] << 8);  // samples 0 and 2; O: samples 1 and 3
+        w.x = __byte_perm(E, O[k], 0x5410);
+        w.y = __byte_perm(E, O[k], 0x7632);
+      }
+      *reinterpret_cast<uint2 *>(dst + 1024 * k) = w;
+    }
+    dst += ldp;
   }
-  uint32_t acc[SB_TB][8];
-#pragma unroll
-  for (int d = 0; d < SB_TB; ++d)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[d][i] = 0;
+}
 
-  int failed = -1;
-  bool pending = false;  // the pattern buffers hold partials some thread may still read
-  for (int k = 0; k < nchunks; ++k) {
-    const int b = k & 1;
-    const bool ok = mbar_wait_bounded(&bars[b], (unsigned)((k >> 1) & 1), err, spin_limit);
-    if (__syncthreads_or(!ok)) {
-      failed = k;
-      break;
+// One warp per trial: lane l owns the sample pairs (words) l + 32 k of the
+// tile.  A row at an even shift adds its words as they lie (E).  At an odd
+// shift 2 m + 1 the words from m on are added as they lie too, into O: a
+// pair's odd-shift sum is the high half of O's word and the low half of the
+// next, so the odd shifts cost one realignment per trial (or flush) instead
+// of one per row.  FLUSH: the sums pass 16 bits; stages marked by the plan
+// add the lanes to 32-bit sums.
+// The rows arrive in a ring of nbuf stage buffers: the last warp issues the
+// bulk copies of a stage once all trial warps have left its buffer, with the
+// row list read two stages ahead.  Waits are bounded; one that gives up sets
+// the error word and `dead`, on which every warp leaves, the issuing warp
+// last, after the copies it has in flight.
+// Bound: the staged rows, about 5 TB/s of bulk copies out of L2 (a row serves
+// the trials of its block that share the pattern, 4 to 5 of 16 at G = 4), then
+// shared-memory loads, 2 bytes per (trial, subband, sample), two instructions
+// per word.  With the copies issued by a trial warp between two CTA barriers
+// and two buffers the 4096-channel case took 50.5 ms, with the ring 27.9.
+template <bool FLUSH>
+__global__ void __launch_bounds__(SS_NT, FLUSH ? 1 : 2)
+    k_sub_sum(const uint16_t *__restrict__ scratch, uint64_t ldp,
+              const uint32_t *__restrict__ stage0, const uint32_t *__restrict__ row0,
+              const uint32_t *__restrict__ stages, const SubRow *__restrict__ rows,
+              const uint32_t *__restrict__ info, uint64_t nsub, uint64_t ntrials, uint64_t seg0,
+              uint64_t segend, float *__restrict__ out, uint64_t ldo, double *__restrict__ part,
+              uint64_t ntiles, int rowcap, int bufbytes, int nbuf, unsigned *err,
+              long long spin_limit) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t full[SS_MAXBUF], empty[SS_MAXBUF];
+  __shared__ uint32_t desc[SS_MAXSTAGES];
+  __shared__ volatile int dead;
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+  const uint64_t tb = blockIdx.x;
+  const uint64_t tile0 = (uint64_t)blockIdx.y * SS_TT;  // from seg0
+  const uint32_t st0 = stage0[tb];
+  const int nst = (int)(stage0[tb + 1] - st0);
+  for (int i = threadIdx.x; i < nst; i += SS_NT) desc[i] = stages[st0 + i];
+  if (threadIdx.x == 0) {
+    dead = 0;
+    for (int i = 0; i < nbuf; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], SS_TB);
     }
-    const uint64_t c0 = (uint64_t)k * cc;
-    const int rows = (int)min((uint64_t)cc, (uint64_t)(nch - c0));
-    const uint8_t *buf = smem + b * bstride;
-    for (int j0 = 0; j0 < rows; j0 += G) {
-      const int gr = min(G, rows - j0);
-      const SbEntry &ent = ents[b][j0 / G];
-      const int npat = ent.npat;
-      if (npat == 0) {
-        for (int r = j0; r < j0 + gr; ++r) {
-          const uint4 *row16 = reinterpret_cast<const uint4 *>(buf + (size_t)r * rowcap);
-#pragma unroll
-          for (int d = 0; d < SB_TB; ++d) add_bytes16(row16, info[b].off[r][d] + 16 * tl, acc[d]);
-        }
-        continue;
-      }
-      // Stage A: pattern partials over [lo, hi + tile) of the reference delay,
-      // once every thread is done reading the previous subband's partials.
-      if (pending) __syncthreads();
-      for (int p = 0; p < npat; ++p) {
-        const int lo = ent.lo[p];
-        const int ngr = (DD_TT + (ent.hi[p] - lo) + 15) >> 4;
-        uint16_t *dst = pbuf + (size_t)p * sbstride;
-        for (int g = tl; g < ngr; g += DD_NT) {
-          uint32_t a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-          for (int r = 0; r < gr; ++r) {
-            const long long abs0 = (long long)t0 + ent.dref_min + lo + 16 * g + ent.rel[p][r];
-            const int off = (int)(abs0 - info[b].base[j0 + r]);
-            add_bytes16(reinterpret_cast<const uint4 *>(buf + (size_t)(j0 + r) * rowcap), off, a);
-          }
-          uint4 *d4 = reinterpret_cast<uint4 *>(dst + 16 * g);
-          d4[0] = make_uint4(a[0], a[1], a[2], a[3]);
-          d4[1] = make_uint4(a[4], a[5], a[6], a[7]);
-        }
-      }
-      __syncthreads();
-      // Stage B: every trial adds its pattern's partial at its shift.
-#pragma unroll
-      for (int d = 0; d < SB_TB; ++d) {
-        const int p = ent.pid[d];
-        add_u16x16(pbuf + (size_t)p * sbstride, ent.roff[d] - ent.lo[p] + 16 * tl, acc[d]);
-      }
-      pending = true;
-    }
-    __syncthreads();  // every thread is done reading buffer b (rows, entries, partials)
-    pending = false;
-    if (tl < 32 && k + 2 < nchunks) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      stage_entries(k + 2, b);
-      issue_stage<SB_TB>(s, ld, ns, nch, dstride, delays, ntrials, d0, t0,
-                         (uint64_t)(k + 2) * cc, cc, smem + b * bstride, rowcap, &info[b],
-                         &bars[b], 0);
-    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (failed >= 0) {
-    if (tl == 0) {
-      mbar_wait_bounded(&bars[failed & 1], (unsigned)((failed >> 1) & 1), err, spin_limit);
-      if (failed + 1 < nchunks)
-        mbar_wait_bounded(&bars[(failed + 1) & 1], (unsigned)(((failed + 1) >> 1) & 1), err,
-                          spin_limit);
+  __syncthreads();
+  auto wait = [&](uint64_t *bar, unsigned parity) -> bool {
+    for (long long i = 0; i < spin_limit; ++i) {
+      if (mbar_try_wait(bar, parity)) return true;
+      if ((i & 63) == 63 && dead) return false;
     }
+    atomicOr(err, 1u);
+    dead = 1;
+    return false;
+  };
+
+  if (warp == SS_TB) {
+    // lane i copies rows i and i + 32 of every stage
+    const SubRow *rl = rows + row0[tb];
+    const uint16_t *src = scratch + tile0;
+    constexpr int H = SS_MAXROWS / 32;
+    SubRow r[2][H];  // the rows of stages k and k + 1
+    int ahead = 0;   // first row of the stage to read next
+    auto fetch = [&](int k, SubRow *x) {
+      const int nr = k < nst ? (int)(desc[k] & 255u) : 0;
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if (lane + 32 * h < nr) x[h] = rl[ahead + lane + 32 * h];
+      ahead += nr;
+    };
+    fetch(0, r[0]);
+    fetch(1, r[1]);
+    int b = 0;
+    unsigned turn = 0;
+    int issued = 0;
+    auto one = [&](int k, SubRow *x) -> bool {
+      if (turn && !__all_sync(0xffffffffu, wait(&empty[b], (turn - 1) & 1))) return false;
+      const int nr = (int)(desc[k] & 255u);
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if (lane + 32 * h < nr) {
+          mbar_expect_tx(&full[b], (unsigned)rowcap);
+          bulk_g2s(smem + (size_t)b * bufbytes + (size_t)(lane + 32 * h) * rowcap,
+                   src + (uint64_t)x[h].row * ldp + x[h].start, (unsigned)rowcap, &full[b]);
+        }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[b]);
+      ++issued;
+      fetch(k + 2, x);
+      if (++b == nbuf) {
+        b = 0;
+        ++turn;
+      }
+      return true;
+    };
+    for (int k = 0; k < nst; k += 2) {
+      if (!one(k, r[0])) break;
+      if (k + 1 < nst && !one(k + 1, r[1])) break;
+    }
+    // leave after the copies of the last nbuf stages issued
+    for (int k = max(0, issued - nbuf); k < issued; ++k)
+      for (long long i = 0; i < spin_limit; ++i)
+        if (mbar_try_wait(&full[k % nbuf], (unsigned)(k / nbuf) & 1)) break;
     return;
   }
 
-  const uint64_t tb = t0 + (uint64_t)tl * DD_TPT;
+  const uint32_t *inf = info + (tb * SS_TB + warp) * nsub;
+  const uint64_t tr = tb * SS_TB + warp;
+  const bool live = tr < ntrials;
+  uint32_t E[SS_K], O[SS_K + 1];
+  uint32_t acc[FLUSH ? 2 * SS_K : 1];
 #pragma unroll
-  for (int d = 0; d < SB_TB; ++d) {
-    const uint64_t tr = d0 + d;
-    float v[16];
-    unsigned long long local = 0;
+  for (int i = 0; i < SS_K; ++i) E[i] = O[i] = 0;
+  O[SS_K] = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      uint32_t lo = acc[d][i] & 0xffffu, hi = acc[d][i] >> 16;
-      bool in0 = tb + 2 * i < n, in1 = tb + 2 * i + 1 < n;
-      v[2 * i] = (float)lo;
-      v[2 * i + 1] = (float)hi;
-      local += (in0 ? lo : 0u) + (in1 ? hi : 0u);
-    }
-    if (tr < ntrials) {
-      float *dst = out + tr * ldo + tb;
-      if (tb + 16 <= n) {
-        float4 *d4 = reinterpret_cast<float4 *>(dst);
+  for (int i = 0; i < (FLUSH ? 2 * SS_K : 1); ++i) acc[i] = 0;
+  // Sums of word k's two samples: E's word plus O's realigned by one sample
+  // (the next word is the next lane's; lane 31's is lane 0's of k + 1).
+  auto merged = [&](int k, uint32_t &v0, uint32_t &v1) {
+    const uint32_t up = __shfl_down_sync(0xffffffffu, O[k], 1);
+    const uint32_t wrap = __shfl_sync(0xffffffffu, O[k + 1], 0);
+    const uint32_t nx = lane == 31 ? wrap : up;
+    v0 = (E[k] & 0xffffu) + (O[k] >> 16);
+    v1 = (E[k] >> 16) + (nx & 0xffffu);
+  };
+  // This trial's words in the stage's buffer: byte offset, bit 0 an odd
+  // shift; lane j holds the stage's subband j.
+  uint32_t nextinf = lane < (int)((desc[0] >> 8) & 255u) ? __ldg(inf + lane) : 0u;
+  int b = 0;
+  unsigned turn = 0;
+  for (int k = 0; k < nst; ++k) {
+    const uint32_t d = desc[k];
+    const int nsubs = (int)((d >> 8) & 255u);
+    const uint32_t myinf = nextinf;
+    inf += nsubs;
+    if (k + 1 < nst && lane < (int)((desc[k + 1] >> 8) & 255u)) nextinf = __ldg(inf + lane);
+    if (!__all_sync(0xffffffffu, wait(&full[b], turn & 1))) return;
+    if (live) {
+      const uint8_t *buf = smem + (size_t)b * bufbytes;
+      for (int j = 0; j < nsubs; ++j) {
+        const uint32_t w = __shfl_sync(0xffffffffu, myinf, j);
+        const uint32_t *q = reinterpret_cast<const uint32_t *>(buf + (w & ~1u));
+        if (w & 1u) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float4 w = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          if (accumulate) {
-            const float4 o = d4[i];
-            w.x += o.x;
-            w.y += o.y;
-            w.z += o.z;
-            w.w += o.w;
-          }
-          d4[i] = w;
+          for (int i = 0; i < SS_K; ++i) O[i] += q[lane + 32 * i];
+          O[SS_K] += q[32 * SS_K];
+        } else {
+#pragma unroll
+          for (int i = 0; i < SS_K; ++i) E[i] += q[lane + 32 * i];
         }
-      } else {
-        for (int i = 0; i < 16; ++i)
-          if (tb + i < n) dst[i] = accumulate ? dst[i] + v[i] : v[i];
+      }
+      if constexpr (FLUSH) {
+        if (d >> 16) {
+#pragma unroll
+          for (int i = 0; i < SS_K; ++i) {
+            uint32_t v0, v1;
+            merged(i, v0, v1);
+            acc[2 * i] += v0;
+            acc[2 * i + 1] += v1;
+          }
+#pragma unroll
+          for (int i = 0; i < SS_K; ++i) E[i] = O[i] = 0;
+          O[SS_K] = 0;
+        }
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[b]);
+    if (++b == nbuf) {
+      b = 0;
+      ++turn;
+    }
+  }
+  if (!live) return;
+  const uint64_t t0 = seg0 + tile0;
+  float *dst = out + tr * ldo + t0;
+  uint32_t local = 0;  // at most 2 SS_K sums below 2^24
 #pragma unroll
-    for (int o = 16; o; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
-    if ((tl & 31) == 0) wsum[tl >> 5][d] = local;
+  for (int k = 0; k < SS_K; ++k) {
+    uint32_t v0, v1;
+    merged(k, v0, v1);
+    if constexpr (FLUSH) {
+      v0 += acc[2 * k];
+      v1 += acc[2 * k + 1];
+    }
+    const int e = 2 * (lane + 32 * k);
+    if (t0 + e + 2 <= segend) {
+      *reinterpret_cast<float2 *>(dst + e) = make_float2((float)v0, (float)v1);
+      local += v0 + v1;
+    } else if (t0 + e < segend) {
+      dst[e] = (float)v0;
+      local += v0;
+    }
   }
-  __syncthreads();
-  if (tl < SB_TB && d0 + tl < ntrials) {
-    unsigned long long t = 0;
-    for (int w = 0; w < DD_NT / 32; ++w) t += wsum[w][tl];
-    double *pp = &part[(d0 + tl) * ntiles + blockIdx.x];
-    *pp = accumulate ? *pp + (double)t : (double)t;
-  }
+  unsigned long long sum = local;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if (lane == 0) part[tr * ntiles + t0 / SS_TT] = (double)sum;
 }
 
 // Reference-order f32 accumulation (one output per thread per trial).
@@ -722,33 +811,43 @@ __global__ void __launch_bounds__(DG_NT)
 // sum |x| < 2^(53+q) (with a margin for the rounding of sum |x| itself).
 // Otherwise the thread re-adds the trial's series sequentially, in the
 // reference's order.
-__global__ void k_reduce_parts(const double *part, uint64_t ntiles, uint64_t ntrials,
-                               uint64_t n, double *sums, float *means, const float *series,
-                               uint64_t ldo, int check) {
-  uint64_t tr = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per trial: the tiles' sums are added 32 lanes wide (one thread per
+// trial took 13 us per 256-trial launch of 65 tiles each, a chain of loads).
+constexpr int RP_NT = 128;
+__global__ void __launch_bounds__(RP_NT)
+    k_reduce_parts(const double *part, uint64_t ntiles, uint64_t ntrials, uint64_t n,
+                   double *sums, float *means, const float *series, uint64_t ldo, int check) {
+  const uint64_t tr = (uint64_t)blockIdx.x * (RP_NT / 32) + (threadIdx.x >> 5);
+  const int lane = (int)(threadIdx.x & 31);
   if (tr >= ntrials) return;
-  double s = 0.0;
-  for (uint64_t i = 0; i < ntiles; ++i) s += part[tr * ntiles + i];
-  if (check) {
-    double a = 0.0, q = (double)kNoQuantum;
-    for (uint64_t i = 0; i < ntiles; ++i) {
+  double s = 0.0, a = 0.0, q = (double)kNoQuantum;
+  for (uint64_t i = lane; i < ntiles; i += 32) {
+    s += part[tr * ntiles + i];
+    if (check) {
       a += part[ntrials * ntiles + tr * ntiles + i];
       q = fmin(q, part[2 * ntrials * ntiles + tr * ntiles + i]);
     }
-    const bool exact = f64_sums_exact(a, (int)q);
-    if (!exact) {  // the reference's order: t = 0, 1, ..., from -0.0
-      const float *x = series + tr * ldo;
-      s = -0.0;
-      uint64_t t = 0;
-      for (; t + 4 <= n; t += 4) {  // rows start 256-byte aligned (ldo % 64 == 0)
-        const float4 v = *reinterpret_cast<const float4 *>(x + t);
-        s += (double)v.x;
-        s += (double)v.y;
-        s += (double)v.z;
-        s += (double)v.w;
-      }
-      for (; t < n; ++t) s += (double)x[t];
+  }
+  for (int o = 16; o; o >>= 1) {
+    s += __shfl_down_sync(0xffffffffu, s, o);
+    if (check) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      q = fmin(q, __shfl_down_sync(0xffffffffu, q, o));
     }
+  }
+  if (lane != 0) return;
+  if (check && !f64_sums_exact(a, (int)q)) {  // the reference's order: t = 0, 1, ..., from -0.0
+    const float *x = series + tr * ldo;
+    s = -0.0;
+    uint64_t t = 0;
+    for (; t + 4 <= n; t += 4) {  // rows start 256-byte aligned (ldo % 64 == 0)
+      const float4 v = *reinterpret_cast<const float4 *>(x + t);
+      s += (double)v.x;
+      s += (double)v.y;
+      s += (double)v.z;
+      s += (double)v.w;
+    }
+    for (; t < n; ++t) s += (double)x[t];
   }
   sums[tr] = s;
   means[tr] = (float)(s / (double)n);
@@ -807,159 +906,368 @@ int launch_series_mean(const float *d_x, uint64_t n, double *d_sum, float *d_mea
 
 uint64_t series_ld(uint64_t n) { return ((n + 63) / 64) * 64; }
 
-// The subband kernel over channel groups (sums of a group stay below 2^16;
-// groups start at multiples of G).  PSR_EINVAL (no error recorded) when the
-// sample range or the shared memory does not fit this path.
-int launch_dedisperse_sb(const DeviceObs &o, const uint32_t *d_delays, uint64_t ntrials,
-                         uint64_t n, float *d_out, uint64_t ldo, double *d_part,
-                         uint64_t max_spread, unsigned *d_err, cudaStream_t st, long long spin,
-                         const SubbandPlan &sb, uint64_t chunk_index) {
-  const int G = sb.G;
-  const double maxv = o.max_value();
-  const uint64_t gch = maxv > 0.0 ? (uint64_t)(65535.0 / maxv) : 0;
-  const uint64_t glen = std::min<uint64_t>((gch / G) * G, ((o.nch + G - 1) / G) * G);
-  if (glen < (uint64_t)G || (double)o.nch * maxv >= 16777216.0) return PSR_EINVAL;
-  const uint64_t ntiles = (n + DD_TT - 1) / DD_TT;
-  const int rowcap = (int)(((uint64_t)DD_TT + max_spread + 64 + 15) & ~(uint64_t)15);
-  const int sbstride = (int)(((uint64_t)DD_TT + max_spread + 40 + 7) & ~(uint64_t)7);
-  int dev = 0;
-  PSR_CUDA(cudaGetDevice(&dev));
-  int smax = 0, smsm = 0;
-  PSR_CUDA(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  PSR_CUDA(cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-  const size_t budget = std::min((size_t)smax, (size_t)smsm / 2) - 4096;
-  const size_t pbytes = (size_t)SB_PMAX * sbstride * 2;
-  if (budget <= pbytes) return PSR_EINVAL;
-  int cc = (int)std::min<uint64_t>((uint64_t)DD_MAXCC, (budget - pbytes) / (2 * (size_t)rowcap));
-  cc = (cc / G) * G;
-  if (cc < G) return PSR_EINVAL;
-  const size_t smem = 2 * (size_t)cc * rowcap + pbytes;
-  const SbEntry *plan = sb.entries.as<SbEntry>();
-  auto kern = G == 4 ? k_dedisp_sb<4> : k_dedisp_sb<8>;
-  if (G != 4 && G != 8) return PSR_EINVAL;
-  PSR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)ntiles, (unsigned)((ntrials + SB_TB - 1) / SB_TB));
-  for (uint64_t c0 = 0; c0 < o.nch; c0 += glen) {
-    const uint64_t ng = std::min(glen, o.nch - c0);
-    const int ccg = (int)std::min<uint64_t>((uint64_t)cc, ((ng + G - 1) / G) * G);
-    kern<<<grid, DD_NT, smem, st>>>(o.samples.as<uint8_t>() + c0 * o.ld, o.ld, o.ns, ng, o.nch,
-                                    d_delays + c0, ntrials, n, d_out, ldo, d_part, ntiles, ccg,
-                                    rowcap, c0 > 0 ? 1 : 0, d_err, spin, plan, sb.nsub, c0 / G,
-                                    sb.block0[chunk_index], sbstride);
-    PSR_CUDA(cudaGetLastError());
+namespace {
+int reduce_parts(const double *d_part, uint64_t ntiles, uint64_t ntrials, uint64_t n,
+                 double *d_sums, float *d_means, const float *d_series, uint64_t ldo, int check,
+                 cudaStream_t st) {
+  constexpr uint64_t per = RP_NT / 32;
+  k_reduce_parts<<<(unsigned)((ntrials + per - 1) / per), RP_NT, 0, st>>>(
+      d_part, ntiles, ntrials, n, d_sums, d_means, d_series, ldo, check);
+  PSR_CUDA(cudaGetLastError());
+  return PSR_OK;
+}
+}  // namespace
+
+namespace {
+std::atomic<int> g_subbands{-1};
+
+// Dynamic shared memory of k_sub_sum's stage buffers: two CTAs per SM without
+// FLUSH, one with it.
+constexpr int SS_SMEM = 106 * 1024, SS_SMEM_FLUSH = 216 * 1024;
+constexpr int SP_MAXSMEM = 72 * 1024;       // k_sub_part: three CTAs per SM
+constexpr uint64_t SUB_SCRATCH = 1ull << 30;  // scratch rows of one segment
+
+// A subband's delays relative to its smallest, 16 bits each.
+struct RelKey {
+  uint64_t a = 0, b = 0;
+  bool operator==(const RelKey &o) const { return a == o.a && b == o.b; }
+};
+
+// The patterns of every subband over one chunk of trials.
+struct ChunkPatterns {
+  std::vector<SubBand> subs;
+  std::vector<RelKey> keys;     // rows, in subband order
+  std::vector<uint16_t> pat;    // [subband][trial of the chunk]
+  std::vector<uint32_t> ref;    // [subband][trial]: smallest delay
+  bool ok = true;
+};
+
+void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta, uint64_t tz,
+                    int G, ChunkPatterns &cp) {
+  const uint64_t nt = tz - ta, nsub = (nch + G - 1) / G;
+  cp = ChunkPatterns();
+  cp.pat.resize(nsub * nt);
+  cp.ref.resize(nsub * nt);
+  uint32_t hsize = 64;
+  while (hsize < 4 * nt) hsize <<= 1;
+  std::vector<uint32_t> slot(hsize, 0);  // 1 + row of the subband's pattern, by generation
+  std::vector<uint32_t> gen(hsize, 0);
+  for (uint64_t j = 0; j < nsub && cp.ok; ++j) {
+    const uint64_t ca = j * G;
+    const int ge = (int)std::min<uint64_t>(G, nch - ca);
+    SubBand sb{};
+    sb.row0 = (int32_t)cp.keys.size();
+    uint32_t dmin = 0xffffffffu, dmax = 0;
+    for (uint64_t t = 0; t < nt && cp.ok; ++t) {
+      const uint32_t *d = &tab[(ta + t) * nch + ca];
+      uint32_t m = d[0], mx = d[0];
+      for (int c = 1; c < ge; ++c) {
+        m = std::min(m, d[c]);
+        mx = std::max(mx, d[c]);
+      }
+      if (mx - m > 4095u) {
+        cp.ok = false;
+        break;
+      }
+      sb.relmax = std::max(sb.relmax, (int32_t)(mx - m));
+      dmin = std::min(dmin, m);
+      dmax = std::max(dmax, m);
+      RelKey k;
+      for (int c = 0; c < ge; ++c) {
+        const uint64_t r = d[c] - m;
+        if (c < 4) k.a |= r << (16 * c);
+        else k.b |= r << (16 * (c - 4));
+      }
+      uint64_t h = (k.a ^ (k.b * 0x9E3779B97F4A7C15ull)) * 0xD6E8FEB86659FD93ull;
+      uint32_t q = (uint32_t)(h >> 40) & (hsize - 1);
+      for (;;) {
+        if (gen[q] != j + 1) {
+          gen[q] = (uint32_t)j + 1;
+          slot[q] = (uint32_t)cp.keys.size();
+          cp.keys.push_back(k);
+          break;
+        }
+        if (cp.keys[slot[q]] == k) break;
+        q = (q + 1) & (hsize - 1);
+      }
+      cp.pat[j * nt + t] = (uint16_t)(slot[q] - (uint32_t)sb.row0);
+      cp.ref[j * nt + t] = m;
+    }
+    sb.dmin = (int32_t)dmin;
+    sb.spread = (int32_t)(dmax - dmin);
+    sb.npat = (int32_t)(cp.keys.size() - (size_t)sb.row0);
+    if (sb.npat > 65535) cp.ok = false;  // pat[] holds 16 bits
+    cp.subs.push_back(sb);
   }
+}
+
+// The two-level kernels against the channel-by-channel one on a chunk of nt
+// trials, per 512 samples, in SM issue slots fitted to times on a GB300 (96,
+// 512 and 4096 channels, 64 to 256 trials, both widths): a channel of a trial
+// costs the channel-by-channel kernel 38 (<= 4-bit samples) or 62; a pattern
+// costs k_sub_part 80 + 50 G or 310 + 38 G (the write of its row included);
+// k_sub_sum is bound by the rows it stages, 280 each, or by 32 per (trial,
+// subband) of shared-memory loads.
+double direct_cost(uint64_t nch, uint64_t nt, double maxv) {
+  return (maxv * 2.0 <= 255.0 ? 38.0 : 62.0) * (double)nch * (double)nt;
+}
+double two_level_cost(const ChunkPatterns &cp, uint64_t nt, int G, double maxv) {
+  const double part = maxv * SUB_GMAX <= 255.0 ? 80.0 + 50.0 * G : 310.0 + 38.0 * G;
+  const uint64_t nsub = cp.subs.size();
+  std::vector<uint32_t> seen(65536, 0);
+  uint32_t gen = 0;
+  uint64_t staged = 0;
+  for (uint64_t j = 0; j < nsub; ++j)
+    for (uint64_t t = 0; t < nt; ++t) {
+      if (t % SS_TB == 0) ++gen;
+      uint32_t &s = seen[cp.pat[j * nt + t]];
+      staged += s != gen;
+      s = gen;
+    }
+  return part * (double)cp.keys.size() +
+         std::max(280.0 * (double)staged, 32.0 * (double)nt * (double)nsub);
+}
+}  // namespace
+
+int dedisp_subbands_default(const DeviceObs &o) {
+  (void)o;
+  return g_subbands.load();
+}
+
+namespace {
+// The plan at width G; plan.G stays 0 when it does not fit.
+int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
+                    const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
+                    cudaStream_t st) {
+  const bool byte_part = maxv * SUB_GMAX <= 255.0;
+  const bool flush = (double)nch * maxv > 65535.0;
+  const size_t nchunks = cstart.size() - 1;
+  const uint64_t nsub = (nch + G - 1) / G;
+  std::vector<SubBand> subs;
+  std::vector<uint16_t> rel;
+  std::vector<uint32_t> stage0, rowlist0, stages, info;
+  std::vector<SubRow> rows;
+  std::vector<SubbandPlan::Chunk> chunks;
+  struct Win {  // a row a trial block uses: offsets [lo, hi] of its trials
+    uint32_t row, lo, hi;
+  };
+  std::vector<Win> wins;
+  std::vector<uint32_t> winpos;     // first window of each (trial block, subband)
+  std::vector<uint8_t> slotof;      // [trial block][subband][16]
+  std::vector<uint32_t> offof;
+  uint64_t max_rows = 0, max_spread = 0;
+  int relmax = 0;
+  uint32_t maxwin = 0;
+  size_t most = 0;
+  for (size_t ci = 0; ci < nchunks; ++ci) {
+    const uint64_t ta = cstart[ci], nt = cstart[ci + 1] - ta;
+    if (nt == 0) return PSR_OK;
+    ChunkPatterns cp;
+    chunk_patterns(tab, nch, ta, ta + nt, G, cp);
+    if (!cp.ok) return PSR_OK;
+    SubbandPlan::Chunk c;
+    c.sub0 = subs.size();
+    c.rel0 = rel.size();
+    c.block0 = 0;
+    c.nblocks = (nt + SS_TB - 1) / SS_TB;
+    c.spread = 0;
+    for (const SubBand &sb : cp.subs) {
+      c.spread = std::max<uint64_t>(c.spread, (uint64_t)sb.spread);
+      relmax = std::max(relmax, sb.relmax);
+      subs.push_back(sb);
+    }
+    max_spread = std::max(max_spread, c.spread);
+    max_rows = std::max<uint64_t>(max_rows, cp.keys.size());
+    for (const RelKey &k : cp.keys)
+      for (int r = 0; r < G; ++r)
+        rel.push_back((uint16_t)((r < 4 ? k.a >> (16 * r) : k.b >> (16 * (r - 4))) & 0xffffu));
+    for (uint64_t tb = 0; tb < c.nblocks; ++tb) {
+      for (uint64_t j = 0; j < nsub; ++j) {
+        const SubBand &sb = cp.subs[j];
+        winpos.push_back((uint32_t)wins.size());
+        const size_t w0 = wins.size();
+        for (int d = 0; d < SS_TB; ++d) {
+          // slots past the chunk's trials repeat its last one
+          const uint64_t t = std::min<uint64_t>(tb * SS_TB + d, nt - 1);
+          const uint32_t row = (uint32_t)sb.row0 + cp.pat[j * nt + t];
+          const uint32_t off = cp.ref[j * nt + t] - (uint32_t)sb.dmin;
+          size_t w = w0;
+          while (w < wins.size() && wins[w].row != row) ++w;
+          if (w == wins.size()) wins.push_back(Win{row, off, off});
+          wins[w].lo = std::min(wins[w].lo, off);
+          wins[w].hi = std::max(wins[w].hi, off);
+          slotof.push_back((uint8_t)(w - w0));
+          offof.push_back(off);
+        }
+        for (size_t w = w0; w < wins.size(); ++w)
+          maxwin = std::max(maxwin, wins[w].hi - (wins[w].lo & ~7u));
+        most = std::max(most, wins.size() - w0);
+      }
+    }
+    chunks.push_back(c);
+  }
+  winpos.push_back((uint32_t)wins.size());
+  // A staged row: the tile, its trials' offsets, and the word past the tile
+  // that an odd shift reads.
+  const uint64_t rowcap = (((uint64_t)SS_TT + maxwin + 2) * 2 + 15) & ~15ull;
+  const uint64_t room = flush ? SS_SMEM_FLUSH : SS_SMEM;
+  const int maxrows = (int)std::min<uint64_t>(
+      SS_MAXROWS, std::max<uint64_t>(most, room / (SS_MAXBUF * rowcap)));
+  const uint64_t bufbytes = ((uint64_t)maxrows * rowcap + 127) & ~127ull;
+  const int nbuf = (int)std::min<uint64_t>(SS_MAXBUF, room / bufbytes);
+  const uint64_t prowcap = ((uint64_t)SP_TT + relmax + 36 + 15) & ~15ull;
+  if (nbuf < 2 || prowcap * G > SP_MAXSMEM) return PSR_OK;
+  // Segments of the series: the scratch of one stays within SUB_SCRATCH.
+  const uint64_t tail = max_spread + rowcap / 2 + 16;
+  uint64_t seg = ((n + SS_TT - 1) / SS_TT) * SS_TT;
+  auto stride = [&](uint64_t sg) { return ((sg + tail + SP_TT - 1) / SP_TT) * SP_TT; };
+  if (max_rows * stride(seg) * 2 > SUB_SCRATCH) {
+    const uint64_t per = SUB_SCRATCH / (2 * max_rows);
+    seg = per > tail + SP_TT ? ((per - tail - SP_TT) / SS_TT) * SS_TT : 0;
+    if (seg < 16 * SS_TT) return PSR_OK;  // rows too many to reuse
+  }
+  const uint64_t ldp = stride(seg);
+  // Stages: subbands in order while their rows fit the buffer; a stage after
+  // which the next could pass 16 bits is marked to flush.
+  size_t wi = 0, si = 0;
+  uint64_t blk = 0;
+  for (size_t ci = 0; ci < nchunks; ++ci) {
+    chunks[ci].block0 = blk;
+    for (uint64_t tb = 0; tb < chunks[ci].nblocks; ++tb, ++blk) {
+      stage0.push_back((uint32_t)stages.size());
+      rowlist0.push_back((uint32_t)rows.size());
+      int nrows = 0, nsubs = 0;
+      double held = 0.0;  // largest sum the 16-bit lanes can hold so far
+      const size_t inf0 = info.size();
+      info.resize(inf0 + SS_TB * nsub);
+      for (uint64_t j = 0; j < nsub; ++j, ++wi) {
+        const int nw = (int)(winpos[wi + 1] - winpos[wi]);
+        const double add = maxv * (double)std::min<uint64_t>(G, nch - j * G);
+        const bool over = held + add > 65535.0;
+        if (nsubs && (nrows + nw > maxrows || nsubs == 32 || over)) {
+          stages.push_back(sub_stage(nrows, nsubs, over ? 1 : 0));
+          if (over) held = 0.0;
+          nrows = nsubs = 0;
+        }
+        held += add;
+        for (int w = 0; w < nw; ++w) {
+          const Win &x = wins[winpos[wi] + w];
+          rows.push_back(SubRow{x.row, x.lo & ~7u});
+        }
+        for (int d = 0; d < SS_TB; ++d, ++si) {
+          const Win &x = wins[winpos[wi] + slotof[si]];
+          const uint32_t o = offof[si] - (x.lo & ~7u);
+          info[inf0 + (size_t)d * nsub + j] =
+              (uint32_t)(nrows + slotof[si]) * (uint32_t)rowcap + (o >> 1) * 4u + (o & 1u);
+        }
+        nrows += nw;
+        nsubs += 1;
+      }
+      stages.push_back(sub_stage(nrows, nsubs, 0));
+      if (stages.size() - stage0.back() > SS_MAXSTAGES) return PSR_OK;
+    }
+  }
+  stage0.push_back((uint32_t)stages.size());
+  auto up = [&](DevBuf &b, const void *src, size_t bytes) -> int {
+    PSR_TRY(b.ensure(bytes));
+    PSR_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
+    return PSR_OK;
+  };
+  PSR_TRY(up(plan.subs, subs.data(), subs.size() * sizeof(SubBand)));
+  PSR_TRY(up(plan.rel, rel.data(), rel.size() * 2));
+  PSR_TRY(up(plan.stage0, stage0.data(), stage0.size() * 4));
+  PSR_TRY(up(plan.stages, stages.data(), stages.size() * 4));
+  PSR_TRY(up(plan.rowlist0, rowlist0.data(), rowlist0.size() * 4));
+  PSR_TRY(up(plan.rows, rows.data(), rows.size() * sizeof(SubRow)));
+  PSR_TRY(up(plan.info, info.data(), info.size() * 4));
+  PSR_TRY(plan.scratch.ensure(max_rows * ldp * 2 + 256));
+  PSR_CUDA(cudaStreamSynchronize(st));
+  plan.G = G;
+  plan.nsub = nsub;
+  plan.byte_part = byte_part;
+  plan.flush = flush;
+  plan.seg = seg;
+  plan.ldp = ldp;
+  plan.rowcap = (int)rowcap;
+  plan.prowcap = (int)prowcap;
+  plan.bufbytes = (int)bufbytes;
+  plan.nbuf = nbuf;
+  plan.chunks = std::move(chunks);
+  return PSR_OK;
+}
+
+}  // namespace
+
+int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
+                       const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
+                       cudaStream_t st) {
+  plan.G = 0;
+  plan.chunks.clear();
+  if (G == 0 || cstart.size() < 2 || !(maxv > 0.0) || maxv > 255.0 ||
+      (double)nch * maxv >= 16777216.0 || n < 2)
+    return PSR_OK;
+  if (G == 4 || G == 8) return subband_plan_at(tab, nch, n, maxv, cstart, G, plan, st);
+  // The widths that are cheaper than the channel-by-channel kernel on the
+  // middle chunk, cheapest first.
+  const size_t mid = (cstart.size() - 2) / 2;
+  const uint64_t nt = cstart[mid + 1] - cstart[mid];
+  std::vector<std::pair<double, int>> pick;
+  for (int g : {8, 4}) {
+    ChunkPatterns cp;
+    chunk_patterns(tab, nch, cstart[mid], cstart[mid + 1], g, cp);
+    if (!cp.ok) continue;
+    const double c = two_level_cost(cp, nt, g, maxv);
+    if (c < direct_cost(nch, nt, maxv)) pick.emplace_back(c, g);
+  }
+  std::sort(pick.begin(), pick.end());
+  for (size_t i = 0; i < pick.size() && plan.G == 0; ++i)
+    PSR_TRY(subband_plan_at(tab, nch, n, maxv, cstart, pick[i].second, plan, st));
   return PSR_OK;
 }
 
 namespace {
-std::atomic<int> g_subbands{-1};
-}
-int dedisp_subbands_default(const DeviceObs &o) {
-  const int g = g_subbands.load();
-  if (g >= 0) return g;
-  // Measured on a GB300 with the word-cache channel-by-channel kernel: the
-  // whole 8000-trial survey search (4096 x 8-bit channels, 2^23 samples)
-  // takes 13.39 s with subbands of 8 and 14.13 s channel by channel; at
-  // 64-1024 8-bit channels subbands cost about 8%, and on <= 4-bit samples
-  // the byte-lane kernel is faster.  Batches tune it per shape class.
-  return o.kind == SAMPLE_U8 && o.h.nbits == 8 && o.nch >= 2048 ? 8 : 0;
-}
-
-// Cost of one (block, subband) in thread instructions per 16 samples, for
-// the choice between stage A/B and direct adds: a shifted 16-byte add is
-// about 33, a shifted 16-sample u16 add about 37, plus two barriers.
-bool subband_pays(int npat, int ge, int tbe) {
-  return npat * ge * 33 + tbe * 37 + 40 < tbe * ge * 33;
-}
-
-int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch,
-                       const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st) {
-  plan.G = 0;
-  plan.nsub = 0;
-  plan.block0.clear();
-  plan.reused = plan.direct = 0;
-  if ((G != 4 && G != 8) || cstart.size() < 2) return PSR_OK;
-  const uint64_t nsub = (nch + G - 1) / G;
-  std::vector<uint64_t> block0;
-  uint64_t nblocks = 0;
-  for (size_t ci = 0; ci + 1 < cstart.size(); ++ci) {
-    block0.push_back(nblocks);
-    nblocks += (cstart[ci + 1] - cstart[ci] + SB_TB - 1) / SB_TB;
-  }
-  std::vector<SbEntry> ent(nblocks * nsub);
-  uint64_t nsb = 0, ndirect = 0;
-  for (size_t ci = 0; ci + 1 < cstart.size(); ++ci) {
-    const uint64_t ta = cstart[ci], tz = cstart[ci + 1];
-    for (uint64_t b = 0; ta + b * SB_TB < tz; ++b) {
-      const uint64_t tb0 = ta + b * SB_TB;
-      const int tbe = (int)std::min<uint64_t>(SB_TB, tz - tb0);
-      for (uint64_t j = 0; j < nsub; ++j) {
-        SbEntry e{};
-        const uint64_t ca = j * G;
-        const int ge = (int)std::min<uint64_t>(G, nch - ca);
-        uint32_t dref[SB_TB];
-        int32_t dmin = INT32_MAX, dmaxr = 0;
-        for (int d = 0; d < SB_TB; ++d) {
-          // trials past the chunk repeat its last trial, as the kernel's staging does
-          const uint64_t tr = tb0 + (uint64_t)std::min(d, tbe - 1);
-          uint32_t m = 0xffffffffu;
-          for (int c = 0; c < ge; ++c) m = std::min(m, tab[tr * nch + ca + c]);
-          dref[d] = m;
-          dmin = std::min(dmin, (int32_t)m);
-          dmaxr = std::max(dmaxr, (int32_t)m);
-        }
-        bool ok = dmaxr - dmin < 65536;
-        int npat = 0;
-        for (int d = 0; d < SB_TB && ok; ++d) {
-          const uint64_t tr = tb0 + (uint64_t)std::min(d, tbe - 1);
-          uint16_t rel[SB_GMAX] = {0};
-          for (int c = 0; c < ge; ++c) {
-            const uint32_t r = tab[tr * nch + ca + c] - dref[d];
-            if (r > 65535u) ok = false;
-            rel[c] = (uint16_t)r;
-          }
-          int p = 0;
-          while (p < npat && std::memcmp(e.rel[p], rel, sizeof(rel)) != 0) ++p;
-          if (p == npat) {
-            if (npat == SB_PMAX) {
-              ok = false;
-              break;
-            }
-            std::memcpy(e.rel[p], rel, sizeof(rel));
-            e.lo[p] = 0xffff;
-            e.hi[p] = 0;
-            ++npat;
-          }
-          const uint16_t ro = (uint16_t)(dref[d] - (uint32_t)dmin);
-          e.pid[d] = (uint8_t)p;
-          e.roff[d] = ro;
-          e.lo[p] = std::min(e.lo[p], ro);
-          e.hi[p] = std::max(e.hi[p], ro);
-        }
-        if (ok && subband_pays(npat, ge, tbe)) {
-          e.npat = (uint8_t)npat;
-          e.dref_min = dmin;
-          ++nsb;
-        } else {
-          e = SbEntry{};
-          ++ndirect;
-        }
-        ent[(block0[ci] + b) * nsub + j] = e;
-      }
-    }
-  }
-  PSR_TRY(plan.entries.ensure(ent.size() * sizeof(SbEntry)));
-  PSR_CUDA(cudaMemcpyAsync(plan.entries.p, ent.data(), ent.size() * sizeof(SbEntry),
-                           cudaMemcpyHostToDevice, st));
-  PSR_CUDA(cudaStreamSynchronize(st));
-  plan.G = G;
-  plan.nsub = nsub;
-  plan.block0 = block0;
-  plan.reused = nsb;
-  plan.direct = ndirect;
+template <int G, bool BYTE>
+int run_part(const DeviceObs &o, const SubbandPlan &sb, const SubbandPlan::Chunk &c,
+             uint64_t seg0, uint64_t seglen, unsigned *d_err, cudaStream_t st, long long spin) {
+  const size_t smem = (size_t)G * sb.prowcap;
+  PSR_CUDA(cudaFuncSetAttribute(k_sub_part<G, BYTE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                SP_MAXSMEM));
+  dim3 grid((unsigned)((seglen + c.spread + 2 + SP_TT - 1) / SP_TT), (unsigned)sb.nsub);
+  k_sub_part<G, BYTE><<<grid, SP_NT, smem, st>>>(
+      o.samples.as<uint8_t>(), o.ld, o.ns, o.nch, sb.subs.as<SubBand>() + c.sub0,
+      sb.rel.as<uint16_t>() + c.rel0, seg0, seglen, sb.scratch.as<uint16_t>(), sb.ldp, sb.prowcap,
+      d_err, spin);
+  PSR_CUDA(cudaGetLastError());
   return PSR_OK;
 }
+
+int launch_dedisperse_sub(const DeviceObs &o, uint64_t ntrials, uint64_t n, float *d_out,
+                          uint64_t ldo, double *d_part, unsigned *d_err, cudaStream_t st,
+                          long long spin, const SubbandPlan &sb, uint64_t chunk_index) {
+  const SubbandPlan::Chunk &c = sb.chunks[chunk_index];
+  const uint64_t ntiles = (n + SS_TT - 1) / SS_TT;
+  auto kern = sb.flush ? k_sub_sum<true> : k_sub_sum<false>;
+  PSR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                sb.flush ? SS_SMEM_FLUSH : SS_SMEM));
+  for (uint64_t seg0 = 0; seg0 < n; seg0 += sb.seg) {
+    const uint64_t len = std::min(sb.seg, n - seg0);
+    if (sb.G == 8)
+      PSR_TRY(sb.byte_part ? (run_part<8, true>(o, sb, c, seg0, len, d_err, st, spin))
+                           : (run_part<8, false>(o, sb, c, seg0, len, d_err, st, spin)));
+    else
+      PSR_TRY(sb.byte_part ? (run_part<4, true>(o, sb, c, seg0, len, d_err, st, spin))
+                           : (run_part<4, false>(o, sb, c, seg0, len, d_err, st, spin)));
+    dim3 grid((unsigned)c.nblocks, (unsigned)((len + SS_TT - 1) / SS_TT));
+    kern<<<grid, SS_NT, (size_t)sb.nbuf * sb.bufbytes, st>>>(
+        sb.scratch.as<uint16_t>(), sb.ldp, sb.stage0.as<uint32_t>() + c.block0,
+        sb.rowlist0.as<uint32_t>() + c.block0, sb.stages.as<uint32_t>(), sb.rows.as<SubRow>(),
+        sb.info.as<uint32_t>() + c.block0 * SS_TB * sb.nsub, sb.nsub, ntrials, seg0, seg0 + len,
+        d_out, ldo, d_part, ntiles, sb.rowcap, sb.bufbytes, sb.nbuf, d_err, spin);
+    PSR_CUDA(cudaGetLastError());
+  }
+  return PSR_OK;
+}
+}  // namespace
 
 int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t ntrials,
                          uint64_t n, float *d_out, uint64_t ldo, double *d_part,
@@ -967,19 +1275,13 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
                          cudaStream_t st, long long spin_limit, int arm_only, bool want_means,
                          const SubbandPlan *sb, uint64_t chunk_index) {
   const long long spin = spin_limit > 0 ? spin_limit : DD_SPIN_LIMIT;
-  if (sb && sb->G && !arm_only && o.kind == SAMPLE_U8 && chunk_index < sb->block0.size()) {
-    int rc = launch_dedisperse_sb(o, d_delays, ntrials, n, d_out, ldo, d_part, max_spread,
-                                  d_err, st, spin, *sb, chunk_index);
-    if (rc == PSR_OK) {
-      if (want_means) {
-        const uint64_t ntiles = (n + DD_TT - 1) / DD_TT;
-        k_reduce_parts<<<(unsigned)((ntrials + 127) / 128), 128, 0, st>>>(
-            d_part, ntiles, ntrials, n, d_sums, d_means, d_out, ldo, 0);
-        PSR_CUDA(cudaGetLastError());
-      }
-      return PSR_OK;
-    }
-    if (rc != PSR_EINVAL) return rc;  // EINVAL: this shape does not fit; take the kernels below
+  if (sb && sb->G && !arm_only && o.kind == SAMPLE_U8 && chunk_index < sb->chunks.size()) {
+    PSR_TRY(launch_dedisperse_sub(o, ntrials, n, d_out, ldo, d_part, d_err, st, spin, *sb,
+                                  chunk_index));
+    if (want_means)
+      PSR_TRY(reduce_parts(d_part, (n + SS_TT - 1) / SS_TT, ntrials, n, d_sums, d_means, d_out,
+                           ldo, 0, st));
+    return PSR_OK;
   }
   // Integer samples: channel groups small enough that a group's sum fits the
   // 16-bit lanes (nch * max <= 65535 when there is one group); the groups'
@@ -1033,11 +1335,8 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
         if (rc != PSR_OK) return rc;
         PSR_CUDA(cudaGetLastError());
       }
-      if (want_means) {
-        k_reduce_parts<<<(unsigned)((ntrials + 127) / 128), 128, 0, st>>>(
-            d_part, ntiles, ntrials, n, d_sums, d_means, d_out, ldo, 0);
-        PSR_CUDA(cudaGetLastError());
-      }
+      if (want_means)
+        PSR_TRY(reduce_parts(d_part, ntiles, ntrials, n, d_sums, d_means, d_out, ldo, 0, st));
       return PSR_OK;
     }
   }
@@ -1060,11 +1359,9 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
                                                       ntiles);
   }
   PSR_CUDA(cudaGetLastError());
-  if (want_means) {
-    k_reduce_parts<<<(unsigned)((ntrials + 127) / 128), 128, 0, st>>>(
-        d_part, ntiles, ntrials, n, d_sums, d_means, d_out, ldo, o.kind == SAMPLE_F32 ? 1 : 0);
-    PSR_CUDA(cudaGetLastError());
-  }
+  if (want_means)
+    PSR_TRY(reduce_parts(d_part, ntiles, ntrials, n, d_sums, d_means, d_out, ldo,
+                         o.kind == SAMPLE_F32 ? 1 : 0, st));
   return PSR_OK;
 }
 

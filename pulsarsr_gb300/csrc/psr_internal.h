@@ -245,26 +245,34 @@ int make_delay_table(const DeviceObs &o, const double *trials, uint64_t ntrials,
 // (packed integer) kernel's waits give up after spin_limit polls (0 = the
 // default limit) and set *d_err; arm_only = 1 arms its barriers without
 // issuing the copies, so every wait runs out (a test of that path).
-// Subband-reuse plan of the staged dedispersion kernel for one DM plan
-// split into outer chunks (k_dedisperse.cu): per block of 8 consecutive
-// trials of a chunk and subband of G adjacent channels, the distinct
-// intra-subband delay patterns.  G = 0: no plan.
+// Two-level dedispersion plan of one DM plan split into outer chunks
+// (k_dedisperse.cu): per chunk and subband of G adjacent channels, the distinct
+// intra-subband delay patterns (rows of `scratch`), and per block of 16 trials
+// the rows to stage and every trial's shift in them.  G = 0: no plan, channel
+// by channel.  `scratch` belongs to the stream that runs the searches.
 struct SubbandPlan {
+  struct Chunk {
+    uint64_t sub0, rel0, block0, nblocks, spread;
+  };
   int G = 0;
+  bool byte_part = false, flush = false;
   uint64_t nsub = 0;
-  DevBuf entries;
-  std::vector<uint64_t> block0;  // first block of each outer chunk
-  uint64_t reused = 0, direct = 0;  // (block, subband) pairs by mode
+  uint64_t seg = 0, ldp = 0;  // samples per segment, row stride of scratch
+  int rowcap = 0, prowcap = 0, bufbytes = 0, nbuf = 0;
+  std::vector<Chunk> chunks;
+  DevBuf subs, rel, stage0, rowlist0, stages, rows, info, scratch;
 };
 // The subband width searches use when not told otherwise: the process-wide
-// setting of psr_set_dedisp_subbands, else the per-sample-kind default.
+// setting of psr_set_dedisp_subbands (-1: chosen from the delay table).
 int dedisp_subbands_default(const DeviceObs &o);
-int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch,
+// n: series length; maxv: largest sample (0: no plan); G: 4, 8, 0 (no plan)
+// or -1 (the cheapest).  A plan that does not fit leaves plan.G = 0.
+int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
                        cudaStream_t st);
 // With want_means = false (series only folded, not searched) the sums and
 // means are left unset.  With a subband plan (8-bit-storage samples), chunk
-// chunk_index of the plan runs the subband-reuse kernel.
+// chunk_index of the plan runs the two-level kernels.
 int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t ntrials,
                          uint64_t n, float *d_out, uint64_t ldo, double *d_part, double *d_sums,
                          float *d_means, uint64_t max_spread, unsigned *d_err, cudaStream_t st,

@@ -64,7 +64,8 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   cstart.push_back(ntrials);
   nchunks = cstart.size() - 1;
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
-  PSR_TRY(build_subband_plan(tab, o.nch, cstart, o.kind == SAMPLE_U8 ? G : 0, sbplan, st));
+  PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
+                             sbplan, st));
   PSR_TRY(chunk_overflow.ensure(nchunks * 4 + 16));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&ev_fft[0], &ev_fft[1], &ev_sel[0], &ev_sel[1]})
