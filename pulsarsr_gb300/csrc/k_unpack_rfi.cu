@@ -211,29 +211,16 @@ __global__ void k_hist_median(const unsigned *__restrict__ hist, uint64_t nch, u
   med[c] = (float)d;
 }
 
-// Exact integer channel totals (for the provably-exact f32 fast path).
-template <class T>
-__global__ void k_chan_total(const T *__restrict__ s, uint64_t ns, uint64_t ld,
-                             unsigned long long *__restrict__ tot) {
-  const T *row = s + (uint64_t)blockIdx.y * ld;
-  unsigned long long acc = 0;
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ns;
-       t += (uint64_t)gridDim.x * blockDim.x)
-    acc += (unsigned long long)row[t];
-  for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&tot[blockIdx.y], acc);
-}
-
 template <class T>
 __device__ __forceinline__ float as_f32(T v) {
   return (float)v;
 }
 
-// Channel means and variances (rfi/src/lib.rs:35-43), in reference order,
-// with the per-sample work taken off the sequential chain: one
-// CTA per channel; warps 1.. write the f32 terms of the next segment into a
-// shared-memory double buffer while thread 0 adds the current segment's terms
-// in reference order.  The chain then costs one FADD latency per sample.
+// A sum of f32 samples in the reference's order where it can fall (negative
+// samples): the per-sample work is taken off the sequential chain, one CTA
+// per channel; warps 1.. write the next segment into a shared-memory double
+// buffer while thread 0 adds the current one.  The chain then costs one FADD
+// latency per sample.
 constexpr int PC_NT = 256;
 constexpr int PC_SEG = 2048;
 
@@ -283,303 +270,438 @@ __device__ float pc_sequential_sum(const T *row, uint64_t ns, float *buf, Term t
   return acc;  // valid in thread 0
 }
 
-template <class T>
-__global__ void __launch_bounds__(PC_NT)
-    k_chan_mean_var_pc(const T *__restrict__ s, uint64_t ns, uint64_t ld,
-                       const unsigned long long *__restrict__ tot, float *__restrict__ means,
-                       float *__restrict__ vars) {
-  __shared__ __align__(16) float buf[2 * PC_SEG];
-  __shared__ float mean_s;
-  const uint64_t c = blockIdx.x;
-  const T *row = s + c * ld;
-  if (sizeof(T) < 4 && tot[c] <= (1ull << 24)) {
-    if (threadIdx.x == 0) mean_s = __fdiv_rn((float)tot[c], (float)ns);
-  } else {
-    const float sum = pc_sequential_sum(row, ns, buf, [](float x) { return x; });
-    if (threadIdx.x == 0) mean_s = __fdiv_rn(sum, (float)ns);
-  }
-  __syncthreads();
-  const float m = mean_s;
-  const float acc = pc_sequential_sum(row, ns, buf, [m](float x) {
-    const float d = __fsub_rn(x, m);
-    return __fmul_rn(d, d);
-  });
-  if (threadIdx.x == 0) {
-    means[c] = m;
-    vars[c] = __fdiv_rn(acc, (float)ns);
-  }
-}
-
 // Reference-order f32 sums of non-negative terms, s = RN(...RN(RN(-0 + t0) +
 // t1)... + t_{n-1}), bit for bit, in parallel.  While s stays in one binade
 // [2^e, 2^(e+1)) every representable value is a multiple of u = 2^(e-23), so
 // s = K u (2^23 <= K < 2^24) and RN(s + t) = (K + inc(t)) u with inc(t) =
 // t/u rounded to nearest: the integer part q of t/u plus one when its
 // fraction exceeds 1/2.  An exact half (a tie) rounds to even: inc = q +
-// ((K + q) mod 2), so it depends on the running K only through its parity,
-// and leaves K even.  The parity after a run of terms is therefore either
-// P xor c (no tie in the run) or a constant (after its last tie): these maps
-// compose, so a warp scans them across its lanes, and the total of a
-// 512-term chunk is a known sum plus, when it holds a tie, one bit that
-// depends on K's parity at the chunk's start.  t >= 0 makes K monotone; a
-// chunk whose total keeps K + total < 2^24 is added at once.  Chunks with a
-// binade crossing, a subnormal, infinite or NaN term, or s still 0 or
-// subnormal are added term by term in order.
-constexpr int ES_L = 512;  // terms per chunk, 16 per lane
+// ((K + q) mod 2), so it depends on the running K through its parity alone.
+// A run of terms is therefore a map from K's parity to an increment, (d0, d1),
+// and maps compose: after (a0, a1), (b0, b1) adds b0 or b1 by the parity of
+// what stands then.  t >= 0 makes K monotone: a run whose increment keeps
+// K + d < 2^24 is added at once.
+//
+// The binade is not known before the sum is, but it can be guessed from plain
+// sums of the terms.  So the pass over the samples is parallel over the whole
+// card, and only a scan over chunks of 512 terms is left per channel:
+//   k_es_sums   plain sums of every chunk's samples and their squares
+//   k_es_guess  binades of the mean's running sum at every chunk
+//   k_es_maps   the map of every chunk at its guessed binade
+//   k_es_scan   one warp per channel: composes 32 chunks' maps at a time;
+//               a chunk whose guess is wrong, or that leaves its binade, is
+//               taken apart into its lanes' 16 terms (maps again at the true
+//               binade, the lane that crosses term by term)
+// and the last two again for the variance, whose binades follow from the mean
+// and the plain sums.  Subnormal, infinite and NaN terms make a run special:
+// it is added term by term.
+constexpr int ES_L = 512;          // terms per chunk, 16 per lane
+constexpr int ES_PER = ES_L / 32;
+constexpr uint32_t ES_SPECIAL = 0xffffffffu;
 
-// One term at unit u = 2^(e - 23): inc = q (+1 above the half), kind 0;
-// kind 1: an exact half (inc = q, the rounding bit comes from K's parity);
-// kind 2: a term the binade arithmetic does not cover.
-__device__ __forceinline__ int es_term(float t, int e, unsigned long long &inc) {
-  const uint32_t b = __float_as_uint(t);
-  const int be = (int)((b >> 23) & 0xff);
-  inc = 0;
-  if (be == 0 || be == 255) return (b & 0x7fffffffu) != 0u ? 2 : 0;  // +-0 adds nothing
-  const uint32_t mt = (b & 0x7fffffu) | 0x800000u;
-  const int sh = (be - 150) - (e - 23);  // t / u = mt 2^sh
-  if (sh >= 0) {
-    // t >= 2^23 u > 2^e would leave the binade: count it as 2^40 units
-    // (any such term fails the K + total < 2^24 test; no 64-bit overflow)
-    inc = sh >= 24 ? (1ull << 40) : ((unsigned long long)mt << sh);
-    return 0;
-  }
-  if (sh <= -25) return 0;  // below half a unit
-  const int r = -sh;
-  const uint32_t rem = mt & ((1u << r) - 1u), half = 1u << (r - 1);
-  inc = (unsigned long long)(mt >> r) + (rem > half ? 1ull : 0ull);
-  return rem == half ? 1 : 0;
-}
-
-// A warp's chunk at unit u: total(P0) = base + (tie ? P0 ^ bit : 0) for K's
-// parity P0 at the chunk's start; special: the chunk must go term by term.
-struct EsChunk {
-  unsigned long long base;
-  int bit;
-  bool tie, special;
-};
-
-template <int PER>
-__device__ __forceinline__ EsChunk es_chunk_warp(const float (&t)[PER], int e, int lane) {
-  // lane map: constant (after a tie in the lane) or xor
-  bool lc = false, lsp = false;
-  uint32_t lv = 0;
-  unsigned long long lsum = 0;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    unsigned long long inc;
-    const int k = es_term(t[j], e, inc);
-    lsum += inc;
-    if (k == 2) {
-      lsp = true;
-    } else if (k == 1) {
-      lc = true;
-      lv = 0;
-    } else {
-      lv ^= (uint32_t)inc & 1u;
-    }
-  }
-  EsChunk c;
-  c.bit = 0;
-  c.tie = __any_sync(0xffffffffu, lc);
-  c.special = __any_sync(0xffffffffu, lsp);
-  if (!c.tie) {  // (most chunks) the total does not depend on K
-#pragma unroll
-    for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    c.base = lsum;
-    return c;
-  }
-  // inclusive scan of the maps, then the map from the chunk start to this lane
-  bool ic = lc;
-  uint32_t v = lv;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const bool pic = __shfl_up_sync(0xffffffffu, ic, o);
-    const uint32_t pv = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) {
-      v = ic ? v : (pv ^ v);
-      ic = ic || pic;
-    }
-  }
-  bool conc = __shfl_up_sync(0xffffffffu, ic, 1);
-  uint32_t P = __shfl_up_sync(0xffffffffu, v, 1);
-  if (lane == 0) {
-    conc = false;
-    P = 0;
-  }
-  // conc: P is K's parity; otherwise K's parity is P0 ^ P
-  unsigned long long base = 0;
-  int fb = -1;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    unsigned long long inc;
-    const int k = es_term(t[j], e, inc);
-    if (k == 1) {
-      if (conc) {
-        base += inc + ((P + (uint32_t)inc) & 1u);
-      } else {  // the chunk's first tie: its bit waits for P0
-        base += inc;
-        fb = (int)((P ^ (uint32_t)inc) & 1u);
-      }
-      P = 0;
-      conc = true;
-    } else if (k == 0) {
-      base += inc;
-      P ^= (uint32_t)inc & 1u;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
-  const unsigned fm = __ballot_sync(0xffffffffu, fb >= 0);
-  c.base = base;
-  c.bit = fm ? __shfl_sync(0xffffffffu, fb, __ffs(fm) - 1) : 0;
-  return c;
-}
-
-// Lane l's 16 consecutive samples of chunk g of a step: one or two aligned
-// 16-byte loads (rows start 64-element aligned; only issued for samples below
-// ns, whose 16-sample run then ends inside the row's padding).
+// Lane l's 16 consecutive samples of a chunk: aligned 16-byte loads (rows
+// start 64-element aligned; only issued for samples below ns, whose 16-sample
+// run then ends inside the row's padding).
 template <class T>
 struct EsRaw {
-  static constexpr int W = 16 * (int)sizeof(T) / 16;
+  static constexpr int W = (int)sizeof(T);
   uint4 r[W];
   __device__ __forceinline__ void load(const T *p, bool ok) {
 #pragma unroll
     for (int k = 0; k < W; ++k)
       r[k] = ok ? __ldg(reinterpret_cast<const uint4 *>(p) + k) : make_uint4(0u, 0u, 0u, 0u);
   }
+  __device__ __forceinline__ uint32_t word(int i) const {
+    const uint4 &q = r[i >> 2];
+    return (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
+  }
   __device__ __forceinline__ float at(int j) const {
-    if constexpr (sizeof(T) == 1) {
-      const uint32_t w = (r[0].x * (j >> 2 == 0)) | (r[0].y * (j >> 2 == 1)) |
-                         (r[0].z * (j >> 2 == 2)) | (r[0].w * (j >> 2 == 3));
-      return (float)((w >> (8 * (j & 3))) & 255u);
-    } else {
-      const uint4 &q = r[j >> 3];
-      const int e = (j >> 1) & 3;
-      const uint32_t w = e == 0 ? q.x : (e == 1 ? q.y : (e == 2 ? q.z : q.w));
-      return (float)((w >> (16 * (j & 1))) & 65535u);
-    }
+    if constexpr (sizeof(T) == 1) return (float)((word(j >> 2) >> (8 * (j & 3))) & 255u);
+    else if constexpr (sizeof(T) == 2) return (float)((word(j >> 1) >> (16 * (j & 1))) & 65535u);
+    else return __uint_as_float(word(j));
   }
 };
 
-constexpr int ES_G = 16;  // chunks per step = warps per CTA
-
-// One CTA of ES_G warps per channel: warp w holds chunk w of every step of
-// ES_G chunks (its samples prefetched a step ahead), computes the chunk's
-// total at the binade of the running s, and the CTA adds the longest run of
-// chunks that stays in the binade (each tie's rounding bit from the running
-// parity); a chunk that cannot be is added term by term, in order, by
-// thread 0.  Returns s in every thread.
-struct EsShared {
-  float stage[ES_L];
-  unsigned long long tot[ES_G];
-  int tie[ES_G], bit[ES_G], special[ES_G];
-  float s;
-};
-
-template <class T, class Term>
-__device__ float exact_seq_sum_cta(const T *__restrict__ row, uint64_t ns, Term term,
-                                   EsShared &sh) {
-  const int lane = (int)(threadIdx.x & 31), g = (int)(threadIdx.x >> 5);
-  constexpr int PER = ES_L / 32;
-  constexpr uint64_t STEP = (uint64_t)ES_G * ES_L;
-  if (threadIdx.x == 0) sh.s = -0.0f;
-  EsRaw<T> raw, nxt;
-  {
-    const uint64_t i0 = (uint64_t)g * ES_L + (uint64_t)lane * PER;
-    raw.load(row + i0, i0 < ns);
+// The map (d0, d1) of N terms at the binade with biased exponent be; true if
+// the run is special or its increment reaches 2^24 (it leaves the binade).
+template <int N>
+__device__ __forceinline__ bool es_run(const float (&t)[N], int be, uint32_t &d0, uint32_t &d1) {
+  bool special = false;
+  d0 = d1 = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t b = __float_as_uint(t[j]) & 0x7fffffffu;
+    const int bt = (int)(b >> 23);
+    special |= bt == 255 || (bt == 0 && b != 0) || bt > be;
+    const uint32_t mt = bt ? (b & 0x7fffffu) | 0x800000u : 0u;
+    const int r = min(max(be - bt, 0), 25);  // t / u = mt 2^-r; below half a unit past 24
+    const uint32_t q = mt >> r, frac = __funnelshift_r(0u, mt, r);
+    const uint32_t inc = q + (frac > 0x80000000u ? 1u : 0u);
+    const uint32_t tie = frac == 0x80000000u ? 1u : 0u;
+    d0 += inc;
+    d0 += d0 & tie;
+    d1 += inc;
+    d1 += ~d1 & tie;
   }
-  __syncthreads();
-  for (uint64_t c0 = 0; c0 < ns; c0 += STEP) {
-    const uint64_t i0 = c0 + (uint64_t)g * ES_L + (uint64_t)lane * PER;
-    nxt.load(row + i0 + STEP, i0 + STEP < ns);
-    float t[PER];
-#pragma unroll
-    for (int j = 0; j < PER; ++j) t[j] = i0 + j < ns ? term(raw.at(j)) : 0.0f;
-    const int nchunk = (int)min((uint64_t)ES_G, (ns - c0 + ES_L - 1) / ES_L);
-    int g0 = 0;
-    while (g0 < nchunk) {  // g0 and sh.s are uniform across the CTA
-      const float s = sh.s;
-      const uint32_t sb = __float_as_uint(s);
-      const int se = (int)((sb >> 23) & 0xff);
-      int g1 = g0;
-      if (se > 0 && se < 255 && !(sb >> 31)) {
-        const int e = se - 127;
-        if (g >= g0) {  // warp-uniform
-          const EsChunk ck = es_chunk_warp<PER>(t, e, lane);
-          if (lane == 0) {
-            sh.tot[g] = ck.base;
-            sh.tie[g] = ck.tie ? 1 : 0;
-            sh.bit[g] = ck.bit;
-            sh.special[g] = ck.special ? 1 : 0;
-          }
-        }
-        __syncthreads();
-        unsigned long long acc = (sb & 0x7fffffu) | 0x800000u;
-        bool stop = false;
-#pragma unroll
-        for (int k = 0; k < ES_G; ++k) {
-          if (k >= g0 && k < nchunk && !stop) {
-            // a chunk with a tie: its first tie rounds by K's parity here
-            const uint32_t rb = ((uint32_t)acc ^ (uint32_t)sh.bit[k]) & 1u;
-            const unsigned long long tk = sh.tot[k] + (sh.tie[k] ? rb : 0u);
-            if (sh.special[k] || acc + tk >= (1ull << 24)) {
-              stop = true;
-            } else {
-              acc += tk;
-              g1 = k + 1;
-            }
-          }
-        }
-        __syncthreads();  // every thread has read sh.s, sh.tot and sh.tie
-        if (g1 > g0 && threadIdx.x == 0)
-          sh.s = __uint_as_float(((uint32_t)(e + 127) << 23) | ((uint32_t)acc & 0x7fffffu));
-      }
-      if (g1 == g0) {  // chunk g0 term by term
-        if (g == g0)
-#pragma unroll
-          for (int j = 0; j < PER; ++j) sh.stage[lane * PER + j] = t[j];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          float a = sh.s;
-          const int cnt = (int)min((uint64_t)ES_L, ns - (c0 + (uint64_t)g0 * ES_L));
-          for (int i = 0; i < cnt; ++i) a = __fadd_rn(a, sh.stage[i]);
-          sh.s = a;
-        }
-        g1 = g0 + 1;
-      }
-      __syncthreads();  // sh.s updated
-      g0 = g1;
-    }
-    raw = nxt;
-  }
-  return sh.s;
+  return special || d0 >= (1u << 24) || d1 >= (1u << 24);
 }
 
-// Channel means and variances (rfi/src/lib.rs:35-43) for integer samples:
-// one warp per channel, the exact parallel reference-order sums above (the
-// mean straight from the exact integer total while it is below 2^24).
-template <class T>
-__global__ void __launch_bounds__(32 * ES_G)
-    k_chan_mean_var_ex(const T *__restrict__ s, uint64_t ns, uint64_t ld,
-                       const unsigned long long *__restrict__ tot, float *__restrict__ means,
-                       float *__restrict__ vars) {
-  __shared__ EsShared sh;
-  const uint64_t c = blockIdx.x;
-  const T *row = s + c * ld;
-  float m;
-  if (tot[c] <= (1ull << 24)) {
-    m = __fdiv_rn((float)tot[c], (float)ns);
-  } else {
-    m = __fdiv_rn(exact_seq_sum_cta(row, ns, [](float x) { return x; }, sh), (float)ns);
-    __syncthreads();  // sh is reused below
+// Inclusive scan of the lanes' maps.
+__device__ __forceinline__ void es_scan_maps(uint32_t &d0, uint32_t &d1, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t a0 = __shfl_up_sync(0xffffffffu, d0, o);
+    const uint32_t a1 = __shfl_up_sync(0xffffffffu, d1, o);
+    if (lane >= o) {
+      const uint32_t b0 = d0, b1 = d1;
+      d0 = a0 + ((a0 & 1u) ? b1 : b0);
+      d1 = a1 + ((a1 & 1u) ? b0 : b1);
+    }
   }
-  const float acc = exact_seq_sum_cta(row, ns, [m](float x) {
-    const float d = __fsub_rn(x, m);
-    return __fmul_rn(d, d);
-  }, sh);
+}
+
+// Adds the longest prefix of the lanes [cur, 32) with `valid` maps that keeps
+// s in its binade (biased exponent be, normal); returns the first lane left.
+__device__ __forceinline__ int es_advance(float &s, int be, bool valid, uint32_t m0, uint32_t m1,
+                                          int cur, int lane) {
+  const unsigned vm = __ballot_sync(0xffffffffu, valid && lane >= cur) >> cur;
+  const int run = vm == 0xffffffffu ? 32 : __ffs(~vm) - 1;
+  const bool in = lane >= cur && lane < cur + run;
+  uint32_t d0 = in ? m0 : 0u, d1 = in ? m1 : 0u;
+  es_scan_maps(d0, d1, lane);
+  const uint32_t K = (__float_as_uint(s) & 0x7fffffu) | 0x800000u;
+  const uint32_t Kn = K + ((K & 1u) ? d1 : d0);
+  const int nok = __popc(__ballot_sync(0xffffffffu, in && Kn < (1u << 24)));
+  if (nok) {
+    const uint32_t Kl = __shfl_sync(0xffffffffu, Kn, cur + nok - 1);
+    s = __uint_as_float((uint32_t)be << 23 | (Kl & 0x7fffffu));
+  }
+  return cur + nok;
+}
+
+// One chunk by a warp: lane l holds terms 16 l .. 16 l + 15 of it (cnt valid
+// terms in all); returns s, in every lane.
+__device__ __noinline__ float es_chunk(const float (&t)[ES_PER], int cnt, float s, int lane) {
+  int cur = 0;
+  while (cur < 32) {
+    const int be = (int)(__float_as_uint(s) >> 23);
+    if (be > 0 && be < 255) {
+      uint32_t d0, d1;
+      const bool bad = es_run(t, be, d0, d1);
+      cur = es_advance(s, be, !bad, d0, d1, cur, lane);
+      if (cur == 32) break;
+    }
+#pragma unroll
+    for (int j = 0; j < ES_PER; ++j) {
+      const float v = __shfl_sync(0xffffffffu, t[j], cur);
+      if (cur * ES_PER + j < cnt) s = __fadd_rn(s, v);
+    }
+    ++cur;
+  }
+  return s;
+}
+
+// Plain sums per chunk: sum[] exact for integer samples (32 bits hold 512
+// 16-bit samples), sq[] and the f32 sums rounded (they only guess binades).
+// neg[c] is set when a channel holds a negative (or NaN) f32 sample.
+// Bound: HBM, one read of the samples.
+constexpr int EK_NT = 256, EK_CPW = 4;  // chunks per warp
+template <class T>
+__global__ void __launch_bounds__(EK_NT)
+    k_es_sums(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t nck,
+              uint32_t *__restrict__ sum, float *__restrict__ sq, unsigned *__restrict__ neg) {
+  const int lane = (int)(threadIdx.x & 31);
+  const T *row = s + (uint64_t)blockIdx.y * ld;
+  const uint64_t k0 = ((uint64_t)blockIdx.x * (EK_NT / 32) + (threadIdx.x >> 5)) * EK_CPW;
+  EsRaw<T> x[EK_CPW];
+#pragma unroll
+  for (int i = 0; i < EK_CPW; ++i) {
+    const uint64_t p = (k0 + i) * ES_L + (uint64_t)lane * ES_PER;
+    x[i].load(row + p, p < ns);
+  }
+  bool below = false;
+#pragma unroll
+  for (int i = 0; i < EK_CPW; ++i) {
+    const uint64_t k = k0 + i;
+    if (k >= nck) break;  // (warp-uniform)
+    const uint64_t at = (uint64_t)blockIdx.y * nck + k;  // (samples past ns are zero)
+    if constexpr (sizeof(T) == 1) {
+      unsigned a = 0, q = 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        a = __dp4a(x[i].word(w), 0x01010101u, a);
+        q = __dp4a(x[i].word(w), x[i].word(w), q);
+      }
+      a = __reduce_add_sync(0xffffffffu, a);
+      q = __reduce_add_sync(0xffffffffu, q);
+      if (lane == 0) {
+        sum[at] = a;
+        sq[at] = (float)q;
+      }
+    } else if constexpr (sizeof(T) == 2) {
+      unsigned a = 0;
+      float q = 0.0f;
+#pragma unroll
+      for (int j = 0; j < ES_PER; ++j) {
+        const float v = x[i].at(j);
+        a += (unsigned)v;
+        q = __fmaf_rn(v, v, q);
+      }
+      a = __reduce_add_sync(0xffffffffu, a);
+      for (int o = 16; o; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
+      if (lane == 0) {
+        sum[at] = a;
+        sq[at] = q;
+      }
+    } else {
+      float a = 0.0f, q = 0.0f;
+#pragma unroll
+      for (int j = 0; j < ES_PER; ++j) {
+        const float v = x[i].at(j);
+        below |= !(v >= 0.0f);
+        a += v;
+        q = __fmaf_rn(v, v, q);
+      }
+      for (int o = 16; o; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        q += __shfl_down_sync(0xffffffffu, q, o);
+      }
+      if (lane == 0) {
+        sum[at] = __float_as_uint(a);
+        sq[at] = q;
+      }
+    }
+  }
+  if (sizeof(T) == 4 && __any_sync(0xffffffffu, below) && lane == 0) atomicOr(&neg[blockIdx.y], 1u);
+}
+
+// Plain sums run in integers (exact) for integer samples and in f32 otherwise
+// (FP64 runs at 1/64 rate here; only the binade is wanted).
+template <class T>
+struct EsPlain {
+  typedef unsigned long long type;
+  static __device__ __forceinline__ type of(uint32_t v) { return v; }
+};
+template <>
+struct EsPlain<float> {
+  typedef float type;
+  static __device__ __forceinline__ float of(uint32_t v) { return __uint_as_float(v); }
+};
+// Biased f32 exponent of a prefix (0: no guess).
+__device__ __forceinline__ uint8_t es_binade(float p) {
+  const uint32_t b = __float_as_uint(p) >> 23;
+  return b > 0 && b < 255 ? (uint8_t)b : (uint8_t)0;
+}
+
+// Binades at the start of every chunk of one channel's running sum of chunk
+// sums f(k), by a CTA of EG_NT threads; returns the total in every thread.
+constexpr int EG_NT = 256;
+template <class A, class F>
+__device__ A es_guess(uint64_t nck, F f, uint8_t *__restrict__ out, A *red) {
+  // contiguous chunks per thread: its sum, a scan of the threads' sums, then
+  // its running sums
+  const uint64_t per = (nck + EG_NT - 1) / EG_NT;
+  const uint64_t a = min((uint64_t)threadIdx.x * per, nck), b = min(a + per, nck);
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+  A t = 0;
+  for (uint64_t k = a; k < b; ++k) t += f(k);
+  A inc = t;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const A v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  __syncthreads();  // red may still be read by an earlier call
+  if (lane == 31) red[warp] = inc;
+  __syncthreads();
+  A p = inc - t, tot = 0;
+  for (int i = 0; i < EG_NT / 32; ++i) {
+    if (i < warp) p += red[i];
+    tot += red[i];
+  }
+  for (uint64_t k = a; k < b; ++k) {
+    out[k] = es_binade((float)p);
+    p += f(k);
+  }
+  return tot;
+}
+
+// What a channel's mean needs: 0 its exact integer total (at most 2^24, every
+// partial sum exact), 1 the maps, 2 the sequential sum (negative samples).
+struct EsChan {
+  int mode;
+};
+
+template <class T>
+__device__ void es_guess_var(const uint32_t *sum, const float *sq, uint64_t nck, uint64_t ns,
+                             float m, uint8_t *guess, float *red) {
+  es_guess<float>(nck, [&](uint64_t k) {
+    const float cnt = (float)min((uint64_t)ES_L, ns - k * ES_L);
+    const float a = (float)EsPlain<T>::of(sum[k]);
+    return fmaxf(__fmaf_rn(m, __fmaf_rn(cnt, m, -2.0f * a), sq[k]), 0.0f);
+  }, guess, red);
+}
+
+// One CTA per channel: the mean's binades, or the mean itself where the total
+// is exact (then the variance's binades).
+template <class T>
+__global__ void __launch_bounds__(EG_NT)
+    k_es_guess(const uint32_t *__restrict__ sum, const float *__restrict__ sq,
+               const unsigned *__restrict__ neg, uint64_t nck, uint64_t ns,
+               uint8_t *__restrict__ guess, EsChan *__restrict__ chan,
+               float *__restrict__ means) {
+  typedef typename EsPlain<T>::type A;
+  __shared__ A red[EG_NT / 32];
+  __shared__ float redf[EG_NT / 32];
+  const uint64_t c = blockIdx.x;
+  sum += c * nck;
+  sq += c * nck;
+  guess += c * nck;
+  const A tot = es_guess<A>(nck, [&](uint64_t k) { return EsPlain<T>::of(sum[k]); }, guess, red);
+  int mode = 1;
+  if (sizeof(T) < 4 && tot <= (A)16777216) mode = 0;
+  if (sizeof(T) == 4 && neg[c]) mode = 2;
+  const float m = __fdiv_rn((float)tot, (float)ns);
   if (threadIdx.x == 0) {
-    means[c] = m;
-    vars[c] = __fdiv_rn(acc, (float)ns);
+    chan[c].mode = mode;
+    if (mode == 0) means[c] = m;
+  }
+  if (mode == 0) es_guess_var<T>(sum, sq, nck, ns, m, guess, redf);
+}
+
+template <bool VAR>
+__device__ __forceinline__ float es_term(float x, float m) {
+  if constexpr (!VAR) return x;
+  const float d = __fsub_rn(x, m);
+  return __fmul_rn(d, d);
+}
+
+// The map of every chunk at its guessed binade.
+// Bound: issue, about 30 instructions per sample.
+// Measured on a GB300 (512 8-bit channels of 1,047,799 samples, means above
+// 2^24): the six kernels 2.3 ms, 0.88 of them in each pass of k_es_maps; one
+// CTA per channel that walked its chunks in order took 6.4 with its totals.
+template <class T, bool VAR>
+__global__ void __launch_bounds__(EK_NT)
+    k_es_maps(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t nck,
+              const uint8_t *__restrict__ guess, const EsChan *__restrict__ chan,
+              const float *__restrict__ means, uint2 *__restrict__ maps) {
+  const uint64_t c = blockIdx.y;
+  if (!VAR && chan[c].mode != 1) return;
+  const int lane = (int)(threadIdx.x & 31);
+  const T *row = s + c * ld;
+  const float m = VAR ? means[c] : 0.0f;
+  const uint64_t k0 = ((uint64_t)blockIdx.x * (EK_NT / 32) + (threadIdx.x >> 5)) * EK_CPW;
+  EsRaw<T> nx;
+  {
+    const uint64_t p = k0 * ES_L + (uint64_t)lane * ES_PER;
+    nx.load(row + p, p < ns);
+  }
+  for (int i = 0; i < EK_CPW; ++i) {
+    const uint64_t k = k0 + i;
+    if (k >= nck) break;
+    const uint64_t p = k * ES_L + (uint64_t)lane * ES_PER;
+    const EsRaw<T> x = nx;
+    if (i + 1 < EK_CPW) nx.load(row + p + ES_L, p + ES_L < ns);
+    const int be = (int)guess[c * nck + k];
+    uint2 out = make_uint2(ES_SPECIAL, ES_SPECIAL);
+    if (be) {
+      float t[ES_PER];
+#pragma unroll
+      for (int j = 0; j < ES_PER; ++j) t[j] = p + j < ns ? es_term<VAR>(x.at(j), m) : 0.0f;
+      uint32_t d0, d1;
+      const bool bad = es_run(t, be, d0, d1);
+      if (!__any_sync(0xffffffffu, bad)) {
+        if (!__any_sync(0xffffffffu, d0 != d1)) {  // no lane depends on the parity
+          d0 = d1 = __reduce_add_sync(0xffffffffu, d0);
+        } else {
+          es_scan_maps(d0, d1, lane);
+          d0 = __shfl_sync(0xffffffffu, d0, 31);
+          d1 = __shfl_sync(0xffffffffu, d1, 31);
+        }
+        if (d0 < (1u << 24) && d1 < (1u << 24)) out = make_uint2(d0, d1);
+      }
+    }
+    if (lane == 0) maps[c * nck + k] = out;
+  }
+}
+
+// The running sum over a channel's chunks; the mean (then the variance's
+// binades) or the variance.  One CTA per channel, the scan by its first warp.
+template <class T, bool VAR>
+__global__ void __launch_bounds__(EG_NT)
+    k_es_scan(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t nck,
+              const uint32_t *__restrict__ sum, const float *__restrict__ sq,
+              uint8_t *__restrict__ guess, const EsChan *__restrict__ chan,
+              const uint2 *__restrict__ maps, float *__restrict__ means,
+              float *__restrict__ vars) {
+  __shared__ float red[EG_NT / 32];
+  __shared__ float mean_s;
+  const uint64_t c = blockIdx.x;
+  if (!VAR && chan[c].mode == 0) return;
+  guess += c * nck;
+  maps += c * nck;
+  const T *row = s + c * ld;
+  if (threadIdx.x < 32 && (VAR || chan[c].mode == 1)) {
+    const int lane = (int)threadIdx.x;
+    const float m = VAR ? means[c] : 0.0f;
+    float acc = -0.0f;
+    uint2 nm = make_uint2(ES_SPECIAL, ES_SPECIAL);
+    int nb = 0;
+    if (lane < (int)min((uint64_t)32, nck)) {
+      nm = maps[lane];
+      nb = (int)guess[lane];
+    }
+    for (uint64_t g0 = 0; g0 < nck; g0 += 32) {
+      const int cnt = (int)min((uint64_t)32, nck - g0);
+      const uint2 mp = nm;
+      const int gb = nb;
+      if (g0 + 32 + lane < nck) {
+        nm = maps[g0 + 32 + lane];
+        nb = (int)guess[g0 + 32 + lane];
+      }
+      int cur = 0;
+      while (cur < cnt) {
+        const int be = (int)(__float_as_uint(acc) >> 23);
+        if (be > 0 && be < 255) {
+          const bool valid = lane < cnt && gb == be && mp.x != ES_SPECIAL;
+          cur = es_advance(acc, be, valid, mp.x, mp.y, cur, lane);
+          if (cur >= cnt) break;
+        }
+        const uint64_t k = g0 + cur, p = k * ES_L + (uint64_t)lane * ES_PER;
+        EsRaw<T> x;
+        x.load(row + p, p < ns);
+        float t[ES_PER];
+#pragma unroll
+        for (int j = 0; j < ES_PER; ++j) t[j] = p + j < ns ? es_term<VAR>(x.at(j), m) : 0.0f;
+        acc = es_chunk(t, (int)min((uint64_t)ES_L, ns - k * ES_L), acc, lane);
+        ++cur;
+      }
+    }
+    if (lane == 0) {
+      const float v = __fdiv_rn(acc, (float)ns);
+      if (VAR) {
+        vars[c] = v;
+      } else {
+        means[c] = v;
+        mean_s = v;
+      }
+    }
+  }
+  if constexpr (!VAR) {
+    __shared__ __align__(16) float buf[sizeof(T) == 4 ? 2 * PC_SEG : 4];
+    if constexpr (sizeof(T) == 4) {
+      if (chan[c].mode == 2) {
+        const float a = pc_sequential_sum(row, ns, buf, [](float x) { return x; });
+        if (threadIdx.x == 0) {
+          mean_s = __fdiv_rn(a, (float)ns);
+          means[c] = mean_s;
+        }
+      }
+    }
+    (void)buf;
+    __syncthreads();
+    es_guess_var<T>(sum + c * nck, sq + c * nck, nck, ns, mean_s, guess, red);
   }
 }
 
@@ -719,6 +841,38 @@ int launch_median_f32(const float *d_vals, uint64_t n, float *d_out, unsigned in
   return PSR_OK;
 }
 
+// Channel means and variances (rfi/src/lib.rs:35-43) into w.means and w.vars.
+template <class T>
+static int enqueue_mean_var(const T *s, uint64_t nch, uint64_t ns, uint64_t ld, RfiWork &w,
+                            cudaStream_t st) {
+  const uint64_t nck = (ns + ES_L - 1) / ES_L;
+  PSR_TRY(w.es_sum.ensure(nch * nck * 4));
+  PSR_TRY(w.es_sq.ensure(nch * nck * 4));
+  PSR_TRY(w.es_guess.ensure(nch * nck));
+  PSR_TRY(w.es_maps.ensure(nch * nck * sizeof(uint2)));
+  PSR_TRY(w.es_chan.ensure(nch * sizeof(EsChan)));
+  PSR_TRY(w.es_neg.ensure(nch * 4));
+  uint32_t *sum = w.es_sum.as<uint32_t>();
+  float *sq = w.es_sq.as<float>(), *means = w.means.as<float>(), *vars = w.vars.as<float>();
+  uint8_t *guess = w.es_guess.as<uint8_t>();
+  EsChan *chan = w.es_chan.as<EsChan>();
+  uint2 *maps = w.es_maps.as<uint2>();
+  if (sizeof(T) == 4) PSR_CUDA(cudaMemsetAsync(w.es_neg.p, 0, nch * 4, st));
+  constexpr uint64_t per = (EK_NT / 32) * EK_CPW;
+  const dim3 grid((unsigned)((nck + per - 1) / per), (unsigned)nch);
+  k_es_sums<T><<<grid, EK_NT, 0, st>>>(s, ns, ld, nck, sum, sq, w.es_neg.as<unsigned>());
+  k_es_guess<T><<<(unsigned)nch, EG_NT, 0, st>>>(sum, sq, w.es_neg.as<unsigned>(), nck, ns, guess,
+                                                 chan, means);
+  k_es_maps<T, false><<<grid, EK_NT, 0, st>>>(s, ns, ld, nck, guess, chan, means, maps);
+  k_es_scan<T, false><<<(unsigned)nch, EG_NT, 0, st>>>(s, ns, ld, nck, sum, sq, guess, chan, maps,
+                                                       means, vars);
+  k_es_maps<T, true><<<grid, EK_NT, 0, st>>>(s, ns, ld, nck, guess, chan, means, maps);
+  k_es_scan<T, true><<<(unsigned)nch, EG_NT, 0, st>>>(s, ns, ld, nck, sum, sq, guess, chan, maps,
+                                                      means, vars);
+  PSR_CUDA(cudaGetLastError());
+  return PSR_OK;
+}
+
 template <class T>
 static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaStream_t st) {
   const uint64_t nch = o.nch, ns = o.ns;
@@ -733,21 +887,9 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   PSR_TRY(w.blkbad.ensure(blocks_n));
   PSR_TRY(w.scratch.ensure(std::max(nch, blocks_n) * 4));
   PSR_TRY(w.flags.ensure(2 * nch));
-  PSR_TRY(w.hist.ensure(nch * 8 + 8));
+  PSR_TRY(w.active.ensure(8));
   T *s = o.samples.as<T>();
-  unsigned long long *tot = w.hist.as<unsigned long long>();
-  PSR_CUDA(cudaMemsetAsync(tot, 0, nch * 8 + 8, st));
-  if (sizeof(T) < 4) {
-    dim3 g((unsigned)std::min<uint64_t>((ns + 255) / 256, 64), (unsigned)nch);
-    k_chan_total<T><<<g, 256, 0, st>>>(s, ns, o.ld, tot);
-  }
-  if constexpr (sizeof(T) < 4)
-    k_chan_mean_var_ex<T><<<(unsigned)nch, 32 * ES_G, 0, st>>>(s, ns, o.ld, tot, w.means.as<float>(),
-                                                       w.vars.as<float>());
-  else
-    k_chan_mean_var_pc<T><<<(unsigned)nch, PC_NT, 0, st>>>(s, ns, o.ld, tot,
-                                                          w.means.as<float>(),
-                                                          w.vars.as<float>());
+  PSR_TRY(enqueue_mean_var<T>(s, nch, ns, o.ld, w, st));
   k_block_sums<T><<<(unsigned)((nch * blocks_n + 127) / 128), 128, 0, st>>>(
       s, ns, o.ld, nch, bs, blocks_n, w.bsum.as<float>());
   if constexpr (sizeof(T) == 1) {
@@ -767,9 +909,10 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   unsigned char *fl = w.flags.as<unsigned char>();
   k_channel_decide<<<1, 1024, 0, st>>>(w.means.as<float>(), w.vars.as<float>(), nch, thr,
                                        w.scratch.as<float>(), fl, fl + nch,
-                                       w.chbad.as<unsigned char>(), tot + nch);
+                                       w.chbad.as<unsigned char>(), w.active.as<unsigned long long>());
   k_block_means<<<(unsigned)((blocks_n + 127) / 128), 128, 0, st>>>(
-      w.bsum.as<float>(), w.chbad.as<unsigned char>(), nch, ns, bs, blocks_n, tot + nch,
+      w.bsum.as<float>(), w.chbad.as<unsigned char>(), nch, ns, bs, blocks_n,
+      w.active.as<unsigned long long>(),
       w.bmeans.as<float>());
   k_block_decide<<<1, 1024, 0, st>>>(w.bmeans.as<float>(), blocks_n, thr,
                                      w.scratch.as<float>(), w.blkbad.as<unsigned char>());
@@ -780,35 +923,14 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   return PSR_OK;
 }
 
-template <class T>
-static int channel_stats_t(const DeviceObs &o, RfiWork &w, cudaStream_t st) {
-  const uint64_t nch = o.nch, ns = o.ns;
-  PSR_TRY(w.means.ensure(nch * 4));
-  PSR_TRY(w.vars.ensure(nch * 4));
-  PSR_TRY(w.hist.ensure(nch * 8 + 8));
-  const T *s = o.samples.as<T>();
-  unsigned long long *tot = w.hist.as<unsigned long long>();
-  PSR_CUDA(cudaMemsetAsync(tot, 0, nch * 8 + 8, st));
-  if constexpr (sizeof(T) < 4) {
-    dim3 g((unsigned)std::min<uint64_t>((ns + 255) / 256, 64), (unsigned)nch);
-    k_chan_total<T><<<g, 256, 0, st>>>(s, ns, o.ld, tot);
-    k_chan_mean_var_ex<T><<<(unsigned)nch, 32 * ES_G, 0, st>>>(s, ns, o.ld, tot, w.means.as<float>(),
-                                                       w.vars.as<float>());
-  } else {
-    k_chan_mean_var_pc<T><<<(unsigned)nch, PC_NT, 0, st>>>(s, ns, o.ld, tot,
-                                                          w.means.as<float>(),
-                                                          w.vars.as<float>());
-  }
-  PSR_CUDA(cudaGetLastError());
-  return PSR_OK;
-}
-
 int rfi_channel_stats(const DeviceObs &o, float *means, float *variances, cudaStream_t st) {
   RfiWork w;
+  PSR_TRY(w.means.ensure(o.nch * 4));
+  PSR_TRY(w.vars.ensure(o.nch * 4));
   switch (o.kind) {
-    case SAMPLE_U8: PSR_TRY(channel_stats_t<uint8_t>(o, w, st)); break;
-    case SAMPLE_U16: PSR_TRY(channel_stats_t<uint16_t>(o, w, st)); break;
-    default: PSR_TRY(channel_stats_t<float>(o, w, st));
+    case SAMPLE_U8: PSR_TRY(enqueue_mean_var(o.samples.as<uint8_t>(), o.nch, o.ns, o.ld, w, st)); break;
+    case SAMPLE_U16: PSR_TRY(enqueue_mean_var(o.samples.as<uint16_t>(), o.nch, o.ns, o.ld, w, st)); break;
+    default: PSR_TRY(enqueue_mean_var(o.samples.as<float>(), o.nch, o.ns, o.ld, w, st));
   }
   PSR_CUDA(cudaMemcpyAsync(means, w.means.p, o.nch * 4, cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaMemcpyAsync(variances, w.vars.p, o.nch * 4, cudaMemcpyDeviceToHost, st));
