@@ -15,12 +15,21 @@
 //   Sub-FFT of size L: Stockham autosort stages with radices
 //   [16]*(q/4) + [2|4|8]; DFT_8 = 2x4 and DFT_16 = 4x4 four-step with the
 //   internal twiddles W_R^(n2*k1).
-// A CTA transforms C columns held in shared memory position-major with one
-// padding slot every 16 (free of bank conflicts for the row-wise global
-// loads, every Stockham access and the drains).  Every size is a template parameter, so all index
-// arithmetic reduces to shifts and masks; each thread owns exactly one
-// radix-16 butterfly per stage.  Stages are in place: every thread loads its
-// inputs, the block synchronises, then stores.
+// A CTA transforms C columns (pass 1) or rows (pass 2) held in shared memory
+// with one padding slot every 16 positions: position-major for columns,
+// row-major for rows, each free of bank conflicts for its stages.  Every size
+// is a template parameter, so all index arithmetic reduces to shifts and
+// masks; each thread owns exactly one radix-16 butterfly per stage.  Stages
+// are in place: every thread loads its inputs, the block synchronises, then
+// stores.  The first stage's inputs come straight from where they lie (the
+// staged series, the work buffer) and the last stage's outputs leave from
+// registers (times the pass-1 twiddle to the work buffer; through the real
+// post-processing to the spectrum), so a sub-FFT of three stages makes two
+// round trips through shared memory.
+// Bound: instruction issue (about 2.5 M warp instructions per 2^20-point
+// trial) at half occupancy (64 registers, 2 CTAs of 512 threads per SM).
+// Measured on a GB300, 2^20 points, 700 trials: pass 1 1.68 -> 1.55 ms, pass 2
+// 1.67 -> 1.34 ms against stages that all went through shared memory.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -33,8 +42,6 @@
 
 namespace psr {
 namespace {
-
-constexpr int LB = 8;  // global loads in flight per thread when staging a tile
 
 __host__ __device__ constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x >> 1); }
 __host__ __device__ constexpr int cols_for(int L) {
@@ -70,17 +77,6 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 w) {
 __device__ __forceinline__ float2 mul_mi(float2 d) { return make_float2(d.y, -d.x); }
 
 // W_N^x for x in [0, N) from the quarter table (lq = log2(N/4)).
-// 8-byte asynchronous global -> shared copy (no registers held while in flight).
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
 __device__ __forceinline__ float2 twN(const float2 *__restrict__ Q, uint32_t x, int lq) {
   const uint32_t q = x >> lq, r = x & ((1u << lq) - 1u);
   const float2 v = __ldg(&Q[r]);
@@ -164,17 +160,8 @@ __device__ __forceinline__ void dft8(float2 *v, const W16 &c) {
     v[k1 + 6] = d;
   }
 }
-__device__ __forceinline__ void dft16(float2 *v, const W16 &c) {
-  float2 u[4][4];
-#pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) {
-    float2 a = v[n2], b = v[n2 + 4], c = v[n2 + 8], d = v[n2 + 12];
-    dft4(a, b, c, d);
-    u[n2][0] = a;
-    u[n2][1] = b;
-    u[n2][2] = c;
-    u[n2][3] = d;
-  }
+// The internal twiddles and second level of dft16.
+__device__ __forceinline__ void dft16_second(float2 (&u)[4][4], float2 *v, const W16 &c) {
   u[1][1] = cmul(u[1][1], c.get<1>());
   u[1][2] = cmul(u[1][2], c.get<2>());
   u[1][3] = cmul(u[1][3], c.get<3>());
@@ -193,6 +180,35 @@ __device__ __forceinline__ void dft16(float2 *v, const W16 &c) {
     v[k1 + 8] = c;
     v[k1 + 12] = d;
   }
+}
+__device__ __forceinline__ void dft16(float2 *v, const W16 &c) {
+  float2 u[4][4];
+#pragma unroll
+  for (int n2 = 0; n2 < 4; ++n2) {
+    float2 a = v[n2], b = v[n2 + 4], c = v[n2 + 8], d = v[n2 + 12];
+    dft4(a, b, c, d);
+    u[n2][0] = a;
+    u[n2][1] = b;
+    u[n2][2] = c;
+    u[n2][3] = d;
+  }
+  dft16_second(u, v, c);
+}
+
+// dft16 of inputs whose second half (v[8..15]) is zero: the first level's sums
+// with zero are skipped (the same values up to the sign of zero, which cannot
+// change |X|^2).
+__device__ __forceinline__ void dft16_half(float2 *v, const W16 &c) {
+  float2 u[4][4];
+#pragma unroll
+  for (int n2 = 0; n2 < 4; ++n2) {
+    const float2 a = v[n2], b = v[n2 + 4], d = mul_mi(b);
+    u[n2][0] = cadd(a, b);
+    u[n2][1] = cadd(a, d);
+    u[n2][2] = csub(a, b);
+    u[n2][3] = csub(a, d);
+  }
+  dft16_second(u, v, c);
 }
 
 template <int R>
@@ -269,16 +285,48 @@ __device__ __forceinline__ void stages16(float2 *sm, const float2 *Wl, const W16
   }
 }
 
-// The stages after the first radix-16 stage (used when stage 0 runs fused
-// with the global loads).
-template <int L, int C, int NT>
-__device__ __forceinline__ void subfft_rest(float2 *sm, const float2 *Wl, const W16 &c) {
-  constexpr int q = ilog2(L);
-  constexpr int NsLast = 1 << (4 * (q / 4));
-  stages16<L, C, NT, 1>(sm, Wl, c);
-  if constexpr (q % 4 == 1) stage<2, L, C, NT, NsLast>(sm, Wl, c);
-  else if constexpr (q % 4 == 2) stage<4, L, C, NT, NsLast>(sm, Wl, c);
-  else if constexpr (q % 4 == 3) stage<8, L, C, NT, NsLast>(sm, Wl, c);
+// Radix and stride (product of the earlier radices) of a sub-FFT's last stage.
+__host__ __device__ constexpr int last_radix(int L) {
+  return ilog2(L) % 4 == 0 ? 16 : 1 << (ilog2(L) % 4);
+}
+
+// The radix-16 stages s, s + 1, .. before the last stage.
+template <int L, int C, int NT, int s>
+__device__ __forceinline__ void stages_mid(float2 *sm, const float2 *Wl, const W16 &c) {
+  if constexpr ((1 << (4 * s)) * last_radix(L) < L) {
+    stage<16, L, C, NT, (1 << (4 * s))>(sm, Wl, c);
+    stages_mid<L, C, NT, s + 1>(sm, Wl, c);
+  }
+}
+
+// The last stage, its outputs handed to emit(j, col, v) instead of stored:
+// butterfly (col, j) leaves v[r] at position j + r L / R.
+template <int L, int C, int NT, class Emit>
+__device__ __forceinline__ void last_stage(const float2 *sm, const float2 *Wl, const W16 &c16,
+                                           Emit emit) {
+  constexpr int R = last_radix(L), nb = L / R, total = nb * C, BPT = (total + NT - 1) / NT;
+#pragma unroll
+  for (int i = 0; i < BPT; ++i) {
+    const int w = (int)threadIdx.x + i * NT;
+    if (total % NT == 0 || w < total) {
+      const int col = w % C, j = w / C;
+      float2 v[R];
+      if constexpr ((nb * C) % 16 == 0) {
+        const float2 *src = sm + lay<C>(j, col);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = src[r * lay_step<C, nb>()];
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = sm[lay<C>(j + r * nb, col)];
+      }
+      if (j != 0) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = cmul(v[r], Wl[r * j]);
+      }
+      dftR<R>(v, c16);
+      emit(j, col, v);
+    }
+  }
 }
 
 template <int L, int C, int NT>
@@ -352,25 +400,32 @@ struct Acc2 {
   }
 };
 
-// Block total of the per-thread (hi, lo) pairs: TwoSum merges across the
-// warp in f32, f64 only for the final per-warp pairs (thread 0).
+// Block total of the per-thread (hi, lo) pairs: TwoSum merges in f32 across
+// the warp, then across the warps; f64 only for the last pair (FP64 runs at
+// 1/64 of the f32 rate: 16 warps' pairs added in f64 by one thread held every
+// CTA of pass 2 for about 1500 cycles).
 template <int NT>
 __device__ __forceinline__ void block_sum_store(Acc2 acc, double *dst) {
-  __shared__ float2 red[NT / 32 > 0 ? NT / 32 : 1];
+  constexpr int NW = NT / 32 > 0 ? NT / 32 : 1;
+  __shared__ float2 red[NW];
+  auto merge = [&](int from) {
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
-    const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
-    acc.add(oh);
-    acc.lo = __fadd_rn(acc.lo, ol);
-  }
+    for (int o = from; o; o >>= 1) {
+      const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
+      const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
+      acc.add(oh);
+      acc.lo = __fadd_rn(acc.lo, ol);
+    }
+  };
+  merge(16);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(acc.hi, acc.lo);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) t += (double)red[w].x + (double)red[w].y;
-    *dst = t;
+  if (threadIdx.x < 32) {
+    const int w = (int)threadIdx.x;
+    acc.hi = w < NW ? red[w].x : 0.0f;
+    acc.lo = w < NW ? red[w].y : 0.0f;
+    merge(NW / 2 > 0 ? NW / 2 : 0);
+    if (w == 0) *dst = (double)acc.hi + (double)acc.lo;
   }
 }
 
@@ -451,7 +506,6 @@ __device__ __forceinline__ void p1_group(float2 *sm, const float2 *Wl, const W16
                                          float2 *__restrict__ out, const float2 *stg,
                                          Hook after_stage0) {
   constexpr int C = cols_for(M1), NT = threads_for(M1, C);
-  constexpr int total = M1 * C;
   const uint64_t nz = (len + 1) / 2;  // complex inputs that can be non-zero
   {
     // Stage 0 (radix 16, Ns = 1) straight from global memory (or the staged
@@ -466,22 +520,23 @@ __device__ __forceinline__ void p1_group(float2 *sm, const float2 *Wl, const W16
       const int w = (int)threadIdx.x + i * NT;
       if (nbt % NT == 0 || w < nbt) {
         const int col = w % C, j = w / C;
+        // (at most half the inputs can be non-zero: r < 8)
         float2 v[16];
         if (stg) {
 #pragma unroll
-          for (int r = 0; r < 16; ++r) {
+          for (int r = 0; r < 8; ++r) {
             const uint64_t n = (uint64_t)(j + r * nb) * M2 + n2_0 + col;
             v[r] = n < nz ? staged_z(stg[(j + r * nb) * C + col], len, n, mean)
                           : make_float2(0.0f, 0.0f);
           }
         } else {
 #pragma unroll
-          for (int r = 0; r < 16; ++r) {
+          for (int r = 0; r < 8; ++r) {
             const uint64_t n = (uint64_t)(j + r * nb) * M2 + n2_0 + col;
             v[r] = n < nz ? load_z(row, len, n, mean) : make_float2(0.0f, 0.0f);
           }
         }
-        dft16(v, c16);
+        dft16_half(v, c16);
         if constexpr (16 % C == 0) {
           // e = (16j + r) C + col with col < C | 16: the padding of r C +
           // col is (r C) / 16, so every r is a constant offset
@@ -497,59 +552,22 @@ __device__ __forceinline__ void p1_group(float2 *sm, const float2 *Wl, const W16
   }
   __syncthreads();
   after_stage0();
-  subfft_rest<M1, C, NT>(sm, Wl, c16);
+  stages_mid<M1, C, NT, 1>(sm, Wl, c16);
   // W_M^(n2*k1) comes from a table laid out like the output, Tw1[k1*M2 +
   // n2] (values identical to the quarter-table lookup): reads coalesce.
-  if constexpr (NT % C == 0 && 16 % C == 0) {
-    // thread t drains column t % C at rows k1 = t / C + i NT / C: slot
-    // lay<C>(k1, col) = C k1 + col + (C k1) / 16 advances by a constant
-    constexpr int KS = NT / C;  // row step
-    const int col = (int)threadIdx.x % C, k10 = (int)threadIdx.x / C;
+  last_stage<M1, C, NT>(sm, Wl, c16, [&](int j, int col, float2 *v) {
+    constexpr int R = last_radix(M1), nb = M1 / R;
     const uint32_t n2 = n2_0 + (uint32_t)col;
-    const float2 *src = sm + C * k10 + col + (C * k10) / 16;
-    const float2 *tws = tw1 + (uint64_t)k10 * M2 + n2;
-    float2 *dst = out + (uint64_t)k10 * M2 + n2;
-    constexpr int NI = M1 / KS;
-#pragma unroll 1
-    for (int i0 = 0; i0 < NI; i0 += LB) {
-      float2 w[LB];
+    const uint64_t at = (uint64_t)j * M2 + n2;
+    float2 w[R];
 #pragma unroll
-      for (int u = 0; u < LB; ++u)
-        w[u] = i0 + u < NI ? __ldg(tws + (uint64_t)(i0 + u) * KS * M2)
-                           : make_float2(1.0f, 0.0f);
+    for (int r = 0; r < R; ++r) w[r] = __ldg(tw1 + at + (uint64_t)r * nb * M2);
 #pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        if (i0 + u < NI) {
-          const int k1 = k10 + (i0 + u) * KS;
-          float2 v = src[(i0 + u) * lay_step<C, KS>()];
-          if (n2 * (uint32_t)k1 != 0) v = cmul(v, w[u]);
-          dst[(uint64_t)(i0 + u) * KS * M2] = v;
-        }
-      }
+    for (int r = 0; r < R; ++r) {
+      if (n2 * (uint32_t)(j + r * nb) != 0) v[r] = cmul(v[r], w[r]);
+      out[at + (uint64_t)r * nb * M2] = v[r];
     }
-  } else {
-#pragma unroll 1
-    for (int base = 0; base < total; base += LB * NT) {
-      float2 w[LB];
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int idx = base + u * NT + (int)threadIdx.x;
-        w[u] = idx < total ? __ldg(&tw1[(uint64_t)(idx / C) * M2 + n2_0 + (idx % C)])
-                           : make_float2(1.0f, 0.0f);
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int idx = base + u * NT + (int)threadIdx.x;
-        if (idx < total) {
-          const int col = idx % C, k1 = idx / C;
-          const uint32_t n2 = n2_0 + (uint32_t)col;
-          float2 v = sm[lay<C>(k1, col)];
-          if (n2 * (uint32_t)k1 != 0) v = cmul(v, w[u]);
-          out[(uint64_t)k1 * M2 + n2] = v;
-        }
-      }
-    }
-  }
+  });
 }
 
 // Pass 1: column groups of every trial, persistent: CTA b takes groups b,
@@ -613,18 +631,83 @@ __global__ void __launch_bounds__(threads_for(M1, cols_for(M1)), 2)
   }
 }
 
+// Pass 2's shared-memory layout: row ci starts at ci * p2_pitch, position pos
+// at pos + pos / 16 of it.  Warps run along a row in the radix-16 stages
+// (conflict-free by the padding); in the last stage a half-warp reads H rows
+// x 16 / H positions, which the pitch (16 / H modulo 16) keeps in 16 different
+// bank pairs.
+template <int L>
+__host__ __device__ constexpr int p2_pitch() {
+  constexpr int H = cols_for(L) / 2, base = L + L / 16;
+  return base + (16 / H + 16 - base % 16) % 16;
+}
+__device__ __forceinline__ int p2_slot(int pos) { return pos + (pos >> 4); }
+
+// One in-place stage on C rows; W1 is the second stage's twiddle table
+// [r][k] = W_L^(r k L / 256) (its lanes' 16 values of k are contiguous).
+template <int R, int L, int C, int NT, int Ns>
+__device__ __forceinline__ void stage_rows(float2 *sm, const float2 *Wl, const float2 *W1,
+                                           const W16 &c16) {
+  constexpr int nb = L / R, total = nb * C, BPT = (total + NT - 1) / NT, P = p2_pitch<L>();
+  float2 v[BPT][R];
+#pragma unroll
+  for (int i = 0; i < BPT; ++i) {
+    const int w = (int)threadIdx.x + i * NT, row = w / nb, j = w % nb;
+    if (total % NT == 0 || w < total) {
+      const float2 *src = sm + row * P;
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[i][r] = src[p2_slot(j + r * nb)];
+      const int k = j % Ns;
+      if (k != 0) {
+#pragma unroll
+        for (int r = 1; r < R; ++r)
+          v[i][r] = cmul(v[i][r], R == 16 && Ns == 16 ? W1[r * 16 + k]
+                                                      : Wl[r * k * (L / (Ns * R))]);
+      }
+      dftR<R>(v[i], c16);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < BPT; ++i) {
+    const int w = (int)threadIdx.x + i * NT, row = w / nb, j = w % nb;
+    if (total % NT == 0 || w < total) {
+      float2 *dst = sm + row * P;
+      const int base = (j / Ns) * Ns * R + j % Ns;
+#pragma unroll
+      for (int r = 0; r < R; ++r) dst[p2_slot(base + r * Ns)] = v[i][r];
+    }
+  }
+  __syncthreads();
+}
+template <int L, int C, int NT, int s>
+__device__ __forceinline__ void stages_rows_mid(float2 *sm, const float2 *Wl, const float2 *W1,
+                                                const W16 &c) {
+  if constexpr ((1 << (4 * s)) * last_radix(L) < L) {
+    stage_rows<16, L, C, NT, (1 << (4 * s))>(sm, Wl, W1, c);
+    stages_rows_mid<L, C, NT, s + 1>(sm, Wl, W1, c);
+  }
+}
+
 // Pass 2 on one row group of one trial: the row sub-FFTs of length M2, then
 // the real post-processing and |X|^2.  Group 0 holds rows 0 and M1/2; group
 // g >= 1 holds rows kb..kb+h-1 (kb = 1 + (g-1)*H) and M1-kb..M1-kb-h+1.
-// Unused columns of the last group are transformed but never read.
-// The row twiddle table Wl is built while the rows are in flight.
+// Unused rows of the last group are zero and never written out.
+// The first stage takes its inputs from the work buffer (16 loads in flight
+// per thread while the CTA builds its twiddle tables).  Bin k2 of row k pairs
+// with bin M2 - 1 - k2 of row M1 - k, and the last stage's butterfly j leaves
+// bins j + r M2 / R: butterfly j of a row and butterfly M2 / R - 1 - j of its
+// mirror hold R whole pairs, so one thread takes both and post-processes them
+// in registers.  (Where the last radix is 16 the two would not fit: the stage
+// goes through shared memory, as group 0's, whose rows pair differently.)
 template <int M1, int M2>
-__device__ __forceinline__ void p2_group(float2 *sm, float2 *Wl, uint32_t N,
+__device__ __forceinline__ void p2_group(float2 *sm, float2 *Wl, float2 *W1, uint32_t N,
                                          const float2 *__restrict__ in, uint32_t g,
                                          const float2 *__restrict__ Q, int lq,
                                          float *__restrict__ out, double *__restrict__ psum_out) {
-  constexpr int C = cols_for(M2), NT = threads_for(M2, C), H = C / 2;
+  constexpr int C = cols_for(M2), NT = threads_for(M2, C), H = C / 2, P = p2_pitch<M2>();
   constexpr uint32_t M = (uint32_t)M1 * M2;
+  constexpr int nb0 = M2 / 16, R = last_radix(M2), nbl = M2 / R;
   int h;
   uint32_t kb = 0;
   if (g == 0) {
@@ -633,121 +716,122 @@ __device__ __forceinline__ void p2_group(float2 *sm, float2 *Wl, uint32_t N,
     kb = 1 + (g - 1) * (uint32_t)H;
     h = (int)min((uint32_t)H, (uint32_t)(M1 / 2 - kb));
   }
-  const int ncols = 2 * h;
-  const int total = M2 * ncols;
   auto row_of = [&](int ci) -> uint32_t {
     if (g == 0) return ci == 0 ? 0u : (uint32_t)(M1 / 2);
-    return ci < h ? kb + (uint32_t)ci : (uint32_t)M1 - (kb + (uint32_t)(ci - h));
+    return ci < H ? kb + (uint32_t)ci : (uint32_t)M1 - (kb + (uint32_t)(ci - H));
   };
-  if constexpr (C == 16 && NT == M2) {
-    // thread t copies position t of every row to slot lay<16>(t, ci) = 17 t + ci
-    const float2 *src = in + threadIdx.x;
-    float2 *dst = sm + 17 * threadIdx.x;
+  {
+    static_assert(nb0 * C == NT, "one first-stage butterfly per thread");
+    const int ci = (int)threadIdx.x / nb0, j = (int)threadIdx.x % nb0;
+    float2 v[16];
+    if (g == 0 ? ci < 2 : ci % H < h) {
+      const float2 *src = in + (uint64_t)row_of(ci) * M2 + j;
 #pragma unroll
-    for (int ci = 0; ci < C; ++ci)
-      if (ci < ncols) cp_async8(dst + ci, src + (uint64_t)row_of(ci) * M2);
-    build_wl<M2>(Wl, N, Q, lq);
-    cp_async_wait_all();
-  } else {
-    build_wl<M2>(Wl, N, Q, lq);
-#pragma unroll 1
-    for (int base = 0; base < total; base += LB * NT) {
-      float2 v[LB];
+      for (int r = 0; r < 16; ++r) v[r] = src[r * nb0];
+    } else {
 #pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int idx = base + u * NT + (int)threadIdx.x;
-        v[u] = idx < total ? in[(uint64_t)row_of(idx / M2) * M2 + idx % M2]
-                           : make_float2(0.0f, 0.0f);
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int idx = base + u * NT + (int)threadIdx.x;
-        if (idx < total) sm[lay<C>(idx % M2, idx / M2)] = v[u];
-      }
+      for (int r = 0; r < 16; ++r) v[r] = make_float2(0.0f, 0.0f);
     }
+    build_wl<M2>(Wl, N, Q, lq);
+    if constexpr (M2 >= 256)
+      for (int t = threadIdx.x; t < 256; t += NT)
+        W1[t] = twN(Q, (uint32_t)((t >> 4) * (t & 15)) * (N / 256), lq);
+    __syncthreads();
+    const W16 c16 = load_w16<M2>(Wl);
+    dft16(v, c16);
+    float2 *dst = sm + ci * P + 17 * j;  // p2_slot(16 j + r) = 17 j + r
+#pragma unroll
+    for (int r = 0; r < 16; ++r) dst[r] = v[r];
   }
   __syncthreads();
   const W16 c16 = load_w16<M2>(Wl);
-  subfft<M2, C, NT>(sm, Wl, c16);
+  stages_rows_mid<M2, C, NT, 1>(sm, Wl, W1, c16);
   Acc2 acc;
-  if (g == 0) {
-    for (uint32_t idx = threadIdx.x; idx < 2 * M2; idx += NT) {
-      const uint32_t k2 = idx % M2, which = idx / M2;
-      uint32_t k, mk2;
-      if (which == 0) {
-        k = M1 * k2;
-        mk2 = (M2 - k2) % M2;
-      } else {
-        k = M1 / 2 + M1 * k2;
-        mk2 = M2 - 1 - k2;
+  if (g != 0 && R < 16) {
+    // Full twiddle of bin k = kb + p + M1 k2: k2 < M2 / 2 (r < R / 2) lies in
+    // the first quarter of the quarter-table's cycle, the rest in the second
+    // (the quadrant rule of twN, fixed per r).  W_N^(M-k) = (-W_N^k.re,
+    // W_N^k.im) holds bit for bit for the lookup (its mirrored half is the
+    // swapped first half), up to the sign of zero components, which cannot
+    // change |X|^2.
+    constexpr int PPT = (H * nbl + NT - 1) / NT;
+    static_assert(R == 16 || (H * nbl) % NT == 0, "whole pairs per thread");
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int idx = (int)threadIdx.x + i * NT, p = idx % H, j = idx / H, jm = nbl - 1 - j;
+      const uint32_t k0 = kb + (uint32_t)p + (uint32_t)M1 * (uint32_t)j;
+      float2 wk[R], a[R], b[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float2 q = __ldg(&Q[k0 + (uint32_t)M1 * (uint32_t)nbl * (r < R / 2 ? r : r - R / 2)]);
+        wk[r] = r < R / 2 ? make_float2(q.x, -q.y) : make_float2(-q.y, -q.x);
       }
-      const float p = post_power(sm[lay<C>(k2, which)], sm[lay<C>(mk2, which)], twN(Q, k, lq));
-      out[k] = p;
-      acc.add(p);
-    }
-    if (threadIdx.x == 0) {  // k = M (Nyquist): a = Z[0], b = conj(Z[0])
-      const float p = post_power(sm[lay<C>(0, 0)], sm[lay<C>(0, 0)], twN(Q, M, lq));
-      out[M] = p;
-      acc.add(p);
+      const float2 *sa = sm + p * P + p2_slot(j), *sb = sm + (H + p) * P + p2_slot(jm);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        a[r] = sa[r * (nbl + nbl / 16)];
+        b[r] = sb[r * (nbl + nbl / 16)];
+      }
+      if (j != 0) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) a[r] = cmul(a[r], Wl[r * j]);
+      }
+      if (jm != 0) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) b[r] = cmul(b[r], Wl[r * jm]);
+      }
+      dftR<R>(a, c16);
+      dftR<R>(b, c16);
+      if (p < h) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t k = k0 + (uint32_t)M1 * (uint32_t)(r * nbl);
+          float pk, pm;
+          post_power_pair(a[r], b[R - 1 - r], wk[r], pk, pm);
+          out[k] = pk;
+          out[M - k] = pm;
+          acc.add(pk);
+          acc.add(pm);
+        }
+      }
     }
   } else {
-    // Bins k = kb + p + M1 k2 and M - k.  W_N^(M-k) = (-W_N^k.re, W_N^k.im)
-    // holds bit for bit for the quarter-table lookup (its mirrored half is
-    // the swapped first half), up to the sign of zero components, which
-    // cannot change |X|^2.  Full groups (h == H) divide by a constant.
-    auto rows = [&](auto hc) {
-      constexpr int HC = decltype(hc)::value;
-      const int hh = HC > 0 ? HC : h;
-      constexpr int PB = LB;
-      const int tot2 = M2 * hh;
-#pragma unroll 1
-      for (int base = 0; base < tot2; base += PB * NT) {
-        float2 wk[PB];
-        uint32_t kk[PB];
-        int pp[PB], k2s[PB];
-        // Full groups: k2 = t / HC + u NT / HC with t / HC < NT / HC and
-        // 4 NT / HC = M2 / 2, so bin k = kb + p + M1 k2 (kb + p < M1 / 2) lies in
-        // the first quarter of the quarter-table's cycle for u < 4 and in the
-        // second for u >= 4: the quadrant rule of twN, fixed per u.
-        constexpr bool QFIX = HC > 0 && PB == 8 && 4 * (NT / (HC > 0 ? HC : 1)) == M2 / 2 &&
-                              (HC > 0 ? NT % HC == 0 : false) && M2 * HC == PB * NT;
-#pragma unroll
-        for (int u = 0; u < PB; ++u) {
-          const int idx = base + u * NT + (int)threadIdx.x;
-          pp[u] = HC > 0 ? idx % HC : idx % hh;
-          k2s[u] = HC > 0 ? idx / HC : idx / hh;
-          kk[u] = kb + (uint32_t)pp[u] + M1 * (uint32_t)k2s[u];
-          if constexpr (QFIX) {
-            if (u < 4) {
-              const float2 v = __ldg(&Q[kk[u]]);
-              wk[u] = make_float2(v.x, -v.y);
-            } else {
-              const float2 v = __ldg(&Q[kk[u] - (1u << lq)]);
-              wk[u] = make_float2(-v.y, -v.x);
-            }
-          } else {
-            wk[u] = idx < tot2 ? twN(Q, kk[u], lq) : make_float2(1.0f, 0.0f);
-          }
+    stage_rows<R, M2, C, NT, nbl>(sm, Wl, W1, c16);
+    if (g == 0) {
+      for (uint32_t idx = threadIdx.x; idx < 2 * M2; idx += NT) {
+        const uint32_t k2 = idx % M2, which = idx / M2;
+        uint32_t k, mk2;
+        if (which == 0) {
+          k = M1 * k2;
+          mk2 = (M2 - k2) % M2;
+        } else {
+          k = M1 / 2 + M1 * k2;
+          mk2 = M2 - 1 - k2;
         }
-#pragma unroll
-        for (int u = 0; u < PB; ++u) {
-          const int idx = base + u * NT + (int)threadIdx.x;
-          if (idx < tot2) {
-            const uint32_t k = kk[u];
-            const float2 zk = sm[lay<C>(k2s[u], pp[u])];
-            const float2 zm = sm[lay<C>(M2 - 1 - k2s[u], hh + pp[u])];
-            float pk, pm;
-            post_power_pair(zk, zm, wk[u], pk, pm);
-            out[k] = pk;
-            out[M - k] = pm;
-            acc.add(pk);
-            acc.add(pm);
-          }
-        }
+        const float2 *row = sm + which * P;
+        const float p = post_power(row[p2_slot((int)k2)], row[p2_slot((int)mk2)], twN(Q, k, lq));
+        out[k] = p;
+        acc.add(p);
       }
-    };
-    if (h == H) rows(std::integral_constant<int, H>{});
-    else rows(std::integral_constant<int, 0>{});
+      if (threadIdx.x == 0) {  // k = M (Nyquist): a = Z[0], b = conj(Z[0])
+        const float p = post_power(sm[0], sm[0], twN(Q, M, lq));
+        out[M] = p;
+        acc.add(p);
+      }
+    } else {
+      for (int idx = (int)threadIdx.x; idx < H * M2; idx += NT) {
+        const int p = idx % H, k2 = idx / H;
+        if (p >= h) continue;
+        const uint32_t k = kb + (uint32_t)p + (uint32_t)M1 * (uint32_t)k2;
+        float pk, pm;
+        post_power_pair(sm[p * P + p2_slot(k2)], sm[(H + p) * P + p2_slot(M2 - 1 - k2)],
+                        twN(Q, k, lq), pk, pm);
+        out[k] = pk;
+        out[M - k] = pm;
+        acc.add(pk);
+        acc.add(pm);
+      }
+    }
   }
   block_sum_store<NT>(acc, psum_out);
 }
@@ -762,7 +846,8 @@ __global__ void __launch_bounds__(threads_for(M2, cols_for(M2)), 2)
   constexpr uint32_t M = (uint32_t)M1 * M2;
   extern __shared__ float2 dyn[];
   float2 *Wl = dyn;       // M2 entries
-  float2 *sm = dyn + M2;  // lay_slots<M2, C>() entries
+  float2 *W1 = Wl + M2;   // 256 entries
+  float2 *sm = W1 + 256;  // C rows of p2_pitch
   const uint64_t trial = blockIdx.y;
   const uint32_t g = blockIdx.x;
   {
@@ -785,7 +870,7 @@ __global__ void __launch_bounds__(threads_for(M2, cols_for(M2)), 2)
       }
     }
   }
-  p2_group<M1, M2>(sm, Wl, N, work + trial * (uint64_t)M, g, Q, lq, power + trial * ldp,
+  p2_group<M1, M2>(sm, Wl, W1, N, work + trial * (uint64_t)M, g, Q, lq, power + trial * ldp,
                    psum + trial * ngroups + g);
 }
 
@@ -861,7 +946,7 @@ int run_four_step(const FftArgs &a) {
   }
   {
     constexpr int C = cols_for(M2);
-    const size_t smem = (size_t)(M2 + lay_slots<M2, C>()) * sizeof(float2);
+    const size_t smem = (size_t)(M2 + 256 + C * p2_pitch<M2>()) * sizeof(float2);
     PSR_CUDA(cudaFuncSetAttribute(k_fft_pass2<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
     const uint32_t ng = 1 + ((uint32_t)M1 / 2 - 1 + C / 2 - 1) / (C / 2);
