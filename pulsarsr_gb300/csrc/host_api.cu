@@ -1611,9 +1611,10 @@ int psr_batch_sync(psr_batch *b) {
     // A raw-candidate overflow makes finish() regrow that session's buffers
     // and redo the chunk; the captured graph would then hold stale pointers,
     // so it is captured again on the next run.
-    const void *raw = s->eng.sw.raw.p, *gq = s->eng.sw.gq.p;
+    const SpecWork &w = s->eng.sw;
+    const void *raw = w.raw.p, *gq = w.gq.p, *xq = w.xq.p;
     PSR_TRY(psr_session_sync(s.get()));
-    regrown = regrown || s->eng.sw.raw.p != raw || s->eng.sw.gq.p != gq;
+    regrown = regrown || w.raw.p != raw || w.gq.p != gq || w.xq.p != xq;
   }
   if (regrown) b->drop_graph();
   return PSR_OK;

@@ -46,9 +46,11 @@ __device__ __forceinline__ int count_le64(const uint32_t *a, uint32_t key) {
   return pos;
 }
 
-// Chunks are stored with a 65-word stride so that threads probing the same
-// index of different chunks hit different banks.
+// Sorted chunks are stored with a 65-word stride so that threads probing the
+// same index of different chunks hit different banks; unsorted ones with a
+// 68-word stride, for 16-byte accesses (8 lanes' quads fill the 32 banks).
 constexpr int SC_STRIDE = 65;
+constexpr int SC_RAW = 68;
 
 struct RawCand {
   double score;
@@ -68,6 +70,7 @@ struct HarmArgs {
   double bin_hz;
   double threshold;
   float t1;  // smallest float v with (double)v - 1.0 >= threshold
+  float lim[6];  // harm_maybe: h + threshold sqrt(h), lowered (-inf: always exact)
   uint64_t first;
   uint64_t end[6];  // end_h for h = 1,2,4,8,16,32 (0 when the h loop is skipped)
   RawCand *raw;
@@ -111,62 +114,6 @@ __device__ __forceinline__ double inv_sqrt_div(double x, int hi) {
   }
 }
 
-// Whether (sum - h) / sqrt(h) can reach thr, without the f64 division where
-// it clearly cannot: x * RN(1/sqrt(h)) is within 2^-50 (relative) of the
-// correctly rounded quotient, so below thr by more than |thr| 2^-49 it is
-// below for certain.  Levels with h = 1, 4, 16 scale exactly: always true.
-__device__ __forceinline__ bool may_reach(double x, int hi, double thr) {
-  if ((hi & 1) == 0) return true;
-  constexpr double r1 = 0.7071067811865476;  // RN(1/sqrt(2)); / 2 and / 4 are exact
-  const double r = hi == 1 ? r1 : hi == 3 ? r1 * 0.5 : r1 * 0.25;
-  return __dmul_rn(x, r) >= thr - fabs(thr) * 0x1p-49;
-}
-
-// Full score of harmonic level hi (h = 1 << hi) at bin k (k in [first, end]).
-__device__ double score_at(const HarmArgs &a, const float *raw, const float *sc, uint64_t k,
-                           int hi) {
-  const int h = 1 << hi;
-  if (h > 1 && pw(a, raw, sc, k) < 4.0f) return -INFINITY;
-  const double off = offset_at(raw, k);
-  const double kf = __dadd_rn((double)k, off);
-  double sum = -0.0;
-  for (int j = 1; j <= h; ++j) {
-    const double pos = __dmul_rn(kf, (double)j);
-    uint64_t idx = (uint64_t)round(pos);
-    if (idx > a.plen - 1) idx = a.plen - 1;
-    sum = __dadd_rn(sum, (double)pw(a, raw, sc, idx));
-  }
-  return inv_sqrt_div(__dsub_rn(sum, (double)h), hi);
-}
-
-// Appends a raw candidate.  The lanes of a warp that emit together (all for
-// the CTA's one trial) take consecutive slots: a ballot of the converged
-// lanes, one atomic by the lowest, the base broadcast by a shuffle and each
-// lane's rank among them.  The order of the raw list does not matter:
-// k_select orders it by (score, h, k).
-__device__ void emit(const HarmArgs &a, uint64_t trial, const float *raw, uint64_t k, int hi,
-                     double score) {
-  const unsigned mask = __activemask();
-  const int lane = (int)(threadIdx.x & 31);
-  const int leader = __ffs(mask) - 1;
-  unsigned base = 0;
-  if (lane == leader) base = atomicAdd(&a.raw_count[trial], (unsigned)__popc(mask));
-  base = __shfl_sync(mask, base, leader);
-  const unsigned slot = base + (unsigned)__popc(mask & ((1u << lane) - 1u));
-  if (slot >= a.raw_cap) {
-    atomicOr(a.overflow, 1u);
-    return;
-  }
-  const double off = offset_at(raw, k);
-  RawCand c;
-  c.score = score;
-  c.freq = __dmul_rn(__dadd_rn((double)k, off), a.bin_hz);
-  c.k = (uint32_t)k;
-  c.h = (uint32_t)hi;
-  a.raw[trial * a.raw_cap + slot] = c;
-}
-
-
 // round(RN(kf * j)) for a positive normal double kf and 1 <= j <= 32, in
 // exact 64-bit integer arithmetic: kf = m * 2^E (53-bit m), the product m*j
 // is exact in 58 bits, rounded to 53 bits (nearest, ties to even) as the FPU
@@ -197,66 +144,91 @@ __device__ __forceinline__ uint64_t round_mul(double kf, uint32_t j) {
   return ip + (fr >= (1ull << (s - 1)) ? 1ull : 0ull);
 }
 
-// All harmonic levels h >= 2 of one gated bin (pw(k) >= 4), one lane per
-// bin: the offset is computed once, the harmonic positions and gathers are
-// issued together, and the f64 sums accumulate in j order (the reference's
-// per-h sums are the same prefix sums).  NL = number of levels (5: h <= 16,
-// 6: h <= 32).
-template <int NL>
-__device__ void harm_item(const HarmArgs &a, uint64_t trial, const float *raw, const float *sc,
-                          uint64_t k) {
-  constexpr int HMAX = 1 << (NL - 1);
-  int hmax = 0;
-#pragma unroll
-  for (int hi = 1; hi < NL; ++hi)
-    if (a.end[hi] != 0 && k + 1 <= a.end[hi]) hmax = hi;
-  if (hmax == 0 || pw(a, raw, sc, k) < 4.0f) return;  // queue entries are a superset
-  const double kf = __dadd_rn((double)k, offset_at(raw, k));
-  const int H = 1 << hmax;
-  float v[HMAX];
-#pragma unroll
-  for (int j = 1; j <= HMAX; ++j) {
-    float x = 0.0f;
-    if (j <= H) {
-      uint64_t idx = round_mul(kf, (uint32_t)j);
-      if (idx > a.plen - 1) idx = a.plen - 1;
-      x = pw(a, raw, sc, idx);
-    }
-    v[j - 1] = x;
-  }
+// Full score of harmonic level hi (h = 1 << hi) at bin k (k in [first, end]);
+// kf = k + the parabolic offset.
+__device__ double score_at(const HarmArgs &a, const float *raw, const float *sc, uint64_t k,
+                           int hi, double &kf) {
+  const int h = 1 << hi;
+  kf = __dadd_rn((double)k, offset_at(raw, k));
+  if (h > 1 && pw(a, raw, sc, k) < 4.0f) return -INFINITY;
   double sum = -0.0;
+  for (int j0 = 1; j0 <= h; j0 += 8) {  // gathers in flight, then the sums in order
+    float v[8];
 #pragma unroll
-  for (int hi = 1; hi < NL; ++hi) {
-    if (hi > hmax) break;
-    const int h = 1 << hi;
-    // harmonics j = h/2+1 .. h (v[j-1]); for h = 2 also j = 1
-#pragma unroll
-    for (int j = (hi == 1 ? 0 : h / 2); j < h; ++j) sum = __dadd_rn(sum, (double)v[j]);
-    const double xs = __dsub_rn(sum, (double)h);
-    if (!may_reach(xs, hi, a.threshold)) continue;
-    const double s = inv_sqrt_div(xs, hi);
-    if (s >= a.threshold) {
-      const double sm = score_at(a, raw, sc, k - 1, hi);
-      const double sp = score_at(a, raw, sc, k + 1, hi);
-      if (s > sm && s >= sp) emit(a, trial, raw, k, hi, s);
+    for (int u = 0; u < 8; ++u) {
+      v[u] = 0.0f;
+      if (j0 + u <= h) {
+        uint64_t idx = round_mul(kf, (uint32_t)(j0 + u));
+        if (idx > a.plen - 1) idx = a.plen - 1;
+        v[u] = pw(a, raw, sc, idx);
+      }
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j0 + u <= h) sum = __dadd_rn(sum, (double)v[u]);
   }
+  return inv_sqrt_div(__dsub_rn(sum, (double)h), hi);
+}
+
+// Appends a raw candidate.  The lanes of a warp that emit together (all for
+// the CTA's one trial) take consecutive slots: a ballot of the converged
+// lanes, one atomic by the lowest, the base broadcast by a shuffle and each
+// lane's rank among them.  The order of the raw list does not matter:
+// k_select orders it by (score, h, k).
+__device__ void emit(const HarmArgs &a, uint64_t trial, uint64_t k, int hi, double score,
+                     double kf) {
+  const unsigned mask = __activemask();
+  const int lane = (int)(threadIdx.x & 31);
+  const int leader = __ffs(mask) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(&a.raw_count[trial], (unsigned)__popc(mask));
+  base = __shfl_sync(mask, base, leader);
+  const unsigned slot = base + (unsigned)__popc(mask & ((1u << lane) - 1u));
+  if (slot >= a.raw_cap) {
+    atomicOr(a.overflow, 1u);
+    return;
+  }
+  RawCand c;
+  c.score = score;
+  c.freq = __dmul_rn(kf, a.bin_hz);
+  c.k = (uint32_t)k;
+  c.h = (uint32_t)hi;
+  a.raw[trial * a.raw_cap + slot] = c;
 }
 
 // Gate queues: per trial the bins that pass the h = 1 gate (q1) and the
-// h >= 2 gate (q2); capacity qcap each, counts n1/n2.
+// h >= 2 gate (q2); capacity qcap each, counts n1/n2.  xq: the (bin, level)
+// pairs left for exact evaluation, k | level << 25, bit 28 set where both
+// neighbours' scores are certainly lower; capacity xcap, count nx.
 struct GateArgs {
-  uint32_t *q1, *q2;
-  unsigned *n1, *n2;
-  uint64_t qcap;
+  uint32_t *q1, *q2, *xq;
+  unsigned *n1, *n2, *nx;
+  uint64_t qcap, xcap;
 };
+constexpr uint32_t XQ_PEAK = 1u << 28;
+
+// The floor of every spectrum's scales (search/src/lib.rs:53-54): 1e-6 of its
+// mean raw power, from the FFT's partial sums.  One warp per trial, before the
+// gate kernel: every CTA of that computed it again, about 1500 cycles of FP64
+// (1/64 of the f32 rate) in front of its first barrier.
+__global__ void __launch_bounds__(128)
+    k_floor(const double *__restrict__ psum, uint32_t npsum, uint64_t ntrials, uint64_t plen,
+            float *__restrict__ floor_out) {
+  const uint64_t trial = (uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = (int)(threadIdx.x & 31);
+  if (trial >= ntrials) return;
+  double s = 0.0;
+  for (uint32_t i = lane; i < npsum; i += 32) s += psum[trial * npsum + i];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) floor_out[trial] = (float)(s / (double)plen * 1e-6);
+}
 
 constexpr int SCG_OWN = SC_G * 64;  // bins of the CTA's own blocks
 constexpr int SCG_LQ = 1024;        // local queue slots (overflow goes to global)
-constexpr size_t SCG_SMEM = (size_t)SC_CH * SC_STRIDE * 4 + (size_t)(SC_G + 4) * 4 +
+constexpr size_t SCG_SMEM = (size_t)SC_CH * SC_RAW * 4 + (size_t)(SC_G + 4) * 4 +
                             (size_t)SCG_LQ * 2 * 2;
 
-// Normalisation scales of 124 blocks per CTA, then the harmonic gates on the
+// Normalisation scales of SC_G blocks per CTA, then the harmonic gates on the
 // CTA's own bins while they are hot in L2.  An h = 1 peak needs
 // max(pw(k), pw(k+1)) >= t1 (t1 = the smallest float whose f64 value minus 1
 // reaches the threshold; score_1(k) is pw(k) - 1 or pw(k+1) - 1), and h >= 2
@@ -266,15 +238,23 @@ constexpr size_t SCG_SMEM = (size_t)SC_CH * SC_STRIDE * 4 + (size_t)(SC_G + 4) *
 // 2e-7 of the correctly rounded quotient); birdies are ignored and the last
 // bin, whose neighbour's scale belongs to the next CTA, is always queued.
 // The item kernel evaluates every queued bin exactly.
+//
+// Median: the rank is counted at a pivot first, the mean of the five chunks'
+// own medians (7 probes per chunk), which is within a few ranks on a locally
+// flat spectrum; a merge walk forwards or backwards over the sorted chunks
+// finishes.  Far pivots fall back to rank-bound skips.
+// Bound: ALU (the sorting network's 1086 min/max per thread of about GATE_I
+// instructions).  Measured on a GB300, 64 spectra of 2^19 bins: 116 us with up
+// to six rounds of skips from rank 0, word-wise staging and f32 gate
+// estimates, GATE_T now.
 __global__ void __launch_bounds__(SC_NT)
-    k_scales_gate(HarmArgs a, const double *__restrict__ psum, uint32_t npsum,
-                  uint64_t nblocks, float *__restrict__ scale_out, GateArgs g) {
+    k_scales_gate(HarmArgs a, const float *__restrict__ floor_in, uint64_t nblocks,
+                  float *__restrict__ scale_out, GateArgs g) {
   extern __shared__ __align__(16) uint32_t dsm[];
   uint32_t *ch = dsm;                                // SC_CH x SC_STRIDE (sorted chunks)
-  float *inv_s = reinterpret_cast<float *>(ch + SC_CH * SC_STRIDE);  // 1/scale per block
+  float *inv_s = reinterpret_cast<float *>(ch + SC_CH * SC_RAW);  // 1/scale per block
   uint16_t *lq1 = reinterpret_cast<uint16_t *>(inv_s + SC_G + 4);
   uint16_t *lq2 = lq1 + SCG_LQ;
-  __shared__ float floor_s;
   __shared__ int c1, c2;
   __shared__ unsigned base1, base2;
   const uint64_t plen = a.plen;
@@ -282,55 +262,56 @@ __global__ void __launch_bounds__(SC_NT)
   const float *raw = a.power + trial * a.ldp;
   const long long b0 = (long long)blockIdx.x * SC_G;
   const long long c_first = b0 - 2;  // chunk index of local chunk 0
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {  // floor: mean of the raw power from the FFT's partial sums
-    double s = 0.0;
-    for (uint32_t i = lane; i < npsum; i += 32) s += psum[trial * npsum + i];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) floor_s = (float)(s / (double)plen * 1e-6);
-  }
+  const float floor_s = __ldg(floor_in + trial);
   if (threadIdx.x == 0) c1 = c2 = 0;
   // Stage the bins of all chunks (16-byte loads, four in flight per thread);
   // out-of-range chunks and bin 0 hold the sentinel 0xffffffff.
   constexpr int NV = SC_CH * 64;
   constexpr int NV4 = NV / 4;
   static_assert(NV4 % (4 * SC_NT) == 0, "staging loop covers the chunks exactly");
-  const long long e_first = c_first * 64;  // a multiple of 4: 16-byte aligned loads
+  // e = (first bin of the CTA's chunks) + 4 i; 32-bit arithmetic: plen < 2^25
+  const int e_first = (int)(c_first * 64), plen_i = (int)plen;
+#pragma unroll 1
   for (int base = 0; base < NV4; base += 4 * SC_NT) {
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long e = e_first + 4ll * (base + u * SC_NT + (int)threadIdx.x);
-      if (e >= 1 && e + 3 < (long long)plen) {
+      const int e = e_first + 4 * (base + u * SC_NT + (int)threadIdx.x);
+      if (e >= 1 && e + 3 < plen_i) {
         v[u] = *reinterpret_cast<const uint4 *>(raw + e);
       } else {
         uint32_t t[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          t[j] = (e + j >= 1 && e + j < (long long)plen) ? fbits(raw[e + j]) : 0xffffffffu;
+          t[j] = (e + j >= 1 && e + j < plen_i) ? fbits(raw[e + j]) : 0xffffffffu;
         v[u] = make_uint4(t[0], t[1], t[2], t[3]);
       }
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int i = 4 * (base + u * SC_NT + (int)threadIdx.x);
-      uint32_t *dst = ch + (i >> 6) * SC_STRIDE + (i & 63);  // one chunk row
-      dst[0] = v[u].x;
-      dst[1] = v[u].y;
-      dst[2] = v[u].z;
-      dst[3] = v[u].w;
+      const int q = base + u * SC_NT + (int)threadIdx.x;  // quad q of the CTA: chunk q / 16
+      *reinterpret_cast<uint4 *>(ch + (q >> 4) * SC_RAW + 4 * (q & 15)) = v[u];
     }
   }
   __syncthreads();
   {
     // Thread t sorts chunk t in registers: Batcher's odd-even merge sort
     // network (543 compare-exchanges for 64 keys), fully unrolled, so every
-    // register index is static and there are no shuffles.  The stride-65
-    // layout makes these row reads bank-conflict free.
+    // register index is static and there are no shuffles.
     uint32_t x[64];
-    uint32_t *row = ch + threadIdx.x * SC_STRIDE;
+    {
+      const uint4 *row = reinterpret_cast<const uint4 *>(ch + threadIdx.x * SC_RAW);
 #pragma unroll
-    for (int i = 0; i < 64; ++i) x[i] = row[i];
+      for (int i = 0; i < 16; ++i) {
+        const uint4 q = row[i];
+        x[4 * i] = q.x;
+        x[4 * i + 1] = q.y;
+        x[4 * i + 2] = q.z;
+        x[4 * i + 3] = q.w;
+      }
+    }
+    __syncthreads();  // the sorted rows overlay the unsorted ones
+    uint32_t *row = ch + threadIdx.x * SC_STRIDE;
     // (merge step (p, k) compares a with a + k for every a >= k % p with
     // (a - k % p) mod 2k < k, both in one block of 2p)
 #pragma unroll
@@ -359,16 +340,71 @@ __global__ void __launch_bounds__(SC_NT)
     // The window is local chunks threadIdx.x .. threadIdx.x + 4 (chunks
     // b-2..b+2), each sorted and padded with sentinels above every value.
     const uint32_t *w = ch + threadIdx.x * SC_STRIDE;
+    // Pivot: the mean of the chunks' middle keys (as floats; a chunk that is
+    // not full may hold a sentinel there).
+    int p[5] = {0, 0, 0, 0, 0};
+    int rr = r;
+    uint32_t med_k = 0;
+    bool found = false;
+    {
+      float sum = 0.0f;
+      int full = 0;
+#pragma unroll
+      for (int d = 0; d < 5; ++d) {
+        const uint32_t m = w[d * SC_STRIDE + 32];
+        if (m < 0x7f800000u) {
+          sum += __uint_as_float(m);
+          ++full;
+        }
+      }
+      const uint32_t y = full ? __float_as_uint(__fdividef(sum, (float)full)) : 0u;
+      if (y > 0u && y < 0x7f800000u) {
+        int c = 0, cnt[5];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) {
+          cnt[d] = count_le64(w + d * SC_STRIDE, y - 1u);  // elements < y
+          c += cnt[d];
+        }
+        if (c <= r) {  // forwards: these c elements lie below the target
+#pragma unroll
+          for (int d = 0; d < 5; ++d) p[d] = cnt[d];
+          rr = r - c;
+        } else if (c - r <= 24) {
+          // backwards: the (c - r)-th largest of the elements below y.  Heads
+          // are keys + 1, 0 where a chunk has none left.
+          uint32_t hd[5];
+#pragma unroll
+          for (int d = 0; d < 5; ++d) hd[d] = cnt[d] ? w[d * SC_STRIDE + cnt[d] - 1] + 1u : 0u;
+          for (int step = c - r; step > 0; --step) {
+            uint32_t m = hd[0];
+            int am = 0;
+#pragma unroll
+            for (int d = 1; d < 5; ++d)
+              if (hd[d] > m) {
+                m = hd[d];
+                am = d;
+              }
+            med_k = m - 1u;
+#pragma unroll
+            for (int d = 0; d < 5; ++d)
+              if (d == am) {
+                --cnt[d];
+                hd[d] = cnt[d] ? w[d * SC_STRIDE + cnt[d] - 1] + 1u : 0u;
+              }
+          }
+          found = true;
+        }
+      }
+    }
+    if (!found) {
     // Rank-bound skips: with p_d elements of chunk d already known to lie
     // below the target and rr = r - sum(p_d), let y = min_d A_d[p_d + rr/5].
     // Each chunk has at most rr/5 unskipped elements below y, so at most rr
     // elements below y remain and the rank-r element is >= y: skip them.
     // Every round shrinks rr geometrically; a short merge walk finishes.
-    int p[5] = {0, 0, 0, 0, 0};
-    int rr = r;
     for (int round = 0; round < 6; ++round) {
       const int q = rr / 5;
-      if (q == 0) break;
+      if (q < 3) break;  // (a walk over up to 14 is cheaper than another round)
       uint32_t y = 0xffffffffu;
 #pragma unroll
       for (int d = 0; d < 5; ++d)
@@ -405,9 +441,10 @@ __global__ void __launch_bounds__(SC_NT)
           hd[d] = p[d] < 64 ? w[d * SC_STRIDE + p[d]] : 0xffffffffu;
         }
     }
-    uint32_t med_k = hd[0];
+    med_k = hd[0];
 #pragma unroll
     for (int d = 1; d < 5; ++d) med_k = min(med_k, hd[d]);
+    }
     const float sc = fmaxf(fmaxf(__fdiv_rn(__uint_as_float(med_k), LN2F), floor_s), 1e-20f);
     inv_s[threadIdx.x] = __frcp_rn(sc);
     scale_out[trial * a.lds + b] = sc;
@@ -417,52 +454,65 @@ __global__ void __launch_bounds__(SC_NT)
   const uint64_t kb0 = (uint64_t)b0 * 64;
   const float t1lo = a.t1 > 0.0f ? a.t1 * (1.0f - 4e-7f) : -INFINITY;
   const float t4lo = 4.0f * (1.0f - 4e-7f);
-  const float tmin = fminf(t1lo, t4lo);
   uint32_t *gq1 = g.q1 + trial * g.qcap, *gq2 = g.q2 + trial * g.qcap;
   // Four consecutive bins per thread (one 16-byte load, one block scale);
-  // the fourth bin's neighbour is the next group's first.
-  for (int i4 = threadIdx.x; i4 < SCG_OWN / 4; i4 += SC_NT) {
-    const int i = 4 * i4;
-    const uint64_t k = kb0 + (uint64_t)i;
-    if (k + 3 < a.first + 1 || k + 1 > a.end[0]) continue;  // no bin in [first+1, end_1 - 1]
-    const float4 r4 = *reinterpret_cast<const float4 *>(raw + k);
-    const float inv = inv_s[i >> 6];
-    const float e[4] = {r4.x * inv, r4.y * inv, r4.z * inv, r4.w * inv};
-    const float nx =
-        (i + 4 < SCG_OWN && k + 4 <= a.end[0]) ? raw[k + 4] * inv_s[(i + 4) >> 6] : 0.0f;
-    // Most groups pass neither gate: every estimate (and the neighbour's)
-    // below both thresholds queues nothing (the CTA's last group excepted).
-    if (i + 4 < SCG_OWN &&
-        fmaxf(fmaxf(fmaxf(e[0], e[1]), fmaxf(e[2], e[3])), nx) < tmin)
-      continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint64_t kj = k + (uint64_t)j;
-      if (kj < a.first + 1 || kj + 1 > a.end[0]) continue;
-      const float e0 = e[j];
-      bool pass1 = true;
-      if (i + j + 1 < SCG_OWN) pass1 = fmaxf(e0, j < 3 ? e[j + 1] : nx) >= t1lo;
-      if (pass1) {
-        const int slot = atomicAdd(&c1, 1);
-        if (slot < SCG_LQ) {
-          lq1[slot] = (uint16_t)(i + j);
-        } else {
-          const unsigned gi = atomicAdd(&g.n1[trial], 1u);
-          if (gi < g.qcap) gq1[gi] = (uint32_t)kj;
-          else atomicOr(a.overflow, 1u);
-        }
+  // the fourth bin's neighbour is the next group's first (the next lane's).
+  // Bins [ilo, ihi] of the CTA are candidates ([first + 1, end_1 - 1]).
+  const int own = SCG_OWN;
+  const int ilo = (int)max((long long)(a.first + 1) - (long long)kb0, 0ll);
+  const int ihi = (int)min((long long)a.end[0] - 1 - (long long)kb0, (long long)own - 1);
+  // About 7% of a noise spectrum's groups hold a gated bin, so nearly every
+  // warp does: each lane makes a 4-bit mask per gate, and the warp's lanes
+  // take their slots from one atomic and the prefix of their counts (in bit
+  // planes of ballots).
+  const int lane = (int)(threadIdx.x & 31);
+  const unsigned below = (1u << lane) - 1u;
+  auto append = [&](unsigned m, int i, int *count, uint16_t *lq, unsigned *gcount, uint32_t *gq) {
+    const unsigned cnt = (unsigned)__popc(m);
+    const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1u);
+    const unsigned b1 = __ballot_sync(0xffffffffu, cnt & 2u);
+    const unsigned b2 = __ballot_sync(0xffffffffu, cnt & 4u);
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2));
+    int slot = __shfl_sync(0xffffffffu, base, 0) + __popc(b0 & below) + 2 * __popc(b1 & below) +
+               4 * __popc(b2 & below);
+    while (m) {
+      const int j = __ffs((int)m) - 1;
+      m &= m - 1;
+      if (slot < SCG_LQ) {
+        lq[slot] = (uint16_t)(i + j);
+      } else {
+        const unsigned gi = atomicAdd(gcount, 1u);
+        if (gi < g.qcap) gq[gi] = (uint32_t)(kb0 + (uint64_t)(i + j));
+        else atomicOr(a.overflow, 1u);
       }
-      if (e0 >= t4lo) {
-        const int slot = atomicAdd(&c2, 1);
-        if (slot < SCG_LQ) {
-          lq2[slot] = (uint16_t)(i + j);
-        } else {
-          const unsigned gi = atomicAdd(&g.n2[trial], 1u);
-          if (gi < g.qcap) gq2[gi] = (uint32_t)kj;
-          else atomicOr(a.overflow, 1u);
-        }
+      ++slot;
+    }
+  };
+  for (int i0 = 0; i0 < own / 4; i0 += SC_NT) {  // (uniform trip count)
+    const int i = 4 * (i0 + (int)threadIdx.x);
+    unsigned m1 = 0, m2 = 0;
+    if (i < own && i + 3 >= ilo && i <= ihi) {
+      const uint64_t k = kb0 + (uint64_t)i;
+      const float4 r4 = *reinterpret_cast<const float4 *>(raw + k);
+      const float inv = inv_s[i >> 6];
+      const float e[4] = {r4.x * inv, r4.y * inv, r4.z * inv, r4.w * inv};
+      const float nx = (i + 4 < own && i + 3 <= ihi) ? raw[k + 4] * inv_s[(i + 4) >> 6] : 0.0f;
+      unsigned mt = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        m2 |= e[j] >= t4lo ? 1u << j : 0u;
+        mt |= fmaxf(e[j], j < 3 ? e[j + 1] : nx) >= t1lo ? 1u << j : 0u;
+      }
+      m1 = mt | (i + 4 < own ? 0u : 8u);  // the CTA's last bin always
+      if (i < ilo || i + 3 > ihi) {
+        const unsigned in = (0xfu << max(ilo - i, 0)) & (0xfu >> max(i + 3 - ihi, 0));
+        m1 &= in;
+        m2 &= in;
       }
     }
+    if (__any_sync(0xffffffffu, m2)) append(m2, i, &c2, lq2, &g.n2[trial], gq2);
+    if (__any_sync(0xffffffffu, m1)) append(m1, i, &c1, lq1, &g.n1[trial], gq1);
   }
   __syncthreads();
   const int m1 = min(c1, SCG_LQ), m2 = min(c2, SCG_LQ);
@@ -478,30 +528,156 @@ __global__ void __launch_bounds__(SC_NT)
     gq2[base2 + i] = (uint32_t)(kb0 + lq2[i]);
 }
 
-// Exact evaluation of the gated bins, one bin per thread: h = 1 peaks for
-// q1 entries, all harmonic levels h >= 2 for q2 entries.
+// The f32 side of the harmonic sums.  The positions round((k + off) j) are found
+// from the f32 parabolic offset with a bound on its error: off is exactly 0
+// where the curvature is certainly not negative, exactly +-1/2 where it is
+// certainly clamped, else off +- eps; ok is false where that cannot be told.
+struct Off {
+  float off, eps;
+  bool ok;
+};
+__device__ __forceinline__ Off off_f32(const float *raw, uint32_t k) {
+  const float a = raw[k - 1], b = raw[k], c = raw[k + 1];
+  const float curv = fmaf(-2.0f, b, a) + c, size = a + 2.0f * b + c;
+  Off o{0.0f, 0.0f, fabsf(curv) > 1.3e-7f * size};  // (false for NaN)
+  if (o.ok && curv < 0.0f) {
+    const float rel = 1.5e-7f * __fdividef(size, -curv) + 1e-6f;
+    if (!(rel <= 0.01f)) o.ok = false;
+    o.off = __fdividef(0.5f * (a - c), curv);
+    if (fabsf(o.off) > 0.5f + rel) {
+      o.off = o.off > 0.0f ? 0.5f : -0.5f;
+    } else {
+      o.eps = fabsf(o.off) * rel;
+      o.off = fminf(fmaxf(o.off, -0.5f), 0.5f);
+    }
+  }
+  return o;
+}
+// raw / scale at harmonic j of bin k, to within 1e-6; `sure` is cleared where
+// the position's rounding is within the offset's error (or the scale is
+// extreme).  Birdies are ignored.
+__device__ __forceinline__ float harm_f32(const float *raw, const float *sc, uint32_t last,
+                                          uint32_t k, const Off &o, int j, bool &sure) {
+  const float p = fmaf(o.off, (float)j, 0.5f), fl = floorf(p), fr = p - fl;
+  const float ej = o.eps > 0.0f ? fmaf(o.eps, (float)j, 4e-6f) : 0.0f;
+  const uint32_t idx = min(k * (uint32_t)j + (uint32_t)(int)fl, last);
+  const float s = sc[idx >> 6];
+  sure &= fr >= ej && fr <= 1.0f - ej && s < 1e30f;
+  return __fdividef(raw[idx], s);
+}
+// Level hi's sum at a neighbour bin against `sum` at the peak: -1 certainly
+// lower, 1 certainly higher, 0 not told.
+__device__ __forceinline__ int neighbour_f32(const float *raw, const float *sc, uint32_t last,
+                                             uint32_t k, int hi, float sum) {
+  const float p = __fdividef(raw[k], sc[k >> 6]);
+  if (p < 4.0f * (1.0f - 1e-5f)) return -1;  // no score below 4
+  if (!(p > 4.0f * (1.0f + 1e-5f))) return 0;
+  const Off o = off_f32(raw, k);
+  bool sure = o.ok;
+  float t = 0.0f;
+  for (int j = 1; j <= (1 << hi); ++j) t += harm_f32(raw, sc, last, k, o, j, sure);
+  if (!sure) return 0;
+  return t < sum * (1.0f - 2e-5f) ? -1 : t > sum * (1.0f + 2e-5f) ? 1 : 0;
+}
+
+// Which (bin, level) pairs of the gated bins need the exact score.  A bin's sum
+// at a level is certain to within 1e-5; the pair is passed on unless the sum
+// is below the level's limit (h + threshold sqrt(h), lowered by 1e-5; birdies
+// only lower a score) or, without birdies, a neighbour's is certainly higher.
+// Every h = 1 bin is passed on.
+// Bound: the gathers.  FP64 runs at 1/64 of the f32 rate here: with every
+// gated bin's levels summed in f64 the items took 155 us for 64 spectra of
+// 2^19 bins (76% of the FP64 pipe), filter and exact scores ITEMS_T now.
 constexpr int HI_NT = 256;
 constexpr int HI_CTAS_PER_TRIAL = 12;
+constexpr int HX_NT = 128, HX_CTAS_PER_TRIAL = 4;
 
 template <int NL>
-__global__ void __launch_bounds__(HI_NT) k_harm_items(HarmArgs a, GateArgs g) {
+__global__ void __launch_bounds__(HI_NT) k_harm_filter(HarmArgs a, GateArgs g) {
+  constexpr int HMAX = 1 << (NL - 1);
   const uint64_t trial = blockIdx.y;
   const float *raw = a.power + trial * a.ldp;
   const float *sc = a.scale + trial * a.lds;
   const unsigned n1 = min(g.n1[trial], (unsigned)g.qcap), n2 = min(g.n2[trial], (unsigned)g.qcap);
   const uint32_t *q1 = g.q1 + trial * g.qcap, *q2 = g.q2 + trial * g.qcap;
-  for (unsigned idx = blockIdx.x * HI_NT + threadIdx.x; idx < n1 + n2;
-       idx += gridDim.x * HI_NT) {
+  uint32_t *xq = g.xq + trial * g.xcap;
+  const int lane = (int)(threadIdx.x & 31);
+  const uint32_t last = (uint32_t)a.plen - 1;
+  for (unsigned base = (blockIdx.x * HI_NT + threadIdx.x) & ~31u; base < n1 + n2;
+       base += gridDim.x * HI_NT) {  // (warp-uniform)
+    const unsigned idx = base + lane;
+    uint32_t entry[NL];  // per level, ~0: none
+#pragma unroll
+    for (int hi = 0; hi < NL; ++hi) entry[hi] = 0xffffffffu;
     if (idx < n1) {
-      const uint64_t k = q1[idx];
-      const double s = score_at(a, raw, sc, k, 0);
-      if (s >= a.threshold) {
-        const double sm = score_at(a, raw, sc, k - 1, 0);
-        const double sp = score_at(a, raw, sc, k + 1, 0);
-        if (s > sm && s >= sp) emit(a, trial, raw, k, 0, s);
+      entry[0] = q1[idx];
+    } else if (idx < n1 + n2) {
+      const uint32_t k = q2[idx - n1];
+      int hmax = 0;
+#pragma unroll
+      for (int hi = 1; hi < NL; ++hi)
+        if (a.end[hi] != 0 && k + 1 <= a.end[hi]) hmax = hi;
+      if (hmax > 0) {
+        const Off o = off_f32(raw, k);
+        bool sure = o.ok;
+        float v[HMAX];
+#pragma unroll
+        for (int j = 1; j <= HMAX; ++j)
+          v[j - 1] = j <= (1 << hmax) ? harm_f32(raw, sc, last, k, o, j, sure) : 0.0f;
+        float sum = v[0];
+#pragma unroll
+        for (int hi = 1; hi < NL; ++hi) {
+#pragma unroll
+          for (int j = 1 << (hi - 1); j < (1 << hi); ++j) sum += v[j];
+          if (hi > hmax) continue;
+          if (!sure) {
+            entry[hi] = k | (uint32_t)hi << 25;
+          } else if (!(sum < a.lim[hi])) {
+            uint32_t x = k | (uint32_t)hi << 25;
+            if (!a.nbirdies) {
+              const int lo = neighbour_f32(raw, sc, last, k - 1, hi, sum);
+              const int up = lo > 0 ? 0 : neighbour_f32(raw, sc, last, k + 1, hi, sum);
+              if (lo > 0 || up > 0) x = 0xffffffffu;
+              else if (lo < 0 && up < 0) x |= XQ_PEAK;
+            }
+            entry[hi] = x;
+          }
+        }
       }
-    } else {
-      harm_item<NL>(a, trial, raw, sc, q2[idx - n1]);
+    }
+#pragma unroll
+    for (int hi = 0; hi < NL; ++hi) {
+      const bool take = entry[hi] != 0xffffffffu;
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (!m) continue;
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(&g.nx[trial], (unsigned)__popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1u));
+      if (take) {
+        if (at < g.xcap) xq[at] = entry[hi];
+        else atomicOr(a.overflow, 1u);
+      }
+    }
+  }
+}
+
+// The exact scores (reference f64 arithmetic) of the filtered pairs.
+__global__ void __launch_bounds__(HX_NT) k_harm_exact(HarmArgs a, GateArgs g) {
+  const uint64_t trial = blockIdx.y;
+  const float *raw = a.power + trial * a.ldp;
+  const float *sc = a.scale + trial * a.lds;
+  const unsigned n = min(g.nx[trial], (unsigned)g.xcap);
+  const uint32_t *xq = g.xq + trial * g.xcap;
+  for (unsigned i = blockIdx.x * HX_NT + threadIdx.x; i < n; i += gridDim.x * HX_NT) {
+    const uint32_t x = xq[i];
+    const uint64_t k = x & 0x1ffffffu;
+    const int hi = (int)((x >> 25) & 7u);
+    double kf, kn;
+    const double s = score_at(a, raw, sc, k, hi, kf);
+    if (s >= a.threshold) {
+      const bool peak = (x & XQ_PEAK) || (s > score_at(a, raw, sc, k - 1, hi, kn) &&
+                                          s >= score_at(a, raw, sc, k + 1, hi, kn));
+      if (peak) emit(a, trial, k, hi, s, kf);
     }
   }
 }
@@ -515,7 +691,7 @@ __device__ __forceinline__ unsigned long long score_key_desc(double s) {
 }
 
 constexpr int SEL_CAP = 2048;
-constexpr int SEL_NT = 1024;
+constexpr int SEL_NT = 512;
 
 struct SelArgs {
   const RawCand *raw;
@@ -533,11 +709,30 @@ __device__ __forceinline__ bool key_less(unsigned long long ka, uint32_t sa,
   return ka < kb || (ka == kb && sa < sb);
 }
 
+// |a - b| < tol, exactly as the f64 comparison, with f32 copies deciding where
+// their rounding (2^-24 of each) cannot matter.
+__device__ __forceinline__ bool near_freq(double a, float af, double b, float bf, double tol,
+                                          float tolf) {
+  const float d = fabsf(af - bf), err = 3e-7f * fmaxf(fabsf(af), fabsf(bf)) + 2e-7f * tolf;
+  if (d > tolf + err) return false;
+  if (d < tolf - err) return true;
+  return fabs(__dsub_rn(a, b)) < tol;
+}
+
+// One CTA per trial: the raw candidates in score order, then the reference's
+// dedupe.  Bitonic sort of (score, order) keys in shared memory: the steps
+// over distances below 64 stay inside a warp's 64-element blocks, so only the
+// wider ones need the block's barrier.  Dedupe by one warp, 32 candidates at a
+// time: each lane tests its candidate against the kept ones, then the lanes
+// left are kept in order, each dropping those near it.
+// Measured on a GB300, 64 GBT-shaped trials: 53 us with a barrier per step and
+// the dedupe one candidate at a time from global memory, SELECT_T now.
 __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
   __shared__ unsigned long long key[SEL_CAP];
   __shared__ uint32_t seq[SEL_CAP];
   __shared__ uint32_t idx[SEL_CAP];
   __shared__ double kept_f[64];
+  __shared__ float kept_s[64];
   __shared__ int nk;
   const uint64_t trial = blockIdx.x;
   const RawCand *rc = a.raw + trial * a.raw_cap;
@@ -546,9 +741,10 @@ __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
   const double dm = a.trial_dm[trial];
   if (threadIdx.x == 0) nk = 0;
   if (n <= SEL_CAP) {
-    unsigned P = 1;
+    const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+    unsigned P = 64;
     while (P < n) P <<= 1;
-    for (unsigned i = threadIdx.x; i < P; i += blockDim.x) {
+    for (unsigned i = threadIdx.x; i < P; i += SEL_NT) {
       if (i < n) {
         key[i] = score_key_desc(rc[i].score);
         seq[i] = (rc[i].h << 24) | rc[i].k;
@@ -560,40 +756,55 @@ __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
       }
     }
     __syncthreads();
-    for (unsigned k = 2; k <= P; k <<= 1)
-      for (unsigned j = k >> 1; j > 0; j >>= 1) {
-        for (unsigned i = threadIdx.x; i < P; i += blockDim.x) {
-          const unsigned l = i ^ j;
-          if (l > i) {
-            const bool up = (i & k) == 0;
-            const bool gt = key_less(key[l], seq[l], key[i], seq[i]);
-            if (gt == up) {
-              unsigned long long tk = key[i];
-              key[i] = key[l];
-              key[l] = tk;
-              uint32_t ts = seq[i];
-              seq[i] = seq[l];
-              seq[l] = ts;
-              uint32_t ti = idx[i];
-              idx[i] = idx[l];
-              idx[l] = ti;
-            }
-          }
+    auto exchange = [&](unsigned i, unsigned l, unsigned k) {
+      const bool up = (i & k) == 0;
+      const unsigned long long ki = key[i], kl = key[l];
+      const uint32_t si = seq[i], sl = seq[l];
+      if (key_less(kl, sl, ki, si) == up) {
+        key[i] = kl;
+        key[l] = ki;
+        seq[i] = sl;
+        seq[l] = si;
+        const uint32_t t = idx[i];
+        idx[i] = idx[l];
+        idx[l] = t;
+      }
+    };
+    for (unsigned k = 2; k <= P; k <<= 1) {
+      unsigned j = k >> 1;
+      for (; j >= 64; j >>= 1) {
+        for (unsigned p = threadIdx.x; p < P / 2; p += SEL_NT) {
+          const unsigned i = 2 * j * (p / j) + p % j;
+          exchange(i, i + j, k);
         }
         __syncthreads();
       }
-    // Sequential dedupe by warp 0 (search/src/lib.rs:131-143).
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      int kc = 0;
-      for (unsigned i = 0; i < n && (uint64_t)kc < a.max_candidates; ++i) {
-        const RawCand c = rc[idx[i]];
-        bool dup = false;
-        for (int q = lane; q < kc; q += 32) dup |= fabs(__dsub_rn(kept_f[q], c.freq)) < a.tol;
-        dup = __any_sync(0xffffffffu, dup);
-        if (!dup) {
-          if (lane == 0) {
+      for (unsigned b = warp; b < P / 64; b += SEL_NT / 32)
+        for (unsigned q = j; q > 0; q >>= 1) {
+          const unsigned i = 64 * b + 2 * q * (lane / q) + lane % q;
+          exchange(i, i + q, k);
+          __syncwarp();
+        }
+      if (k >= 64) __syncthreads();  // (below, a block stays with its warp)
+    }
+    // Dedupe (search/src/lib.rs:131-143) by warp 0.
+    if (warp == 0) {
+      const float tolf = (float)a.tol;
+      unsigned kc = 0;
+      for (unsigned i0 = 0; i0 < n && kc < a.max_candidates; i0 += 32) {
+        const bool in = i0 + lane < n;
+        RawCand c{};
+        if (in) c = rc[idx[i0 + lane]];
+        const float cf = (float)c.freq;
+        bool alive = in;
+        for (unsigned q = 0; q < kc; ++q)
+          alive = alive && !near_freq(kept_f[q], kept_s[q], c.freq, cf, a.tol, tolf);
+        unsigned m = __ballot_sync(0xffffffffu, alive);
+        while (m && kc < a.max_candidates) {
+          const int w = __ffs((int)m) - 1;
+          if (lane == w) {
             kept_f[kc] = c.freq;
+            kept_s[kc] = cf;
             psr_candidate o;
             o.frequency_hz = c.freq;
             o.period_s = __ddiv_rn(1.0, c.freq);
@@ -601,12 +812,15 @@ __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
             o.harmonics = 1ull << c.h;
             o.score = c.score;
             out[kc] = o;
+            alive = false;
           }
-          ++kc;
           __syncwarp();
+          if (alive) alive = !near_freq(kept_f[kc], kept_s[kc], c.freq, cf, a.tol, tolf);
+          ++kc;
+          m = __ballot_sync(0xffffffffu, alive);
         }
       }
-      if (lane == 0) a.kept_count[trial] = (unsigned)kc;
+      if (lane == 0) a.kept_count[trial] = kc;
     }
     return;
   }
@@ -705,13 +919,14 @@ int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint
   PSR_TRY(w.scale.ensure(outer * w.lds * 4));
   (void)inner;
   PSR_TRY(w.raw.ensure(outer * w.raw_cap * sizeof(RawCand)));
-  PSR_TRY(w.raw_count.ensure(outer * 4));
-  PSR_TRY(w.overflow.ensure(16));
+  PSR_TRY(w.counts.ensure((4 * outer + 4) * 4));
+  PSR_TRY(w.floors.ensure(outer * 4));
   // Gated bins are ~2% of a noise spectrum; a quarter of the bins is ample
   // and an overflow (flagged) reruns the chunk with room for every bin.
   w.qcap = w.queue_full ? plen : plen / 4 + 1024;
+  w.xcap = w.queue_full ? 6 * plen : w.qcap;  // every level of every bin at most
   PSR_TRY(w.gq.ensure(2 * outer * w.qcap * 4));
-  PSR_TRY(w.gn.ensure(2 * outer * 4 + 16));
+  PSR_TRY(w.xq.ensure(outer * w.xcap * 4));
   PSR_TRY(w.birdies.ensure(std::max<size_t>(c.birdies.size(), 2) * 8));
   if (!c.birdies.empty())
     PSR_CUDA(cudaMemcpyAsync(w.birdies.p, c.birdies.data(), c.birdies.size() * 8,
@@ -719,10 +934,9 @@ int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint
   return PSR_OK;
 }
 
+// counts: overflow word, then raw, q1, q2 and exact-list counts per trial.
 int spectrum_reset(SpecWork &w, uint64_t outer_trials, cudaStream_t st) {
-  PSR_CUDA(cudaMemsetAsync(w.raw_count.p, 0, outer_trials * 4, st));
-  PSR_CUDA(cudaMemsetAsync(w.overflow.p, 0, 16, st));
-  PSR_CUDA(cudaMemsetAsync(w.gn.p, 0, 2 * outer_trials * 4, st));
+  PSR_CUDA(cudaMemsetAsync(w.counts.p, 0, (4 * outer_trials + 4) * 4, st));
   w.outer_trials = outer_trials;
   return PSR_OK;
 }
@@ -756,9 +970,9 @@ HarmArgs harm_args(const FftPlan &p, const SpecConfig &c, const float *d_power, 
     a.end[hi] = (e <= first + 1) ? 0 : e;
   }
   a.raw = w.raw.as<RawCand>();
-  a.raw_count = w.raw_count.as<unsigned>();
+  a.raw_count = w.counts.as<unsigned>() + 4;
   a.raw_cap = w.raw_cap;
-  a.overflow = w.overflow.as<unsigned>();
+  a.overflow = w.counts.as<unsigned>();
   // exact f32 form of the h = 1 prefilter (double)max(pw) - 1.0 >= threshold
   float v = (float)(c.threshold + 1.0);
   if (std::isnan(v)) v = INFINITY;
@@ -767,6 +981,10 @@ HarmArgs harm_args(const FftPlan &p, const SpecConfig &c, const float *d_power, 
   for (int it = 0; it < 64 && !((double)v - 1.0 >= c.threshold); ++it)
     v = std::nextafter(v, INFINITY);
   a.t1 = v;
+  for (int hi = 0; hi < 6; ++hi) {
+    const double h = (double)(1 << hi), l = h + c.threshold * std::sqrt(h);
+    a.lim[hi] = l > 1e-3 && l < 1e30 ? (float)(l * (1.0 - 1e-5)) : -INFINITY;
+  }
   return a;
 }
 GateArgs gate_args(SpecWork &w, uint64_t slot0) {
@@ -774,8 +992,12 @@ GateArgs gate_args(SpecWork &w, uint64_t slot0) {
   g.qcap = w.qcap;
   g.q1 = w.gq.as<uint32_t>() + slot0 * w.qcap;
   g.q2 = w.gq.as<uint32_t>() + (w.outer_trials + slot0) * w.qcap;
-  g.n1 = w.gn.as<unsigned>() + slot0;
-  g.n2 = w.gn.as<unsigned>() + w.outer_trials + slot0;
+  g.xq = w.xq.as<uint32_t>() + slot0 * w.xcap;
+  g.xcap = w.xcap;
+  unsigned *n = w.counts.as<unsigned>() + 4 + slot0;
+  g.n1 = n + w.outer_trials;
+  g.n2 = n + 2 * w.outer_trials;
+  g.nx = n + 3 * w.outer_trials;
   return g;
 }
 }  // namespace
@@ -792,7 +1014,9 @@ int spectrum_gate(const FftPlan &p, const SpecConfig &c, const float *d_power, u
   PSR_CUDA(cudaFuncSetAttribute(k_scales_gate, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)SCG_SMEM));
   dim3 grid((unsigned)((nblocks + SC_G - 1) / SC_G), (unsigned)ntrials);
-  k_scales_gate<<<grid, SC_NT, SCG_SMEM, st>>>(a, d_psum, npsum, nblocks,
+  float *floors = w.floors.as<float>() + slot0;
+  k_floor<<<(unsigned)((ntrials + 3) / 4), 128, 0, st>>>(d_psum, npsum, ntrials, plen, floors);
+  k_scales_gate<<<grid, SC_NT, SCG_SMEM, st>>>(a, floors, nblocks,
                                                w.scale.as<float>() + slot0 * w.lds, g);
   PSR_CUDA(cudaGetLastError());
   return PSR_OK;
@@ -804,10 +1028,10 @@ int spectrum_items(const FftPlan &p, const SpecConfig &c, const float *d_power, 
   HarmArgs a = harm_args(p, c, d_power, ldp, w);
   if (a.end[0] == 0) return PSR_OK;
   dim3 grid(HI_CTAS_PER_TRIAL, (unsigned)ntrials);
-  if (c.levels == 6)
-    k_harm_items<6><<<grid, HI_NT, 0, st>>>(a, gate_args(w, 0));
-  else
-    k_harm_items<5><<<grid, HI_NT, 0, st>>>(a, gate_args(w, 0));
+  const GateArgs g = gate_args(w, 0);
+  if (c.levels == 6) k_harm_filter<6><<<grid, HI_NT, 0, st>>>(a, g);
+  else k_harm_filter<5><<<grid, HI_NT, 0, st>>>(a, g);
+  k_harm_exact<<<dim3(HX_CTAS_PER_TRIAL, (unsigned)ntrials), HX_NT, 0, st>>>(a, g);
   PSR_CUDA(cudaGetLastError());
   return PSR_OK;
 }
@@ -818,7 +1042,7 @@ int spectrum_select(const FftPlan &p, const SpecConfig &c, const double *d_trial
                     cudaStream_t st) {
   SelArgs s{};
   s.raw = w.raw.as<RawCand>();
-  s.raw_count = w.raw_count.as<unsigned>();
+  s.raw_count = w.counts.as<unsigned>() + 4;
   s.raw_cap = w.raw_cap;
   s.trial_dm = d_trial_dm;
   s.tol = 1.0 / ((double)p.len * c.tsamp);

@@ -216,8 +216,9 @@ struct SpecConfig {
   int levels = 5;               // harmonic sums h = 1 .. 2^(levels-1)
 };
 struct SpecWork {
-  DevBuf scale, raw, raw_count, birdies, overflow, gq, gn;
-  uint64_t qcap = 0;          // gate queue capacity per trial
+  DevBuf scale, raw, counts, floors, birdies, gq, xq;
+  uint64_t qcap = 0, xcap = 0;  // gate queue and exact list capacities per trial
+  const unsigned *overflow() const { return counts.as<unsigned>(); }
   bool queue_full = false;    // size the gate queues for every bin
   uint64_t outer_trials = 0;  // trials of the chunk being processed
   uint64_t raw_cap = 0;  // raw (pre-dedupe) candidates per trial

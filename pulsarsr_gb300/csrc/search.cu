@@ -115,7 +115,7 @@ int SearchEngine::enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st
                           kept.as<psr_candidate>() + t0 * maxc, kept_count.as<unsigned>() + t0,
                           aux));
   PSR_TRY(record(ST_SPEC, false, aux));
-  PSR_CUDA(cudaMemcpyAsync(chunk_overflow.as<unsigned>() + ci, sw.overflow.p, 4,
+  PSR_CUDA(cudaMemcpyAsync(chunk_overflow.as<unsigned>() + ci, sw.overflow(), 4,
                            cudaMemcpyDeviceToDevice, aux));
   PSR_CUDA(cudaEventRecord(ev_sel[b], aux));
   sel_pending[b] = true;
