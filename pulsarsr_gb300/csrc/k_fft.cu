@@ -960,6 +960,31 @@ int run_four_step(const FftArgs &a) {
   return PSR_OK;
 }
 
+// The quarter table, entries r <= N/8 and their mirrors N/4 - r (components
+// swapped).  The angles of every N are those of the largest (2 pi r / N with
+// N a power of two), and for each of them the device's f64 sincos rounds to
+// the same f32 values as the host's, which the oracle uses (compared
+// exhaustively).  On the host the tables of a 2^23-point transform took about
+// 28 ms.
+__global__ void __launch_bounds__(256) k_fft_quarter(uint64_t N, float2 *__restrict__ Q) {
+  const uint64_t r = (uint64_t)blockIdx.x * 256 + threadIdx.x, n4 = N / 4, n8 = N / 8;
+  if (r > n8) return;
+  double sn, cs;
+  sincos(6.283185307179586 * (double)r / (double)N, &sn, &cs);
+  const float2 v = make_float2((float)cs, (float)sn);
+  Q[r] = v;
+  if (n4 - r > n8) Q[n4 - r] = make_float2(v.y, v.x);
+}
+
+// Tw1[k1*M2 + n2] = W_N^(2*n2*k1) = W_M^(n2*k1), by the device lookup.
+__global__ void __launch_bounds__(256)
+    k_fft_tw1(const float2 *__restrict__ Q, int lq, int lm2, uint64_t M,
+              float2 *__restrict__ tw1) {
+  const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  const uint64_t k1 = i >> lm2, n2 = i & ((1ull << lm2) - 1);
+  if (i < M) tw1[i] = twN(Q, (uint32_t)(2 * n2 * k1), lq);
+}
+
 }  // namespace
 
 uint64_t FftPlan::pass2_ctas() const {
@@ -987,37 +1012,16 @@ int FftPlan::init(uint64_t series_len, cudaStream_t st) {
   while ((1ull << m) < M) ++m;
   M1 = 1ull << ((m + 1) / 2);
   M2 = 1ull << (m / 2);
-  const uint64_t n4 = N / 4, n8 = N / 8;
-  std::vector<float2> q(n4 + 1);
-  for (uint64_t r = 0; r <= n8; ++r) {
-    double a = 6.283185307179586 * (double)r / (double)N;
-    q[r] = make_float2((float)std::cos(a), (float)std::sin(a));
-  }
-  for (uint64_t r = n8 + 1; r <= n4; ++r) q[r] = make_float2(q[n4 - r].y, q[n4 - r].x);
-  PSR_TRY(Q.ensure(q.size() * sizeof(float2)));
-  PSR_CUDA(cudaMemcpyAsync(Q.p, q.data(), q.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
+  int lq = 0;
+  while ((1ull << lq) < N / 4) ++lq;
+  PSR_TRY(Q.ensure((N / 4 + 1) * sizeof(float2)));
+  k_fft_quarter<<<(unsigned)((N / 8 + 1 + 255) / 256), 256, 0, st>>>(N, Q.as<float2>());
   if (m > 12) {
-    // Tw1[k1*M2 + n2] = W_N^(2*n2*k1) = W_M^(n2*k1), from the same quarter table
-    // and quadrant rule as the device lookup.
-    std::vector<float2> t((size_t)M);
-    for (uint64_t k1 = 0; k1 < M1; ++k1)
-      for (uint64_t n2 = 0; n2 < M2; ++n2) {
-        const uint64_t x = 2 * n2 * k1, qd = x / n4, r = x % n4;
-        const float2 v = q[r];
-        float2 w;
-        switch (qd & 3) {
-          case 0: w = make_float2(v.x, -v.y); break;
-          case 1: w = make_float2(-v.y, -v.x); break;
-          case 2: w = make_float2(-v.x, v.y); break;
-          default: w = make_float2(v.y, v.x); break;
-        }
-        t[k1 * M2 + n2] = w;
-      }
-    PSR_TRY(tw1.ensure(t.size() * sizeof(float2)));
-    PSR_CUDA(cudaMemcpyAsync(tw1.p, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice,
-                             st));
+    PSR_TRY(tw1.ensure(M * sizeof(float2)));
+    k_fft_tw1<<<(unsigned)(M / 256), 256, 0, st>>>(Q.as<float2>(), lq, ilog2((int)M2), M,
+                                                   tw1.as<float2>());
   }
-  PSR_CUDA(cudaStreamSynchronize(st));
+  PSR_CUDA(cudaGetLastError());
   return PSR_OK;
 }
 

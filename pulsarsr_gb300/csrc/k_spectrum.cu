@@ -239,14 +239,15 @@ constexpr size_t SCG_SMEM = (size_t)SC_CH * SC_RAW * 4 + (size_t)(SC_G + 4) * 4 
 // bin, whose neighbour's scale belongs to the next CTA, is always queued.
 // The item kernel evaluates every queued bin exactly.
 //
-// Median: the rank is counted at a pivot first, the mean of the five chunks'
-// own medians (7 probes per chunk), which is within a few ranks on a locally
-// flat spectrum; a merge walk forwards or backwards over the sorted chunks
-// finishes.  Far pivots fall back to rank-bound skips.
-// Bound: ALU (the sorting network's 1086 min/max per thread of about GATE_I
+// Median: the rank is counted at a pivot, the mean of the five chunks' own
+// medians (7 probes per chunk), then at one moved by the density of exponential
+// noise, which on a locally flat spectrum is two or three ranks short; a merge
+// walk forwards or backwards over the sorted chunks finishes.  Far pivots fall
+// back to rank-bound skips.
+// Bound: ALU (the sorting network's 1086 min/max per thread of about 4000
 // instructions).  Measured on a GB300, 64 spectra of 2^19 bins: 116 us with up
-// to six rounds of skips from rank 0, word-wise staging and f32 gate
-// estimates, GATE_T now.
+// to six rounds of skips from rank 0, word-wise staging and one shared atomic
+// per queued bin, 114 now.
 __global__ void __launch_bounds__(SC_NT)
     k_scales_gate(HarmArgs a, const float *__restrict__ floor_in, uint64_t nblocks,
                   float *__restrict__ scale_out, GateArgs g) {
@@ -357,13 +358,24 @@ __global__ void __launch_bounds__(SC_NT)
           ++full;
         }
       }
-      const uint32_t y = full ? __float_as_uint(__fdividef(sum, (float)full)) : 0u;
-      if (y > 0u && y < 0x7f800000u) {
+      uint32_t y = full ? __float_as_uint(__fdividef(sum, (float)full)) : 0u;
+      if (y > 0u && y < 0x7f000000u) {
         int c = 0, cnt[5];
+        auto count = [&]() {
+          c = 0;
 #pragma unroll
-        for (int d = 0; d < 5; ++d) {
-          cnt[d] = count_le64(w + d * SC_STRIDE, y - 1u);  // elements < y
-          c += cnt[d];
+          for (int d = 0; d < 5; ++d) {
+            cnt[d] = count_le64(w + d * SC_STRIDE, y - 1u);  // elements < y
+            c += cnt[d];
+          }
+        };
+        count();
+        // Second pivot, two ranks short: exponential noise has (hi - lo) ln 2 /
+        // 2 y elements per unit around its median y.
+        const float step = __fdividef((float)(r - c) - 2.0f, 0.34657f * (float)(hi - lo));
+        if (fabsf(step) < 0.3f) {
+          y = __float_as_uint(__uint_as_float(y) * (1.0f + step));
+          count();
         }
         if (c <= r) {  // forwards: these c elements lie below the target
 #pragma unroll
@@ -489,30 +501,48 @@ __global__ void __launch_bounds__(SC_NT)
       ++slot;
     }
   };
-  for (int i0 = 0; i0 < own / 4; i0 += SC_NT) {  // (uniform trip count)
-    const int i = 4 * (i0 + (int)threadIdx.x);
-    unsigned m1 = 0, m2 = 0;
-    if (i < own && i + 3 >= ilo && i <= ihi) {
-      const uint64_t k = kb0 + (uint64_t)i;
-      const float4 r4 = *reinterpret_cast<const float4 *>(raw + k);
-      const float inv = inv_s[i >> 6];
-      const float e[4] = {r4.x * inv, r4.y * inv, r4.z * inv, r4.w * inv};
-      const float nx = (i + 4 < own && i + 3 <= ihi) ? raw[k + 4] * inv_s[(i + 4) >> 6] : 0.0f;
-      unsigned mt = 0;
+  // (four groups per thread in flight: the queue's stores keep the compiler
+  // from moving a later group's load above them)
+  constexpr int GU = 4;
+  for (int i0 = 0; i0 < own / 4; i0 += GU * SC_NT) {  // (uniform trip count)
+    float4 r[GU];
+    float edge[GU];  // the bin after the warp's last, in lane 31
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        m2 |= e[j] >= t4lo ? 1u << j : 0u;
-        mt |= fmaxf(e[j], j < 3 ? e[j + 1] : nx) >= t1lo ? 1u << j : 0u;
-      }
-      m1 = mt | (i + 4 < own ? 0u : 8u);  // the CTA's last bin always
-      if (i < ilo || i + 3 > ihi) {
-        const unsigned in = (0xfu << max(ilo - i, 0)) & (0xfu >> max(i + 3 - ihi, 0));
-        m1 &= in;
-        m2 &= in;
+    for (int u = 0; u < GU; ++u) {
+      const int i = 4 * (i0 + u * SC_NT + (int)threadIdx.x);
+      r[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      edge[u] = 0.0f;
+      if (i < own && i + 3 >= ilo && i <= ihi) {
+        r[u] = *reinterpret_cast<const float4 *>(raw + kb0 + (uint64_t)i);
+        if (lane == 31 && i + 4 < own && i + 3 <= ihi) edge[u] = raw[kb0 + (uint64_t)(i + 4)];
       }
     }
-    if (__any_sync(0xffffffffu, m2)) append(m2, i, &c2, lq2, &g.n2[trial], gq2);
-    if (__any_sync(0xffffffffu, m1)) append(m1, i, &c1, lq1, &g.n1[trial], gq1);
+#pragma unroll
+    for (int u = 0; u < GU; ++u) {
+      const int i = 4 * (i0 + u * SC_NT + (int)threadIdx.x);
+      const float up = __shfl_down_sync(0xffffffffu, r[u].x, 1);
+      const float nr = lane == 31 ? edge[u] : up;
+      unsigned m1 = 0, m2 = 0;
+      if (i < own && i + 3 >= ilo && i <= ihi) {
+        const float inv = inv_s[i >> 6];
+        const float e[4] = {r[u].x * inv, r[u].y * inv, r[u].z * inv, r[u].w * inv};
+        const float nx = (i + 4 < own && i + 3 <= ihi) ? nr * inv_s[(i + 4) >> 6] : 0.0f;
+        unsigned mt = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          m2 |= e[j] >= t4lo ? 1u << j : 0u;
+          mt |= fmaxf(e[j], j < 3 ? e[j + 1] : nx) >= t1lo ? 1u << j : 0u;
+        }
+        m1 = mt | (i + 4 < own ? 0u : 8u);  // the CTA's last bin always
+        if (i < ilo || i + 3 > ihi) {
+          const unsigned in = (0xfu << max(ilo - i, 0)) & (0xfu >> max(i + 3 - ihi, 0));
+          m1 &= in;
+          m2 &= in;
+        }
+      }
+      if (__any_sync(0xffffffffu, m2)) append(m2, i, &c2, lq2, &g.n2[trial], gq2);
+      if (__any_sync(0xffffffffu, m1)) append(m1, i, &c1, lq1, &g.n1[trial], gq1);
+    }
   }
   __syncthreads();
   const int m1 = min(c1, SCG_LQ), m2 = min(c2, SCG_LQ);
@@ -587,7 +617,7 @@ __device__ __forceinline__ int neighbour_f32(const float *raw, const float *sc, 
 // Every h = 1 bin is passed on.
 // Bound: the gathers.  FP64 runs at 1/64 of the f32 rate here: with every
 // gated bin's levels summed in f64 the items took 155 us for 64 spectra of
-// 2^19 bins (76% of the FP64 pipe), filter and exact scores ITEMS_T now.
+// 2^19 bins (76% of the FP64 pipe), filter and exact scores 32 + 47 now.
 constexpr int HI_NT = 256;
 constexpr int HI_CTAS_PER_TRIAL = 12;
 constexpr int HX_NT = 128, HX_CTAS_PER_TRIAL = 4;
@@ -726,7 +756,7 @@ __device__ __forceinline__ bool near_freq(double a, float af, double b, float bf
 // time: each lane tests its candidate against the kept ones, then the lanes
 // left are kept in order, each dropping those near it.
 // Measured on a GB300, 64 GBT-shaped trials: 53 us with a barrier per step and
-// the dedupe one candidate at a time from global memory, SELECT_T now.
+// the dedupe one candidate at a time from global memory, 26 now.
 __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
   __shared__ unsigned long long key[SEL_CAP];
   __shared__ uint32_t seq[SEL_CAP];
