@@ -835,11 +835,11 @@ int psr_raw_power(const float *series, uint64_t len, float *out) {
   DevBuf ser, sums, work, power, psum;
   PSR_TRY(ser.ensure(ldo * 4 + 256));
   PSR_TRY(sums.ensure(8));
-  PSR_TRY(work.ensure(p.M * 8 + 16));
+  PSR_TRY(work.ensure(std::max<uint64_t>(p.M * 8 + 16, series_mean_scratch(len))));
   PSR_TRY(power.ensure((p.M + 1 + 64) * 4));
   PSR_TRY(psum.ensure(p.pass2_ctas() * 8 + 8));
   PSR_CUDA(cudaMemcpyAsync(ser.p, series, len * 4, cudaMemcpyHostToDevice, s.s));
-  PSR_TRY(launch_series_mean(ser.as<float>(), len, nullptr, sums.as<float>(), s.s));
+  PSR_TRY(launch_series_mean(ser.as<float>(), len, nullptr, sums.as<float>(), work.p, s.s));
   PSR_TRY(launch_raw_power_ex(p, ser.as<float>(), ldo, sums.as<float>(), 1, work.as<float2>(),
                               power.as<float>(), ((p.M + 1 + 63) / 64) * 64, psum.as<double>(),
                               s.s));

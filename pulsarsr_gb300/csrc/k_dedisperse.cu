@@ -801,18 +801,83 @@ __global__ void __launch_bounds__(DG_NT)
   }
 }
 
-// Reduction of per-tile partial sums into the series sum per trial and the
-// f32 mean the FFT subtracts (search/src/lib.rs:36-40).  The reference's
-// mean is a sequential f64 sum starting from -0.0.  Integer samples make
-// every partial sum an exact integer below 2^53, so any order gives it.  For
-// f32 samples (check = true) the tiles also recorded sum |x| and the finest
-// quantum 2^q among the outputs: every partial sum, in any order, is then a
-// multiple of 2^q no larger than sum |x|, so it is exact in f64 while
-// sum |x| < 2^(53+q) (with a margin for the rounding of sum |x| itself).
-// Otherwise the thread re-adds the trial's series sequentially, in the
-// reference's order.
-// One warp per trial: the tiles' sums are added 32 lanes wide (one thread per
-// trial took 13 us per 256-trial launch of 65 tiles each, a chain of loads).
+// ---------------------------------------------------------------------------
+// The series sum per trial and the f32 mean the FFT subtracts
+// (search/src/lib.rs:36-40).  The reference's mean is a sequential f64 sum
+// starting from -0.0.  Integer samples make every partial sum an exact integer
+// below 2^53, so any order gives it.  Otherwise the series is taken in segments
+// of which the sum, sum |x| and the finest quantum 2^q among the values are
+// known.  A running sum s that is a multiple of 2^qs stays exact through a
+// segment, in any order inside it, while |s| + sum |x| < 2^(53 + min(q, qs))
+// (with a margin for the rounding of sum |x|): every partial sum is a multiple
+// of that quantum below 2^53 of it.  Such segments are added at once, 32 at a
+// time where that holds for all of them together; the others sample by sample
+// in order.
+
+// 2^(53 + q) (q within f32 exponents' reach; larger: no limit).
+__device__ __forceinline__ double exact_limit(int q) {
+  return q > 200 ? INFINITY : __longlong_as_double((long long)(53 + q + 1023) << 52);
+}
+// Quantum exponent of a finite f64 (zero constrains nothing).
+__device__ __forceinline__ int quantum_exponent64(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & ~(1ull << 63);
+  if (b == 0) return kNoQuantum;
+  const int e = (int)(b >> 52);
+  unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+  if (e) m |= 1ull << 52;
+  return (e ? e : 1) - 1075 + (__ffsll((long long)m) - 1);
+}
+// Whether s passes exactly through values of magnitude sum `mag` and quantum q.
+__device__ __forceinline__ bool passes(double s, double mag, int q) {
+  const int qs = quantum_exponent64(s);
+  return fabs(s) + mag * (1.0 + 0x1p-20) < exact_limit(min(q, qs));
+}
+
+// The sequential sum s + x[..] over segments [g0, g1) by one warp; segment i
+// covers samples [i len, (i + 1) len) of x[0, n) and seg(i, S, A, q) gives its
+// sum, sum |x| and quantum.  All lanes hold s and return the sum.
+template <class Seg>
+__device__ double sequential_sum(const float *__restrict__ x, uint64_t n, uint64_t len,
+                                 uint64_t g0, uint64_t nseg, Seg seg, int lane, double s) {
+  for (uint64_t g = g0; g < nseg; g += 32) {
+    double S = 0.0, A = 0.0;
+    int q = kNoQuantum;
+    if (g + lane < nseg) seg(g + lane, S, A, q);
+    double St = S, At = A;
+    int qt = q;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      St += __shfl_xor_sync(0xffffffffu, St, o);
+      At += __shfl_xor_sync(0xffffffffu, At, o);
+      qt = min(qt, __shfl_xor_sync(0xffffffffu, qt, o));
+    }
+    if (passes(s, At, qt)) {
+      s += St;
+      continue;
+    }
+    const int cnt = (int)min((uint64_t)32, nseg - g);
+    for (int i = 0; i < cnt; ++i) {
+      const double Si = __shfl_sync(0xffffffffu, S, i), Ai = __shfl_sync(0xffffffffu, A, i);
+      const int qi = __shfl_sync(0xffffffffu, q, i);
+      if (passes(s, Ai, qi)) {
+        s += Si;
+        continue;
+      }
+      const uint64_t a = (g + i) * len, b = min(a + len, n);
+      for (uint64_t t0 = a; t0 < b; t0 += 32) {
+        const float v = t0 + lane < b ? x[t0 + lane] : 0.0f;
+        const int m = (int)min((uint64_t)32, b - t0);
+        for (int u = 0; u < m; ++u) s += (double)__shfl_sync(0xffffffffu, v, u);
+      }
+    }
+  }
+  return s;
+}
+
+// Per-tile partial sums into sums and means: one warp per trial.  Integer
+// samples: the tiles' sums added 32 lanes wide.  f32 samples (check): the
+// sequential sum, tiles of 1024 samples as segments (the one-thread re-addition
+// that inexact series took before costs about 30 us per 1000 samples).
 constexpr int RP_NT = 128;
 __global__ void __launch_bounds__(RP_NT)
     k_reduce_parts(const double *part, uint64_t ntiles, uint64_t ntrials, uint64_t n,
@@ -820,86 +885,130 @@ __global__ void __launch_bounds__(RP_NT)
   const uint64_t tr = (uint64_t)blockIdx.x * (RP_NT / 32) + (threadIdx.x >> 5);
   const int lane = (int)(threadIdx.x & 31);
   if (tr >= ntrials) return;
-  double s = 0.0, a = 0.0, q = (double)kNoQuantum;
-  for (uint64_t i = lane; i < ntiles; i += 32) {
-    s += part[tr * ntiles + i];
-    if (check) {
-      a += part[ntrials * ntiles + tr * ntiles + i];
-      q = fmin(q, part[2 * ntrials * ntiles + tr * ntiles + i]);
-    }
-  }
-  for (int o = 16; o; o >>= 1) {
-    s += __shfl_down_sync(0xffffffffu, s, o);
-    if (check) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      q = fmin(q, __shfl_down_sync(0xffffffffu, q, o));
-    }
+  double s = 0.0;
+  if (check) {
+    const double *ps = part + tr * ntiles, *pa = ps + ntrials * ntiles,
+                 *pq = pa + ntrials * ntiles;
+    s = sequential_sum(series + tr * ldo, n, DG_TT, 0, ntiles,
+                       [&](uint64_t i, double &S, double &A, int &q) {
+                         S = ps[i];
+                         A = pa[i];
+                         q = (int)pq[i];
+                       }, lane, -0.0);
+  } else {
+    for (uint64_t i = lane; i < ntiles; i += 32) s += part[tr * ntiles + i];
+    for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   }
   if (lane != 0) return;
-  if (check && !f64_sums_exact(a, (int)q)) {  // the reference's order: t = 0, 1, ..., from -0.0
-    const float *x = series + tr * ldo;
-    s = -0.0;
-    uint64_t t = 0;
-    for (; t + 4 <= n; t += 4) {  // rows start 256-byte aligned (ldo % 64 == 0)
-      const float4 v = *reinterpret_cast<const float4 *>(x + t);
-      s += (double)v.x;
-      s += (double)v.y;
-      s += (double)v.z;
-      s += (double)v.w;
-    }
-    for (; t < n; ++t) s += (double)x[t];
-  }
   sums[tr] = s;
   means[tr] = (float)(s / (double)n);
 }
 
-// One CTA: the series sum and mean of launch_series_mean.
-constexpr int SM_NT = 1024;
+// launch_series_mean: segments of SM_SEG samples, one warp each, and blocks of
+// SM_B segments, one CTA each; then one warp over 32 blocks at a time, which
+// opens a block that does not pass into its segments.  Measured on a GB300:
+// 3,000,001 samples 2.56 ms by one CTA that read the series, 0.02 + 0.01 now.
+constexpr int SM_SEG = 256, SM_B = 32, SM_NT = 32 * SM_B;
+struct SegSum {
+  double S, A;
+  int q, pad;
+};
 __global__ void __launch_bounds__(SM_NT)
-    k_series_mean(const float *__restrict__ x, uint64_t n, double *sum_out, float *mean_out) {
-  __shared__ double ss[SM_NT / 32], sa[SM_NT / 32];
-  __shared__ int sq[SM_NT / 32];
-  double s = 0.0, a = 0.0;
+    k_series_segs(const float *__restrict__ x, uint64_t n, uint64_t nseg,
+                  SegSum *__restrict__ seg, SegSum *__restrict__ blk) {
+  __shared__ SegSum sh[SM_B];
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+  const uint64_t i = (uint64_t)blockIdx.x * SM_B + warp;
+  float v[SM_SEG / 32];
+#pragma unroll
+  for (int u = 0; u < SM_SEG / 32; ++u) {
+    const uint64_t t = i * SM_SEG + 32 * u + lane;
+    v[u] = t < n ? x[t] : 0.0f;
+  }
+  double S = 0.0;
+  float A = 0.0f;  // an upper bound is all it is used for
   int q = kNoQuantum;
-  for (uint64_t i = threadIdx.x; i < n; i += SM_NT) {
-    const float v = x[i];
-    s += (double)v;
-    a += fabs((double)v);
-    q = min(q, quantum_exponent(v));
+#pragma unroll
+  for (int u = 0; u < SM_SEG / 32; ++u) {
+    S += (double)v[u];
+    A = __fadd_ru(A, fabsf(v[u]));
+    q = min(q, quantum_exponent(v[u]));
   }
-  for (int o = 16; o; o >>= 1) {
-    s += __shfl_down_sync(0xffffffffu, s, o);
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    q = min(q, __shfl_down_sync(0xffffffffu, q, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    ss[threadIdx.x >> 5] = s;
-    sa[threadIdx.x >> 5] = a;
-    sq[threadIdx.x >> 5] = q;
+  // (where S itself is inexact, A and q make passes() fail for any s)
+  auto reduce = [&]() {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      S += __shfl_xor_sync(0xffffffffu, S, o);
+      A = __fadd_ru(A, __shfl_xor_sync(0xffffffffu, A, o));
+    }
+    q = __reduce_min_sync(0xffffffffu, q);
+  };
+  reduce();
+  if (lane == 0) {
+    sh[warp] = SegSum{S, (double)A, q, 0};
+    if (i < nseg) seg[i] = sh[warp];
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  s = 0.0;
-  a = 0.0;
-  q = kNoQuantum;
-  for (int w = 0; w < SM_NT / 32; ++w) {
-    s += ss[w];
-    a += sa[w];
-    q = min(q, sq[w]);
+  if (warp != 0) return;
+  S = sh[lane].S;
+  A = (float)sh[lane].A;  // (was a float)
+  q = sh[lane].q;
+  reduce();
+  if (lane == 0) blk[blockIdx.x] = SegSum{S, (double)A, q, 0};
+}
+__global__ void __launch_bounds__(32)
+    k_series_mean(const float *__restrict__ x, uint64_t n, const SegSum *__restrict__ seg,
+                  uint64_t nseg, const SegSum *__restrict__ blk, uint64_t nblk, double *sum_out,
+                  float *mean_out) {
+  const int lane = (int)threadIdx.x;
+  double s = -0.0;
+  for (uint64_t g = 0; g < nblk; g += 32) {
+    SegSum b{0.0, 0.0, kNoQuantum, 0};
+    if (g + lane < nblk) b = blk[g + lane];
+    double St = b.S, At = b.A;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      St += __shfl_xor_sync(0xffffffffu, St, o);
+      At += __shfl_xor_sync(0xffffffffu, At, o);
+    }
+    if (passes(s, At, __reduce_min_sync(0xffffffffu, b.q))) {
+      s += St;
+      continue;
+    }
+    const int cnt = (int)min((uint64_t)32, nblk - g);
+    for (int i = 0; i < cnt; ++i) {
+      const double Si = __shfl_sync(0xffffffffu, b.S, i), Ai = __shfl_sync(0xffffffffu, b.A, i);
+      if (passes(s, Ai, __shfl_sync(0xffffffffu, b.q, i))) {
+        s += Si;
+        continue;
+      }
+      s = sequential_sum(x, n, SM_SEG, (g + i) * SM_B, min((g + i + 1) * SM_B, nseg),
+                         [&](uint64_t j, double &S, double &A, int &q) {
+                           const SegSum e = seg[j];
+                           S = e.S;
+                           A = e.A;
+                           q = e.q;
+                         }, lane, s);
+    }
   }
-  if (!f64_sums_exact(a, q)) {  // the reference's order, from -0.0
-    s = -0.0;
-    for (uint64_t i = 0; i < n; ++i) s += (double)x[i];
-  }
+  if (lane != 0) return;
   if (sum_out) *sum_out = s;
   *mean_out = (float)(s / (double)n);
 }
 
 }  // namespace
 
+size_t series_mean_scratch(uint64_t n) {
+  const uint64_t nseg = (n + SM_SEG - 1) / SM_SEG;
+  return (size_t)(nseg + (nseg + SM_B - 1) / SM_B) * sizeof(SegSum);
+}
+
 int launch_series_mean(const float *d_x, uint64_t n, double *d_sum, float *d_mean,
-                       cudaStream_t st) {
-  k_series_mean<<<1, SM_NT, 0, st>>>(d_x, n, d_sum, d_mean);
+                       void *d_scratch, cudaStream_t st) {
+  const uint64_t nseg = (n + SM_SEG - 1) / SM_SEG, nblk = (nseg + SM_B - 1) / SM_B;
+  SegSum *seg = static_cast<SegSum *>(d_scratch), *blk = seg + nseg;
+  k_series_segs<<<(unsigned)nblk, SM_NT, 0, st>>>(d_x, n, nseg, seg, blk);
+  k_series_mean<<<1, 32, 0, st>>>(d_x, n, seg, nseg, blk, nblk, d_sum, d_mean);
   PSR_CUDA(cudaGetLastError());
   return PSR_OK;
 }
@@ -1304,7 +1413,9 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
     // The CTA's delay block ([trials per CTA][channels of the group], u32) is
     // preloaded into shared memory when it takes at most 16 KB.
     const int group = (int)(255.0 / maxv);
-    const size_t dly_bytes = (size_t)(group >= 2 ? DD_DB8 : DD_DB) * glen * 4;
+    // (one trial takes a kernel for one: the block of 8 would add it 8 times)
+    const bool one = ntrials == 1;
+    const size_t dly_bytes = (size_t)(one ? 1 : group >= 2 ? DD_DB8 : DD_DB) * glen * 4;
     const int preload = dly_bytes <= 16384 && dly_bytes + 2 * (size_t)rowcap <= budget;
     if (preload) budget -= dly_bytes;
     int cc = (int)std::min<uint64_t>({(uint64_t)DD_MAXCC, glen, budget / (2 * (size_t)rowcap)});
@@ -1326,7 +1437,13 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
           return PSR_OK;
         };
         int rc;
-        if (group >= 2)
+        if (one && group >= 2)
+          rc = preload ? run(k_dedisp_u8<true, 1, true>, 1, group)
+                       : run(k_dedisp_u8<true, 1, false>, 1, group);
+        else if (one)
+          rc = preload ? run(k_dedisp_u8<false, 1, true>, 1, 1)
+                       : run(k_dedisp_u8<false, 1, false>, 1, 1);
+        else if (group >= 2)
           rc = preload ? run(k_dedisp_u8<true, DD_DB8, true>, DD_DB8, group)
                        : run(k_dedisp_u8<true, DD_DB8, false>, DD_DB8, group);
         else

@@ -182,8 +182,9 @@ extern "C" int psr_raw_power_noalloc(const float *series, uint64_t len, float *o
   float *d_mean = reinterpret_cast<float *>(base + NA_MEAN);
   float *d_pow = reinterpret_cast<float *>(base + NA_POW);
   PSR_CUDA(cudaMemcpyAsync(d_ser, series, len * 4, cudaMemcpyHostToDevice, st));
-  // The mean as psr_raw_power takes it (one CTA, no scratch of its own).
-  PSR_TRY(launch_series_mean(d_ser, len, nullptr, d_mean, st));
+  // The mean as psr_raw_power takes it; its segment sums (24 bytes per 256
+  // samples) lie in the work region, which pass 1 writes afterwards.
+  PSR_TRY(launch_series_mean(d_ser, len, nullptr, d_mean, base + NA_WORK, st));
   const uint64_t lds = series_ld(len), ldp = ((M + 1 + 63) / 64) * 64;
   PSR_TRY(launch_raw_power_tables(len, N, reinterpret_cast<const float2 *>(base + NA_Q),
                                   reinterpret_cast<const float2 *>(base + NA_TW1), d_ser, lds,

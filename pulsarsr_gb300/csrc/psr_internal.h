@@ -283,10 +283,11 @@ int launch_dedisperse_ex(const DeviceObs &o, const uint32_t *d_delays, uint64_t 
 uint64_t dedisperse_part_count(const DeviceObs &o, uint64_t n);
 // The f64 sum of a device series and the f32 mean search::periodicity
 // subtracts (search/src/lib.rs:36), bit-identical to the reference's
-// sequential sum: added in parallel where that is exact, else in order.  One
-// CTA; d_sum may be null.
+// sequential sum: segments added at once where that is exact, else in order.
+// d_scratch holds series_mean_scratch(n) bytes; d_sum may be null.
+size_t series_mean_scratch(uint64_t n);
 int launch_series_mean(const float *d_x, uint64_t n, double *d_sum, float *d_mean,
-                       cudaStream_t st);
+                       void *d_scratch, cudaStream_t st);
 int launch_raw_power_ex(const FftPlan &p, const float *d_series, uint64_t lds,
                         const float *d_means, uint64_t ntrials, float2 *d_work, float *d_power,
                         uint64_t ldp, double *d_psum, cudaStream_t st);
