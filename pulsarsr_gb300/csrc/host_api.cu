@@ -371,6 +371,18 @@ struct psr_session {
 };
 
 namespace psr {
+// Rows of n floats, ld apart, packed without gaps.  A pitched device-to-host
+// copy into pageable memory goes row by row at about 1.2 GB/s here (36 ms for
+// 21 rows of 2.1 MB); packed first, one flat copy runs at link speed.
+__global__ void k_pack_rows(const float *__restrict__ in, uint64_t ld, uint64_t n,
+                            float *__restrict__ out) {
+  in += blockIdx.y * ld;
+  out += blockIdx.y * n;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = in[i];
+}
+
 template <class T>
 __global__ void k_to_f32(const T *s, uint64_t ld, uint64_t ns, uint64_t nch, float *out) {
   const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -776,8 +788,20 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
   PSR_TRY(launch_dedisperse_ex(o, dd.as<uint32_t>(), ntrials, length, ser.as<float>(), ldo,
                                parts.as<double>(), sums.as<double>(), means.as<float>(), spread,
                                err.as<unsigned>(), st, 0, 0, sums_out != nullptr, &sbp, 0));
-  PSR_CUDA(cudaMemcpy2DAsync(out, length * 4, ser.p, ldo * 4, length * 4, ntrials,
-                             cudaMemcpyDeviceToHost, st));
+  // (launched in blocks of 65535 rows)
+  const float *rows = ser.as<float>();
+  DevBuf packed;
+  if (ldo != length && ntrials > 1) {
+    PSR_TRY(packed.ensure(ntrials * length * 4));
+    for (uint64_t r = 0; r < ntrials; r += 65535) {
+      const unsigned nr = (unsigned)std::min<uint64_t>(65535, ntrials - r);
+      k_pack_rows<<<dim3((unsigned)std::min<uint64_t>((length + 255) / 256, 256), nr), 256, 0,
+                    st>>>(rows + r * ldo, ldo, length, packed.as<float>() + r * length);
+    }
+    PSR_CUDA(cudaGetLastError());
+    rows = packed.as<float>();
+  }
+  PSR_CUDA(cudaMemcpyAsync(out, rows, ntrials * length * 4, cudaMemcpyDeviceToHost, st));
   if (sums_out)
     PSR_CUDA(cudaMemcpyAsync(sums_out, sums.p, ntrials * 8, cudaMemcpyDeviceToHost, st));
   unsigned e = 0;
