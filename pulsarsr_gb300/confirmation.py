@@ -82,10 +82,15 @@ class Outcome:
 
     def json(self, pretty: bool = False) -> str:
         L = lib()
-        n = L.psr_outcome_json(self._o, C.c_int(int(pretty)), None, C.c_uint64(0))
-        buf = C.create_string_buffer(n + 1)
-        L.psr_outcome_json(self._o, C.c_int(int(pretty)), buf, C.c_uint64(n + 1))
-        return buf.value.decode()
+        # Room for the compact text (about 110 bytes per trial's response and
+        # 8 KiB of profiles at 64 bins): the text is made once, not also to size it.
+        cap = 4096 + self.ncandidates * (160 * self.trial_count + 16384)
+        while True:
+            buf = C.create_string_buffer(cap)
+            n = L.psr_outcome_json(self._o, C.c_int(int(pretty)), buf, C.c_uint64(cap))
+            if n < cap:
+                return C.string_at(buf, n).decode()
+            cap = n + 1
 
     @property
     def data(self) -> dict:

@@ -510,6 +510,7 @@ using psrjson::Value;
 
 Value candidate_json(const psr_candidate &c) {
   Value v = Value::object();
+  v.reserve(5);
   v.set("frequency_hz", Value::num(c.frequency_hz));
   v.set("period_s", Value::num(c.period_s));
   v.set("dm", Value::num(c.dm));
@@ -537,6 +538,7 @@ Value window_json(const psr_window &w) {
 }
 Value f32_array(const std::vector<float> &x) {
   Value a = Value::array();
+  a.reserve(x.size());
   for (float f : x) a.push(Value::num32(f));
   return a;
 }
@@ -579,8 +581,10 @@ Value confirmed_json(const Confirmed &r) {
   v.set("time_profiles", std::move(tpr));
   v.set("subband_profiles", std::move(sbr));
   Value resp = Value::array();
+  resp.reserve(r.dm_response.size());
   for (const DmPoint &p : r.dm_response) {
     Value q = Value::object();
+    q.reserve(4);
     q.set("dm", Value::num(p.dm));
     q.set("spectral_score", p.matched ? Value::num(p.spectral_score) : Value::null());
     q.set("spectral_frequency_hz",
@@ -590,6 +594,7 @@ Value confirmed_json(const Confirmed &r) {
   }
   v.set("dm_response", std::move(resp));
   Value mem = Value::array();
+  mem.reserve(r.members.size());
   for (const psr_candidate &c : r.members) mem.push(candidate_json(c));
   v.set("harmonic_members", std::move(mem));
   v.set("accepted", Value::boolean(r.s.accepted != 0));

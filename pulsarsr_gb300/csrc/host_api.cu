@@ -12,6 +12,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -29,6 +30,69 @@ const double K_DM = 4148.808;  // dedisperse/src/lib.rs:3
 
 void set_error(const std::string &msg) { g_error = msg; }
 const std::string &last_error() { return g_error; }
+
+// ---------------------------------------------- temporary buffers' pool
+namespace {
+thread_local PoolScope *t_scope = nullptr;
+std::mutex g_pool_mutex;
+std::map<int, cudaMemPool_t> g_pools;  // by device; null where it has none
+
+cudaMemPool_t device_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  auto it = g_pools.find(dev);
+  if (it != g_pools.end()) return it->second;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = POOL_KEEP;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    if (pool) cudaMemPoolDestroy(pool);
+    pool = nullptr;
+    cudaGetLastError();
+  }
+  return g_pools[dev] = pool;
+}
+}  // namespace
+
+PoolScope::PoolScope(cudaStream_t s) : st(s), outer(t_scope) { t_scope = this; }
+PoolScope::~PoolScope() { t_scope = outer; }
+PoolScope *PoolScope::current() { return t_scope; }
+
+cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled) {
+  pooled = false;
+  if (t_scope && n <= POOL_BLOCK) {
+    const cudaMemPool_t pool = device_pool();
+    if (pool && cudaMallocFromPoolAsync(p, n, pool, t_scope->st) == cudaSuccess) {
+      st = t_scope->st;
+      pooled = true;
+      return cudaSuccess;
+    }
+    cudaGetLastError();
+  }
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    bool trimmed = false;
+    {
+      int dev = 0;
+      cudaGetDevice(&dev);
+      std::lock_guard<std::mutex> lock(g_pool_mutex);
+      const auto it = g_pools.find(dev);
+      if (it != g_pools.end() && it->second)
+        trimmed = cudaMemPoolTrimTo(it->second, 0) == cudaSuccess;
+    }
+    if (trimmed) {
+      cudaGetLastError();
+      e = cudaMalloc(p, n);
+    }
+  }
+  return e;
+}
 
 // ------------------------------------------------------- fbank header
 namespace {
@@ -204,8 +268,9 @@ int parse_header_fields(const uint8_t *b, uint64_t len, psr_header &h,
 }
 
 // dedisperse::delays (dedisperse/src/lib.rs:9-34); powi(-2) is 1/(f*f).
-bool host_delays(const double *f, size_t n, double tsamp, double dm, std::vector<uint64_t> &out) {
-  bool bad = n == 0 || !std::isfinite(tsamp) || tsamp <= 0.0 || !std::isfinite(dm) || dm < 0.0;
+// Channel i's delay in samples is round(K_DM * dm * g[i] / tsamp).
+bool delay_factors(const double *f, size_t n, double tsamp, std::vector<double> &g) {
+  bool bad = n == 0 || !std::isfinite(tsamp) || tsamp <= 0.0;
   for (size_t i = 0; i < n && !bad; ++i) bad = !std::isfinite(f[i]) || f[i] <= 0.0;
   if (bad) {
     set_error(
@@ -215,9 +280,46 @@ bool host_delays(const double *f, size_t n, double tsamp, double dm, std::vector
   double ref = 0.0;
   for (size_t i = 0; i < n; ++i) ref = std::fmax(ref, f[i]);
   const double rinv = 1.0 / (ref * ref);
+  g.resize(n);
+  for (size_t i = 0; i < n; ++i) g[i] = 1.0 / (f[i] * f[i]) - rinv;
+  return true;
+}
+
+// One trial's row of a delay table: delays, capped to 32 bits, and the largest.
+bool delay_row(const double *g, size_t n, double tsamp, double dm, uint32_t *out,
+               uint64_t &max_delay) {
+  if (!std::isfinite(dm) || dm < 0.0) {
+    set_error(
+        "invalid dedispersion input: positive frequencies/tsamp and nonnegative DM required");
+    return false;
+  }
+  const double k = K_DM * dm;
+  double top = 0.0;
+  for (size_t i = 0; i < n; ++i) {
+    const double s = std::round(k * g[i] / tsamp);
+    top = s > top ? s : top;
+    const double v = s > 0.0 ? s : 0.0;
+    out[i] = (uint32_t)(v < 4294967295.0 ? v : 4294967295.0);
+  }
+  if (top > 18446744073709551615.0) {
+    set_error("invalid dedispersion input: delay overflow");
+    return false;
+  }
+  max_delay = std::max(max_delay, (uint64_t)top);
+  return true;
+}
+
+bool host_delays(const double *f, size_t n, double tsamp, double dm, std::vector<uint64_t> &out) {
+  std::vector<double> g;
+  if (!delay_factors(f, n, tsamp, g)) return false;
+  if (!std::isfinite(dm) || dm < 0.0) {
+    set_error(
+        "invalid dedispersion input: positive frequencies/tsamp and nonnegative DM required");
+    return false;
+  }
   out.resize(n);
   for (size_t i = 0; i < n; ++i) {
-    const double s = std::round(K_DM * dm * (1.0 / (f[i] * f[i]) - rinv) / tsamp);
+    const double s = std::round(K_DM * dm * g[i] / tsamp);
     if (s > 18446744073709551615.0) {
       set_error("invalid dedispersion input: delay overflow");
       return false;
@@ -729,6 +831,7 @@ int dedisperse_delays(const DeviceObs &o, const uint64_t *d, int64_t length, flo
   std::vector<uint32_t> tab(o.nch);
   for (uint64_t c = 0; c < o.nch; ++c) tab[c] = (uint32_t)d[c];
   uint64_t spread = 0;
+  PoolScope scope(st);
   DevBuf dd, ser, parts, sums, means, err;
   PSR_TRY(dd.ensure(o.nch * 4));
   PSR_CUDA(cudaMemcpyAsync(dd.p, tab.data(), o.nch * 4, cudaMemcpyHostToDevice, st));
@@ -765,6 +868,7 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
   }
   const DeviceObs &o = fb->o;
   cudaStream_t st = fb->stream.s;
+  PoolScope scope(st);
   std::vector<uint32_t> tab;
   uint64_t spread = 0, maxd = 0;
   PSR_TRY(make_delay_table(o, trials, ntrials, tab, spread, maxd));
@@ -853,6 +957,7 @@ int psr_raw_power(const float *series, uint64_t len, float *out) {
     return PSR_EINVAL;
   }
   Stream s;
+  PoolScope scope(s.s);
   FftPlan p;
   PSR_TRY(p.init(len, s.s));
   const uint64_t ldo = series_ld_(len);
@@ -882,6 +987,7 @@ int psr_periodicity(const float *series, uint64_t len, double tsamp, double dm,
   }
   // A one-channel f32 filterbank with zero delay reproduces the series.
   Stream s;
+  PoolScope scope(s.s);
   DeviceObs o;
   PSR_TRY(obs_from_f32(series, 1, len, tsamp, o, s.s));
   SearchEngine e;
@@ -902,6 +1008,7 @@ int psr_search_trials(const psr_fb *fb, const double *trials, uint64_t ntrials,
     return PSR_EINVAL;
   }
   cudaStream_t st = fb->stream.s;
+  PoolScope scope(st);
   SearchEngine e;
   PSR_TRY(e.prepare(fb->o, trials, ntrials, discovery, to_spec(cfg, fb->o.h.tsamp), st));
   PSR_TRY(e.enqueue(fb->o, st));
@@ -916,6 +1023,7 @@ int psr_analyze(const psr_fb *fb, const double *trials, uint64_t ntrials,
     set_error("analyze: null argument");
     return PSR_EINVAL;
   }
+  PoolScope scope(fb->stream.s);
   psr_rules r;
   psr_rules_default(&r);
   std::unique_ptr<psr_outcome> o(new psr_outcome());
@@ -961,6 +1069,7 @@ int psr_refine_objective(const psr_fb *fb, uint64_t n, const psr_timing *theta,
     set_error("refine: null argument");
     return PSR_EINVAL;
   }
+  PoolScope scope(fb->stream.s);
   RefineWork w;
   RefineEval ev;
   PSR_TRY(w.evaluate(fb->o, n, *theta, ro, 1.0, ev, fb->stream.s));
@@ -987,6 +1096,7 @@ int psr_refine_cube_objective(const psr_fb *fb, uint64_t n, const psr_timing *re
     return PSR_EINVAL;
   }
   std::vector<double> g(3 * npoints);
+  PoolScope scope(fb->stream.s);
   PSR_TRY(cube_objective(fb->o, n, *reference, theta, npoints, ro, J, g.data(), fb->stream.s));
   if (grad) {
     // (nu, nudot) = (1/P, -Pdot/P^2): the chain rule to (P, Pdot).
@@ -1011,6 +1121,7 @@ int psr_refine_gradient(const psr_fb *fb, uint64_t n, const psr_timing *start, u
     set_error("refine: null argument");
     return PSR_EINVAL;
   }
+  PoolScope scope(fb->stream.s);
   if (ro.exact) {
     RefineWork w;
     for (uint64_t i = 0; i < ncand; ++i) {
@@ -1089,6 +1200,7 @@ int psr_refine_grid(const psr_fb *fb, uint64_t n, const psr_timing *start, uint6
     set_error("refine_grid: resolution >= 0, dm_step > 0, 0 <= dm_lo <= dm_hi, bins >= 4");
     return PSR_EINVAL;
   }
+  PoolScope scope(fb->stream.s);
   for (uint64_t i = 0; i < ncand; ++i) {
     double r = 0.0;
     PSR_TRY(grid_refine_one(fb->o, n, start[i], resolution_hz, dm_step, dm_lo, dm_hi, bins,
@@ -1144,6 +1256,7 @@ int psr_profile_at(const float *series, uint64_t n, double tsamp, double period,
     return PSR_EINVAL;
   }
   Stream s;
+  PoolScope scope(s.s);
   DevBuf x;
   PSR_TRY(x.ensure(n * 4));
   PSR_CUDA(cudaMemcpyAsync(x.p, series, n * 4, cudaMemcpyHostToDevice, s.s));
@@ -1165,6 +1278,7 @@ int psr_refine(const float *series, uint64_t n, double tsamp, double frequency, 
     periods[i] = 1.0 / f;
   }
   Stream s;
+  PoolScope scope(s.s);
   DevBuf x;
   PSR_TRY(x.ensure(n * 4));
   PSR_CUDA(cudaMemcpyAsync(x.p, series, n * 4, cudaMemcpyHostToDevice, s.s));
@@ -1196,6 +1310,7 @@ int psr_measure(const float *x, uint64_t n, uint64_t offset, double tsamp, doubl
     return PSR_EINVAL;
   }
   Stream s;
+  PoolScope scope(s.s);
   DevBuf d;
   PSR_TRY(d.ensure(n * 4));
   PSR_CUDA(cudaMemcpyAsync(d.p, x, n * 4, cudaMemcpyHostToDevice, s.s));

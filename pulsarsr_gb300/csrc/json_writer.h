@@ -22,41 +22,54 @@ namespace detail {
 template <typename T>
 inline std::string pretty(T v, int max_kk, int min_kk_exclusive) {
   if (!std::isfinite(v)) return "null";
-  std::string sign = std::signbit(v) ? "-" : "";
-  if (v == 0) return sign + "0.0";
-  char buf[64];
+  char out[96], *o = out;  // at most a sign, 17 digits and 16 zeros
+  if (std::signbit(v)) *o++ = '-';
+  if (v == 0) return std::string(out, o) + "0.0";
+  char buf[64], digits[40];
   auto r = std::to_chars(buf, buf + sizeof buf, std::fabs(v), std::chars_format::scientific);
-  std::string s(buf, r.ptr);
-  const size_t e = s.find('e');
-  std::string mant = s.substr(0, e);
-  const int exp10 = std::atoi(s.c_str() + e + 1);
-  std::string digits;
-  for (char c : mant)
-    if (c != '.') digits += c;
-  const int length = (int)digits.size();
-  const int kk = exp10 + 1;  // 10^(kk-1) <= v < 10^kk
+  *r.ptr = '\0';
+  int length = 0;
+  const char *e = buf;
+  for (; *e != 'e'; ++e)
+    if (*e != '.') digits[length++] = *e;
+  const int kk = std::atoi(e + 1) + 1;  // 10^(kk-1) <= v < 10^kk
   const int k = kk - length;
-  std::string out;
+  auto put = [&](int a, int b) {
+    for (; a < b; ++a) *o++ = digits[a];
+  };
+  auto zeros = [&](int n) {
+    for (; n > 0; --n) *o++ = '0';
+  };
   if (k >= 0 && kk <= max_kk) {
-    out = digits + std::string((size_t)k, '0') + ".0";
+    put(0, length);
+    zeros(k);
+    *o++ = '.';
+    *o++ = '0';
   } else if (kk > 0 && kk <= max_kk) {
-    out = digits.substr(0, (size_t)kk) + "." + digits.substr((size_t)kk);
+    put(0, kk);
+    *o++ = '.';
+    put(kk, length);
   } else if (kk > min_kk_exclusive && kk <= 0) {
-    out = "0." + std::string((size_t)(-kk), '0') + digits;
-  } else if (length == 1) {
-    out = digits + "e" + std::to_string(kk - 1);
+    *o++ = '0';
+    *o++ = '.';
+    zeros(-kk);
+    put(0, length);
   } else {
-    out = digits.substr(0, 1) + "." + digits.substr(1) + "e" + std::to_string(kk - 1);
+    put(0, 1);
+    if (length > 1) *o++ = '.';
+    put(1, length);
+    *o++ = 'e';
+    o = std::to_chars(o, out + sizeof out, kk - 1).ptr;
   }
-  return sign + out;
+  return std::string(out, o);
 }
 }  // namespace detail
 
 inline std::string f64(double v) { return detail::pretty<double>(v, 16, -5); }
 inline std::string f32(float v) { return detail::pretty<float>(v, 13, -6); }
 
-inline std::string quote(const std::string &s) {
-  std::string o = "\"";
+inline void quote_to(std::string &o, const std::string &s) {
+  o += '"';
   for (unsigned char c : s) {
     switch (c) {
       case '"': o += "\\\""; break;
@@ -74,7 +87,12 @@ inline std::string quote(const std::string &s) {
         }
     }
   }
-  return o + "\"";
+  o += '"';
+}
+inline std::string quote(const std::string &s) {
+  std::string o;
+  quote_to(o, s);
+  return o;
 }
 
 // A JSON value: scalars keep their serialised text.
@@ -105,6 +123,11 @@ struct Value {
     Value v;
     v.kind = OBJECT;
     return v;
+  }
+  Value &reserve(size_t n) {
+    if (kind == ARRAY) items.reserve(n);
+    if (kind == OBJECT) fields.reserve(n);
+    return *this;
   }
   Value &push(Value v) {
     items.push_back(std::move(v));
@@ -149,7 +172,7 @@ inline void dump_to(const Value &v, std::string &o, bool pretty, int depth) {
       o += nl;
       for (size_t i = 0; i < v.fields.size(); ++i) {
         o += ind;
-        o += quote(v.fields[i].first);
+        quote_to(o, v.fields[i].first);
         o += pretty ? ": " : ":";
         dump_to(v.fields[i].second, o, pretty, depth + 1);
         if (i + 1 < v.fields.size()) o += ",";

@@ -1055,20 +1055,30 @@ void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta,
                     int G, ChunkPatterns &cp) {
   const uint64_t nt = tz - ta, nsub = (nch + G - 1) / G;
   cp = ChunkPatterns();
+  cp.subs.reserve(nsub);
   cp.pat.resize(nsub * nt);
   cp.ref.resize(nsub * nt);
   uint32_t hsize = 64;
   while (hsize < 4 * nt) hsize <<= 1;
   std::vector<uint32_t> slot(hsize, 0);  // 1 + row of the subband's pattern, by generation
   std::vector<uint32_t> gen(hsize, 0);
+  // The table's rows are nch apart: a strip of 64 channels is copied first.
+  constexpr uint64_t STRIP = 64;
+  std::vector<uint32_t> strip(nt * STRIP);
   for (uint64_t j = 0; j < nsub && cp.ok; ++j) {
     const uint64_t ca = j * G;
     const int ge = (int)std::min<uint64_t>(G, nch - ca);
+    if (ca % STRIP == 0) {
+      const uint64_t w = std::min<uint64_t>(STRIP, nch - ca);
+      for (uint64_t t = 0; t < nt; ++t)
+        std::copy_n(&tab[(ta + t) * nch + ca], w, &strip[t * STRIP]);
+    }
     SubBand sb{};
     sb.row0 = (int32_t)cp.keys.size();
     uint32_t dmin = 0xffffffffu, dmax = 0;
+    RelKey last;
     for (uint64_t t = 0; t < nt && cp.ok; ++t) {
-      const uint32_t *d = &tab[(ta + t) * nch + ca];
+      const uint32_t *d = &strip[t * STRIP + ca % STRIP];
       uint32_t m = d[0], mx = d[0];
       for (int c = 1; c < ge; ++c) {
         m = std::min(m, d[c]);
@@ -1087,6 +1097,12 @@ void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta,
         if (c < 4) k.a |= r << (16 * c);
         else k.b |= r << (16 * (c - 4));
       }
+      cp.ref[j * nt + t] = m;
+      if (t && k == last) {  // as the trial before
+        cp.pat[j * nt + t] = cp.pat[j * nt + t - 1];
+        continue;
+      }
+      last = k;
       uint64_t h = (k.a ^ (k.b * 0x9E3779B97F4A7C15ull)) * 0xD6E8FEB86659FD93ull;
       uint32_t q = (uint32_t)(h >> 40) & (hsize - 1);
       for (;;) {
@@ -1100,7 +1116,6 @@ void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta,
         q = (q + 1) & (hsize - 1);
       }
       cp.pat[j * nt + t] = (uint16_t)(slot[q] - (uint32_t)sb.row0);
-      cp.ref[j * nt + t] = m;
     }
     sb.dmin = (int32_t)dmin;
     sb.spread = (int32_t)(dmax - dmin);
@@ -1144,10 +1159,12 @@ int dedisp_subbands_default(const DeviceObs &o) {
 }
 
 namespace {
-// The plan at width G; plan.G stays 0 when it does not fit.
+// The plan at width G; plan.G stays 0 when it does not fit.  `known`: the
+// patterns of chunk known_ci at this width, or null.
 int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                     const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                    cudaStream_t st) {
+                    cudaStream_t st, const ChunkPatterns *known = nullptr,
+                    size_t known_ci = 0) {
   const bool byte_part = maxv * SUB_GMAX <= 255.0;
   const bool flush = (double)nch * maxv > 65535.0;
   const size_t nchunks = cstart.size() - 1;
@@ -1171,8 +1188,10 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
   for (size_t ci = 0; ci < nchunks; ++ci) {
     const uint64_t ta = cstart[ci], nt = cstart[ci + 1] - ta;
     if (nt == 0) return PSR_OK;
-    ChunkPatterns cp;
-    chunk_patterns(tab, nch, ta, ta + nt, G, cp);
+    ChunkPatterns own;
+    const bool have = known && ci == known_ci;
+    if (!have) chunk_patterns(tab, nch, ta, ta + nt, G, own);
+    const ChunkPatterns &cp = have ? *known : own;
     if (!cp.ok) return PSR_OK;
     SubbandPlan::Chunk c;
     c.sub0 = subs.size();
@@ -1180,6 +1199,8 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
     c.block0 = 0;
     c.nblocks = (nt + SS_TB - 1) / SS_TB;
     c.spread = 0;
+    slotof.reserve(slotof.size() + c.nblocks * nsub * SS_TB);
+    offof.reserve(offof.size() + c.nblocks * nsub * SS_TB);
     for (const SubBand &sb : cp.subs) {
       c.spread = std::max<uint64_t>(c.spread, (uint64_t)sb.spread);
       relmax = std::max(relmax, sb.relmax);
@@ -1321,16 +1342,19 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
   const size_t mid = (cstart.size() - 2) / 2;
   const uint64_t nt = cstart[mid + 1] - cstart[mid];
   std::vector<std::pair<double, int>> pick;
+  ChunkPatterns cp[2];  // at widths 8, 4
   for (int g : {8, 4}) {
-    ChunkPatterns cp;
-    chunk_patterns(tab, nch, cstart[mid], cstart[mid + 1], g, cp);
-    if (!cp.ok) continue;
-    const double c = two_level_cost(cp, nt, g, maxv);
+    ChunkPatterns &p = cp[g == 4];
+    chunk_patterns(tab, nch, cstart[mid], cstart[mid + 1], g, p);
+    if (!p.ok) continue;
+    const double c = two_level_cost(p, nt, g, maxv);
     if (c < direct_cost(nch, nt, maxv)) pick.emplace_back(c, g);
   }
   std::sort(pick.begin(), pick.end());
-  for (size_t i = 0; i < pick.size() && plan.G == 0; ++i)
-    PSR_TRY(subband_plan_at(tab, nch, n, maxv, cstart, pick[i].second, plan, st));
+  for (size_t i = 0; i < pick.size() && plan.G == 0; ++i) {
+    const int g = pick[i].second;
+    PSR_TRY(subband_plan_at(tab, nch, n, maxv, cstart, g, plan, st, &cp[g == 4], mid));
+  }
   return PSR_OK;
 }
 

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <cstdlib>
 
 #include <string>
 #include <vector>
@@ -58,18 +59,47 @@ __host__ __device__ inline bool f64_sums_exact(double mag, int q) {
   return q >= kNoQuantum || mag * (1.0 + 0x1p-20) < ldexp(1.0, 53 + q);
 }
 
-// Owning device allocation (sized once, reused).
+// Temporary buffers of a one-shot call.  While a PoolScope lives, the buffers
+// that this thread allocates come, up to POOL_BLOCK bytes each, from a memory
+// pool of the library's own: they are allocated and freed in the order of
+// `st`, and the driver keeps up to POOL_KEEP bytes of them mapped between
+// calls.  Measured against cudaMalloc, cudaFree and page-locked staging made
+// and dropped in each call: the search of a 32,583-sample series 0.59 -> 0.32
+// ms, a fold refinement of 263,571 samples 0.45 -> 0.24 ms, the power spectrum
+// of 3,000,001 samples 0.83 -> 0.43 ms; an analysis of five families made 690
+// allocations, 10 of its 56 ms.
+// A scope is declared after the stream it names and before the buffers, so that
+// every buffer is returned while the stream exists; a buffer that another
+// stream uses is returned only once that stream is idle.  Handles that live
+// on (filterbanks, sessions, batches) take cudaMalloc as before.  An
+// allocation that fails gives the pool's idle memory back and is tried again.
+constexpr size_t POOL_BLOCK = 64ull << 20, POOL_KEEP = 256ull << 20;
+struct PoolScope {
+  explicit PoolScope(cudaStream_t st);
+  ~PoolScope();
+  PoolScope(const PoolScope &) = delete;
+  PoolScope &operator=(const PoolScope &) = delete;
+  cudaStream_t st;
+  PoolScope *outer;
+  static PoolScope *current();  // this thread's innermost scope, or null
+};
+// cudaMalloc, or the current scope's pool (pooled is set then).
+cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled);
+
 // Page-locked host memory, grown on demand and kept across calls (device
 // copies into it run at full link speed, with no staging and no page faults).
+// In a one-shot call, which would page-lock it for a single copy, plain memory.
 struct HostBuf {
   void *p = nullptr;
   size_t bytes = 0;
+  bool pinned = true;
   HostBuf() = default;
   HostBuf(const HostBuf &) = delete;
   HostBuf &operator=(const HostBuf &) = delete;
   ~HostBuf() { release(); }
   void release() {
-    if (p) cudaFreeHost(p);
+    if (p && pinned) cudaFreeHost(p);
+    if (p && !pinned) std::free(p);
     p = nullptr;
     bytes = 0;
   }
@@ -77,7 +107,10 @@ struct HostBuf {
     if (n <= bytes && p) return PSR_OK;
     release();
     if (n == 0) n = 16;
-    cudaError_t e = cudaHostAlloc(&p, n, cudaHostAllocDefault);
+    pinned = !PoolScope::current();
+    if (!pinned) p = std::malloc(n);
+    const cudaError_t e = pinned ? cudaHostAlloc(&p, n, cudaHostAllocDefault)
+                                 : (p ? cudaSuccess : cudaErrorMemoryAllocation);
     if (e != cudaSuccess) {
       p = nullptr;
       set_error(std::string("CUDA error in cudaHostAlloc(") + std::to_string(n) +
@@ -93,15 +126,19 @@ struct HostBuf {
   }
 };
 
+// Owning device allocation (sized once, reused).
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
+  cudaStream_t st = nullptr;  // of a pooled allocation
+  bool pooled = false;
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p && pooled) cudaFreeAsync(p, st);
+    if (p && !pooled) cudaFree(p);
     p = nullptr;
     bytes = 0;
   }
@@ -109,7 +146,7 @@ struct DevBuf {
     if (n <= bytes && p) return PSR_OK;
     release();
     if (n == 0) n = 16;
-    cudaError_t e = cudaMalloc(&p, n);
+    cudaError_t e = device_alloc(&p, n, st, pooled);
     if (e != cudaSuccess) {
       p = nullptr;
       set_error(std::string("CUDA error in cudaMalloc(") + std::to_string(n) +
@@ -162,6 +199,9 @@ int inject_rfi(DeviceObs &o, const psr_synth_rfi &r, cudaStream_t st);
 int pack_payload_u8(const DeviceObs &src, uint8_t *d_payload, cudaStream_t st);
 
 // Host-side restatements that stay on the host (FP64 tables, small sorts).
+bool delay_factors(const double *f, size_t n, double tsamp, std::vector<double> &g);
+bool delay_row(const double *g, size_t n, double tsamp, double dm, uint32_t *out,
+               uint64_t &max_delay);
 bool host_delays(const double *f, size_t n, double tsamp, double dm,
                  std::vector<uint64_t> &out);
 int parse_header(const uint8_t *b, uint64_t len, psr_header &h);

@@ -163,7 +163,10 @@ SearchEngine::~SearchEngine() {
   }
   for (cudaEvent_t e : {ev_fft[0], ev_fft[1], ev_sel[0], ev_sel[1]})
     if (e) cudaEventDestroy(e);
-  if (aux) cudaStreamDestroy(aux);
+  if (aux) {
+    cudaStreamSynchronize(aux);  // its buffers go back to st's pool now
+    cudaStreamDestroy(aux);
+  }
 }
 
 int SearchEngine::enqueue(const DeviceObs &o, cudaStream_t st) {
@@ -248,31 +251,41 @@ int make_delay_table(const DeviceObs &o, const double *trials, uint64_t ntrials,
   std::vector<double> freqs(o.nch);
   for (uint64_t c = 0; c < o.nch; ++c) freqs[c] = o.h.fch1 + (double)c * o.h.foff;
   tab.assign(ntrials * o.nch, 0);
-  std::vector<uint64_t> d;
+  std::vector<double> g;
   max_delay = 0;
-  for (uint64_t i = 0; i < ntrials; ++i) {
-    if (!host_delays(freqs.data(), o.nch, o.h.tsamp, trials[i], d)) return PSR_EDEDISPERSE;
-    for (uint64_t c = 0; c < o.nch; ++c) {
-      max_delay = std::max(max_delay, d[c]);
-      tab[i * o.nch + c] = (uint32_t)std::min<uint64_t>(d[c], 0xffffffffull);
-    }
-  }
+  if (ntrials && !delay_factors(freqs.data(), o.nch, o.h.tsamp, g)) return PSR_EDEDISPERSE;
+  for (uint64_t i = 0; i < ntrials; ++i)
+    if (!delay_row(g.data(), o.nch, o.h.tsamp, trials[i], &tab[i * o.nch], max_delay))
+      return PSR_EDEDISPERSE;
   if (max_delay > o.ns) {
     set_error("invalid dedispersion input: delay exceeds observation");
     return PSR_EDEDISPERSE;
   }
   // Widest delay spread of any channel over any 8 consecutive trials (an
   // upper bound for every trial block of at most 8, whatever its alignment).
-  max_spread = 0;
-  for (uint64_t b = 0; b < ntrials; ++b)
-    for (uint64_t c = 0; c < o.nch; ++c) {
-      uint32_t lo = 0xffffffffu, hi = 0;
-      for (uint64_t i = b; i < std::min<uint64_t>(b + 8, ntrials); ++i) {
-        lo = std::min(lo, tab[i * o.nch + c]);
-        hi = std::max(hi, tab[i * o.nch + c]);
+  // Extremes over 2, 4 and 8 trials in turn, for a strip of channels at a time.
+  constexpr uint64_t STRIP = 64;
+  std::vector<uint32_t> lo(ntrials * STRIP), hi;
+  uint32_t widest = 0;
+  for (uint64_t c0 = 0; c0 < o.nch; c0 += STRIP) {
+    const uint64_t w = std::min<uint64_t>(STRIP, o.nch - c0);
+    for (uint64_t i = 0; i < ntrials; ++i)
+      for (uint64_t c = 0; c < w; ++c) lo[i * STRIP + c] = tab[i * o.nch + c0 + c];
+    hi = lo;
+    for (uint64_t step : {1, 2, 4})
+      for (uint64_t i = 0; i + step < ntrials; ++i) {
+        uint32_t *l = &lo[i * STRIP], *h = &hi[i * STRIP];
+        const uint32_t *l2 = l + step * STRIP, *h2 = h + step * STRIP;
+        for (uint64_t c = 0; c < STRIP; ++c) {
+          l[c] = std::min(l[c], l2[c]);
+          h[c] = std::max(h[c], h2[c]);
+        }
       }
-      max_spread = std::max<uint64_t>(max_spread, hi - lo);
-    }
+    for (uint64_t i = 0; i < ntrials; ++i)
+      for (uint64_t c = 0; c < w; ++c)
+        widest = std::max(widest, hi[i * STRIP + c] - lo[i * STRIP + c]);
+  }
+  max_spread = widest;
   return PSR_OK;
 }
 
