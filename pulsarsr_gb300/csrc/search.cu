@@ -60,7 +60,9 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   const uint64_t tail = chunk >= 16 && ntrials > chunk ? chunk / 8 : 0;
   cstart.clear();
   for (uint64_t t = 0; t < ntrials - tail; t += chunk) cstart.push_back(t);
-  if (tail) cstart.push_back(ntrials - tail);
+  // (a piece before it of under chunk / 4 trials joins it: the subband
+  // patterns are summed once per chunk)
+  if (tail && ntrials - tail - cstart.back() >= chunk / 4) cstart.push_back(ntrials - tail);
   cstart.push_back(ntrials);
   nchunks = cstart.size() - 1;
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
