@@ -36,7 +36,7 @@ namespace psr {
 
 // Device buffers of one cube, reused by every group of a refinement call.
 struct CubeWork {
-  DevBuf cube, R, chsum, tau, kc, cands, prof, g, grad;
+  DevBuf cube, R, chsum, tau, kc, ref, dsh, anchors, prof, g;
   uint64_t rows = 0;
   double var = 1.0;
 };
@@ -58,7 +58,7 @@ constexpr int CB_MAXB = 1024;
 // j folds a contiguous stretch of runs of the subint, prefetching its next run
 // while it folds the current one.  Samples of a boundary run outside [t0, t1) are
 // zeroed.  Phases are fixed-point fractions of a cycle (u64, 2^-64 cycle
-// resolution): one CTA-wide f64 anchor at the first run, then per-thread
+// resolution): an f64 anchor at the first run (k_cube_anchors), then per-thread
 // offsets and per-stride advances by exact integer second differences, so no
 // thread does f64 work per run.  Inside a run the bin position u (in bins)
 // advances in f32; for du < 1 bin per sample the bin index is walked
@@ -171,42 +171,148 @@ struct RunSums {
     s += s32;
     q += q32;
   }
-  __device__ __forceinline__ double sum() const { return (double)s; }
-  __device__ __forceinline__ double sq() const { return (double)q; }
+  __device__ __forceinline__ void end_tile(const uint4 *, int) {}
+  // Lane 0: the warp's sums (integers below 2^53).
+  __device__ __forceinline__ void warp_total(double &sum, double &sq) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      s += __shfl_down_sync(0xffffffffu, s, o);
+      q += __shfl_down_sync(0xffffffffu, q, o);
+    }
+    sum = (double)s;
+    sq = (double)q;
+  }
 };
+// f32 sums of v and v^2 over a chunk of 4 (or a run of 32) join (hi, lo)
+// pairs by TwoSum, which keep 38 bits or more of any number of terms where each
+// term has 24; only what passes f32's range goes to f64 (FP64 runs at 1/64 of the
+// f32 rate: two conversions and two sums per chunk and f64 shuffles were half
+// of the time of the fold).
 template <>
 struct RunSums<float> {
-  double s = 0.0, q = 0.0;
+  struct Pair {
+    float h = 0.0f, l = 0.0f;
+    __device__ __forceinline__ void add(float x) {
+      const float t = __fadd_rn(h, x), b = __fsub_rn(t, h);
+      l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(x, b)));
+      h = t;
+    }
+    __device__ __forceinline__ void add(const Pair &o) {
+      add(o.h);
+      l = __fadd_rn(l, o.l);
+    }
+    __device__ __forceinline__ bool finite() const { return isfinite(h) && isfinite(l); }
+    __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+  };
+  Pair ps, pq, ts, tq;       // so far; of the open tile
+  double s = 0.0, q = 0.0;  // what passed f32's range
+  __device__ __forceinline__ void join(const Pair &a, const Pair &b) {
+    const Pair os = ps, oq = pq;
+    ps.add(a);
+    pq.add(b);
+    if (!(ps.finite() && pq.finite())) {
+      s += os.value() + a.value();
+      q += oq.value() + b.value();
+      ps = pq = Pair();
+    }
+  }
   __device__ __forceinline__ void add(const RunRegs<float> &x) {
-    float ps = 0.0f, pq = 0.0f;
+    Pair a, b;
 #pragma unroll
     for (int i = 0; i < CB_RUN; ++i) {
       const float v = run_sample<float>(x, i);
-      ps += v;
-      pq = fmaf(v, v, pq);
+      a.h += v;
+      b.h = fmaf(v, v, b.h);
     }
-    s += (double)ps;
-    q += (double)pq;
+    join(a, b);
   }
-  __device__ __forceinline__ void add_chunk(const uint4 &v) {
-    float ps = 0.0f, pq = 0.0f;
+  static __device__ __forceinline__ void chunk_sums(const uint4 &v, float &cs, float &cq) {
+    cs = cq = 0.0f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float x = __uint_as_float(word_of(v, e));
-      ps += x;
-      pq = fmaf(x, x, pq);
+      cs += x;
+      cq = fmaf(x, x, cq);
     }
-    s += (double)ps;
-    q += (double)pq;
   }
-  __device__ __forceinline__ double sum() const { return s; }
-  __device__ __forceinline__ double sq() const { return q; }
+  __device__ __forceinline__ void add_chunk(const uint4 &v) {
+    float cs, cq;
+    chunk_sums(v, cs, cq);
+    ts.add(cs);
+    tq.add(cq);
+  }
+  // The lane's chunks of a tile (every 32nd of n) are done.
+  __device__ __forceinline__ void end_tile(const uint4 *tile, int n) {
+    if (ts.finite() && tq.finite()) {
+      join(ts, tq);
+    } else {
+      for (int i = (int)(threadIdx.x & 31); i < n; i += 32) {
+        float cs, cq;
+        chunk_sums(tile[i], cs, cq);
+        s += (double)cs;
+        q += (double)cq;
+      }
+    }
+    ts = tq = Pair();
+  }
+  // Lane 0: the warp's sums.
+  __device__ __forceinline__ void warp_total(double &sum, double &sq) {
+    Pair a = ps, b = pq;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      Pair x, y;
+      x.h = __shfl_down_sync(0xffffffffu, a.h, o);
+      x.l = __shfl_down_sync(0xffffffffu, a.l, o);
+      y.h = __shfl_down_sync(0xffffffffu, b.h, o);
+      y.l = __shfl_down_sync(0xffffffffu, b.l, o);
+      a.add(x);
+      b.add(y);
+    }
+    const bool wide = __shfl_sync(0xffffffffu, !(a.finite() && b.finite()), 0);
+    sum = wide ? 0.0 : a.value();
+    sq = wide ? 0.0 : b.value();
+    if (wide || __any_sync(0xffffffffu, s != 0.0 || q != 0.0)) {
+      if (wide) {
+        s += ps.value();
+        q += pq.value();
+      }
+      for (int o = 16; o; o >>= 1) {
+        s += __shfl_down_sync(0xffffffffu, s, o);
+        q += __shfl_down_sync(0xffffffffu, q, o);
+      }
+      sum += s;
+      sq += q;
+    }
+  }
 };
 
 // frac(x) as a u64 fraction of a cycle.
 __device__ __forceinline__ unsigned long long fix_frac(double x) {
   const double f = x - floor(x);
   return __double2ull_rz(ldexp(f, 64));
+}
+
+// Phase anchors of every (channel, subint) in units of `unit` samples, at the
+// unit that holds the subint's first sample: fx[0] phase, fx[1] cycles per sample
+// there, fx[2] unit 1 - unit 0, fx[3] its change per unit, fx[4] the change of
+// fx[1] per unit.  In a kernel of their own: one thread's f64 chain held a fold CTA
+// for a fifth of its time.
+__global__ void __launch_bounds__(CB_NT)
+    k_cube_anchors(uint64_t n, int S, uint64_t nrows, double unit, double tsamp, double nu,
+                   double nudot, const double *__restrict__ tau,
+                   unsigned long long *__restrict__ anchors) {
+  const uint64_t r = (uint64_t)blockIdx.x * CB_NT + threadIdx.x;
+  if (r >= nrows) return;
+  const uint64_t c = r / (uint64_t)S, s = r % (uint64_t)S;
+  const uint64_t u0 = (n * s) / (uint64_t)S / (uint64_t)unit;
+  const double td = (double)(u0 * (uint64_t)unit) * tsamp - tau[c];
+  const double f = (nu + nudot * td) * tsamp, g = nudot * tsamp * tsamp;
+  unsigned long long *fx = anchors + 5 * r;
+  fx[0] = fix_frac(nu * td + 0.5 * nudot * td * td);
+  fx[1] = fix_frac(f);
+  fx[2] = fix_frac(unit * f + 0.5 * g * unit * unit);
+  fx[3] = fix_frac(g * unit * unit);
+  fx[4] = fix_frac(g * unit);
 }
 
 // Bin accumulators of one CTA.  PrivateBins: one column per thread,
@@ -392,9 +498,8 @@ __device__ __forceinline__ void fold_run(const RunRegs<uint8_t> &x, float u, flo
 // of 32, at most CB_NT.
 template <class T, bool PRIV>
 __global__ void __launch_bounds__(CB_NT)
-    k_cube_fold(const T *__restrict__ x, uint64_t ld, uint64_t n, int S, int B, double tsamp,
-                double nu, double nudot, const double *__restrict__ tau,
-                float *__restrict__ cube, double *__restrict__ chsum) {
+    k_cube_fold(const T *__restrict__ x, uint64_t ld, uint64_t n, int S, int B,
+                const unsigned long long *__restrict__ anchors, float *__restrict__ cube, double *__restrict__ chsum) {
   extern __shared__ float hist[];
   __shared__ unsigned long long fx[5];
   __shared__ double red[2][CB_NT / 32];
@@ -406,18 +511,7 @@ __global__ void __launch_bounds__(CB_NT)
   for (int i = tid; i < hn; i += nt) hist[i] = 0.0f;
   const uint64_t t0 = (n * (uint64_t)s) / (uint64_t)S, t1 = (n * (uint64_t)(s + 1)) / (uint64_t)S;
   const uint64_t rlo = t0 / CB_RUN, rhi = (t1 + CB_RUN - 1) / CB_RUN;  // runs [rlo, rhi)
-  if (tid == 0) {
-    // Phase (cycles) at sample m of the channel: nu td + nudot td^2 / 2,
-    // td = m tsamp - tau_c; f = d phase / d sample, g = d f / d sample.
-    const double td = (double)(rlo * CB_RUN) * tsamp - tau[c];
-    const double f = (nu + nudot * td) * tsamp, g = nudot * tsamp * tsamp;
-    const double R = (double)CB_RUN;
-    fx[0] = fix_frac(nu * td + 0.5 * nudot * td * td);  // phase at the first run
-    fx[1] = fix_frac(f);                                // cycles/sample there
-    fx[2] = fix_frac(R * f + 0.5 * g * R * R);          // run 1 - run 0
-    fx[3] = fix_frac(g * R * R);                        // its change per run
-    fx[4] = fix_frac(g * R);                            // f change per run
-  }
+  if (tid < 5) fx[tid] = anchors[5 * (c * (uint64_t)S + (uint64_t)s) + tid];
   __syncthreads();
   // Thread j folds the contiguous runs [rlo + j q, rlo + (j + 1) q) so that
   // the open bin carries from run to run.  Phase at run m (from rlo):
@@ -457,11 +551,8 @@ __global__ void __launch_bounds__(CB_NT)
     cur = nxt;
   }
   if (ob.bin >= 0) flush_bins(bins, ob.bin, B, ob.a0, ob.a1);
-  double sum = sums.sum(), sq = sums.sq();
-  for (int o = 16; o; o >>= 1) {
-    sum += __shfl_down_sync(0xffffffffu, sum, o);
-    sq += __shfl_down_sync(0xffffffffu, sq, o);
-  }
+  double sum, sq;
+  sums.warp_total(sum, sq);
   if ((tid & 31) == 0) {
     red[0][tid >> 5] = sum;
     red[1][tid >> 5] = sq;
@@ -471,7 +562,7 @@ __global__ void __launch_bounds__(CB_NT)
     double a = 0.0;
     for (int w2 = 0; w2 < nt / 32; ++w2) a += red[tid][w2];
     chsum[(c * (uint64_t)S + (uint64_t)s) * 2 + tid] = a;
-    if (tid == 0) mean_s = (float)(a / (double)B);
+    if (tid == 0) mean_s = (float)(B & (B - 1) ? a / (double)B : a * (1.0 / (double)B));
   }
   __syncthreads();
   float *dst = cube + (c * (uint64_t)S + (uint64_t)s) * (uint64_t)B;
@@ -497,6 +588,12 @@ __global__ void __launch_bounds__(CB_NT)
   }
 }
 
+// A sample as f32 (integers exactly, without the conversion pipe).
+__device__ __forceinline__ float sample_float(float v) { return v; }
+__device__ __forceinline__ float sample_float(unsigned v) {
+  return __fsub_rn(__uint_as_float(0x4B000000u + v), 8388608.0f);
+}
+
 // Bin-owner fold for 1/31 <= du < 1 bins per sample (each bin holds 1 to 31
 // consecutive samples per period).  Each warp stages tiles of CB_TL samples
 // of the subint in shared memory; lane l owns bins l, l + 32, ... < B and,
@@ -506,38 +603,46 @@ __global__ void __launch_bounds__(CB_NT)
 // phase linear across the tile).  Adjacent bins use the same Q, so every
 // sample is counted once.  The lane keeps S_b = sum v and T_b = sum (u - m) v
 // in registers; at the end bin b of the cloud-in-cell fold is S_b - T_b +
-// T_(b-1).  No atomics, no per-sample branches.
+// T_(b-1).  No atomics, no per-sample branches: an interval is read four
+// samples at a time, those past its end as zeros.
+// One warp per tile up to 16 tiles (a subint of 16,384 samples touches 9: with 8
+// warps, seven of them waited for the one with two tiles), 8 warps above; the
+// warps' sums go into their own tiles' memory, so that three CTAs fit an SM.
+// Bound: issue; conversions and ceilings, on the quarter-rate pipe, are done by
+// sums at 2^23.  Measured on a GB300, 256 channels of 1,048,576 f32 samples, 0.3
+// bins per sample: 1.05 ms before, 0.50 now (0.16 for the bytes).
 constexpr int CB_TL = 2048;
 constexpr int CB_BO_MAXB = 256;
 constexpr int CB_BO_NB = CB_BO_MAXB / 32;
+constexpr int CB_BO_SLOTS = 8;   // tile i adds to the sums of slot i mod 8
+constexpr int CB_BO_WARPS = 16;  // warps of a CTA, at most
+// ceil(x) for |x| < 2^22
+__device__ __forceinline__ int ceil_int(float x) {
+  return (int)__float_as_uint(__fadd_ru(x, 12582912.0f)) - 0x4B400000;
+}
+// (float)i for 0 <= i < 2^23
+__device__ __forceinline__ float float_of(int i) {
+  return __fsub_rn(__uint_as_float(0x4B000000u + (unsigned)i), 8388608.0f);
+}
 
 template <class T>
-__global__ void __launch_bounds__(CB_NT)
-    k_cube_fold_bo(const T *__restrict__ x, uint64_t ld, uint64_t n, int S, int B, double tsamp,
-                   double nu, double nudot, const double *__restrict__ tau,
-                   float *__restrict__ cube, double *__restrict__ chsum) {
+__global__ void __launch_bounds__(32 * CB_BO_WARPS)
+    k_cube_fold_bo(const T *__restrict__ x, uint64_t ld, uint64_t n, int S, int B,
+                   const unsigned long long *__restrict__ anchors, float *__restrict__ cube, double *__restrict__ chsum) {
   extern __shared__ __align__(16) unsigned char smem_bo[];
-  T *tiles = reinterpret_cast<T *>(smem_bo);  // [warp][CB_TL]
-  float *wS = reinterpret_cast<float *>(smem_bo + (size_t)(CB_NT / 32) * CB_TL * sizeof(T));
-  float *wT = wS + (CB_NT / 32) * B;
+  T *tiles = reinterpret_cast<T *>(smem_bo);  // [warp][CB_TL], then [warp][S, T][B]
+  static_assert(2 * CB_BO_MAXB * 4 <= CB_TL, "a warp's sums fit its tile");
+  auto sums_of = [&](int w) { return reinterpret_cast<float *>(tiles + (size_t)w * CB_TL); };
   __shared__ unsigned long long fx[5];
-  __shared__ double red[2][CB_NT / 32];
+  __shared__ double red[2][CB_BO_WARPS];
   __shared__ float mean_s;
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nw = (int)blockDim.x >> 5;
   const int s = blockIdx.x;
   const uint64_t c = blockIdx.y;
   const uint64_t t0 = (n * (uint64_t)s) / (uint64_t)S, t1 = (n * (uint64_t)(s + 1)) / (uint64_t)S;
   const uint64_t k0 = t0 / CB_TL, k1 = (t1 + CB_TL - 1) / CB_TL;  // tiles [k0, k1)
-  if (tid == 0) {
-    const double td = (double)(k0 * CB_TL) * tsamp - tau[c];
-    const double f = (nu + nudot * td) * tsamp, g = nudot * tsamp * tsamp;
-    const double L = (double)CB_TL;
-    fx[0] = fix_frac(nu * td + 0.5 * nudot * td * td);  // phase at tile k0
-    fx[1] = fix_frac(f);                                // cycles/sample there
-    fx[2] = fix_frac(L * f + 0.5 * g * L * L);          // tile 1 - tile 0
-    fx[3] = fix_frac(g * L * L);                        // its change per tile
-    fx[4] = fix_frac(g * L);                            // f change per tile
-  }
+  if (tid < 5) fx[tid] = anchors[5 * (c * (uint64_t)S + (uint64_t)s) + tid];
   __syncthreads();
   const float Bs = (float)B * 5.42101086242752217e-20f;  // B 2^-64
   const float fB = (float)B;
@@ -548,8 +653,17 @@ __global__ void __launch_bounds__(CB_NT)
   for (int j = 0; j < CB_BO_NB; ++j) Sb[j] = Tb[j] = 0.0f;
   RunSums<T> sums;
   constexpr int PER = 16 / (int)sizeof(T);  // samples per 16-byte chunk
-  for (uint64_t k = k0 + warp; k < k1; k += CB_NT / 32) {
+  for (uint64_t k = k0 + warp; k < k1; k += nw) {
     const uint64_t ta = k * CB_TL;
+    if (ta >= t0 && ta + CB_TL <= t1) {
+      const uint4 *src = reinterpret_cast<const uint4 *>(row + ta);
+#pragma unroll 8
+      for (int q = lane; q < CB_TL / PER; q += 32) {
+        const uint4 v = __ldg(src + q);
+        reinterpret_cast<uint4 *>(tile)[q] = v;
+        sums.add_chunk(v);
+      }
+    } else
     // Stage the tile (chunks wholly outside [t0, t1) are not loaded).
     for (int q = lane; q < CB_TL / PER; q += 32) {
       const uint64_t cs = ta + (uint64_t)q * PER;
@@ -568,6 +682,7 @@ __global__ void __launch_bounds__(CB_NT)
       reinterpret_cast<uint4 *>(tile)[q] = v;
       sums.add_chunk(v);
     }
+    sums.end_tile(reinterpret_cast<const uint4 *>(tile), CB_TL / PER);
     __syncwarp();
     // Phase of the tile: fixed-point at its first sample, linear across it.
     const unsigned long long kk = k - k0;
@@ -589,43 +704,50 @@ __global__ void __launch_bounds__(CB_NT)
       const int b = lane + 32 * j;
       if (b >= B) break;
       // first unwrapped m = b + k B >= mfirst (0 <= mfirst < B)
-      int m = b >= mfirst ? b : b + B;
+      float m = float_of(b >= mfirst ? b : b + B);
       float sj = 0.0f, tj = 0.0f;
-      for (; (float)m < uend; m += B) {
-        const int i0 = max(0, (int)ceilf(((float)m - ua) * inv));
-        const int i1 = min(CB_TL, (int)ceilf(((float)(m + 1) - ua) * inv));
+      for (; m < uend; m += fB) {
+        const int i0 = max(0, ceil_int((m - ua) * inv));
+        const int i1 = min(CB_TL, ceil_int(((m + 1.0f) - ua) * inv));
         // sum v and sum (i - i0) v of the bin's samples, then its weights
         // w_i = w_0 + (i - i0) du, w_0 = ua + i0 du - m
-        float sl = 0.0f, il = 0.0f, fq = 0.0f;
-        for (int q = 0; q < cmax; ++q) {
-          if (i0 + q >= i1) break;
-          const float v = (float)tile[i0 + q];
+        const T *p = tile + i0;
+        const int len = i1 - i0;
+        float sl = 0.0f, il = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float v = e < len ? sample_float(std::conditional_t<std::is_same<T, float>::value, float, unsigned>(p[e])) : 0.0f;
           sl += v;
-          il = fmaf(fq, v, il);
-          fq += 1.0f;
+          il = fmaf((float)e, v, il);
+        }
+        for (int q = 4; q < cmax; q += 4) {
+          const float fq = float_of(q);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float v = q + e < len ? sample_float(std::conditional_t<std::is_same<T, float>::value, float, unsigned>(p[q + e])) : 0.0f;
+            sl += v;
+            il = fmaf(fq + (float)e, v, il);
+          }
         }
         sj += sl;
-        tj = fmaf(fmaf((float)i0, du, ua) - (float)m, sl, fmaf(du, il, tj));
+        tj = fmaf(fmaf(float_of(i0), du, ua) - m, sl, fmaf(du, il, tj));
       }
       Sb[j] += sj;
       Tb[j] += tj;
     }
     __syncwarp();
   }
-  // Per-warp bin sums to shared memory, then across warps.
+  // Per-warp bin sums into the warp's own tile, then across warps.
 #pragma unroll
   for (int j = 0; j < CB_BO_NB; ++j) {
     const int b = lane + 32 * j;
     if (b < B) {
-      wS[warp * B + b] = Sb[j];
-      wT[warp * B + b] = Tb[j];
+      sums_of(warp)[b] = Sb[j];
+      sums_of(warp)[B + b] = Tb[j];
     }
   }
-  double sum = sums.sum(), sq = sums.sq();
-  for (int o = 16; o; o >>= 1) {
-    sum += __shfl_down_sync(0xffffffffu, sum, o);
-    sq += __shfl_down_sync(0xffffffffu, sq, o);
-  }
+  double sum, sq;
+  sums.warp_total(sum, sq);
   if (lane == 0) {
     red[0][warp] = sum;
     red[1][warp] = sq;
@@ -633,19 +755,24 @@ __global__ void __launch_bounds__(CB_NT)
   __syncthreads();
   if (tid < 2) {
     double a = 0.0;
-    for (int w2 = 0; w2 < CB_NT / 32; ++w2) a += red[tid][w2];
+    for (int w2 = 0; w2 < nw; ++w2) a += red[tid][w2];
     chsum[(c * (uint64_t)S + (uint64_t)s) * 2 + tid] = a;
-    if (tid == 0) mean_s = (float)(a / (double)B);
+    if (tid == 0) mean_s = (float)(B & (B - 1) ? a / (double)B : a * (1.0 / (double)B));
   }
   __syncthreads();
   float *dst = cube + (c * (uint64_t)S + (uint64_t)s) * (uint64_t)B;
-  for (int b = tid; b < B; b += CB_NT) {
+  for (int b = tid; b < B; b += nw * 32) {
     const int bp = b == 0 ? B - 1 : b - 1;
+    // slot w holds the sums of tiles w and w + 8 (of every eighth with 8 warps)
+    auto slot = [&](int w, int i) {
+      const float x = sums_of(w)[i];
+      return w + CB_BO_SLOTS < nw ? x + sums_of(w + CB_BO_SLOTS)[i] : x;
+    };
     float sb = 0.0f, tb = 0.0f, tp = 0.0f;
-    for (int w2 = 0; w2 < CB_NT / 32; ++w2) {
-      sb += wS[w2 * B + b];
-      tb += wT[w2 * B + b];
-      tp += wT[w2 * B + bp];
+    for (int w2 = 0; w2 < min(nw, CB_BO_SLOTS); ++w2) {
+      sb += slot(w2, b);
+      tb += slot(w2, B + b);
+      tp += slot(w2, B + bp);
     }
     dst[b] = sb - tb + tp - mean_s;
   }
@@ -665,14 +792,20 @@ int cube_fold_threads(int B, bool &priv) {
 template <class T>
 int launch_cube_fold(dim3 grid, int B, cudaStream_t st, const T *x, uint64_t ld, uint64_t n,
                      int S, double tsamp, double nu, double nudot, const double *tau,
-                     float *cube, double *chsum) {
+                     unsigned long long *anchors, float *cube, double *chsum) {
   const double du = nu * tsamp * (double)B;
-  if (du >= 1.0 / 31.0 && du < 1.0 && B <= CB_BO_MAXB) {
-    const size_t sm = (size_t)(CB_NT / 32) * CB_TL * sizeof(T) + (size_t)2 * (CB_NT / 32) * B * 4;
+  const bool owner = du >= 1.0 / 31.0 && du < 1.0 && B <= CB_BO_MAXB;
+  const uint64_t nrows = (uint64_t)grid.x * grid.y;
+  k_cube_anchors<<<(unsigned)((nrows + CB_NT - 1) / CB_NT), CB_NT, 0, st>>>(
+      n, S, nrows, owner ? (double)CB_TL : (double)CB_RUN, tsamp, nu, nudot, tau, anchors);
+  if (owner) {
+    // tiles that a subint's samples can touch
+    const uint64_t tiles = ((n + S - 1) / S + CB_TL - 2) / CB_TL + 1;
+    const int nw = tiles <= CB_BO_WARPS ? (int)tiles : CB_BO_SLOTS;
+    const size_t sm = (size_t)nw * CB_TL * sizeof(T);
     PSR_CUDA(cudaFuncSetAttribute(k_cube_fold_bo<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sm));
-    k_cube_fold_bo<T><<<grid, CB_NT, sm, st>>>(x, ld, n, S, B, tsamp, nu, nudot, tau, cube,
-                                              chsum);
+    k_cube_fold_bo<T><<<grid, nw * 32, sm, st>>>(x, ld, n, S, B, anchors, cube, chsum);
     return PSR_OK;
   }
   // Below 1/31 bins per sample runs rarely change bin: one shared row with
@@ -681,163 +814,240 @@ int launch_cube_fold(dim3 grid, int B, cudaStream_t st, const T *x, uint64_t ld,
   const int nt = du < 1.0 ? CB_NT : cube_fold_threads(B, priv);
   if (priv)
     k_cube_fold<T, true><<<grid, nt, (size_t)(B + 1) * nt * 4, st>>>(
-        x, ld, n, S, B, tsamp, nu, nudot, tau, cube, chsum);
+        x, ld, n, S, B, anchors, cube, chsum);
   else
-    k_cube_fold<T, false><<<grid, nt, (size_t)(B + 1) * 4, st>>>(x, ld, n, S, B, tsamp, nu,
-                                                                nudot, tau, cube, chsum);
+    k_cube_fold<T, false><<<grid, nt, (size_t)(B + 1) * 4, st>>>(x, ld, n, S, B, anchors, cube,
+                                                                chsum);
   return PSR_OK;
 }
 
 struct CandDev {
   double nu, nudot, dm;
 };
+// The candidates of a launch, as a kernel argument.
+constexpr int CB_CANDS = 64;
+struct CandBatch {
+  CandDev c[CB_CANDS];
+};
 
-__device__ __forceinline__ double cube_shift(const CandDev &q, double nu_r, double nudot_r,
-                                             double dm_r, double Ts, double kc, double B,
-                                             double &tdq) {
-  const double taur = kc * dm_r, tauq = kc * q.dm;
-  const double tdr = Ts - taur;
-  tdq = Ts - tauq;
-  const double phr = nu_r * tdr + 0.5 * nudot_r * tdr * tdr;
-  const double phq = q.nu * tdq + 0.5 * q.nudot * tdq * tdq;
-  return (phq - phr) * B;
+// x - floor(x) for 0 <= x < 2^23, the floor by a sum rounded down at 2^23 (floorf
+// runs on the quarter-rate pipe).
+__device__ __forceinline__ float frac_pos(float x) {
+  return x - __fsub_rn(__fadd_rd(x, 8388608.0f), 8388608.0f);
 }
 
-// Shift of row r = (c, s) for a candidate, in bins, and T_s - tau_c(DM).
-__device__ __forceinline__ double row_shift(const CandDev &q, double nu_r, double nudot_r,
-                                            double dm_r, double Tsub, const double *kc, int S,
-                                            int B, uint64_t r, double &tdq, double &kcc) {
-  const uint64_t c = r / (uint64_t)S;
-  const int s = (int)(r % (uint64_t)S);
-  const double Ts = ((double)s + 0.5) * Tsub;
-  kcc = kc[c];
-  return cube_shift(q, nu_r, nudot_r, dm_r, Ts, kcc, (double)B, tdq);
+__device__ __forceinline__ double row_time(uint32_t r, int S, double Tsub) {
+  return ((double)(r % (uint32_t)S) + 0.5) * Tsub;  // T_s of row r = (channel, subint s)
+}
+
+// ref[r] = phase of row r at the reference (cycles), T_s - tau_c(DM_ref).
+__global__ void __launch_bounds__(CB_NT)
+    k_cube_ref(uint32_t rows, int S, const double *__restrict__ kc, double Tsub, double nu_r,
+               double nudot_r, double dm_r, double *__restrict__ ref) {
+  const uint32_t r = blockIdx.x * CB_NT + threadIdx.x;
+  if (r >= rows) return;
+  const double tdr = row_time(r, S, Tsub) - kc[r / (uint32_t)S] * dm_r;
+  ref[r] = nu_r * tdr + 0.5 * nudot_r * tdr * tdr;
 }
 
 // R[r][k-1] = sum_b C[r][b] e^(-2 pi i k b / B), k = 1..B/2; one CTA per
-// CB_ROWS rows, twiddles from a shared table.
+// CB_ROWS rows, twiddles from a shared table.  A thread takes one harmonic of
+// four rows, so that a twiddle (gathered, with bank conflicts) is read once for
+// them.  With one thread per (row, harmonic), a row at a time: 16,384 rows of 64
+// harmonics 101 us; 41 now.
 constexpr int CB_ROWS = 32;
+// Rows staged at a time: 16 KB of shared memory, a multiple of 4.
+__host__ __device__ inline int cube_dft_group(int B) {
+  const int g = 4096 / B & ~3;
+  return g < 4 ? 4 : (g > CB_ROWS ? CB_ROWS : g);
+}
 __global__ void __launch_bounds__(CB_NT)
     k_cube_dft(const float *__restrict__ cube, uint64_t rows, int B, float2 *__restrict__ R) {
   __shared__ float2 tw[CB_MAXB];
-  __shared__ float row[CB_MAXB];
+  extern __shared__ __align__(16) float row[];  // [rows of a group][B], zeros past the last row
   for (int m = threadIdx.x; m < B; m += blockDim.x) {
     float sn, cs;
     sincospif(-2.0f * (float)m / (float)B, &sn, &cs);
     tw[m] = make_float2(cs, sn);
   }
   const int K = B / 2;
+  const int group = cube_dft_group(B);
   const uint64_t r1 = min((uint64_t)(blockIdx.x + 1) * CB_ROWS, rows);
-  for (uint64_t r = (uint64_t)blockIdx.x * CB_ROWS; r < r1; ++r) {
+  for (uint64_t r = (uint64_t)blockIdx.x * CB_ROWS; r < r1; r += group) {
+    const int nr = (int)min((uint64_t)group, r1 - r);
     __syncthreads();
-    for (int b = threadIdx.x; b < B; b += blockDim.x) row[b] = cube[r * (uint64_t)B + b];
+    for (int i = threadIdx.x; i < group * B; i += blockDim.x)
+      row[i] = i < nr * B ? cube[r * (uint64_t)B + i] : 0.0f;
     __syncthreads();
-    for (int k = threadIdx.x + 1; k <= K; k += blockDim.x) {
-      float re = 0.0f, im = 0.0f;
+    for (int i = threadIdx.x; i < (nr + 3) / 4 * K; i += blockDim.x) {
+      const int g = i / K, k = i - g * K + 1;
+      const float *x = row + 4 * g * B;
+      float re[4], im[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) re[j] = im[j] = 0.0f;
       int m = 0;
+#pragma unroll 4
       for (int b = 0; b < B; ++b) {
         const float2 w = tw[m];
-        re += row[b] * w.x;
-        im += row[b] * w.y;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          re[j] += x[j * B + b] * w.x;
+          im[j] += x[j * B + b] * w.y;
+        }
         m += k;
         if (m >= B) m -= B;
       }
-      R[r * (uint64_t)K + (k - 1)] = make_float2(re, im);
+      for (int j = 0; j < min(4, nr - 4 * g); ++j)
+        R[(r + 4 * g + j) * (uint64_t)K + (k - 1)] = make_float2(re[j], im[j]);
     }
   }
 }
 
-// P[cand][k] for every candidate: CTA (chunk of rows, candidate); thread k
-// accumulates its harmonic over the chunk's rows, then one f64 atomic pair.
-__global__ void __launch_bounds__(CB_NT)
-    k_cube_harmonics(const float2 *__restrict__ R, uint64_t rows, int S, int B,
-                     const double *__restrict__ kc, double Tsub, double nu_r, double nudot_r,
-                     double dm_r, const CandDev *__restrict__ cands, int rows_per_cta,
+// P[cand][k]: CTA (256 rows, candidate).  The CTA first computes its rows'
+// shifts (the only f64 work: about 16 operations per row and candidate, the
+// reference's phase coming from k_cube_ref; the gradient reads them back
+// from dsh), then takes sub-blocks of rows: every thread turns (row, harmonic)
+// entries by their phase into shared memory, one thread per harmonic component
+// adds a sub-block in row order, and one f64 atomic per component ends the CTA.
+// Bound: issue, about 65 instructions per entry, most of them sincospif's.
+// With one thread per harmonic walking the 256 rows, and the phases of both
+// ends computed in f64 per row and candidate here and again in the gradient,
+// the 22 evaluations of a group of 16 (16,384 rows of 64 harmonics) took 0.77 ms
+// here and 0.95 in the gradient; 0.64 and 0.65 now.  Two candidates per CTA
+// read R half as often and issue a sixth less, but left the SMs at 27 warps:
+// 0.76 and 0.80.
+constexpr int CB_HROWS = CB_NT;  // rows per CTA
+constexpr int CB_HITEMS = 2048;  // (row, harmonic) entries of a sub-block
+__global__ void __launch_bounds__(CB_NT, 8)
+    k_cube_harmonics(const float2 *__restrict__ R, uint32_t rows, int S, int B,
+                     const double *__restrict__ kc, const double *__restrict__ ref, double Tsub,
+                     const __grid_constant__ CandBatch cands, float *__restrict__ dsh,
                      double *__restrict__ P) {
-  __shared__ float dsh[CB_NT];  // shift / B, reduced to [0, 1)
-  const int k = blockIdx.y;
-  const CandDev q = cands[k];
-  const int K = B / 2;
-  const uint64_t r0 = (uint64_t)blockIdx.x * rows_per_cta;
-  const int nr = (int)min((uint64_t)rows_per_cta, rows - r0);
-  if (threadIdx.x < nr) {
-    double tdq, kcc;
-    const double d = row_shift(q, nu_r, nudot_r, dm_r, Tsub, kc, S, B, r0 + threadIdx.x, tdq,
-                               kcc) / (double)B;
-    dsh[threadIdx.x] = (float)(d - floor(d));
+  __shared__ float d[CB_HROWS];  // shift / B, reduced to [0, 1)
+  __shared__ float2 z[CB_HITEMS];
+  constexpr int ACC = CB_MAXB / CB_NT;  // components per thread
+  const int tid = (int)threadIdx.x;
+  const int cand = (int)blockIdx.y;
+  const uint32_t K = (uint32_t)B / 2;
+  const uint32_t r0 = blockIdx.x * CB_HROWS;
+  const int nr = (int)min((uint32_t)CB_HROWS, rows - r0);
+  if (tid < nr) {
+    const uint32_t r = r0 + (uint32_t)tid;
+    const CandDev q = cands.c[cand];
+    const double tdq = row_time(r, S, Tsub) - kc[r / (uint32_t)S] * q.dm;
+    double x = q.nu * tdq + 0.5 * q.nudot * tdq * tdq - ref[r];
+    // shift in bins over B: the two roundings cancel at powers of two
+    if (B & (B - 1)) x = x * (double)B / (double)B;
+    const float f = (float)(x - floor(x));
+    d[tid] = f;
+    dsh[(uint64_t)cand * rows + r] = f;
   }
+  float acc[ACC];
+#pragma unroll
+  for (int j = 0; j < ACC; ++j) acc[j] = 0.0f;
+  const int RB = (int)min((uint32_t)CB_HITEMS / K, (uint32_t)CB_HROWS);
+  // idx / K = idx * inv >> 20 exactly for idx < 2048, 2 <= K <= 512
+  const uint32_t inv = ((1u << 20) + K - 1) / K;
+  const int comps = 2 * (int)K;
   __syncthreads();
-  for (int h = threadIdx.x + 1; h <= K; h += blockDim.x) {
-    float re = 0.0f, im = 0.0f;
-    for (int i = 0; i < nr; ++i) {
+  for (int i0 = 0; i0 < nr; i0 += RB) {
+    const int m = min(RB, nr - i0), items = m * (int)K;
+    const float2 *src = R + (uint64_t)(r0 + (uint32_t)i0) * K;
+#pragma unroll 1  // (unrolled four times: 0.71 ms)
+    for (int idx = tid; idx < items; idx += CB_NT) {
+      const int row = (int)((uint32_t)idx * inv >> 20);
+      const float h = (float)(idx - row * (int)K + 1);
+      const float2 v = src[idx];
       // e^(-2 pi i h d) with h d reduced mod 1 in f32
-      float x = (float)h * dsh[i];
-      x -= floorf(x);
+      const float x = frac_pos(h * d[i0 + row]);
       float sn, cs;
       sincospif(-2.0f * x, &sn, &cs);
-      const float2 v = R[(r0 + i) * (uint64_t)K + (h - 1)];
-      re += v.x * cs - v.y * sn;
-      im += v.x * sn + v.y * cs;
+      z[idx] = make_float2(v.x * cs - v.y * sn, v.x * sn + v.y * cs);
     }
-    atomicAdd(&P[((uint64_t)k * K + (h - 1)) * 2], (double)re);
-    atomicAdd(&P[((uint64_t)k * K + (h - 1)) * 2 + 1], (double)im);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ACC; ++j) {
+      const int t = tid + j * CB_NT;
+      if (t >= comps) break;
+      const float *p = reinterpret_cast<const float *>(z) + t;
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) acc[j] += p[(uint32_t)i * 2 * K];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < ACC; ++j) {
+    const int t = tid + j * CB_NT;
+    if (t >= comps) break;
+    atomicAdd(&P[(uint64_t)cand * 2 * K + t], (double)acc[j]);
   }
 }
 
-// Gradient: each warp takes 32 rows at a time; lane l computes row l's shift
-// (the only f64 work), then the warp walks the 32 rows with the lanes
-// splitting each row's harmonics.
+// A[cand][h - 1] = 2 w_h conj(P_h) / (B n v).
 __global__ void __launch_bounds__(CB_NT)
-    k_cube_grad(const float2 *__restrict__ R, uint64_t rows, int S, int B,
-                const double *__restrict__ kc, double Tsub, double nu_r, double nudot_r,
-                double dm_r, const CandDev *__restrict__ cands, const float2 *__restrict__ A,
+    k_cube_coefficients(const double *__restrict__ P, int K, int entries, double norm,
+                        float2 *__restrict__ A) {
+  const int i = (int)(blockIdx.x * CB_NT + threadIdx.x);
+  if (i >= entries) return;
+  const double wk = i % K + 1 < K ? 2.0 : 1.0;
+  A[i] = make_float2((float)(2.0 * wk * P[2 * i] / norm), (float)(-2.0 * wk * P[2 * i + 1] / norm));
+}
+
+// Gradient: a warp takes 32 rows of a candidate; the lanes split each row's
+// harmonics, then lane l adds row l's 32 partial sums (as the tree over lane
+// distances 16, 8, 4, 2, 1) and does its f64 terms.
+constexpr int CB_GNT = 128;
+__global__ void __launch_bounds__(CB_GNT)
+    k_cube_grad(const float2 *__restrict__ R, uint32_t rows, int S, int B,
+                const double *__restrict__ kc, double Tsub, const float *__restrict__ dsh,
+                const __grid_constant__ CandBatch cands, const float2 *__restrict__ A,
                 double *__restrict__ grad) {
-  __shared__ double red[3][CB_NT / 32];
-  const int k = blockIdx.y;
-  const CandDev q = cands[k];
+  __shared__ float part[CB_GNT / 32][32][33];
+  __shared__ double red[3][CB_GNT / 32];
+  const int cand = (int)blockIdx.y;
   const int K = B / 2;
-  const float2 *Ak = A + (uint64_t)k * K;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t nwarps = (uint64_t)gridDim.x * (CB_NT / 32);
+  const float2 *Ak = A + (uint64_t)cand * K;
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
   const float twopi_b = 6.283185307179586f / (float)B;
+  const uint32_t r0 = (blockIdx.x * (CB_GNT / 32) + warp) * 32;
+  const int nr = r0 < rows ? (int)min(32u, rows - r0) : 0;
+  const float dl = lane < nr ? dsh[(uint64_t)cand * rows + r0 + lane] : 0.0f;
+#pragma unroll 2
+  for (int i = 0; i < nr; ++i) {
+    const float2 *Rr = R + (uint64_t)(r0 + i) * K;
+    const float d = __shfl_sync(0xffffffffu, dl, i);
+    float g = 0.0f;
+    for (int h = lane + 1; h <= K; h += 32) {
+      const float2 v = Rr[h - 1];
+      const float x = frac_pos((float)h * d);
+      float sn, cs;
+      sincospif(-2.0f * x, &sn, &cs);
+      // z = R e^(-2 pi i h d) (-2 pi i h / B); contribution Re(A_h z)
+      const float zr = v.x * cs - v.y * sn, zi = v.x * sn + v.y * cs;
+      const float f = twopi_b * (float)h;
+      const float2 a = Ak[h - 1];
+      g += a.x * (zi * f) - a.y * (-zr * f);
+    }
+    part[warp][i][lane] = g;
+  }
+  __syncwarp();
   double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-  for (uint64_t r0 = ((uint64_t)blockIdx.x * (CB_NT / 32) + warp) * 32; r0 < rows;
-       r0 += nwarps * 32) {
-    const uint64_t rl = r0 + lane;
-    double tdq = 0.0, kcc = 0.0;
-    float dl = 0.0f;
-    if (rl < rows) {
-      const double dd = row_shift(q, nu_r, nudot_r, dm_r, Tsub, kc, S, B, rl, tdq, kcc) /
-                        (double)B;
-      dl = (float)(dd - floor(dd));
-    }
-    float gl = 0.0f;  // this lane's row's dJ/dd, assembled below
-    const int nr = (int)min((uint64_t)32, rows - r0);
-    for (int i = 0; i < nr; ++i) {
-      const float d = __shfl_sync(0xffffffffu, dl, i);
-      const float2 *Rr = R + (r0 + i) * (uint64_t)K;
-      float g = 0.0f;
-      for (int h = lane + 1; h <= K; h += 32) {
-        float x = (float)h * d;
-        x -= floorf(x);
-        float sn, cs;
-        sincospif(-2.0f * x, &sn, &cs);
-        const float2 v = Rr[h - 1];
-        // z = R e^(-2 pi i h d) (-2 pi i h / B); contribution Re(A_h z)
-        const float zr = v.x * cs - v.y * sn, zi = v.x * sn + v.y * cs;
-        const float f = twopi_b * (float)h;
-        const float2 a = Ak[h - 1];
-        g += a.x * (zi * f) - a.y * (-zr * f);
-      }
-      for (int o = 16; o; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-      if (lane == i) gl = g;
-    }
-    if (rl < rows) {
-      const double Bd = (double)B, gg = (double)gl;
-      a0 += gg * Bd * tdq;
-      a1 += gg * Bd * 0.5 * tdq * tdq;
-      a2 += gg * (-Bd * (q.nu + q.nudot * tdq) * kcc);
-    }
+  if (lane < nr) {
+    const float *p = part[warp][lane];
+    float t[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) t[j] = p[j] + p[j + 16];
+#pragma unroll
+    for (int o = 8; o; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < o; ++j) t[j] = t[j] + t[j + o];
+    const uint32_t r = r0 + (uint32_t)lane;
+    const CandDev q = cands.c[cand];
+    const double kcc = kc[r / (uint32_t)S], tdq = row_time(r, S, Tsub) - kcc * q.dm;
+    const double Bd = (double)B, gg = (double)t[0];
+    a0 = gg * Bd * tdq;
+    a1 = gg * Bd * 0.5 * tdq * tdq;
+    a2 = gg * (-Bd * (q.nu + q.nudot * tdq) * kcc);
   }
   for (int o = 16; o; o >>= 1) {
     a0 += __shfl_xor_sync(0xffffffffu, a0, o);
@@ -852,11 +1062,10 @@ __global__ void __launch_bounds__(CB_NT)
   __syncthreads();
   if (threadIdx.x < 3) {
     double x = 0.0;
-    for (int w = 0; w < CB_NT / 32; ++w) x += red[threadIdx.x][w];
-    atomicAdd(&grad[(uint64_t)k * 3 + threadIdx.x], x);
+    for (int w = 0; w < CB_GNT / 32; ++w) x += red[threadIdx.x][w];
+    atomicAdd(&grad[(uint64_t)cand * 3 + threadIdx.x], x);
   }
 }
-
 
 // v = sum over channels of each channel's sample variance (the variance of a
 // sum of independent channels), from the per-(channel, subint) sums.
@@ -867,6 +1076,7 @@ __global__ void __launch_bounds__(CB_NT)
   double v = 0.0;
   for (uint64_t c = threadIdx.x; c < nch; c += CB_NT) {
     double s1 = 0.0, s2 = 0.0;
+#pragma unroll 8
     for (int s = 0; s < S; ++s) {
       s1 += chsum[(c * S + s) * 2];
       s2 += chsum[(c * S + s) * 2 + 1];
@@ -903,27 +1113,34 @@ int build_cube(const DeviceObs &o, uint64_t n, int S, int B, double nu, double n
   PSR_CUDA(cudaMemcpyAsync(w.tau.p, tau.data(), nch * 8, cudaMemcpyHostToDevice, st));
   PSR_CUDA(cudaMemcpyAsync(w.kc.p, kc.data(), nch * 8, cudaMemcpyHostToDevice, st));
   dim3 grid((unsigned)S, (unsigned)nch);
+  PSR_TRY(w.anchors.ensure(w.rows * 5 * 8));
+  unsigned long long *ap = w.anchors.as<unsigned long long>();
   const double *tp = w.tau.as<double>();
   float *cp = w.cube.as<float>();
   double *sp = w.chsum.as<double>();
   switch (o.kind) {
     case SAMPLE_U8:
       PSR_TRY(launch_cube_fold(grid, B, st, o.samples.as<uint8_t>(), o.ld, n, S, o.h.tsamp, nu,
-                               nudot, tp, cp, sp));
+                               nudot, tp, ap, cp, sp));
       break;
     case SAMPLE_U16:
       PSR_TRY(launch_cube_fold(grid, B, st, o.samples.as<uint16_t>(), o.ld, n, S, o.h.tsamp, nu,
-                               nudot, tp, cp, sp));
+                               nudot, tp, ap, cp, sp));
       break;
     default:
       PSR_TRY(launch_cube_fold(grid, B, st, o.samples.as<float>(), o.ld, n, S, o.h.tsamp, nu,
-                               nudot, tp, cp, sp));
+                               nudot, tp, ap, cp, sp));
   }
   PSR_CUDA(cudaGetLastError());
   PSR_TRY(w.R.ensure(w.rows * (uint64_t)(B / 2) * sizeof(float2)));
-  k_cube_dft<<<(unsigned)((w.rows + CB_ROWS - 1) / CB_ROWS), CB_NT, 0, st>>>(
+  k_cube_dft<<<(unsigned)((w.rows + CB_ROWS - 1) / CB_ROWS), CB_NT,
+               (size_t)cube_dft_group(B) * B * 4, st>>>(
       w.cube.as<float>(), w.rows, B, w.R.as<float2>());
   PSR_CUDA(cudaGetLastError());
+  const double Tsub = (double)n * o.h.tsamp / (double)S;
+  PSR_TRY(w.ref.ensure(w.rows * 8));
+  k_cube_ref<<<(unsigned)((w.rows + CB_NT - 1) / CB_NT), CB_NT, 0, st>>>(
+      (uint32_t)w.rows, S, w.kc.as<double>(), Tsub, nu, nudot, dm, w.ref.as<double>());
   PSR_TRY(w.prof.ensure(16));
   k_cube_var<<<1, CB_NT, 0, st>>>(w.chsum.as<double>(), nch, S, n, w.prof.as<double>());
   PSR_CUDA(cudaGetLastError());
@@ -934,54 +1151,50 @@ int build_cube(const DeviceObs &o, uint64_t n, int S, int B, double nu, double n
   return PSR_OK;
 }
 
-// J and gradient (in nu, nudot, DM) of every candidate.
-int eval_cube(const DeviceObs &o, uint64_t n, int S, int B, double nu_r, double nudot_r,
-              double dm_r, const std::vector<CandDev> &cand, CubeWork &w, std::vector<double> &J,
-              std::vector<double> &grad, cudaStream_t st) {
-  const int K = (int)cand.size();
+// J and gradient (in nu, nudot, DM) of every candidate, relative to the
+// reference that the cube was built at.  P and the gradients come back in one
+// copy.
+int eval_cube(const DeviceObs &o, uint64_t n, int S, int B, const std::vector<CandDev> &cand,
+              CubeWork &w, std::vector<double> &J, std::vector<double> &grad, cudaStream_t st) {
+  const size_t K = cand.size();
   const int H = B / 2;
   const double Tsub = (double)n * o.h.tsamp / (double)S;
-  PSR_TRY(w.cands.ensure(K * sizeof(CandDev)));
-  PSR_TRY(w.prof.ensure((size_t)K * H * 2 * 8));
-  PSR_TRY(w.g.ensure((size_t)K * H * sizeof(float2)));
-  PSR_TRY(w.grad.ensure((size_t)K * 3 * 8));
-  PSR_CUDA(cudaMemcpyAsync(w.cands.p, cand.data(), K * sizeof(CandDev), cudaMemcpyHostToDevice,
-                           st));
-  PSR_CUDA(cudaMemsetAsync(w.prof.p, 0, (size_t)K * H * 2 * 8, st));
-  PSR_CUDA(cudaMemsetAsync(w.grad.p, 0, (size_t)K * 3 * 8, st));
-  const int rows_per_cta = CB_NT;
-  dim3 gp((unsigned)((w.rows + rows_per_cta - 1) / rows_per_cta), (unsigned)K);
-  k_cube_harmonics<<<gp, CB_NT, 0, st>>>(w.R.as<float2>(), w.rows, S, B, w.kc.as<double>(), Tsub,
-                                         nu_r, nudot_r, dm_r, w.cands.as<CandDev>(),
-                                         rows_per_cta, w.prof.as<double>());
-  PSR_CUDA(cudaGetLastError());
-  std::vector<double> P((size_t)K * H * 2);
-  PSR_CUDA(cudaMemcpyAsync(P.data(), w.prof.p, P.size() * 8, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaStreamSynchronize(st));
+  const uint32_t rows = (uint32_t)w.rows;
+  const size_t np = K * H * 2, nout = np + K * 3;
   const double norm = (double)B * (double)n * w.var;
-  std::vector<float2> A((size_t)K * H);
+  PSR_TRY(w.prof.ensure(nout * 8));
+  PSR_TRY(w.g.ensure(std::min<size_t>(K, CB_CANDS) * H * sizeof(float2)));
+  PSR_TRY(w.dsh.ensure(std::min<size_t>(K, CB_CANDS) * w.rows * 4));
+  PSR_CUDA(cudaMemsetAsync(w.prof.p, 0, nout * 8, st));
+  for (size_t c0 = 0; c0 < K; c0 += CB_CANDS) {
+    const int nc = (int)std::min<size_t>(CB_CANDS, K - c0);
+    CandBatch cb{};
+    std::copy_n(cand.begin() + c0, nc, cb.c);
+    double *P = w.prof.as<double>() + c0 * H * 2;
+    const unsigned gy = (unsigned)nc;
+    k_cube_harmonics<<<dim3((rows + CB_HROWS - 1) / CB_HROWS, gy), CB_NT, 0, st>>>(
+        w.R.as<float2>(), rows, S, B, w.kc.as<double>(), w.ref.as<double>(), Tsub, cb,
+        w.dsh.as<float>(), P);
+    k_cube_coefficients<<<(unsigned)((nc * H + CB_NT - 1) / CB_NT), CB_NT, 0, st>>>(
+        P, H, nc * H, norm, w.g.as<float2>());
+    k_cube_grad<<<dim3((rows + CB_GNT - 1) / CB_GNT, gy), CB_GNT, 0, st>>>(
+        w.R.as<float2>(), rows, S, B, w.kc.as<double>(), Tsub, w.dsh.as<float>(), cb,
+        w.g.as<float2>(), w.prof.as<double>() + np + c0 * 3);
+    PSR_CUDA(cudaGetLastError());
+  }
+  std::vector<double> out(nout);
+  PSR_CUDA(cudaMemcpyAsync(out.data(), w.prof.p, nout * 8, cudaMemcpyDeviceToHost, st));
+  PSR_CUDA(cudaStreamSynchronize(st));
   J.assign(K, 0.0);
-  for (int k = 0; k < K; ++k) {
+  for (size_t k = 0; k < K; ++k) {
     double j = 0.0;
     for (int h = 1; h <= H; ++h) {
-      const double re = P[((size_t)k * H + h - 1) * 2], im = P[((size_t)k * H + h - 1) * 2 + 1];
-      const double wk = h < H ? 2.0 : 1.0;
-      j += wk * (re * re + im * im);
-      A[(size_t)k * H + h - 1] = make_float2((float)(2.0 * wk * re / norm),
-                                             (float)(-2.0 * wk * im / norm));
+      const double re = out[(k * H + h - 1) * 2], im = out[(k * H + h - 1) * 2 + 1];
+      j += (h < H ? 2.0 : 1.0) * (re * re + im * im);
     }
     J[k] = j / norm;
   }
-  PSR_CUDA(cudaMemcpyAsync(w.g.p, A.data(), A.size() * sizeof(float2), cudaMemcpyHostToDevice,
-                           st));
-  dim3 gg((unsigned)std::min<uint64_t>((w.rows + 255) / 256, 1024), (unsigned)K);
-  k_cube_grad<<<gg, CB_NT, 0, st>>>(w.R.as<float2>(), w.rows, S, B, w.kc.as<double>(), Tsub,
-                                    nu_r, nudot_r, dm_r, w.cands.as<CandDev>(),
-                                    w.g.as<float2>(), w.grad.as<double>());
-  PSR_CUDA(cudaGetLastError());
-  grad.resize((size_t)K * 3);
-  PSR_CUDA(cudaMemcpyAsync(grad.data(), w.grad.p, grad.size() * 8, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaStreamSynchronize(st));
+  grad.assign(out.begin() + np, out.end());
   return PSR_OK;
 }
 
@@ -1030,7 +1243,7 @@ int cube_objective(const DeviceObs &o, uint64_t n, const psr_timing &ref, const 
     cand[k].dm = theta[k].dm;
   }
   std::vector<double> J, grad;
-  PSR_TRY(eval_cube(o, n, S, B, nu_r, nudot_r, ref.dm, cand, w, J, grad, st));
+  PSR_TRY(eval_cube(o, n, S, B, cand, w, J, grad, st));
   for (uint64_t k = 0; k < K; ++k) {
     Jout[k] = J[k];
     if (gout) {
@@ -1107,7 +1320,7 @@ int refine_cube_group(const DeviceObs &o, uint64_t n, const psr_timing *start, u
       who.push_back(k);
     }
     if (batch.empty()) break;
-    PSR_TRY(eval_cube(o, n, S, B, nu_r, nudot_r, dm_r, batch, w, J, grad, st));
+    PSR_TRY(eval_cube(o, n, S, B, batch, w, J, grad, st));
     for (size_t i = 0; i < who.size(); ++i) {
       Opt &s = st8[who[i]];
       ++s.evals;
