@@ -363,8 +363,8 @@ __device__ float pc_sequential_sum(const T *row, uint64_t ns, float *buf, Term t
 //               taken apart into its lanes' 16 terms (maps again at the true
 //               binade, the lane that crosses term by term)
 // and the last two again for the variance, whose binades follow from the mean
-// and the plain sums.  Subnormal, infinite and NaN terms make a run special:
-// it is added term by term.
+// and the plain sums.  An infinite or NaN term makes a run special: it is added
+// term by term.
 constexpr int ES_L = 512;          // terms per chunk, 16 per lane
 constexpr int ES_PER = ES_L / 32;
 constexpr uint32_t ES_SPECIAL = 0xffffffffu;
@@ -386,34 +386,36 @@ struct EsRaw {
     return (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
   }
   __device__ __forceinline__ float at(int j) const {
-    if constexpr (sizeof(T) == 1) return (float)((word(j >> 2) >> (8 * (j & 3))) & 255u);
-    else if constexpr (sizeof(T) == 2) return (float)((word(j >> 1) >> (16 * (j & 1))) & 65535u);
+    // integers exactly: 2^23 + v assembled by a byte permute, less 2^23
+    if constexpr (sizeof(T) == 1)
+      return __uint_as_float(__byte_perm(word(j >> 2), 0x4B000000u, 0x7540u | (j & 3))) -
+             8388608.0f;
+    else if constexpr (sizeof(T) == 2)
+      return __uint_as_float(
+                 __byte_perm(word(j >> 1), 0x4B000000u, (j & 1) ? 0x7532u : 0x7510u)) -
+             8388608.0f;
     else return __uint_as_float(word(j));
   }
 };
 
-// The map (d0, d1) of N terms at the binade with biased exponent be; true if
-// the run is special or its increment reaches 2^24 (it leaves the binade).
+// The map (d0, d1) of N terms >= 0 at the binade with biased exponent be (1 to
+// 254); true if the run does not fit it (it adds 2^23 units or more, or a term
+// is infinite or NaN).  The f32 unit makes the map: two running sums, from
+// the binade's first value (K = 2^23, even) and its second (odd), see the
+// roundings of any even and odd K as long as they stay in the binade.
 template <int N>
 __device__ __forceinline__ bool es_run(const float (&t)[N], int be, uint32_t &d0, uint32_t &d1) {
-  bool special = false;
-  d0 = d1 = 0;
+  const uint32_t k0 = (uint32_t)be << 23;
+  float s0 = __uint_as_float(k0), s1 = __uint_as_float(k0 + 1);
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    const uint32_t b = __float_as_uint(t[j]) & 0x7fffffffu;
-    const int bt = (int)(b >> 23);
-    special |= bt == 255 || (bt == 0 && b != 0) || bt > be;
-    const uint32_t mt = bt ? (b & 0x7fffffu) | 0x800000u : 0u;
-    const int r = min(max(be - bt, 0), 25);  // t / u = mt 2^-r; below half a unit past 24
-    const uint32_t q = mt >> r, frac = __funnelshift_r(0u, mt, r);
-    const uint32_t inc = q + (frac > 0x80000000u ? 1u : 0u);
-    const uint32_t tie = frac == 0x80000000u ? 1u : 0u;
-    d0 += inc;
-    d0 += d0 & tie;
-    d1 += inc;
-    d1 += ~d1 & tie;
+    s0 = __fadd_rn(s0, t[j]);
+    s1 = __fadd_rn(s1, t[j]);
   }
-  return special || d0 >= (1u << 24) || d1 >= (1u << 24);
+  const uint32_t b0 = __float_as_uint(s0), b1 = __float_as_uint(s1);
+  d0 = b0 - k0;
+  d1 = b1 - k0 - 1;
+  return (int)(b0 >> 23) != be || (int)(b1 >> 23) != be;
 }
 
 // Inclusive scan of the lanes' maps.
@@ -647,10 +649,12 @@ __device__ __forceinline__ float es_term(float x, float m) {
 }
 
 // The map of every chunk at its guessed binade.
-// Bound: issue, about 30 instructions per sample.
+// Bound: issue, about 8 instructions per sample, twice the time of the bytes.
 // Measured on a GB300 (512 8-bit channels of 1,047,799 samples, means above
-// 2^24): the six kernels 2.3 ms, 0.88 of them in each pass of k_es_maps; one
-// CTA per channel that walked its chunks in order took 6.4 with its totals.
+// 2^24): the six kernels 0.59 ms, 0.20 and 0.17 of them in the two passes of
+// k_es_maps (0.88 each with the increments computed in integers, bound by the
+// half-rate pipe); one CTA per channel that walked its chunks in order took 6.4
+// with its totals.
 template <class T, bool VAR>
 __global__ void __launch_bounds__(EK_NT)
     k_es_maps(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t nck,
@@ -662,6 +666,7 @@ __global__ void __launch_bounds__(EK_NT)
   const T *row = s + c * ld;
   const float m = VAR ? means[c] : 0.0f;
   const uint64_t k0 = ((uint64_t)blockIdx.x * (EK_NT / 32) + (threadIdx.x >> 5)) * EK_CPW;
+  const uint64_t whole = ns / ES_L;  // chunks of 512 terms
   EsRaw<T> nx;
   {
     const uint64_t p = k0 * ES_L + (uint64_t)lane * ES_PER;
@@ -678,7 +683,13 @@ __global__ void __launch_bounds__(EK_NT)
     if (be) {
       float t[ES_PER];
 #pragma unroll
-      for (int j = 0; j < ES_PER; ++j) t[j] = p + j < ns ? es_term<VAR>(x.at(j), m) : 0.0f;
+      for (int j = 0; j < ES_PER; ++j) t[j] = es_term<VAR>(x.at(j), m);
+      if (k >= whole) {
+        const int left = p < ns ? (int)min((uint64_t)ES_PER, ns - p) : 0;
+#pragma unroll
+        for (int j = 0; j < ES_PER; ++j)
+          if (j >= left) t[j] = 0.0f;
+      }
       uint32_t d0, d1;
       const bool bad = es_run(t, be, d0, d1);
       if (!__any_sync(0xffffffffu, bad)) {
