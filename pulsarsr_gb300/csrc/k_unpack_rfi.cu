@@ -342,19 +342,36 @@ __global__ void __launch_bounds__(MH_NT)
 }
 
 // Element of rank ns / 2 from each row's histogram (one thread per row).
-__global__ void k_hist_median(const unsigned *__restrict__ hist, uint64_t nch, uint64_t ns,
-                              float *__restrict__ med) {
-  const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per channel: 8 bins per lane, a prefix over the lanes.
+__global__ void __launch_bounds__(128)
+    k_hist_median(const unsigned *__restrict__ hist, uint64_t nch, uint64_t ns,
+                  float *__restrict__ med) {
+  const uint64_t c = (uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (c >= nch) return;
-  const uint64_t r = ns / 2;
-  uint64_t cum = 0;
-  int d = 255;
-  for (int k = 0; k < 256; ++k) {
-    cum += hist[c * 256 + k];
-    if (cum > r) {
-      d = k;
-      break;
-    }
+  const int lane = (int)(threadIdx.x & 31);
+  const unsigned long long r = ns / 2;
+  unsigned h[8];
+  unsigned long long t = 0;
+  const uint4 *q = reinterpret_cast<const uint4 *>(hist + c * 256 + 8 * lane);
+  *reinterpret_cast<uint4 *>(h) = q[0];
+  *reinterpret_cast<uint4 *>(h + 4) = q[1];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) t += h[k];
+  unsigned long long cum = t;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, cum, o);
+    if (lane >= o) cum += v;
+  }
+  const unsigned past = __ballot_sync(0xffffffffu, cum > r);
+  if (lane != (past ? __ffs((int)past) - 1 : 31)) return;
+  cum -= t;
+  int d = 8 * lane + 7;
+#pragma unroll
+  for (int k = 7; k >= 0; --k) {
+    unsigned long long upto = cum;
+    for (int j = 0; j <= k; ++j) upto += h[j];
+    if (upto > r) d = 8 * lane + k;
   }
   med[c] = (float)d;
 }
@@ -918,55 +935,111 @@ __global__ void __launch_bounds__(256)
   if (lane == 0) bsum[id] = (float)acc;
 }
 
-// The element of rank r among n <= 32 N keys key(i), by one warp: the largest
-// value with at most r keys below it, bit by bit, N keys per lane in registers
-// and one warp reduction per bit.  A radix selection's four rounds over 32
-// histograms took about 13 us in a 1024-thread block whatever n is; the channel
-// and block decisions of 32 channels and 164 blocks went from 57 and 25 us to
-// under 10 each, those of 512 channels from 80 to 35.
-template <int N, class KeyFn>
-__device__ uint32_t warp_rank(KeyFn key, int n, int r, int lane) {
-  uint32_t k[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) k[i] = 32 * i + lane < n ? key(32 * i + lane) : 0xffffffffu;
-  uint32_t p = 0;
-  for (int bit = 31; bit >= 0; --bit) {
-    const uint32_t cand = p | (1u << bit);
-    unsigned below = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) below += k[i] < cand ? 1u : 0u;
-    if ((int)__reduce_add_sync(0xffffffffu, below) <= r) p = cand;
-  }
-  return p;
-}
-constexpr int RANK_MAX = 2048;  // 64 keys per lane
-// The same for the block: warp 0 selects, every thread returns the key.
-template <class KeyFn>
-__device__ uint32_t block_rank(KeyFn key, int n, int r, uint32_t *bc) {
-  const int lane = (int)threadIdx.x;
-  if (lane < 32) {
-    const uint32_t k = n <= 256    ? warp_rank<8>(key, n, r, lane)
-                       : n <= 1024 ? warp_rank<32>(key, n, r, lane)
-                                   : warp_rank<RANK_MAX / 32>(key, n, r, lane);
-    if (lane == 0) bc[0] = k;
-  }
-  __syncthreads();
-  const uint32_t k = bc[0];
-  __syncthreads();
-  return k;
+// Counters of NW warps that select together.
+struct RankShared {
+  uint32_t lo, hi;
+  unsigned below[32];
+};
+template <int NW>
+__device__ __forceinline__ void rank_sync() {
+  if constexpr (NW > 1) __syncthreads();
+  else __syncwarp();
 }
 
-// rfi::outliers (rfi/src/lib.rs:13-22) for one vector, inside one block; hist
-// holds 32 x 256 words.
+// The element of rank r among n keys, key 32 NW i + tid in k[i] of the group's
+// thread tid (padded with 0xffffffff, above all others): the largest value with at
+// most r keys below it, bit by bit below the bits that all keys share, one warp
+// reduction (and, for a group of warps, one barrier) per bit.
+template <int N, int NW>
+__device__ uint32_t group_rank(const uint32_t (&k)[N], int n, int r, int tid, RankShared &sh) {
+  uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (32 * NW * i + tid < n) {
+      lo = min(lo, k[i]);
+      hi = max(hi, k[i]);
+    }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if constexpr (NW > 1) {
+    if (tid < 32) sh.below[tid] = 0;
+    if (tid == 0) {
+      sh.lo = 0xffffffffu;
+      sh.hi = 0;
+    }
+    __syncthreads();
+    if ((tid & 31) == 0) {
+      atomicMin(&sh.lo, lo);
+      atomicMax(&sh.hi, hi);
+    }
+    __syncthreads();
+    lo = sh.lo;
+    hi = sh.hi;
+  }
+  uint32_t p = lo;
+  if (lo != hi) {
+    const int top = 31 - __clz((int)(lo ^ hi));  // highest bit in which keys differ
+    p = top == 31 ? 0u : lo >> (top + 1) << (top + 1);
+    for (int bit = top; bit >= 0; --bit) {
+      const uint32_t cand = p | (1u << bit);
+      unsigned b0 = 0, b1 = 0;
+#pragma unroll
+      for (int i = 0; i < N; i += 2) {
+        b0 += k[i] < cand ? 1u : 0u;
+        if (i + 1 < N) b1 += k[i + 1] < cand ? 1u : 0u;
+      }
+      unsigned below = __reduce_add_sync(0xffffffffu, b0 + b1);
+      if constexpr (NW > 1) {
+        if ((tid & 31) == 0) atomicAdd(&sh.below[bit], below);
+        __syncthreads();
+        below = sh.below[bit];
+      }
+      if ((int)below <= r) p = cand;
+    }
+  }
+  rank_sync<NW>();
+  return p;
+}
+
+// rfi::outliers (rfi/src/lib.rs:13-22) for n <= 32 NW N values by NW warps, the
+// keys in registers through both selections.  A radix selection's four rounds
+// over 32 histograms took about 13 us in a 1024-thread block whatever n is; the
+// channel and block decisions of 512 channels and 1048 blocks took 35 and 21 us
+// with two selections by one warp of a block and scratch in between, 13 and 9 now.
+template <int N, int NW>
+__device__ void group_outliers(const float *v, int n, float threshold, unsigned char *flags,
+                               int tid, RankShared &sh) {
+  uint32_t k[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int j = 32 * NW * i + tid;
+    k[i] = j < n ? fkey(v[j]) : 0xffffffffu;
+  }
+  const float center = n > 0 ? fkey_inv(group_rank<N, NW>(k, n, n / 2, tid, sh)) : 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (32 * NW * i + tid < n) k[i] = fkey(fabsf(__fsub_rn(fkey_inv(k[i]), center)));
+  const float mad = n > 0 ? fkey_inv(group_rank<N, NW>(k, n, n / 2, tid, sh)) : 0.0f;
+  const float scale =
+      fmaxf(fmaxf(__fmul_rn(1.4826f, mad), __fmul_rn(fabsf(center), 1e-4f)), 1e-6f);
+  const float lim = __fmul_rn(threshold, scale);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int j = 32 * NW * i + tid;
+    if (j < n) flags[j] = fkey_inv(k[i]) > lim ? 1 : 0;
+  }
+}
+constexpr int CH_RANK_MAX = 1024;   // channels: a warp per vector
+constexpr int BL_RANK_MAX = 2048, BL_NW = 4;  // blocks: four warps
+
+// The same for any n, by one block; hist holds 32 x 256 words.
 __device__ void block_outliers(const float *v, uint64_t n, float threshold,
                                float *dev_scratch, unsigned char *flags,
                                unsigned *hist, uint32_t *bc) {
-  const bool counted = n <= RANK_MAX;
   float center = 0.0f;
   if (n > 0) {
     auto key = [&](uint64_t i) { return fkey(v[i]); };
-    center = fkey_inv(counted ? block_rank(key, (int)n, (int)(n / 2), bc)
-                              : block_select(key, n, n / 2, 24, hist, bc));
+    center = fkey_inv(block_select(key, n, n / 2, 24, hist, bc));
   }
   for (uint64_t i = threadIdx.x; i < n; i += blockDim.x)
     dev_scratch[i] = fabsf(__fsub_rn(v[i], center));
@@ -974,8 +1047,7 @@ __device__ void block_outliers(const float *v, uint64_t n, float threshold,
   float mad = 0.0f;
   if (n > 0) {
     auto key = [&](uint64_t i) { return fkey(dev_scratch[i]); };
-    mad = fkey_inv(counted ? block_rank(key, (int)n, (int)(n / 2), bc)
-                           : block_select(key, n, n / 2, 24, hist, bc));
+    mad = fkey_inv(block_select(key, n, n / 2, 24, hist, bc));
   }
   float scale = fmaxf(fmaxf(__fmul_rn(1.4826f, mad), __fmul_rn(fabsf(center), 1e-4f)), 1e-6f);
   float lim = __fmul_rn(threshold, scale);
@@ -992,8 +1064,21 @@ __global__ void __launch_bounds__(DEC_NT) k_channel_decide(const float *means, c
                                  unsigned long long *active) {
   __shared__ unsigned hist[32 * 256];
   __shared__ uint32_t bc[3];
-  block_outliers(means, nch, threshold, scratch, f1, hist, bc);
-  block_outliers(vars, nch, threshold, scratch, f2, hist, bc);
+  if (nch <= CH_RANK_MAX) {
+    __shared__ RankShared sh;  // (not used by one warp)
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+    if (warp < 2) {
+      const float *v = warp ? vars : means;
+      unsigned char *f = warp ? f2 : f1;
+      if (nch <= 256) group_outliers<8, 1>(v, (int)nch, threshold, f, lane, sh);
+      else if (nch <= 512) group_outliers<16, 1>(v, (int)nch, threshold, f, lane, sh);
+      else group_outliers<CH_RANK_MAX / 32, 1>(v, (int)nch, threshold, f, lane, sh);
+    }
+    __syncthreads();
+  } else {
+    block_outliers(means, nch, threshold, scratch, f1, hist, bc);
+    block_outliers(vars, nch, threshold, scratch, f2, hist, bc);
+  }
   __shared__ unsigned good;
   if (threadIdx.x == 0) good = 0;
   __syncthreads();
@@ -1007,37 +1092,43 @@ __global__ void __launch_bounds__(DEC_NT) k_channel_decide(const float *means, c
 }
 
 // Block means over good channels in channel order (rfi/src/lib.rs:55-69): a CTA
-// takes 32 blocks; its warps load tiles of 64 channels (double buffered) and
-// warp 0 adds them in order, so the chain is one FADD per channel (one thread
-// per block that loads as it adds took 130 us at 512 channels).
-constexpr int BM_NT = 256, BM_C = 64;
+// takes 32 blocks; its other warps load tiles of 64 channels (double buffered,
+// masked channels as zeros, which change no sum) while warp 0 adds in order,
+// so the chain is one FADD per channel (one thread per block that loads as it
+// adds took 130 us at 512 channels, with warp 0 loading too and a test per
+// channel 38, 17 now).
+constexpr int BM_L = 8, BM_C = 64;  // loading warps, channels of a tile
+constexpr int BM_NT = 32 * (1 + BM_L);
 __global__ void __launch_bounds__(BM_NT)
     k_block_means(const float *bsum, const unsigned char *chbad, uint64_t nch, uint64_t ns,
                   uint64_t bs, uint64_t blocks_n, const unsigned long long *active,
                   float *bmeans) {
   __shared__ float tile[2][BM_C][32];
-  __shared__ unsigned char bad[2][BM_C];
   const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
   const uint64_t b = (uint64_t)blockIdx.x * 32 + lane;
-  auto load = [&](uint64_t c0, int k) {
+  auto load = [&](uint64_t c0, int k) {  // warps 1 and up
+    constexpr int R = BM_C / BM_L;
+    float v[R];
+    bool use[R];
 #pragma unroll
-    for (int i = 0; i < BM_C / (BM_NT / 32); ++i) {
-      const int r = warp * (BM_C / (BM_NT / 32)) + i;
-      const uint64_t c = c0 + r;
-      tile[k][r][lane] = c < nch && b < blocks_n ? bsum[c * blocks_n + b] : 0.0f;
-      if (lane == 0) bad[k][r] = c < nch ? chbad[c] : 1;
+    for (int i = 0; i < R; ++i) {
+      const uint64_t c = c0 + (warp - 1) * R + i;
+      use[i] = c < nch && !chbad[c];
+      v[i] = c < nch && b < blocks_n ? bsum[c * blocks_n + b] : 0.0f;
     }
+#pragma unroll
+    for (int i = 0; i < R; ++i) tile[k][(warp - 1) * R + i][lane] = use[i] ? v[i] : 0.0f;
   };
-  load(0, 0);
+  if (warp) load(0, 0);
   __syncthreads();
   float sum = 0.0f;
   int k = 0;
   for (uint64_t c0 = 0; c0 < nch; c0 += BM_C, k ^= 1) {
-    if (c0 + BM_C < nch) load(c0 + BM_C, k ^ 1);
-    if (warp == 0) {
-#pragma unroll 16
-      for (int r = 0; r < BM_C; ++r)
-        if (!bad[k][r]) sum = __fadd_rn(sum, tile[k][r][lane]);
+    if (warp) {
+      if (c0 + BM_C < nch) load(c0 + BM_C, k ^ 1);
+    } else {
+#pragma unroll
+      for (int r = 0; r < BM_C; ++r) sum = __fadd_rn(sum, tile[k][r][lane]);
     }
     __syncthreads();
   }
@@ -1048,20 +1139,35 @@ __global__ void __launch_bounds__(BM_NT)
   bmeans[b] = __fdiv_rn(sum, (float)((end - start) * a));
 }
 
-__global__ void __launch_bounds__(DEC_NT) k_block_decide(const float *bmeans, uint64_t blocks_n, float threshold,
-                               float *scratch, unsigned char *blkbad) {
+__global__ void __launch_bounds__(DEC_NT)
+    k_block_decide(const float *bmeans, uint64_t blocks_n, float threshold, float *scratch,
+                   unsigned char *blkbad) {
   __shared__ unsigned hist[32 * 256];
   __shared__ uint32_t bc[3];
   block_outliers(bmeans, blocks_n, threshold, scratch, blkbad, hist, bc);
 }
+// The same for at most BL_RANK_MAX blocks.
+__global__ void __launch_bounds__(32 * BL_NW)
+    k_block_decide_few(const float *bmeans, int blocks_n, float threshold,
+                       unsigned char *blkbad) {
+  __shared__ RankShared sh;
+  const int tid = (int)threadIdx.x;
+  if (blocks_n <= 64 * BL_NW) group_outliers<2, BL_NW>(bmeans, blocks_n, threshold, blkbad, tid, sh);
+  else if (blocks_n <= 256 * BL_NW)
+    group_outliers<8, BL_NW>(bmeans, blocks_n, threshold, blkbad, tid, sh);
+  else
+    group_outliers<BL_RANK_MAX / (32 * BL_NW), BL_NW>(bmeans, blocks_n, threshold, blkbad, tid, sh);
+}
 
 // Replace masked samples with the channel median (rfi/src/lib.rs:76-89): CTA
-// (group of FILL_B blocks, channel) writes the masked blocks of its group and
-// leaves at once where there are none.  Testing every sample's block took 0.64
-// ms on 512 channels of 1,047,799 samples (GB300), this 0.022.
-constexpr int FILL_B = 64;
+// (group of FILL_B blocks, channel) writes the masked blocks of its group, a warp
+// per block in 16-byte stores, and leaves at once where there are none.
+// Testing every sample's block took 0.64 ms on 512 channels of 1,047,799
+// samples (GB300), this 0.022; 64 channels of 262,144 samples 27 us with sample
+// stores, 4 now.
+constexpr int FILL_B = 64, FILL_NT = 256;
 template <class T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(FILL_NT)
     k_fill(T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t bs, uint64_t blocks_n,
            const unsigned char *__restrict__ chbad, const unsigned char *__restrict__ blkbad,
            const float *__restrict__ med) {
@@ -1070,12 +1176,23 @@ __global__ void __launch_bounds__(128)
   const bool whole = chbad[c] != 0;
   const uint64_t mine = b0 + threadIdx.x;
   if (!__syncthreads_or(whole || (mine < b1 && blkbad[mine]))) return;
+  constexpr uint64_t PER = 16 / sizeof(T);
   const T typical = (T)med[c];
-  T *row = s + c * ld;
-  for (uint64_t b = b0; b < b1; ++b) {
+  T same[PER];
+#pragma unroll
+  for (int i = 0; i < (int)PER; ++i) same[i] = typical;
+  uint4 v;
+  memcpy(&v, same, 16);
+  T *row = s + c * ld;  // 16-byte aligned, as is every PER-th sample
+  const uint64_t lane = threadIdx.x & 31;
+  for (uint64_t b = b0 + (threadIdx.x >> 5); b < b1; b += FILL_NT / 32) {
     if (!whole && !blkbad[b]) continue;
-    const uint64_t end = min((b + 1) * bs, ns);
-    for (uint64_t t = b * bs + threadIdx.x; t < end; t += blockDim.x) row[t] = typical;
+    const uint64_t t0 = b * bs, t1 = min(t0 + bs, ns);
+    const uint64_t a0 = min((t0 + PER - 1) / PER * PER, t1), a1 = max(t1 / PER * PER, a0);
+    if (t0 + lane < a0) row[t0 + lane] = typical;  // (fewer than PER <= 16 samples)
+    for (uint64_t t = a0 + PER * lane; t < a1; t += 32 * PER)
+      *reinterpret_cast<uint4 *>(row + t) = v;
+    if (a1 + lane < t1) row[a1 + lane] = typical;
   }
 }
 
@@ -1190,7 +1307,7 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
                                   (int)MH_SMEM));
     k_chan_hist_u8<<<dim3((unsigned)nsplit, (unsigned)nch), MH_NT, MH_SMEM, st>>>(
         s, ns, o.ld, w.mhist.as<unsigned>());
-    k_hist_median<<<(unsigned)((nch + 127) / 128), 128, 0, st>>>(w.mhist.as<unsigned>(), nch, ns,
+    k_hist_median<<<(unsigned)((nch + 3) / 4), 128, 0, st>>>(w.mhist.as<unsigned>(), nch, ns,
                                                                  w.med.as<float>());
   } else {
     const size_t hb = nch * sizeof(unsigned) << MD_BITS;
@@ -1213,9 +1330,13 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
       w.bsum.as<float>(), w.chbad.as<unsigned char>(), nch, ns, bs, blocks_n,
       w.active.as<unsigned long long>(),
       w.bmeans.as<float>());
-  k_block_decide<<<1, DEC_NT, 0, st>>>(w.bmeans.as<float>(), blocks_n, thr,
-                                     w.scratch.as<float>(), w.blkbad.as<unsigned char>());
-  k_fill<T><<<dim3((unsigned)((blocks_n + FILL_B - 1) / FILL_B), (unsigned)nch), 128, 0, st>>>(
+  if (blocks_n <= (uint64_t)BL_RANK_MAX)
+    k_block_decide_few<<<1, 32 * BL_NW, 0, st>>>(w.bmeans.as<float>(), (int)blocks_n, thr,
+                                                 w.blkbad.as<unsigned char>());
+  else
+    k_block_decide<<<1, DEC_NT, 0, st>>>(w.bmeans.as<float>(), blocks_n, thr,
+                                         w.scratch.as<float>(), w.blkbad.as<unsigned char>());
+  k_fill<T><<<dim3((unsigned)((blocks_n + FILL_B - 1) / FILL_B), (unsigned)nch), FILL_NT, 0, st>>>(
       s, ns, o.ld, bs, blocks_n, w.chbad.as<unsigned char>(), w.blkbad.as<unsigned char>(),
       w.med.as<float>());
   PSR_CUDA(cudaGetLastError());
