@@ -57,7 +57,9 @@ __global__ void k_unpack(const T *__restrict__ payload, T *__restrict__ out, uin
 // row, which keeps the 32 lanes' stores (channels 4 l + i) in 32 banks.
 // Bound: HBM, payload read and samples written once.  Measured on a GB300: 512
 // 8-bit channels of 1,047,799 samples (1.07 GB moved) 0.86 ms with one byte per
-// thread and access, 0.34 now; 96 4-bit channels of 531,000 0.100 and 0.037.
+// thread and access, 0.34 with a bit address per word, 0.19 with whole words
+// where the channel count is a multiple of 4; 96 4-bit channels of 531,000
+// samples 0.100 and 0.037.
 constexpr int UP_T = 128, UP_C = 128, UP_NT = 256;
 
 template <int B>
@@ -90,16 +92,25 @@ __global__ void __launch_bounds__(UP_NT)
   const uint32_t cmask = c + 4 <= nch ? 0xffffffffu
                          : c < nch    ? 0xffffffffu >> (8 * (4 - (int)(nch - c)))
                                       : 0u;
+  const bool words = nch % 4 == 0;
+  const uint64_t step = nch * B, bit0 = ((t0 + 4 * warp) * nch + c) * B;
 #pragma unroll
   for (int h = 0; h < UP_T / 4 / (UP_NT / 32); ++h) {
     const int q = warp + h * (UP_NT / 32);
     uint32_t v[4];
+    if (B == 8 && words) {  // four channels of a time are a word of the payload
+      const uint64_t t = t0 + 4 * q;
+      const uint32_t *w = payload + (t * nch + c) / 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = t + i < ns && cmask ? __ldg(w + i * (nch / 4)) : 0u;
+    } else
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint64_t t = t0 + 4 * q + i;
       uint32_t x = 0;
       if (t < ns && cmask) {
-        const uint64_t bit = (t * nch + c) * B;
+        const uint64_t bit = bit0 + (uint64_t)(32 * h + i) * step;
         const uint32_t *w = payload + (bit >> 5);
         const unsigned sh = (unsigned)bit & 31u;
         // the second word only where the 4 B bits reach it (it may be the
@@ -300,7 +311,8 @@ __global__ void __launch_bounds__(MD_NT)
 // of word t mod 64, so a warp's 32 columns are 32 banks).  A column is added
 // to the row's global histogram before 255 samples could overflow it.
 // Measured on a GB300: 512 channels of 1,047,799 samples 0.52 ms with 16-bit
-// columns (128 threads in the same 64 KB), 0.30 now.
+// columns (128 threads in the same 64 KB), 0.30 with one sample at a time in the
+// chain of a thread's counts, 0.27 now.
 constexpr int MH_NT = 256;
 constexpr int MH_RUNS = 15;  // 16-sample loads per thread between additions
 constexpr size_t MH_SMEM = 256 * MH_NT;
@@ -328,9 +340,21 @@ __global__ void __launch_bounds__(MH_NT)
       const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + i));
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
       const int m = (int)min((uint64_t)16, r1 - i);
+      if (m == 16) {
+        // two samples at a time: both counts are read before either is written
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
-        if (k < m) mine[((w[k >> 2] >> (8 * (k & 3))) & 255u) * MH_NT] += 1;
+        for (int k = 0; k < 16; k += 2) {
+          const uint32_t v = w[k >> 2] >> (8 * (k & 3));
+          uint8_t *p0 = mine + (v & 255u) * MH_NT, *p1 = mine + (v >> 8 & 255u) * MH_NT;
+          const uint8_t c0 = *p0 + 1, c1 = *p1 + 1;
+          *p0 = c0;
+          *p1 = p0 == p1 ? c0 + 1 : c1;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          if (k < m) mine[((w[k >> 2] >> (8 * (k & 3))) & 255u) * MH_NT] += 1;
+      }
     }
     __syncthreads();
 #pragma unroll 8
@@ -897,34 +921,37 @@ __global__ void k_block_sums(const T *__restrict__ s, uint64_t ns, uint64_t ld,
 }
 
 // The same for integer samples whose block totals stay at most 2^24 (every
-// partial sum exact, so any order): a warp per (channel, block), 16-byte loads
+// partial sum exact, so any order): a warp per (block, channel), 16-byte loads
 // with the samples outside the block masked.  Measured on a GB300: 512 8-bit
 // channels of 1,047,799 samples, blocks of 1000: 0.62 ms with a thread per
-// block, 0.165 now.
+// block, 0.165 with 64-bit indices, a division per warp and masks sample by
+// sample, 0.108 now.
+constexpr int BS_W = 8;  // warps (blocks) per CTA
+// The low min(max(x, 0), 4) bytes of a word.
+__device__ __forceinline__ uint32_t low_bytes(int x) {
+  return x >= 4 ? 0xffffffffu : x <= 0 ? 0u : 0xffffffffu >> (32 - 8 * x);
+}
 template <class T>
-__global__ void __launch_bounds__(256)
-    k_block_sums_int(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t nch, uint64_t bs,
+__global__ void __launch_bounds__(32 * BS_W)
+    k_block_sums_int(const T *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t bs,
                      uint64_t blocks_n, float *__restrict__ bsum) {
-  const uint64_t id = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (id >= nch * blocks_n) return;
+  const uint64_t b = (uint64_t)blockIdx.x * BS_W + (threadIdx.x >> 5), c = blockIdx.y;
+  if (b >= blocks_n) return;
   const int lane = (int)(threadIdx.x & 31);
-  const uint64_t c = id / blocks_n, b = id % blocks_n;
-  const uint64_t start = b * bs, end = min(start + bs, ns);
   constexpr int PER = 16 / (int)sizeof(T);
-  const T *row = s + c * ld;
+  const uint64_t start = b * bs, base = start & ~(uint64_t)(PER - 1);
+  const T *p = s + c * ld + base;
+  // samples [head, stop) from base: a block is at most 2^24 samples
+  const int head = (int)(start - base), stop = head + (int)min(bs, ns - start);
   unsigned acc = 0;
-  for (uint64_t p = (start & ~(uint64_t)(PER - 1)) + (uint64_t)lane * PER; p < end;
-       p += 32 * PER) {
-    uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + p));
-    if (p < start || p + PER > end) {
-      T e[PER];
-      memcpy(e, &v, 16);
+  for (int i = lane * PER; i < stop; i += 32 * PER) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + i));
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    if (i < head || i + PER > stop) {
+      const int lo = (head - i) * (int)sizeof(T), hi = (stop - i) * (int)sizeof(T);
 #pragma unroll
-      for (int u = 0; u < PER; ++u)
-        if (p + u < start || p + u >= end) e[u] = 0;
-      memcpy(&v, e, 16);
+      for (int u = 0; u < 4; ++u) w[u] &= low_bytes(hi - 4 * u) & ~low_bytes(lo - 4 * u);
     }
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if constexpr (sizeof(T) == 1) acc = __dp4a(w[u], 0x01010101u, acc);
@@ -932,7 +959,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   acc = __reduce_add_sync(0xffffffffu, acc);
-  if (lane == 0) bsum[id] = (float)acc;
+  if (lane == 0) bsum[c * blocks_n + b] = (float)acc;
 }
 
 // Counters of NW warps that select together.
@@ -1291,8 +1318,8 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   PSR_TRY(enqueue_mean_var<T>(s, nch, ns, o.ld, w, st));
   if constexpr (sizeof(T) < 4) {
     if (bs <= (1u << 24) / (sizeof(T) == 1 ? 255u : 65535u))
-      k_block_sums_int<T><<<(unsigned)((nch * blocks_n + 7) / 8), 256, 0, st>>>(
-          s, ns, o.ld, nch, bs, blocks_n, w.bsum.as<float>());
+      k_block_sums_int<T><<<dim3((unsigned)((blocks_n + BS_W - 1) / BS_W), (unsigned)nch),
+                            32 * BS_W, 0, st>>>(s, ns, o.ld, bs, blocks_n, w.bsum.as<float>());
   }
   if (sizeof(T) == 4 || bs > (1u << 24) / (sizeof(T) == 1 ? 255u : 65535u))
     k_block_sums<T><<<(unsigned)((nch * blocks_n + 127) / 128), 128, 0, st>>>(
