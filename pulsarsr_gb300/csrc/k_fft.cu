@@ -976,6 +976,37 @@ __global__ void __launch_bounds__(256) k_fft_quarter(uint64_t N, float2 *__restr
   if (n4 - r > n8) Q[n4 - r] = make_float2(v.y, v.x);
 }
 
+// From QS_MIN points on by angle sums: 2 pi j / 2^25, j = 2^11 h + l <= 2^22, from
+// 2049 + 2048 angles' f64 sines and cosines, which are a tenth of the f64
+// work (FP64, 1/64 of the f32 rate, bounds the kernel).  Every N's angles are
+// among these, and for each of them the product rounds to the f32 values of the
+// direct evaluation (compared exhaustively).  Measured on a GB300, N = 2^23: 73 us
+// direct, 3 + 14 now.
+constexpr int QS_LO = 11, QS_TOP = 25;
+constexpr uint64_t QS_MIN = 1ull << 17;
+constexpr int QS_H = (1 << (QS_TOP - 3 - QS_LO)) + 1, QS_L = 1 << QS_LO;
+__global__ void __launch_bounds__(256) k_fft_angles(double2 *__restrict__ T) {
+  const int i = (int)(blockIdx.x * 256 + threadIdx.x);
+  if (i >= QS_H + QS_L) return;
+  const double j = i < QS_H ? (double)((uint64_t)i << QS_LO) : (double)(i - QS_H);
+  double sn, cs;
+  sincos(6.283185307179586 * j / (double)(1ull << QS_TOP), &sn, &cs);
+  T[i] = make_double2(cs, sn);
+}
+__global__ void __launch_bounds__(256)
+    k_fft_quarter_split(uint64_t N, int up, const double2 *__restrict__ T,
+                        float2 *__restrict__ Q) {
+  const uint64_t r = (uint64_t)blockIdx.x * 256 + threadIdx.x, n4 = N / 4, n8 = N / 8;
+  if (r > n8) return;
+  const uint32_t j = (uint32_t)(r << up);
+  const double2 a = T[j >> QS_LO], b = T[QS_H + (j & (QS_L - 1))];
+  const double cs = __fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y));
+  const double sn = __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y));
+  const float2 v = make_float2((float)cs, (float)sn);
+  Q[r] = v;
+  if (n4 - r > n8) Q[n4 - r] = make_float2(v.y, v.x);
+}
+
 // Tw1[k1*M2 + n2] = W_N^(2*n2*k1) = W_M^(n2*k1), by the device lookup.
 __global__ void __launch_bounds__(256)
     k_fft_tw1(const float2 *__restrict__ Q, int lq, int lm2, uint64_t M,
@@ -1015,9 +1046,18 @@ int FftPlan::init(uint64_t series_len, cudaStream_t st) {
   int lq = 0;
   while ((1ull << lq) < N / 4) ++lq;
   PSR_TRY(Q.ensure((N / 4 + 1) * sizeof(float2)));
-  k_fft_quarter<<<(unsigned)((N / 8 + 1 + 255) / 256), 256, 0, st>>>(N, Q.as<float2>());
+  if (m > 12) PSR_TRY(tw1.ensure(M * sizeof(float2)));
+  const unsigned qctas = (unsigned)((N / 8 + 1 + 255) / 256);
+  if (N >= QS_MIN) {
+    // (the angles lie in tw1's memory, 512 KB or more, until its own kernel)
+    double2 *T = tw1.as<double2>();
+    static_assert(QS_MIN / 2 * sizeof(float2) >= (QS_H + QS_L) * sizeof(double2), "room");
+    k_fft_angles<<<(QS_H + QS_L + 255) / 256, 256, 0, st>>>(T);
+    k_fft_quarter_split<<<qctas, 256, 0, st>>>(N, QS_TOP - (lq + 2), T, Q.as<float2>());
+  } else {
+    k_fft_quarter<<<qctas, 256, 0, st>>>(N, Q.as<float2>());
+  }
   if (m > 12) {
-    PSR_TRY(tw1.ensure(M * sizeof(float2)));
     k_fft_tw1<<<(unsigned)(M / 256), 256, 0, st>>>(Q.as<float2>(), lq, ilog2((int)M2), M,
                                                    tw1.as<float2>());
   }
