@@ -35,6 +35,12 @@ struct FoldPhase {
   uint32_t margin, pad;
 };
 
+// The rows' phases of a launch, as a kernel argument.
+constexpr uint64_t FOLD_ROWS = 64;
+struct FoldPhases {
+  FoldPhase p[FOLD_ROWS];
+};
+
 // x 2^128 modulo 2^128 for a finite x >= 0.
 unsigned __int128 fixed128(double x) {
   int e = 0;
@@ -107,14 +113,14 @@ __device__ __forceinline__ bool as_count(T x, uint32_t &v) {
 template <class T>
 __global__ void __launch_bounds__(FOLD_NT, 4)
     k_fold(const T *__restrict__ x, uint64_t xstride, uint64_t n, uint64_t offset,
-           const FoldPhase *__restrict__ ph, int phstride, uint32_t bins, int copies,
+           const __grid_constant__ FoldPhases ph, int phstride, uint32_t bins, int copies,
            uint64_t per_cta, double *__restrict__ psums, unsigned long long *__restrict__ pcounts) {
   extern __shared__ unsigned char sm_raw[];
   constexpr int VEC = 4 / (int)sizeof(T);        // samples per 32-bit load
   constexpr int PER = 8192 / FOLD_NT / VEC;      // loads per thread (per_cta <= 8192)
   const uint64_t row = blockIdx.y;
   x += row * xstride;
-  const FoldPhase p = ph[row * phstride];
+  const FoldPhase p = ph.p[row * phstride];
   const uint64_t t0 = (uint64_t)blockIdx.x * per_cta, t1 = min(t0 + per_cta, n);
   // 32 bits of samples from t (rows of 8- and 16-bit samples are 64-element
   // aligned and padded)
@@ -530,33 +536,35 @@ int fold_profiles_ex(const float *d_x, uint64_t xstride, uint64_t n, double tsam
   const uint64_t nparts = (n + f.per_cta - 1) / f.per_cta;
   const uint64_t nser = xstride ? nper : 1;
   const uint32_t mparts = (uint32_t)((n + MOM_PER - 1) / MOM_PER);
-  DevBuf dper, psums, pcounts, sums, cnts, mom;
-  PSR_TRY(dper.ensure(nper * sizeof(FoldPhase)));
-  PSR_TRY(psums.ensure(nper * nparts * bins * 8));
-  PSR_TRY(pcounts.ensure(nper * nparts * bins * 8));
-  PSR_TRY(sums.ensure(nper * bins * 8));
-  PSR_TRY(cnts.ensure(nper * bins * 8));
-  PSR_TRY(mom.ensure((size_t)nser * mparts * 24));
-  std::vector<FoldPhase> phases(nper);
-  for (uint64_t p = 0; p < nper; ++p) phases[p] = fold_phase(tsamp, periods[p], n + offset, bins);
-  PSR_CUDA(cudaMemcpyAsync(dper.p, phases.data(), nper * sizeof(FoldPhase),
-                           cudaMemcpyHostToDevice, st));
-  k_fold<float><<<dim3((unsigned)nparts, (unsigned)nper), FOLD_NT, f.smem, st>>>(
-      d_x, xstride, n, offset, dper.as<FoldPhase>(), 1, (uint32_t)bins, f.copies, f.per_cta,
-      psums.as<double>(), pcounts.as<unsigned long long>());
+  // partial sums and counts; then sums, counts and moments, read back in one copy
+  const size_t nb = (size_t)(nper * bins), np = nb * nparts, nm = (size_t)nser * mparts * 3;
+  DevBuf parts, res;
+  PSR_TRY(parts.ensure(2 * np * 8));
+  PSR_TRY(res.ensure((2 * nb + nm) * 8));
+  double *psums = parts.as<double>(), *sums = res.as<double>();
+  unsigned long long *pcounts = parts.as<unsigned long long>() + np;
+  unsigned long long *cnts = res.as<unsigned long long>() + nb, *mom = cnts + nb;
+  FoldPhases ph{};
+  for (uint64_t r0 = 0; r0 < nper; r0 += FOLD_ROWS) {
+    const uint64_t nr = std::min(FOLD_ROWS, nper - r0);
+    for (uint64_t p = 0; p < nr; ++p)
+      ph.p[p] = fold_phase(tsamp, periods[r0 + p], n + offset, bins);
+    k_fold<float><<<dim3((unsigned)nparts, (unsigned)nr), FOLD_NT, f.smem, st>>>(
+        d_x + r0 * xstride, xstride, n, offset, ph, 1, (uint32_t)bins, f.copies, f.per_cta,
+        psums + r0 * nparts * bins, pcounts + r0 * nparts * bins);
+  }
   PSR_CUDA(cudaGetLastError());
-  k_fold_reduce<<<(unsigned)((nper * bins + 255) / 256), 256, 0, st>>>(
-      psums.as<double>(), pcounts.as<unsigned long long>(), nparts, bins, nper,
-      sums.as<double>(), cnts.as<unsigned long long>());
-  k_series_moments<<<dim3(mparts, (unsigned)nser), MI_NT, 0, st>>>(
-      d_x, xstride, n, MOM_PER, mom.as<unsigned long long>());
+  k_fold_reduce<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(psums, pcounts, nparts, bins, nper,
+                                                             sums, cnts);
+  k_series_moments<<<dim3(mparts, (unsigned)nser), MI_NT, 0, st>>>(d_x, xstride, n, MOM_PER, mom);
   PSR_CUDA(cudaGetLastError());
-  std::vector<double> hs(nper * bins), hm(2 * nser);
-  std::vector<unsigned long long> hc(nper * bins), hmom((size_t)nser * mparts * 3);
-  PSR_CUDA(cudaMemcpyAsync(hs.data(), sums.p, nper * bins * 8, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaMemcpyAsync(hc.data(), cnts.p, nper * bins * 8, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaMemcpyAsync(hmom.data(), mom.p, hmom.size() * 8, cudaMemcpyDeviceToHost, st));
+  std::vector<unsigned long long> back(2 * nb + nm), hc(nb), hmom(nm);
+  std::vector<double> hs(nb), hm(2 * nser);
+  PSR_CUDA(cudaMemcpyAsync(back.data(), res.p, back.size() * 8, cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(hs.data(), back.data(), nb * 8);
+  std::memcpy(hc.data(), back.data() + nb, nb * 8);
+  std::memcpy(hmom.data(), back.data() + 2 * nb, nm * 8);
   bool ints = true;
   for (size_t i = 0; i < hmom.size(); i += 3) ints = ints && hmom[i + 2] != 0;
   if (ints) {
@@ -800,19 +808,18 @@ int fold_channels(const DeviceObs &o, uint64_t n, double tsamp, double period, u
   }
   const FoldShape f = fold_shape(bins);
   const uint64_t nparts = (n + f.per_cta - 1) / f.per_cta;
-  DevBuf dper, psums, pcounts, sums, cnts;
-  PSR_TRY(dper.ensure(sizeof(FoldPhase)));
-  PSR_TRY(psums.ensure(o.nch * nparts * bins * 8));
-  PSR_TRY(pcounts.ensure(o.nch * nparts * bins * 8));
-  PSR_TRY(sums.ensure(o.nch * bins * 8));
-  PSR_TRY(cnts.ensure(o.nch * bins * 8));
-  const FoldPhase phase = fold_phase(tsamp, period, n, bins);
-  PSR_CUDA(cudaMemcpyAsync(dper.p, &phase, sizeof(phase), cudaMemcpyHostToDevice, st));
+  const size_t nb = (size_t)(o.nch * bins), np = nb * nparts;
+  DevBuf parts, res;
+  PSR_TRY(parts.ensure(2 * np * 8));
+  PSR_TRY(res.ensure(2 * nb * 8));
+  double *psums = parts.as<double>();
+  unsigned long long *pcounts = parts.as<unsigned long long>() + np;
+  FoldPhases ph{};
+  ph.p[0] = fold_phase(tsamp, period, n, bins);
   const dim3 grid((unsigned)nparts, (unsigned)o.nch);
   auto run = [&](auto *x) {
-    k_fold<<<grid, FOLD_NT, f.smem, st>>>(x, o.ld, n, (uint64_t)0, dper.as<FoldPhase>(), 0,
-                                          (uint32_t)bins, f.copies, f.per_cta,
-                                          psums.as<double>(), pcounts.as<unsigned long long>());
+    k_fold<<<grid, FOLD_NT, f.smem, st>>>(x, o.ld, n, (uint64_t)0, ph, 0, (uint32_t)bins,
+                                          f.copies, f.per_cta, psums, pcounts);
   };
   switch (o.kind) {
     case SAMPLE_U8: run(o.samples.as<const uint8_t>()); break;
@@ -820,15 +827,15 @@ int fold_channels(const DeviceObs &o, uint64_t n, double tsamp, double period, u
     default: run(o.samples.as<const float>());
   }
   PSR_CUDA(cudaGetLastError());
-  k_fold_reduce<<<(unsigned)((o.nch * bins + 255) / 256), 256, 0, st>>>(
-      psums.as<double>(), pcounts.as<unsigned long long>(), nparts, bins, o.nch,
-      sums.as<double>(), cnts.as<unsigned long long>());
+  k_fold_reduce<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(
+      psums, pcounts, nparts, bins, o.nch, res.as<double>(), res.as<unsigned long long>() + nb);
   PSR_CUDA(cudaGetLastError());
-  std::vector<double> hs(o.nch * bins);
-  std::vector<unsigned long long> hc(o.nch * bins);
-  PSR_CUDA(cudaMemcpyAsync(hs.data(), sums.p, hs.size() * 8, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaMemcpyAsync(hc.data(), cnts.p, hc.size() * 8, cudaMemcpyDeviceToHost, st));
+  std::vector<unsigned long long> back(2 * nb), hc(nb);
+  std::vector<double> hs(nb);
+  PSR_CUDA(cudaMemcpyAsync(back.data(), res.p, back.size() * 8, cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(hs.data(), back.data(), nb * 8);
+  std::memcpy(hc.data(), back.data() + nb, nb * 8);
   values.resize(o.nch * bins);
   for (uint64_t i = 0; i < o.nch * bins; ++i)
     values[i] = hc[i] > 0 ? (float)(hs[i] / (double)hc[i]) : 0.0f;
