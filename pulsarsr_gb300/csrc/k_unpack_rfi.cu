@@ -1309,8 +1309,8 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   PSR_TRY(w.med.ensure(nch * 4));
   PSR_TRY(w.bsum.ensure(nch * blocks_n * 4));
   PSR_TRY(w.bmeans.ensure(blocks_n * 4));
-  PSR_TRY(w.chbad.ensure(nch));
-  PSR_TRY(w.blkbad.ensure(blocks_n));
+  PSR_TRY(w.bad.ensure(nch + blocks_n));  // of the channels, then of the blocks
+  unsigned char *chbad = w.bad.as<unsigned char>(), *blkbad = chbad + nch;
   PSR_TRY(w.scratch.ensure(std::max(nch, blocks_n) * 4));
   PSR_TRY(w.flags.ensure(2 * nch));
   PSR_TRY(w.active.ensure(8));
@@ -1352,19 +1352,19 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
   unsigned char *fl = w.flags.as<unsigned char>();
   k_channel_decide<<<1, DEC_NT, 0, st>>>(w.means.as<float>(), w.vars.as<float>(), nch, thr,
                                        w.scratch.as<float>(), fl, fl + nch,
-                                       w.chbad.as<unsigned char>(), w.active.as<unsigned long long>());
+                                       chbad, w.active.as<unsigned long long>());
   k_block_means<<<(unsigned)((blocks_n + 31) / 32), BM_NT, 0, st>>>(
-      w.bsum.as<float>(), w.chbad.as<unsigned char>(), nch, ns, bs, blocks_n,
+      w.bsum.as<float>(), chbad, nch, ns, bs, blocks_n,
       w.active.as<unsigned long long>(),
       w.bmeans.as<float>());
   if (blocks_n <= (uint64_t)BL_RANK_MAX)
     k_block_decide_few<<<1, 32 * BL_NW, 0, st>>>(w.bmeans.as<float>(), (int)blocks_n, thr,
-                                                 w.blkbad.as<unsigned char>());
+                                                 blkbad);
   else
     k_block_decide<<<1, DEC_NT, 0, st>>>(w.bmeans.as<float>(), blocks_n, thr,
-                                         w.scratch.as<float>(), w.blkbad.as<unsigned char>());
+                                         w.scratch.as<float>(), blkbad);
   k_fill<T><<<dim3((unsigned)((blocks_n + FILL_B - 1) / FILL_B), (unsigned)nch), FILL_NT, 0, st>>>(
-      s, ns, o.ld, bs, blocks_n, w.chbad.as<unsigned char>(), w.blkbad.as<unsigned char>(),
+      s, ns, o.ld, bs, blocks_n, chbad, blkbad,
       w.med.as<float>());
   PSR_CUDA(cudaGetLastError());
   return PSR_OK;
@@ -1398,10 +1398,10 @@ int rfi_enqueue(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaStream_t s
 }
 
 int rfi_collect(const DeviceObs &o, uint64_t bs, RfiWork &w, cudaStream_t st, RfiResult &res) {
-  std::vector<unsigned char> ch(o.nch), bl(w.blocks_n);
-  PSR_CUDA(cudaMemcpyAsync(ch.data(), w.chbad.p, o.nch, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaMemcpyAsync(bl.data(), w.blkbad.p, w.blocks_n, cudaMemcpyDeviceToHost, st));
+  std::vector<unsigned char> ch(o.nch + w.blocks_n);
+  PSR_CUDA(cudaMemcpyAsync(ch.data(), w.bad.p, ch.size(), cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaStreamSynchronize(st));
+  const unsigned char *bl = ch.data() + o.nch;
   res.channels.clear();
   res.blocks.clear();
   for (uint64_t c = 0; c < o.nch; ++c)

@@ -214,7 +214,7 @@ int launch_unpack(const DeviceObs &o, unsigned long long *d_err_index,
 
 // RFI mask (rfi::mask) on the device samples.  Scratch is owned by RfiWork.
 struct RfiWork {
-  DevBuf means, vars, med, bsum, bmeans, chbad, blkbad, scratch, flags, active, mhist;
+  DevBuf means, vars, med, bsum, bmeans, bad, scratch, flags, active, mhist;
   DevBuf es_sum, es_sq, es_guess, es_maps, es_chan, es_neg;  // reference-order sums
   uint64_t blocks_n = 0;
 };

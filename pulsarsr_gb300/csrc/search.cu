@@ -52,11 +52,7 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   PSR_TRY(power.ensure(2 * chunk * ldp * 4));
   PSR_TRY(psum.ensure(2 * chunk * npsum * 8));
   PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
-  const uint64_t maxc = std::max<uint64_t>(cfg.max_candidates, 1);
-  PSR_TRY(kept.ensure(ntrials * maxc * sizeof(psr_candidate)));
-  PSR_TRY(kept_count.ensure(ntrials * 4));
-  PSR_TRY(err.ensure(16));
-  PSR_CUDA(cudaMemsetAsync(err.p, 0, 16, st));
+  PSR_TRY(kept.ensure(list_bytes() + ntrials * 4));
   const uint64_t tail = chunk >= 16 && ntrials > chunk ? chunk / 8 : 0;
   cstart.clear();
   for (uint64_t t = 0; t < ntrials - tail; t += chunk) cstart.push_back(t);
@@ -68,7 +64,8 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
   PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
                              sbplan, st));
-  PSR_TRY(chunk_overflow.ensure(nchunks * 4 + 16));
+  PSR_TRY(status.ensure(nchunks * 4 + 16));
+  PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&ev_fft[0], &ev_fft[1], &ev_sel[0], &ev_sel[1]})
     if (!*e) PSR_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
@@ -82,7 +79,7 @@ int SearchEngine::enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st
   PSR_TRY(record(ST_DEDISP, true, st));
   PSR_TRY(launch_dedisperse_ex(o, delays.as<uint32_t>() + t0 * o.nch, nt, n, series.as<float>(),
                                ldo, parts.as<double>(), sums.as<double>(), means.as<float>(),
-                               max_spread, err.as<unsigned>(), st, 0, 0, true, &sbplan, ci));
+                               max_spread, err(), st, 0, 0, true, &sbplan, ci));
   PSR_TRY(record(ST_DEDISP, false, st));
   // aux runs after everything st has queued so far (the previous chunk's
   // work is ordered on aux already), then resets the candidate queues.
@@ -114,10 +111,10 @@ int SearchEngine::enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st
   PSR_TRY(record(ST_SPEC, true, aux));
   PSR_TRY(spectrum_items(fft, spec, pw, ldp, nt, sw, aux));
   PSR_TRY(spectrum_select(fft, spec, trial_dm.as<double>() + t0, nt, sw,
-                          kept.as<psr_candidate>() + t0 * maxc, kept_count.as<unsigned>() + t0,
+                          kept.as<psr_candidate>() + t0 * maxc, kept_count() + t0,
                           aux));
   PSR_TRY(record(ST_SPEC, false, aux));
-  PSR_CUDA(cudaMemcpyAsync(chunk_overflow.as<unsigned>() + ci, sw.overflow(), 4,
+  PSR_CUDA(cudaMemcpyAsync(status.as<unsigned>() + ci, sw.overflow(), 4,
                            cudaMemcpyDeviceToDevice, aux));
   PSR_CUDA(cudaEventRecord(ev_sel[b], aux));
   sel_pending[b] = true;
@@ -180,8 +177,7 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
   // per-chunk overflow words, then the dedispersion error word
   PSR_TRY(h_status.ensure((nchunks + 1) * 4));
   unsigned *hs = h_status.as<unsigned>();
-  PSR_CUDA(cudaMemcpyAsync(hs, chunk_overflow.p, nchunks * 4, cudaMemcpyDeviceToHost, st));
-  PSR_CUDA(cudaMemcpyAsync(hs + nchunks, err.p, 4, cudaMemcpyDeviceToHost, st));
+  PSR_CUDA(cudaMemcpyAsync(hs, status.p, (nchunks + 1) * 4, cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaStreamSynchronize(st));
   std::vector<unsigned> ov(hs, hs + nchunks);
   const unsigned e = hs[nchunks];
@@ -204,7 +200,7 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
       PSR_TRY(enqueue_chunk(o, ci, st));
       PSR_TRY(join(st));
       unsigned v = 0;
-      PSR_CUDA(cudaMemcpyAsync(&v, chunk_overflow.as<unsigned>() + ci, 4,
+      PSR_CUDA(cudaMemcpyAsync(&v, status.as<unsigned>() + ci, 4,
                                cudaMemcpyDeviceToHost, st));
       PSR_CUDA(cudaStreamSynchronize(st));
       ov[ci] = v;
@@ -216,14 +212,11 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
 int SearchEngine::collect(cudaStream_t st, uint64_t *counts, psr_candidate *out, uint64_t cap,
                           uint64_t *n_total) {
   const uint64_t maxc = std::max<uint64_t>(spec.max_candidates, 1);
-  PSR_TRY(h_kept_count.ensure(ntrials * 4));
-  PSR_TRY(h_kept.ensure(ntrials * maxc * sizeof(psr_candidate)));
-  PSR_CUDA(cudaMemcpyAsync(h_kept_count.p, kept_count.p, ntrials * 4, cudaMemcpyDeviceToHost,
-                           st));
-  PSR_CUDA(cudaMemcpyAsync(h_kept.p, kept.p, ntrials * maxc * sizeof(psr_candidate),
-                           cudaMemcpyDeviceToHost, st));
+  const uint64_t bytes = list_bytes() + ntrials * 4;
+  PSR_TRY(h_kept.ensure(bytes));
+  PSR_CUDA(cudaMemcpyAsync(h_kept.p, kept.p, bytes, cudaMemcpyDeviceToHost, st));
   PSR_CUDA(cudaStreamSynchronize(st));
-  const unsigned *kc = h_kept_count.as<unsigned>();
+  const unsigned *kc = reinterpret_cast<unsigned *>(h_kept.as<char>() + list_bytes());
   const psr_candidate *all = h_kept.as<psr_candidate>();
   uint64_t k = 0;
   for (uint64_t i = 0; i < ntrials; ++i) {

@@ -38,12 +38,21 @@ struct SearchEngine {
   double stage_ms[ST_COUNT] = {0, 0, 0};
   uint64_t stage_launches[ST_COUNT] = {0, 0, 0};
   int record(int stage, bool begin, cudaStream_t st);
+  uint64_t list_bytes() const {
+    return ntrials * (spec.max_candidates < 1 ? 1 : (uint64_t)spec.max_candidates) *
+           sizeof(psr_candidate);
+  }
+  unsigned *kept_count() const {
+    return reinterpret_cast<unsigned *>(kept.as<char>() + list_bytes());
+  }
+  unsigned *err() const { return status.as<unsigned>() + nchunks; }
   int harvest();  // after a sync: add elapsed times, forget the events
   ~SearchEngine();
-  DevBuf delays, trial_dm, series, parts, sums, means, work, power, psum, kept, kept_count, err,
-      chunk_overflow;
-  HostBuf h_kept, h_kept_count;  // collect()'s staging of the kept lists
-  HostBuf h_status;              // finish(): overflow and error words
+  DevBuf delays, trial_dm, series, parts, sums, means, work, power, psum;
+  DevBuf kept;    // every trial's list, then every trial's count
+  DevBuf status;  // per-chunk overflow words, then the dedispersion error word
+  HostBuf h_kept;  // collect()'s staging of kept
+  HostBuf h_status;  // finish()'s of status
   // The gates, harmonic items and selection of a chunk run on `aux`, so that
   // they overlap the FFTs of the following inner chunks and of the next
   // chunk on the caller's stream.  ev_fft[i % 2]: FFT of inner chunk i done.
