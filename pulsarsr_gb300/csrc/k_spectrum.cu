@@ -185,7 +185,7 @@ __device__ void emit(const HarmArgs &a, uint64_t trial, uint64_t k, int hi, doub
   base = __shfl_sync(mask, base, leader);
   const unsigned slot = base + (unsigned)__popc(mask & ((1u << lane) - 1u));
   if (slot >= a.raw_cap) {
-    atomicOr(a.overflow, 1u);
+    atomicOr(a.overflow, OVERFLOW_RAW);
     return;
   }
   RawCand c;
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(SC_NT)
       } else {
         const unsigned gi = atomicAdd(gcount, 1u);
         if (gi < g.qcap) gq[gi] = (uint32_t)(kb0 + (uint64_t)(i + j));
-        else atomicOr(a.overflow, 1u);
+        else atomicOr(a.overflow, OVERFLOW_QUEUE);
       }
       ++slot;
     }
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(SC_NT)
     base2 = atomicAdd(&g.n2[trial], (unsigned)m2);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && (base1 + m1 > g.qcap || base2 + m2 > g.qcap)) atomicOr(a.overflow, 1u);
+  if (threadIdx.x == 0 && (base1 + m1 > g.qcap || base2 + m2 > g.qcap)) atomicOr(a.overflow, OVERFLOW_QUEUE);
   for (int i = threadIdx.x; i < m1 && base1 + i < g.qcap; i += SC_NT)
     gq1[base1 + i] = (uint32_t)(kb0 + lq1[i]);
   for (int i = threadIdx.x; i < m2 && base2 + i < g.qcap; i += SC_NT)
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(HI_NT) k_harm_filter(HarmArgs a, GateArgs g) {
       at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1u));
       if (take) {
         if (at < g.xcap) xq[at] = entry[hi];
-        else atomicOr(a.overflow, 1u);
+        else atomicOr(a.overflow, OVERFLOW_QUEUE);
       }
     }
   }
@@ -952,7 +952,8 @@ int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint
   PSR_TRY(w.counts.ensure((4 * outer + 4) * 4));
   PSR_TRY(w.floors.ensure(outer * 4));
   // Gated bins are ~2% of a noise spectrum; a quarter of the bins is ample
-  // and an overflow (flagged) reruns the chunk with room for every bin.
+  // and an overflow (flagged) reruns the chunk with room for every bin.  Raw lists
+  // overflow on their own where a bright pulsar peaks in many bins.
   w.qcap = w.queue_full ? plen : plen / 4 + 1024;
   w.xcap = w.queue_full ? 6 * plen : w.qcap;  // every level of every bin at most
   PSR_TRY(w.gq.ensure(2 * outer * w.qcap * 4));

@@ -255,6 +255,8 @@ struct SpecConfig {
   std::vector<double> birdies;  // pairs
   int levels = 5;               // harmonic sums h = 1 .. 2^(levels-1)
 };
+// Bits of the overflow word: raw candidate lists; gate queues or exact lists.
+constexpr unsigned OVERFLOW_RAW = 1, OVERFLOW_QUEUE = 2;
 struct SpecWork {
   DevBuf scale, raw, counts, floors, birdies, gq, xq;
   uint64_t qcap = 0, xcap = 0;  // gate queue and exact list capacities per trial

@@ -107,6 +107,29 @@ int SearchEngine::enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st
                           aux));
     PSR_TRY(record(ST_SPEC, false, aux));
   }
+  PSR_TRY(enqueue_select(ci));
+  if (profile == 2) PSR_CUDA(cudaStreamWaitEvent(st, ev_sel[b], 0));
+  return PSR_OK;
+}
+
+int SearchEngine::enqueue_spectrum(uint64_t ci, cudaStream_t st) {
+  const uint64_t nt = cstart[ci + 1] - cstart[ci];
+  const int b = (int)(ci & 1);
+  const float *pw = power.as<float>() + (uint64_t)b * chunk * ldp;
+  const double *ps = psum.as<double>() + (uint64_t)b * chunk * npsum;
+  PSR_CUDA(cudaEventRecord(ev_fft[1], st));
+  PSR_CUDA(cudaStreamWaitEvent(aux, ev_fft[1], 0));
+  PSR_TRY(spectrum_reset(sw, nt, aux));
+  PSR_TRY(record(ST_SPEC, true, aux));
+  PSR_TRY(spectrum_gate(fft, spec, pw, ldp, ps, npsum, nt, 0, sw, aux));
+  PSR_TRY(record(ST_SPEC, false, aux));
+  return enqueue_select(ci);
+}
+
+int SearchEngine::enqueue_select(uint64_t ci) {
+  const uint64_t t0 = cstart[ci], nt = cstart[ci + 1] - t0;
+  const int b = (int)(ci & 1);
+  const float *pw = power.as<float>() + (uint64_t)b * chunk * ldp;
   const uint64_t maxc = std::max<uint64_t>(spec.max_candidates, 1);
   PSR_TRY(record(ST_SPEC, true, aux));
   PSR_TRY(spectrum_items(fft, spec, pw, ldp, nt, sw, aux));
@@ -118,7 +141,6 @@ int SearchEngine::enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st
                            cudaMemcpyDeviceToDevice, aux));
   PSR_CUDA(cudaEventRecord(ev_sel[b], aux));
   sel_pending[b] = true;
-  if (profile == 2) PSR_CUDA(cudaStreamWaitEvent(st, ev_sel[b], 0));
   return PSR_OK;
 }
 
@@ -186,18 +208,22 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
     return PSR_ETIMEOUT;
   }
   PSR_TRY(harvest());
-  for (uint64_t ci = 0; ci < nchunks; ++ci) {
+  // A chunk whose lists overflowed: grow what did and redo it.  The power
+  // spectra of the last two chunks still stand (those of others are made again), so
+  // the last come first.
+  for (uint64_t ci = nchunks; ci-- > 0;) {
+    bool stands = ci + 2 >= nchunks;
     int guard = 0;
     while (ov[ci]) {
-      // Raw candidate storage overflowed for this chunk: grow it and redo.
-      if (++guard > 8) {
+      if (++guard > 9) {
         set_error("search: raw candidate storage overflow");
         return PSR_ECAPACITY;
       }
-      sw.raw_cap *= 4;
-      sw.queue_full = true;
+      if (ov[ci] & OVERFLOW_RAW) sw.raw_cap *= 4;
+      if (ov[ci] & OVERFLOW_QUEUE) sw.queue_full = true;
       PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
-      PSR_TRY(enqueue_chunk(o, ci, st));
+      PSR_TRY(stands ? enqueue_spectrum(ci, st) : enqueue_chunk(o, ci, st));
+      stands = true;
       PSR_TRY(join(st));
       unsigned v = 0;
       PSR_CUDA(cudaMemcpyAsync(&v, status.as<unsigned>() + ci, 4,

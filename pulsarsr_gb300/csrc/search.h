@@ -66,6 +66,11 @@ struct SearchEngine {
   int prepare(const DeviceObs &o, const double *trials, uint64_t ntrials, uint64_t n,
               const SpecConfig &cfg, cudaStream_t st);
   int enqueue_chunk(const DeviceObs &o, uint64_t ci, cudaStream_t st);
+  // The chunk's spectrum work alone, on power spectra that still stand in its
+  // half of the buffers.
+  int enqueue_spectrum(uint64_t ci, cudaStream_t st);
+  // Items and selection of a chunk whose gates are queued on aux.
+  int enqueue_select(uint64_t ci);
   // All chunks, asynchronously (joined back into st).
   int enqueue(const DeviceObs &o, cudaStream_t st);
   // Make st wait for the aux-stream work queued so far.
