@@ -888,7 +888,7 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
   PSR_CUDA(cudaMemsetAsync(err.p, 0, 8, st));
   SubbandPlan sbp;
   PSR_TRY(build_subband_plan(tab, o.nch, length, o.kind == SAMPLE_U8 ? o.max_value() : 0.0,
-                             {0, ntrials}, dedisp_subbands_default(o), sbp, st));
+                             {0, ntrials}, dedisp_subbands_default(o), sbp, st, true));
   PSR_TRY(launch_dedisperse_ex(o, dd.as<uint32_t>(), ntrials, length, ser.as<float>(), ldo,
                                parts.as<double>(), sums.as<double>(), means.as<float>(), spread,
                                err.as<unsigned>(), st, 0, 0, sums_out != nullptr, &sbp, 0));
@@ -1010,6 +1010,7 @@ int psr_search_trials(const psr_fb *fb, const double *trials, uint64_t ntrials,
   cudaStream_t st = fb->stream.s;
   PoolScope scope(st);
   SearchEngine e;
+  e.once = true;
   PSR_TRY(e.prepare(fb->o, trials, ntrials, discovery, to_spec(cfg, fb->o.h.tsamp), st));
   PSR_TRY(e.enqueue(fb->o, st));
   PSR_TRY(e.finish(fb->o, st));

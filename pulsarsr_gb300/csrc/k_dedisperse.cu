@@ -1565,13 +1565,21 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
 
 int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool once) {
   plan.G = 0;
   plan.chunks.clear();
   if (G == 0 || cstart.size() < 2 || !(maxv > 0.0) || maxv > 255.0 ||
       (double)nch * maxv >= 16777216.0 || n < 2)
     return PSR_OK;
   if (G == 4 || G == 8) return subband_plan_at(tab, nch, n, maxv, cstart, G, plan, st);
+  // A plan for one pass has to save more than it takes to make: 25 ns per
+  // channel and trial, 150 us for its buffers and copies (299 channels, 59 trials
+  // of 131,000 to 400,000 samples: 0.3 to 0.5 ms, the kernels saved 0.1).  Seconds
+  // per unit of the costs below: 512 samples, four issue slots a clock of 152 SMs.
+  const double unit = (double)n / 512.0 / 1.155e12;
+  const uint64_t total = cstart.back() - cstart.front();
+  const double making = once ? 150e-6 + 25e-9 * (double)(nch * total) : 0.0;
+  if (once && 0.8 * unit * direct_cost(nch, total, maxv) < making) return PSR_OK;
   // The widths that are cheaper than the channel-by-channel kernel on the
   // middle chunk, cheapest first.
   const size_t mid = (cstart.size() - 2) / 2;
@@ -1583,7 +1591,8 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
     chunk_patterns(tab, nch, cstart[mid], cstart[mid + 1], g, p);
     if (!p.ok) continue;
     const double c = two_level_cost(p, nt, g, maxv);
-    if (c < direct_cost(nch, nt, maxv)) pick.emplace_back(c, g);
+    const double saved = direct_cost(nch, nt, maxv) - c;
+    if (saved > 0.0 && unit * saved * (double)total / (double)nt > making) pick.emplace_back(c, g);
   }
   std::sort(pick.begin(), pick.end());
   for (size_t i = 0; i < pick.size() && plan.G == 0; ++i) {

@@ -310,10 +310,11 @@ struct SubbandPlan {
 // setting of psr_set_dedisp_subbands (-1: chosen from the delay table).
 int dedisp_subbands_default(const DeviceObs &o);
 // n: series length; maxv: largest sample (0: no plan); G: 4, 8, 0 (no plan)
-// or -1 (the cheapest).  A plan that does not fit leaves plan.G = 0.
+// or -1 (the cheapest; with `once`, counting what the plan takes to make).  A plan
+// that does not fit leaves plan.G = 0.
 int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st);
+                       cudaStream_t st, bool once = false);
 // With want_means = false (series only folded, not searched) the sums and
 // means are left unset.  With a subband plan (8-bit-storage samples), chunk
 // chunk_index of the plan runs the two-level kernels.

@@ -63,7 +63,7 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   nchunks = cstart.size() - 1;
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
   PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
-                             sbplan, st));
+                             sbplan, st, once));
   PSR_TRY(status.ensure(nchunks * 4 + 16));
   PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));

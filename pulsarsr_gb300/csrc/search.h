@@ -15,6 +15,7 @@ struct SearchEngine {
   // channel, 4 or 8 = subband reuse, -1 = the library default
   // (dedisp_subbands_default()).
   int subbands = -1;
+  bool once = false;  // one pass only: a subband plan has to pay for itself
   SubbandPlan sbplan;
   uint64_t ntrials = 0, n = 0, nch = 0, ldo = 0, ldp = 0, nparts = 0, nchunks = 0;
   // Outer chunk ci covers trials [cstart[ci], cstart[ci + 1]).  A search of
