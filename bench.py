@@ -330,11 +330,12 @@ def run_ours(args):
     D = st["dedisperse"][1] // 2
     F = st["fft"][1] // 2
     fft_kernels = 2 if N // 2 > 4096 else 1
-    # unpack + 9 RFI kernels (8-bit storage: totals, mean/variance, block sums,
-    # median histograms + pick, channel and block decisions, block means,
-    # fill); per outer chunk dedispersion + part reduction + harmonic items +
-    # selection; per inner chunk the FFT pass(es) and the scales/gates kernel
-    launches = 1 + 9 + D * 4 + F * (fft_kernels + 1)
+    # unpack + 13 RFI kernels (8-bit storage: sums, guesses, two passes of maps
+    # and scans, block sums, median histograms + pick, channel and block
+    # decisions, block means, fill); per outer chunk dedispersion (one kernel more
+    # where it takes two levels) + part reduction + harmonic filter + exact scores
+    # + selection; per inner chunk the FFT pass(es), the floors and the gates
+    launches = 1 + 13 + D * 5 + F * (fft_kernels + 2)
     if rank != 0:
         if dist:
             dist.destroy_process_group()

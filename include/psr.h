@@ -223,8 +223,8 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials,
  * per distinct intra-subband delay pattern of a block of trials and added
  * shifted to every trial that shares it (identical results; a plan whose
  * patterns repeat too little falls back to 0); -1 (initial): the cheapest of
- * the three for the plan.  Process-wide; affects searches prepared
- * afterwards. */
+ * the three for the plan (calls that use it once count making it).
+ * Process-wide; affects searches prepared afterwards. */
 int psr_set_dedisp_subbands(int subbands);
 
 /* Test hook, no reference counterpart: one dedispersion launch (DM 0, up to
