@@ -306,62 +306,43 @@ __global__ void __launch_bounds__(MD_NT)
 }
 
 // 8-bit rows: the median from a 256-bin histogram (one pass).  Each row is
-// split over several CTAs; every thread counts into its own byte column of a
-// [256][MH_NT] table in shared memory (no atomics; thread t's byte is t / 64
-// of word t mod 64, so a warp's 32 columns are 32 banks).  A column is added
-// to the row's global histogram before 255 samples could overflow it.
+// split over several CTAs; a CTA's table has a column per lane, so that a warp's 32
+// counts, shared-memory atomics without a result, always fall in 32 banks.
+// Bound: the atomics, one per 32 samples.
 // Measured on a GB300: 512 channels of 1,047,799 samples 0.52 ms with 16-bit
-// columns (128 threads in the same 64 KB), 0.30 with one sample at a time in the
-// chain of a thread's counts, 0.27 now.
-constexpr int MH_NT = 256;
-constexpr int MH_RUNS = 15;  // 16-sample loads per thread between additions
-constexpr size_t MH_SMEM = 256 * MH_NT;
+// columns per thread, 0.27 with byte columns, read, incremented and written,
+// that were added up before they could overflow, 0.21 now; 64 channels of 262,144
+// samples 17 us, 11 now.
+constexpr int MH_NT = 256, MH_COL = 32;
+constexpr uint64_t MH_MIN = 16384, MH_MAX = 131072;  // samples per CTA
 
 __global__ void __launch_bounds__(MH_NT)
-    k_chan_hist_u8(const uint8_t *__restrict__ s, uint64_t ns, uint64_t ld,
+    k_chan_hist_u8(const uint8_t *__restrict__ s, uint64_t ns, uint64_t ld, uint64_t per,
                    unsigned *__restrict__ hist) {
-  extern __shared__ uint32_t h32[];
-  uint8_t *h8 = reinterpret_cast<uint8_t *>(h32);
+  __shared__ unsigned h[256 * MH_COL];
   const int tid = (int)threadIdx.x;
-  uint8_t *mine = h8 + (tid & 63) * 4 + (tid >> 6);
+  unsigned *mine = h + (tid & (MH_COL - 1));
   const uint8_t *row = s + (uint64_t)blockIdx.y * ld;
   // this CTA's range [a, b), a a multiple of 16 (rows are 64-byte aligned
   // and padded by >= 64 bytes, so whole 16-byte loads stay in the row)
-  const uint64_t per = (((ns + gridDim.x - 1) / gridDim.x) + 15) & ~15ull;
   const uint64_t a = (uint64_t)blockIdx.x * per, b = min(ns, a + per);
-  unsigned total = 0;  // of bin tid
-  for (uint64_t r0 = a; r0 < b; r0 += (uint64_t)MH_RUNS * MH_NT * 16) {
-#pragma unroll 4
-    for (int i = tid; i < 256 * MH_NT / 16; i += MH_NT)
-      reinterpret_cast<uint4 *>(h32)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    const uint64_t r1 = min(b, r0 + (uint64_t)MH_RUNS * MH_NT * 16);
-    for (uint64_t i = r0 + (uint64_t)tid * 16; i < r1; i += (uint64_t)MH_NT * 16) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + i));
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      const int m = (int)min((uint64_t)16, r1 - i);
-      if (m == 16) {
-        // two samples at a time: both counts are read before either is written
 #pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-          const uint32_t v = w[k >> 2] >> (8 * (k & 3));
-          uint8_t *p0 = mine + (v & 255u) * MH_NT, *p1 = mine + (v >> 8 & 255u) * MH_NT;
-          const uint8_t c0 = *p0 + 1, c1 = *p1 + 1;
-          *p0 = c0;
-          *p1 = p0 == p1 ? c0 + 1 : c1;
-        }
-      } else {
+  for (int i = tid; i < 256 * MH_COL / 4; i += MH_NT)
+    reinterpret_cast<uint4 *>(h)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+#pragma unroll 2
+  for (uint64_t i = a + (uint64_t)tid * 16; i < b; i += (uint64_t)MH_NT * 16) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + i));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const int m = (int)min((uint64_t)16, b - i);
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (k < m) mine[((w[k >> 2] >> (8 * (k & 3))) & 255u) * MH_NT] += 1;
-      }
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int j = 0; j < 64; ++j)
-      total = __dp4a(h32[tid * 64 + ((j + tid) & 63)], 0x01010101u, total);
-    __syncthreads();
+    for (int k = 0; k < 16; ++k)
+      if (k < m) atomicAdd(&mine[((w[k >> 2] >> (8 * (k & 3))) & 255u) * MH_COL], 1u);
   }
+  __syncthreads();
+  unsigned total = 0;  // of bin tid
+#pragma unroll 8
+  for (int j = 0; j < MH_COL; ++j) total += h[tid * MH_COL + ((j + tid) & (MH_COL - 1))];
   if (total) atomicAdd(&hist[(uint64_t)blockIdx.y * 256 + tid], total);
 }
 
@@ -1325,15 +1306,14 @@ static int rfi_enqueue_t(DeviceObs &o, uint64_t bs, float thr, RfiWork &w, cudaS
     k_block_sums<T><<<(unsigned)((nch * blocks_n + 127) / 128), 128, 0, st>>>(
         s, ns, o.ld, nch, bs, blocks_n, w.bsum.as<float>());
   if constexpr (sizeof(T) == 1) {
-    // a few column additions per CTA, and enough CTAs for every SM
-    constexpr uint64_t turn = (uint64_t)MH_RUNS * MH_NT * 16;
-    const uint64_t nsplit = std::max<uint64_t>(1, (ns + 2 * turn - 1) / (2 * turn));
+    // long shares (a table is cleared and added up per CTA), but enough CTAs for
+    // every SM
+    const uint64_t share = std::min(MH_MAX, std::max(MH_MIN, ns * nch / 1200));
+    const uint64_t per = (share + 15) / 16 * 16;
     PSR_TRY(w.mhist.ensure(nch * 256 * 4));
     PSR_CUDA(cudaMemsetAsync(w.mhist.p, 0, nch * 256 * 4, st));
-    PSR_CUDA(cudaFuncSetAttribute(k_chan_hist_u8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)MH_SMEM));
-    k_chan_hist_u8<<<dim3((unsigned)nsplit, (unsigned)nch), MH_NT, MH_SMEM, st>>>(
-        s, ns, o.ld, w.mhist.as<unsigned>());
+    k_chan_hist_u8<<<dim3((unsigned)((ns + per - 1) / per), (unsigned)nch), MH_NT, 0, st>>>(
+        s, ns, o.ld, per, w.mhist.as<unsigned>());
     k_hist_median<<<(unsigned)((nch + 3) / 4), 128, 0, st>>>(w.mhist.as<unsigned>(), nch, ns,
                                                                  w.med.as<float>());
   } else {
