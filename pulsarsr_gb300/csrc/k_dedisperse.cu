@@ -521,11 +521,15 @@ __global__ void __launch_bounds__(SP_NT)
 // row list read two stages ahead.  Waits are bounded; one that gives up sets
 // the error word and `dead`, on which every warp leaves, the issuing warp
 // last, after the copies it has in flight.
-// Bound: the staged rows, about 5 TB/s of bulk copies out of L2 (a row serves
-// the trials of its block that share the pattern, 4 to 5 of 16 at G = 4), then
-// shared-memory loads, 2 bytes per (trial, subband, sample), two instructions
-// per word.  With the copies issued by a trial warp between two CTA barriers
-// and two buffers the 4096-channel case took 50.5 ms, with the ring 27.9.
+// Bound: shared-memory loads, 2 bytes per (trial, subband, sample) in two
+// instructions per word: two thirds of the wavefronts and of the issue slots at
+// 512 channels, with 16 trial warps per SM to hide the rest (the copies out of L2 take
+// a tenth of the crossbar; a row serves the trials of its block that share the
+// pattern, 4 to 5 of 16 at G = 4).  With the copies issued by a trial warp between
+// two CTA barriers and two buffers the 4096-channel case took 50.5 ms, with the ring
+// 27.9; with 24 trials per CTA 33.8 (72 registers leave fewer loads in flight),
+// with two trials per warp on one window of words 56.5, with several tiles per CTA
+// 32.3 (CTAs of one tile no longer run side by side, and rows miss L2).
 template <bool FLUSH>
 __global__ void __launch_bounds__(SS_NT, FLUSH ? 1 : 2)
     k_sub_sum(const uint16_t *__restrict__ scratch, uint64_t ldp,
@@ -1365,8 +1369,7 @@ void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta,
 // 512 and 4096 channels, 64 to 256 trials, both widths): a channel of a trial
 // costs the channel-by-channel kernel 38 (<= 4-bit samples) or 62; a pattern
 // costs k_sub_part 80 + 50 G or 310 + 38 G (the write of its row included);
-// k_sub_sum is bound by the rows it stages, 280 each, or by 32 per (trial,
-// subband) of shared-memory loads.
+// k_sub_sum 280 per row it stages, or 32 per (trial, subband), whichever is more.
 double direct_cost(uint64_t nch, uint64_t nt, double maxv) {
   return (maxv * 2.0 <= 255.0 ? 38.0 : 62.0) * (double)nch * (double)nt;
 }
