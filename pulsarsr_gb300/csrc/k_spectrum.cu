@@ -512,7 +512,9 @@ __global__ void __launch_bounds__(SC_NT)
       const int i = 4 * (i0 + u * SC_NT + (int)threadIdx.x);
       r[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       edge[u] = 0.0f;
-      if (i < own && i + 3 >= ilo && i <= ihi) {
+      // (one bin past the last candidate: the group before it, if full, takes
+      // its last bin's neighbour from here; at most bin plen + 1 of the padded row)
+      if (i < own && i + 3 >= ilo && i <= ihi + 1) {
         r[u] = *reinterpret_cast<const float4 *>(raw + kb0 + (uint64_t)i);
         if (lane == 31 && i + 4 < own && i + 3 <= ihi) edge[u] = raw[kb0 + (uint64_t)(i + 4)];
       }
