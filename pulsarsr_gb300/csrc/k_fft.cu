@@ -400,32 +400,28 @@ struct Acc2 {
   }
 };
 
-// Block total of the per-thread (hi, lo) pairs: TwoSum merges in f32 across
-// the warp, then across the warps; f64 only for the last pair (FP64 runs at
-// 1/64 of the f32 rate: 16 warps' pairs added in f64 by one thread held every
-// CTA of pass 2 for about 1500 cycles).
+// Block total of the per-thread (hi, lo) pairs: TwoSum merges across the warp in
+// f32, the warps' pairs in f64, a lane each (FP64 runs at 1/64 of the f32 rate:
+// 16 pairs added by one thread held every CTA of pass 2 for about 1500 cycles).
 template <int NT>
 __device__ __forceinline__ void block_sum_store(Acc2 acc, double *dst) {
   constexpr int NW = NT / 32 > 0 ? NT / 32 : 1;
   __shared__ float2 red[NW];
-  auto merge = [&](int from) {
 #pragma unroll
-    for (int o = from; o; o >>= 1) {
-      const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
-      const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
-      acc.add(oh);
-      acc.lo = __fadd_rn(acc.lo, ol);
-    }
-  };
-  merge(16);
+  for (int o = 16; o; o >>= 1) {
+    const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
+    const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
+    acc.add(oh);
+    acc.lo = __fadd_rn(acc.lo, ol);
+  }
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(acc.hi, acc.lo);
   __syncthreads();
   if (threadIdx.x < 32) {
     const int w = (int)threadIdx.x;
-    acc.hi = w < NW ? red[w].x : 0.0f;
-    acc.lo = w < NW ? red[w].y : 0.0f;
-    merge(NW / 2 > 0 ? NW / 2 : 0);
-    if (w == 0) *dst = (double)acc.hi + (double)acc.lo;
+    double t = w < NW ? (double)red[w].x + (double)red[w].y : 0.0;
+#pragma unroll
+    for (int o = NW / 2; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (w == 0) *dst = t;
   }
 }
 
