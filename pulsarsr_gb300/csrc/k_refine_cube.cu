@@ -183,41 +183,58 @@ struct RunSums {
     sq = (double)q;
   }
 };
-// f32 sums of v and v^2 over a chunk of 4 (or a run of 32) join (hi, lo)
-// pairs by TwoSum, which keep 38 bits or more of any number of terms where each
-// term has 24; only what passes f32's range goes to f64 (FP64 runs at 1/64 of the
-// f32 rate: two conversions and two sums per chunk and f64 shuffles were half
-// of the time of the fold).
+// f32 sums of v and v^2 over a chunk of 4 (or a run of 32) join sums of three
+// f32 words, each the exact error of the one before (TwoSum): with the 24 bits
+// of the terms nothing is lost that an f64 sum keeps.  What passes f32's range
+// goes to f64 (FP64 runs at 1/64 of the f32 rate: two conversions and two sums
+// per chunk and f64 shuffles were half of the time of the fold).
+struct Sum3 {
+  float h = 0.0f, l = 0.0f, m = 0.0f;
+  // a + b, the error left in b
+  static __device__ __forceinline__ void two_sum(float &a, float &b) {
+    const float t = __fadd_rn(a, b), v = __fsub_rn(t, a);
+    b = __fadd_rn(__fsub_rn(a, __fsub_rn(t, v)), __fsub_rn(b, v));
+    a = t;
+  }
+  __device__ __forceinline__ void add(float x) {
+    two_sum(h, x);
+    two_sum(l, x);
+    m = __fadd_rn(m, x);
+  }
+  __device__ __forceinline__ void add(const Sum3 &o) {
+    add(o.h);
+    float x = o.l;
+    two_sum(l, x);
+    m = __fadd_rn(m, __fadd_rn(x, o.m));
+  }
+  __device__ __forceinline__ bool finite() const { return isfinite(h) && isfinite(l) && isfinite(m); }
+  __device__ __forceinline__ double value() const {
+    return (double)h + ((double)l + (double)m);
+  }
+  __device__ __forceinline__ Sum3 from(int o) const {  // the lane o above's
+    Sum3 x;
+    x.h = __shfl_down_sync(0xffffffffu, h, o);
+    x.l = __shfl_down_sync(0xffffffffu, l, o);
+    x.m = __shfl_down_sync(0xffffffffu, m, o);
+    return x;
+  }
+};
 template <>
 struct RunSums<float> {
-  struct Pair {
-    float h = 0.0f, l = 0.0f;
-    __device__ __forceinline__ void add(float x) {
-      const float t = __fadd_rn(h, x), b = __fsub_rn(t, h);
-      l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(x, b)));
-      h = t;
-    }
-    __device__ __forceinline__ void add(const Pair &o) {
-      add(o.h);
-      l = __fadd_rn(l, o.l);
-    }
-    __device__ __forceinline__ bool finite() const { return isfinite(h) && isfinite(l); }
-    __device__ __forceinline__ double value() const { return (double)h + (double)l; }
-  };
-  Pair ps, pq, ts, tq;       // so far; of the open tile
+  Sum3 ps, pq, ts, tq;      // so far; of the open tile
   double s = 0.0, q = 0.0;  // what passed f32's range
-  __device__ __forceinline__ void join(const Pair &a, const Pair &b) {
-    const Pair os = ps, oq = pq;
+  __device__ __forceinline__ void join(const Sum3 &a, const Sum3 &b) {
+    const Sum3 os = ps, oq = pq;
     ps.add(a);
     pq.add(b);
     if (!(ps.finite() && pq.finite())) {
       s += os.value() + a.value();
       q += oq.value() + b.value();
-      ps = pq = Pair();
+      ps = pq = Sum3();
     }
   }
   __device__ __forceinline__ void add(const RunRegs<float> &x) {
-    Pair a, b;
+    Sum3 a, b;
 #pragma unroll
     for (int i = 0; i < CB_RUN; ++i) {
       const float v = run_sample<float>(x, i);
@@ -253,20 +270,15 @@ struct RunSums<float> {
         q += (double)cq;
       }
     }
-    ts = tq = Pair();
+    ts = tq = Sum3();
   }
   // Lane 0: the warp's sums.
   __device__ __forceinline__ void warp_total(double &sum, double &sq) {
-    Pair a = ps, b = pq;
+    Sum3 a = ps, b = pq;
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
-      Pair x, y;
-      x.h = __shfl_down_sync(0xffffffffu, a.h, o);
-      x.l = __shfl_down_sync(0xffffffffu, a.l, o);
-      y.h = __shfl_down_sync(0xffffffffu, b.h, o);
-      y.l = __shfl_down_sync(0xffffffffu, b.l, o);
-      a.add(x);
-      b.add(y);
+      a.add(a.from(o));
+      b.add(b.from(o));
     }
     const bool wide = __shfl_sync(0xffffffffu, !(a.finite() && b.finite()), 0);
     sum = wide ? 0.0 : a.value();
