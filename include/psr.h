@@ -235,6 +235,15 @@ int psr_set_dedisp_subbands(int subbands);
  * kernel (f32, or sums that could pass 2^24).  The CUDA context stays usable. */
 int psr_test_stage_timeout(const psr_fb *fb, uint64_t spin_limit);
 
+/* Test hook, no reference counterpart; needs no device: the two-level plan that
+ * the delays [ntrials][nch] of `chunk` trials at a time would get for series of n
+ * samples of at most max_value, `subbands` as in psr_set_dedisp_subbands (once: as
+ * in a call that uses the plan once).  info: width (0: channel by channel),
+ * whether the 16-bit sums are flushed, samples per segment, segments, bytes of
+ * scratch. */
+int psr_test_subband_plan(const uint32_t *delays, uint64_t nch, uint64_t ntrials, uint64_t chunk,
+                          uint64_t n, double max_value, int subbands, int once, uint64_t *info);
+
 /* ------------------------------------------------------------ search */
 /* The raw power spectrum of search::periodicity (search/src/lib.rs:35-44):
  * mean removal, zero padding to N = 2*next_pow2(len), real FFT, |X|^2.

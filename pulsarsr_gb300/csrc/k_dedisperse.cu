@@ -1397,21 +1397,28 @@ int dedisp_subbands_default(const DeviceObs &o) {
 }
 
 namespace {
-// The plan at width G; plan.G stays 0 when it does not fit.  `known`: the
-// patterns of chunk known_ci at this width, or null.
-int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
-                    const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                    cudaStream_t st, const ChunkPatterns *known = nullptr,
-                    size_t known_ci = 0) {
-  const bool byte_part = maxv * SUB_GMAX <= 255.0;
-  const bool flush = (double)nch * maxv > 65535.0;
-  const size_t nchunks = cstart.size() - 1;
-  const uint64_t nsub = (nch + G - 1) / G;
+// A plan's tables on the host, and the shape that the plan takes from them.
+struct SubbandTables {
+  SubbandPlan::Shape shape;
   std::vector<SubBand> subs;
   std::vector<uint16_t> rel;
   std::vector<uint32_t> stage0, rowlist0, stages, info;
   std::vector<SubRow> rows;
   std::vector<SubbandPlan::Chunk> chunks;
+};
+constexpr uint64_t SUB_GRID = 65535;  // tiles of a segment: grid.y
+static_assert(32 * SS_MAXSTAGES <= SUB_GRID, "as do the subbands of any plan that fits");
+
+// The tables at width G; false when the plan does not fit.  `known`: the
+// patterns of chunk known_ci at this width, or null.
+bool subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
+                    const std::vector<uint64_t> &cstart, int G, SubbandTables &out,
+                    const ChunkPatterns *known = nullptr, size_t known_ci = 0) {
+  const bool flush = (double)nch * maxv > 65535.0;
+  const size_t nchunks = cstart.size() - 1;
+  const uint64_t nsub = (nch + G - 1) / G;
+  out = SubbandTables();
+  auto &[shape, subs, rel, stage0, rowlist0, stages, info, rows, chunks] = out;
   struct Win {  // a row a trial block uses: offsets [lo, hi] of its trials
     uint32_t row, lo, hi;
   };
@@ -1425,12 +1432,12 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
   size_t most = 0;
   for (size_t ci = 0; ci < nchunks; ++ci) {
     const uint64_t ta = cstart[ci], nt = cstart[ci + 1] - ta;
-    if (nt == 0) return PSR_OK;
+    if (nt == 0) return false;
     ChunkPatterns own;
     const bool have = known && ci == known_ci;
     if (!have) chunk_patterns(tab, nch, ta, ta + nt, G, own);
     const ChunkPatterns &cp = have ? *known : own;
-    if (!cp.ok) return PSR_OK;
+    if (!cp.ok) return false;
     SubbandPlan::Chunk c;
     c.sub0 = subs.size();
     c.rel0 = rel.size();
@@ -1484,15 +1491,16 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
   const uint64_t bufbytes = ((uint64_t)maxrows * rowcap + 127) & ~127ull;
   const int nbuf = (int)std::min<uint64_t>(SS_MAXBUF, room / bufbytes);
   const uint64_t prowcap = ((uint64_t)SP_TT + relmax + 36 + 15) & ~15ull;
-  if (nbuf < 2 || prowcap * G > SP_MAXSMEM) return PSR_OK;
-  // Segments of the series: the scratch of one stays within SUB_SCRATCH.
+  if (nbuf < 2 || prowcap * G > SP_MAXSMEM) return false;
+  // Segments of the series: the scratch of one stays within SUB_SCRATCH, its
+  // tiles within a grid.
   const uint64_t tail = max_spread + rowcap / 2 + 16;
-  uint64_t seg = ((n + SS_TT - 1) / SS_TT) * SS_TT;
+  uint64_t seg = std::min((n + SS_TT - 1) / SS_TT, SUB_GRID) * SS_TT;
   auto stride = [&](uint64_t sg) { return ((sg + tail + SP_TT - 1) / SP_TT) * SP_TT; };
   if (max_rows * stride(seg) * 2 > SUB_SCRATCH) {
     const uint64_t per = SUB_SCRATCH / (2 * max_rows);
     seg = per > tail + SP_TT ? ((per - tail - SP_TT) / SS_TT) * SS_TT : 0;
-    if (seg < 16 * SS_TT) return PSR_OK;  // rows too many to reuse
+    if (seg < 16 * SS_TT) return false;  // rows too many to reuse
   }
   const uint64_t ldp = stride(seg);
   // Stages: subbands in order while their rows fit the buffer; a stage after
@@ -1532,49 +1540,42 @@ int subband_plan_at(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
         nsubs += 1;
       }
       stages.push_back(sub_stage(nrows, nsubs, 0));
-      if (stages.size() - stage0.back() > SS_MAXSTAGES) return PSR_OK;
+      if (stages.size() - stage0.back() > SS_MAXSTAGES) return false;
     }
   }
   stage0.push_back((uint32_t)stages.size());
-  auto up = [&](DevBuf &b, const void *src, size_t bytes) -> int {
-    PSR_TRY(b.ensure(bytes));
-    PSR_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
-    return PSR_OK;
-  };
-  PSR_TRY(up(plan.subs, subs.data(), subs.size() * sizeof(SubBand)));
-  PSR_TRY(up(plan.rel, rel.data(), rel.size() * 2));
-  PSR_TRY(up(plan.stage0, stage0.data(), stage0.size() * 4));
-  PSR_TRY(up(plan.stages, stages.data(), stages.size() * 4));
-  PSR_TRY(up(plan.rowlist0, rowlist0.data(), rowlist0.size() * 4));
-  PSR_TRY(up(plan.rows, rows.data(), rows.size() * sizeof(SubRow)));
-  PSR_TRY(up(plan.info, info.data(), info.size() * 4));
-  PSR_TRY(plan.scratch.ensure(max_rows * ldp * 2 + 256));
-  PSR_CUDA(cudaStreamSynchronize(st));
-  plan.G = G;
-  plan.nsub = nsub;
-  plan.byte_part = byte_part;
-  plan.flush = flush;
-  plan.seg = seg;
-  plan.ldp = ldp;
-  plan.rowcap = (int)rowcap;
-  plan.prowcap = (int)prowcap;
-  plan.bufbytes = (int)bufbytes;
-  plan.nbuf = nbuf;
-  plan.chunks = std::move(chunks);
-  return PSR_OK;
+  shape.G = G;
+  shape.nsub = nsub;
+  shape.byte_part = maxv * SUB_GMAX <= 255.0;
+  shape.flush = flush;
+  shape.seg = seg;
+  shape.ldp = ldp;
+  shape.scratch_bytes = max_rows * ldp * 2 + 256;
+  shape.rowcap = (int)rowcap;
+  shape.prowcap = (int)prowcap;
+  shape.bufbytes = (int)bufbytes;
+  shape.nbuf = nbuf;
+  return true;
 }
 
-}  // namespace
-
-int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
-                       const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st, bool once) {
-  plan.G = 0;
-  plan.chunks.clear();
+// The tables at width G (4 or 8), or at the cheapest that pays (-1); shape.G is 0
+// where there is no plan.
+void choose_subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
+                           const std::vector<uint64_t> &cstart, int G, bool once,
+                           SubbandTables &t) {
+  t = SubbandTables();
   if (G == 0 || cstart.size() < 2 || !(maxv > 0.0) || maxv > 255.0 ||
       (double)nch * maxv >= 16777216.0 || n < 2)
-    return PSR_OK;
-  if (G == 4 || G == 8) return subband_plan_at(tab, nch, n, maxv, cstart, G, plan, st);
+    return;
+  auto take = [&](int g, const ChunkPatterns *known, size_t known_ci) {
+    const bool fits = subband_tables(tab, nch, n, maxv, cstart, g, t, known, known_ci);
+    if (!fits) t = SubbandTables();
+    return fits;
+  };
+  if (G == 4 || G == 8) {
+    take(G, nullptr, 0);
+    return;
+  }
   // A plan for one pass has to save more than it takes to make: 25 ns per
   // channel and trial, 150 us for its buffers and copies (299 channels, 59 trials
   // of 131,000 to 400,000 samples: 0.3 to 0.5 ms, the kernels saved 0.1).  Seconds
@@ -1582,7 +1583,7 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
   const double unit = (double)n / 512.0 / 1.155e12;
   const uint64_t total = cstart.back() - cstart.front();
   const double making = once ? 150e-6 + 25e-9 * (double)(nch * total) : 0.0;
-  if (once && 0.8 * unit * direct_cost(nch, total, maxv) < making) return PSR_OK;
+  if (once && 0.8 * unit * direct_cost(nch, total, maxv) < making) return;
   // The widths that are cheaper than the channel-by-channel kernel on the
   // middle chunk, cheapest first.
   const size_t mid = (cstart.size() - 2) / 2;
@@ -1598,10 +1599,36 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
     if (saved > 0.0 && unit * saved * (double)total / (double)nt > making) pick.emplace_back(c, g);
   }
   std::sort(pick.begin(), pick.end());
-  for (size_t i = 0; i < pick.size() && plan.G == 0; ++i) {
-    const int g = pick[i].second;
-    PSR_TRY(subband_plan_at(tab, nch, n, maxv, cstart, g, plan, st, &cp[g == 4], mid));
-  }
+  for (const auto &p : pick)
+    if (take(p.second, &cp[p.second == 4], mid)) return;
+}
+
+}  // namespace
+
+int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
+                       const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
+                       cudaStream_t st, bool once) {
+  SubbandTables t;
+  choose_subband_tables(tab, nch, n, maxv, cstart, G, once, t);
+  static_cast<SubbandPlan::Shape &>(plan) = SubbandPlan::Shape();
+  plan.chunks.clear();
+  if (t.shape.G == 0) return PSR_OK;
+  auto up = [&](DevBuf &b, const auto &v) -> int {
+    PSR_TRY(b.ensure(v.size() * sizeof(v[0])));
+    PSR_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st));
+    return PSR_OK;
+  };
+  PSR_TRY(up(plan.subs, t.subs));
+  PSR_TRY(up(plan.rel, t.rel));
+  PSR_TRY(up(plan.stage0, t.stage0));
+  PSR_TRY(up(plan.stages, t.stages));
+  PSR_TRY(up(plan.rowlist0, t.rowlist0));
+  PSR_TRY(up(plan.rows, t.rows));
+  PSR_TRY(up(plan.info, t.info));
+  PSR_TRY(plan.scratch.ensure(t.shape.scratch_bytes));
+  PSR_CUDA(cudaStreamSynchronize(st));
+  static_cast<SubbandPlan::Shape &>(plan) = t.shape;
+  plan.chunks = std::move(t.chunks);
   return PSR_OK;
 }
 
@@ -1779,6 +1806,28 @@ uint64_t dedisperse_part_count(const DeviceObs &o, uint64_t n) {
 }
 
 }  // namespace psr
+
+extern "C" int psr_test_subband_plan(const uint32_t *delays, uint64_t nch, uint64_t ntrials,
+                                     uint64_t chunk, uint64_t n, double max_value, int subbands,
+                                     int once, uint64_t *info) {
+  if (!delays || !info || nch == 0 || ntrials == 0 || chunk == 0) {
+    psr::set_error("test_subband_plan: a delay table and room for the result");
+    return PSR_EINVAL;
+  }
+  std::vector<uint64_t> cstart;
+  for (uint64_t t = 0; t < ntrials; t += chunk) cstart.push_back(t);
+  cstart.push_back(ntrials);
+  psr::SubbandTables t;
+  psr::choose_subband_tables(std::vector<uint32_t>(delays, delays + nch * ntrials), nch, n,
+                             max_value, cstart, subbands, once != 0, t);
+  const psr::SubbandPlan::Shape &p = t.shape;
+  info[0] = (uint64_t)p.G;
+  info[1] = p.flush;
+  info[2] = p.seg;
+  info[3] = p.seg ? (n + p.seg - 1) / p.seg : 0;
+  info[4] = p.scratch_bytes;
+  return PSR_OK;
+}
 
 extern "C" int psr_set_dedisp_subbands(int subbands) {
   if (subbands != -1 && subbands != 0 && subbands != 4 && subbands != 8) {

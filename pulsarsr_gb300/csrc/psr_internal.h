@@ -294,15 +294,19 @@ int make_delay_table(const DeviceObs &o, const double *trials, uint64_t ntrials,
 // intra-subband delay patterns (rows of `scratch`), and per block of 16 trials
 // the rows to stage and every trial's shift in them.  G = 0: no plan, channel
 // by channel.  `scratch` belongs to the stream that runs the searches.
-struct SubbandPlan {
-  struct Chunk {
-    uint64_t sub0, rel0, block0, nblocks, spread;
-  };
+struct SubbandShape {
   int G = 0;
   bool byte_part = false, flush = false;
   uint64_t nsub = 0;
   uint64_t seg = 0, ldp = 0;  // samples per segment, row stride of scratch
+  uint64_t scratch_bytes = 0;
   int rowcap = 0, prowcap = 0, bufbytes = 0, nbuf = 0;
+};
+struct SubbandPlan : SubbandShape {
+  typedef SubbandShape Shape;
+  struct Chunk {
+    uint64_t sub0, rel0, block0, nblocks, spread;
+  };
   std::vector<Chunk> chunks;
   DevBuf subs, rel, stage0, rowlist0, stages, rows, info, scratch;
 };
