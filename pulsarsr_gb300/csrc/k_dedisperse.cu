@@ -1323,7 +1323,7 @@ void chunk_patterns(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t ta,
         m = std::min(m, d[c]);
         mx = std::max(mx, d[c]);
       }
-      if (mx - m > 4095u) {
+      if (mx - m > 4095u || mx > (uint32_t)INT32_MAX) {  // SubBand holds 31 bits
         cp.ok = false;
         break;
       }

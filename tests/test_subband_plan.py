@@ -31,6 +31,11 @@ def test_tiles_of_a_segment(subbands, tiles):
     assert (nseg - 1) * seg < n <= nseg * seg
 
 
+@pytest.mark.parametrize("delay,want", [(2 ** 31 - 1, 4), (2 ** 31, 0), (2 ** 32 - 1, 0)])
+def test_delays_of_31_bits(delay, want):
+    assert plan(np.full((3, 6), delay), 5000, 255.0, 4)[0] == want
+
+
 @pytest.mark.gpu
 def test_more_tiles_than_a_grid(gpu):
     from pulsarsr_gb300 import dedisperse, synth
