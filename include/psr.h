@@ -227,6 +227,12 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials,
  * Process-wide; affects searches prepared afterwards. */
 int psr_set_dedisp_subbands(int subbands);
 
+/* Test hook, no reference counterpart: the device memory that buffers made on the
+ * calling thread hold, the most they held and the cudaMalloc calls they took since
+ * the last call of this; from now on the thread's allocations fail as out of memory
+ * that would take it past `limit` bytes (0: no limit).  Any pointer may be NULL. */
+int psr_test_device_memory(uint64_t limit, uint64_t *held, uint64_t *peak, uint64_t *mallocs);
+
 /* Test hook, no reference counterpart: one dedispersion launch (DM 0, up to
  * 8192 samples) whose staged kernel arms its TMA barriers but issues no
  * copy, so every bounded wait runs out after spin_limit polls (1..2^26) with

@@ -64,7 +64,15 @@ PoolScope::PoolScope(cudaStream_t s) : st(s), outer(t_scope) { t_scope = this; }
 PoolScope::~PoolScope() { t_scope = outer; }
 PoolScope *PoolScope::current() { return t_scope; }
 
-cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled) {
+namespace {
+// What this thread's buffers hold, for tests (psr_test_device_memory).
+struct ThreadMemory {
+  int64_t held = 0, peak = 0, limit = INT64_MAX;
+  uint64_t mallocs = 0;
+};
+thread_local ThreadMemory t_mem;
+
+cudaError_t alloc_raw(void **p, size_t n, cudaStream_t &st, bool &pooled) {
   pooled = false;
   if (t_scope && n <= POOL_BLOCK) {
     const cudaMemPool_t pool = device_pool();
@@ -92,6 +100,24 @@ cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled) {
     }
   }
   return e;
+}
+}  // namespace
+
+cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled) {
+  if ((int64_t)n > t_mem.limit - t_mem.held) return cudaErrorMemoryAllocation;
+  const cudaError_t e = alloc_raw(p, n, st, pooled);
+  if (e == cudaSuccess) {
+    t_mem.held += (int64_t)n;
+    t_mem.peak = std::max(t_mem.peak, t_mem.held);
+    t_mem.mallocs += !pooled;
+  }
+  return e;
+}
+
+void device_free(void *p, size_t n, cudaStream_t st, bool pooled) {
+  if (pooled) cudaFreeAsync(p, st);
+  else cudaFree(p);
+  t_mem.held -= (int64_t)n;
 }
 
 // ------------------------------------------------------- fbank header
@@ -915,6 +941,16 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
     set_error("dedispersion: a bounded wait for a staged tile gave up");
     return PSR_ETIMEOUT;
   }
+  return PSR_OK;
+}
+
+int psr_test_device_memory(uint64_t limit, uint64_t *held, uint64_t *peak, uint64_t *mallocs) {
+  if (held) *held = (uint64_t)std::max<int64_t>(t_mem.held, 0);
+  if (peak) *peak = (uint64_t)std::max<int64_t>(t_mem.peak, 0);
+  if (mallocs) *mallocs = t_mem.mallocs;
+  t_mem.limit = limit && limit < (uint64_t)INT64_MAX ? (int64_t)limit : INT64_MAX;
+  t_mem.peak = t_mem.held;
+  t_mem.mallocs = 0;
   return PSR_OK;
 }
 

@@ -1618,15 +1618,23 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
     PSR_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st));
     return PSR_OK;
   };
-  PSR_TRY(up(plan.subs, t.subs));
-  PSR_TRY(up(plan.rel, t.rel));
-  PSR_TRY(up(plan.stage0, t.stage0));
-  PSR_TRY(up(plan.stages, t.stages));
-  PSR_TRY(up(plan.rowlist0, t.rowlist0));
-  PSR_TRY(up(plan.rows, t.rows));
-  PSR_TRY(up(plan.info, t.info));
-  PSR_TRY(plan.scratch.ensure(t.shape.scratch_bytes));
-  PSR_CUDA(cudaStreamSynchronize(st));
+  auto all = [&]() -> int {
+    PSR_TRY(plan.scratch.ensure(t.shape.scratch_bytes));
+    PSR_TRY(up(plan.subs, t.subs));
+    PSR_TRY(up(plan.rel, t.rel));
+    PSR_TRY(up(plan.stage0, t.stage0));
+    PSR_TRY(up(plan.stages, t.stages));
+    PSR_TRY(up(plan.rowlist0, t.rowlist0));
+    PSR_TRY(up(plan.rows, t.rows));
+    PSR_TRY(up(plan.info, t.info));
+    PSR_CUDA(cudaStreamSynchronize(st));
+    return PSR_OK;
+  };
+  if (all() != PSR_OK) {  // no memory for it: channel by channel
+    cudaGetLastError();
+    plan.release();
+    return PSR_OK;
+  }
   static_cast<SubbandPlan::Shape &>(plan) = t.shape;
   plan.chunks = std::move(t.chunks);
   return PSR_OK;

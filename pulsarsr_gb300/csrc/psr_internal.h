@@ -85,6 +85,7 @@ struct PoolScope {
 };
 // cudaMalloc, or the current scope's pool (pooled is set then).
 cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled);
+void device_free(void *p, size_t n, cudaStream_t st, bool pooled);
 
 // Page-locked host memory, grown on demand and kept across calls (device
 // copies into it run at full link speed, with no staging and no page faults).
@@ -137,8 +138,7 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p && pooled) cudaFreeAsync(p, st);
-    if (p && !pooled) cudaFree(p);
+    if (p) device_free(p, bytes, st, pooled);
     p = nullptr;
     bytes = 0;
   }
@@ -309,13 +309,18 @@ struct SubbandPlan : SubbandShape {
   };
   std::vector<Chunk> chunks;
   DevBuf subs, rel, stage0, rowlist0, stages, rows, info, scratch;
+  void release() {
+    for (DevBuf *b : {&subs, &rel, &stage0, &rowlist0, &stages, &rows, &info, &scratch})
+      b->release();
+  }
 };
 // The subband width searches use when not told otherwise: the process-wide
 // setting of psr_set_dedisp_subbands (-1: chosen from the delay table).
 int dedisp_subbands_default(const DeviceObs &o);
 // n: series length; maxv: largest sample (0: no plan); G: 4, 8, 0 (no plan)
 // or -1 (the cheapest; with `once`, counting what the plan takes to make).  A plan
-// that does not fit leaves plan.G = 0.
+// that does not fit, or for which there is no device memory, leaves plan.G = 0 and
+// plan's buffers empty.
 int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
                        cudaStream_t st, bool once = false);

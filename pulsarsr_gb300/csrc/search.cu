@@ -61,11 +61,11 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   if (tail && ntrials - tail - cstart.back() >= chunk / 4) cstart.push_back(ntrials - tail);
   cstart.push_back(ntrials);
   nchunks = cstart.size() - 1;
+  PSR_TRY(status.ensure(nchunks * 4 + 16));
+  PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
   PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
                              sbplan, st, once));
-  PSR_TRY(status.ensure(nchunks * 4 + 16));
-  PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&ev_fft[0], &ev_fft[1], &ev_sel[0], &ev_sel[1]})
     if (!*e) PSR_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));

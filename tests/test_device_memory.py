@@ -1,0 +1,56 @@
+"""Device memory of the searches: what is only a faster way gives way where it does
+not fit, and buffers that a plan no longer needs are returned."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+MIB = 1 << 20
+
+
+def memory(limit=0):
+    """(held, peak, cudaMalloc calls) of this thread's buffers since the last call; a
+    limit in bytes from now on."""
+    from pulsarsr_gb300._lib import check, lib
+    v = [C.c_uint64() for _ in range(3)]
+    check(lib().psr_test_device_memory(C.c_uint64(limit), *(C.byref(x) for x in v)))
+    return tuple(int(x.value) for x in v)
+
+
+@pytest.fixture
+def observation(gpu):
+    """64 8-bit channels x 60,000 samples and 48 trials a sample apart; all limits
+    and widths back to their defaults afterwards."""
+    from pulsarsr_gb300 import dedisperse, synth
+    fb = synth.device(64, 8, 60000, 64e-6, 1500.0, -4.0, seed=3, noise_mean=100.0,
+                      noise_sigma=20.0, pulsars=[synth.Pulsar(0.01, 20.0, 0.1, 3.0)])
+    trials = dedisperse.dm_step(fb.header.frequencies(), 64e-6) * np.arange(48)
+    yield fb, trials
+    memory(0)
+    dedisperse.set_subbands(-1)
+
+
+def config():
+    from pulsarsr_gb300 import search
+    return search.Config(min_hz=2.0, max_hz=3000.0, threshold=7.0)
+
+
+@pytest.mark.gpu
+def test_plan_that_does_not_fit(observation):
+    """The two-level plan's scratch past the memory left: channel by channel."""
+    from pulsarsr_gb300 import dedisperse, search
+    fb, trials = observation
+    for call in (lambda: dedisperse.apply_trials(fb, trials, 50000),
+                 lambda: search.search_trials(fb, trials, 50000, config())):
+        dedisperse.set_subbands(0)
+        held = memory()[0]
+        want = call()
+        need = memory()[1] - held
+        dedisperse.set_subbands(4)
+        with_plan = call()
+        assert memory(held + need + MIB)[1] - held > need + MIB  # (the plan takes more)
+        got = call()
+        assert memory()[0] == held
+        for w, p, g in zip(want, with_plan, got):
+            assert np.asarray(w).tobytes() == np.asarray(p).tobytes()
+            assert np.asarray(w).tobytes() == np.asarray(g).tobytes()
