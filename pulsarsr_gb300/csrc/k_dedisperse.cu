@@ -1612,7 +1612,10 @@ int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t 
   choose_subband_tables(tab, nch, n, maxv, cstart, G, once, t);
   static_cast<SubbandPlan::Shape &>(plan) = SubbandPlan::Shape();
   plan.chunks.clear();
-  if (t.shape.G == 0) return PSR_OK;
+  if (t.shape.G == 0) {
+    plan.release();
+    return PSR_OK;
+  }
   auto up = [&](DevBuf &b, const auto &v) -> int {
     PSR_TRY(b.ensure(v.size() * sizeof(v[0])));
     PSR_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st));

@@ -54,3 +54,26 @@ def test_plan_that_does_not_fit(observation):
         for w, p, g in zip(want, with_plan, got):
             assert np.asarray(w).tobytes() == np.asarray(p).tobytes()
             assert np.asarray(w).tobytes() == np.asarray(g).tobytes()
+
+
+@pytest.mark.gpu
+def test_plan_dropped(observation):
+    """A batch prepared again without a plan gives the plan's buffers back."""
+    from pulsarsr_gb300 import batch, dedisperse, fbank
+    fb, trials = observation
+    h = fbank.HeaderInfo(64, 8, 64e-6, 1500.0, -4.0, 0)
+    obs = [dict(header=h, nsamples=60000, trials=trials, discovery=50000, config=config(),
+                rfi_block=0)]
+    held = {}
+    for width in (0, 4):
+        dedisperse.set_subbands(width)
+        before = memory()[0]
+        b = batch.Batch(obs)
+        b.set_chunking(0, 48, 48)
+        held[width] = memory()[0] - before
+        if width == 4:
+            assert held[4] > held[0] + MIB
+            dedisperse.set_subbands(0)
+            b.set_chunking(0, 48, 48)
+            assert memory()[0] - before == held[0]
+        del b
