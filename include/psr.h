@@ -516,8 +516,9 @@ int psr_session_analyze(psr_session *s, uint64_t limit, uint64_t bins,
  * batching itself.  Each observation keeps its own session; psr_batch_run
  * captures all of them, concurrently, into one graph on first use and
  * launches that graph afterwards.  hbm_budget_bytes bounds the dedispersed
- * series and spectra held at once (0: 64 GiB): it sets the trials per
- * dedispersion block. */
+ * series, spectra, candidate bins' lists and dedispersion scratch held at once
+ * (0: 64 GiB): it sets the trials per dedispersion block; the scratch takes an
+ * eighth of it at most. */
 typedef struct {
   psr_header header;
   uint64_t nsamples;

@@ -1357,12 +1357,13 @@ int psr_measure(const float *x, uint64_t n, uint64_t offset, double tsamp, doubl
 
 // ------------------------------------------------------------ session
 namespace {
-// psr_session_create with the engine's outer chunk fixed up front (0: the
-// default), so that a batch allocates each session's buffers once.
+// psr_session_create with the engine's outer chunk (0: the default) and its bytes
+// for a subband plan fixed up front, so that a batch allocates each session's
+// buffers once.
 int session_create(const psr_header *header, uint64_t nsamples, const double *trials,
                    uint64_t ntrials, uint64_t discovery, const psr_search_config *cfg,
                    uint64_t rfi_block_samples, float rfi_threshold, uint64_t chunk,
-                   psr_session **out) {
+                   uint64_t scratch, psr_session **out) {
   if (!header || !trials || !valid_config(cfg) || !out || nsamples < 2 || header->nchans <= 0) {
     set_error("session: invalid arguments");
     return PSR_EINVAL;
@@ -1382,6 +1383,7 @@ int session_create(const psr_header *header, uint64_t nsamples, const double *tr
   s->discovery = discovery;
   s->spec = to_spec(cfg, header->tsamp);
   s->eng.chunk = chunk;
+  s->eng.scratch = scratch;
   PSR_TRY(s->eng.prepare(o, trials, ntrials, discovery, s->spec, s->stream.s));
   PSR_TRY(s->errbuf.ensure(8));
   PSR_CUDA(cudaStreamSynchronize(s->stream.s));
@@ -1394,7 +1396,7 @@ int psr_session_create(const psr_header *header, uint64_t nsamples, const double
                        uint64_t ntrials, uint64_t discovery, const psr_search_config *cfg,
                        uint64_t rfi_block_samples, float rfi_threshold, psr_session **out) {
   return session_create(header, nsamples, trials, ntrials, discovery, cfg, rfi_block_samples,
-                        rfi_threshold, 0, out);
+                        rfi_threshold, 0, SUB_SCRATCH, out);
 }
 
 int psr_session_load(psr_session *s, const uint8_t *payload, uint64_t nbytes) {
@@ -1573,18 +1575,25 @@ struct psr_batch {
 };
 
 namespace {
-// Trials per dedispersion launch so that the batch's dedispersed series and
-// spectra stay within `budget` bytes of HBM (at least 16 per observation).
-uint64_t chunk_for_budget(const psr_batch_obs *obs, uint64_t n, double budget) {
-  double per_trial = 0.0;
+// Trials per dedispersion launch so that the batch's dedispersed series, spectra
+// and exact lists, and every observation's dedispersion scratch (up to `scratch`
+// bytes: an eighth of the budget, shared evenly), stay within `budget` bytes of
+// HBM (at least 16 trials per observation).
+uint64_t chunk_for_budget(const psr_batch_obs *obs, uint64_t n, double budget,
+                          uint64_t &scratch) {
+  scratch = std::min(SUB_SCRATCH, (uint64_t)(budget / 8.0 / (double)n));
+  double per_trial = 0.0, fixed = 0.0;
   for (uint64_t i = 0; i < n; ++i) {
     const uint64_t len = obs[i].discovery;
     uint64_t p = 1;
     while (p < len) p <<= 1;
-    // series, two halves of power spectra, FFT work buffer (complex, p points)
-    per_trial += 4.0 * (double)series_ld(len) + 8.0 * (double)(p + 64) + 8.0 * (double)p;
+    // series, two halves of power spectra, FFT work buffer (complex, p points),
+    // exact lists (a quarter of the bins)
+    per_trial += 4.0 * (double)series_ld(len) + 8.0 * (double)(p + 64) + 8.0 * (double)p +
+                 4.0 * ((double)p / 4.0 + 1024.0);
+    if (obs[i].header.nbits <= 8) fixed += (double)scratch;
   }
-  const double c = per_trial > 0.0 ? budget / per_trial : 256.0;
+  const double c = per_trial > 0.0 ? (budget - fixed) / per_trial : 256.0;
   return (uint64_t)std::max(16.0, std::min(256.0, std::floor(c)));
 }
 
@@ -1607,12 +1616,13 @@ int psr_batch_create(const psr_batch_obs *obs, uint64_t n, uint64_t hbm_budget_b
   }
   std::unique_ptr<psr_batch> b(new psr_batch());
   const double budget = hbm_budget_bytes ? (double)hbm_budget_bytes : 64.0 * (1ull << 30);
-  const uint64_t chunk = chunk_for_budget(obs, n, budget);
+  uint64_t scratch = 0;
+  const uint64_t chunk = chunk_for_budget(obs, n, budget, scratch);
   for (uint64_t i = 0; i < n; ++i) {
     const psr_batch_obs &q = obs[i];
     psr_session *s = nullptr;
     PSR_TRY(session_create(&q.header, q.nsamples, q.trials, q.ntrials, q.discovery, &q.config,
-                           q.rfi_block_samples, q.rfi_threshold, chunk, &s));
+                           q.rfi_block_samples, q.rfi_threshold, chunk, scratch, &s));
     b->obs.emplace_back(s);
     b->chunk.push_back(s->eng.chunk);
     b->inner.push_back(s->eng.inner);

@@ -1273,7 +1273,6 @@ std::atomic<int> g_subbands{-1};
 // FLUSH, one with it.
 constexpr int SS_SMEM = 106 * 1024, SS_SMEM_FLUSH = 216 * 1024;
 constexpr int SP_MAXSMEM = 72 * 1024;       // k_sub_part: three CTAs per SM
-constexpr uint64_t SUB_SCRATCH = 1ull << 30;  // scratch rows of one segment
 
 // A subband's delays relative to its smallest, 16 bits each.
 struct RelKey {
@@ -1412,8 +1411,9 @@ static_assert(32 * SS_MAXSTAGES <= SUB_GRID, "as do the subbands of any plan tha
 // The tables at width G; false when the plan does not fit.  `known`: the
 // patterns of chunk known_ci at this width, or null.
 bool subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
-                    const std::vector<uint64_t> &cstart, int G, SubbandTables &out,
-                    const ChunkPatterns *known = nullptr, size_t known_ci = 0) {
+                    const std::vector<uint64_t> &cstart, int G, uint64_t scratch,
+                    SubbandTables &out, const ChunkPatterns *known = nullptr,
+                    size_t known_ci = 0) {
   const bool flush = (double)nch * maxv > 65535.0;
   const size_t nchunks = cstart.size() - 1;
   const uint64_t nsub = (nch + G - 1) / G;
@@ -1492,13 +1492,13 @@ bool subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
   const int nbuf = (int)std::min<uint64_t>(SS_MAXBUF, room / bufbytes);
   const uint64_t prowcap = ((uint64_t)SP_TT + relmax + 36 + 15) & ~15ull;
   if (nbuf < 2 || prowcap * G > SP_MAXSMEM) return false;
-  // Segments of the series: the scratch of one stays within SUB_SCRATCH, its
-  // tiles within a grid.
+  // Segments of the series: the rows of one stay within `scratch`, its tiles
+  // within a grid.
   const uint64_t tail = max_spread + rowcap / 2 + 16;
   uint64_t seg = std::min((n + SS_TT - 1) / SS_TT, SUB_GRID) * SS_TT;
   auto stride = [&](uint64_t sg) { return ((sg + tail + SP_TT - 1) / SP_TT) * SP_TT; };
-  if (max_rows * stride(seg) * 2 > SUB_SCRATCH) {
-    const uint64_t per = SUB_SCRATCH / (2 * max_rows);
+  if (max_rows * stride(seg) * 2 > scratch) {
+    const uint64_t per = scratch / (2 * max_rows);
     seg = per > tail + SP_TT ? ((per - tail - SP_TT) / SS_TT) * SS_TT : 0;
     if (seg < 16 * SS_TT) return false;  // rows too many to reuse
   }
@@ -1562,13 +1562,13 @@ bool subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, 
 // where there is no plan.
 void choose_subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                            const std::vector<uint64_t> &cstart, int G, bool once,
-                           SubbandTables &t) {
+                           uint64_t scratch, SubbandTables &t) {
   t = SubbandTables();
   if (G == 0 || cstart.size() < 2 || !(maxv > 0.0) || maxv > 255.0 ||
       (double)nch * maxv >= 16777216.0 || n < 2)
     return;
   auto take = [&](int g, const ChunkPatterns *known, size_t known_ci) {
-    const bool fits = subband_tables(tab, nch, n, maxv, cstart, g, t, known, known_ci);
+    const bool fits = subband_tables(tab, nch, n, maxv, cstart, g, scratch, t, known, known_ci);
     if (!fits) t = SubbandTables();
     return fits;
   };
@@ -1607,9 +1607,9 @@ void choose_subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint6
 
 int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st, bool once) {
+                       cudaStream_t st, bool once, uint64_t scratch) {
   SubbandTables t;
-  choose_subband_tables(tab, nch, n, maxv, cstart, G, once, t);
+  choose_subband_tables(tab, nch, n, maxv, cstart, G, once, scratch, t);
   static_cast<SubbandPlan::Shape &>(plan) = SubbandPlan::Shape();
   plan.chunks.clear();
   if (t.shape.G == 0) {
@@ -1830,7 +1830,7 @@ extern "C" int psr_test_subband_plan(const uint32_t *delays, uint64_t nch, uint6
   cstart.push_back(ntrials);
   psr::SubbandTables t;
   psr::choose_subband_tables(std::vector<uint32_t>(delays, delays + nch * ntrials), nch, n,
-                             max_value, cstart, subbands, once != 0, t);
+                             max_value, cstart, subbands, once != 0, psr::SUB_SCRATCH, t);
   const psr::SubbandPlan::Shape &p = t.shape;
   info[0] = (uint64_t)p.G;
   info[1] = p.flush;

@@ -321,9 +321,11 @@ int dedisp_subbands_default(const DeviceObs &o);
 // or -1 (the cheapest; with `once`, counting what the plan takes to make).  A plan
 // that does not fit, or for which there is no device memory, leaves plan.G = 0 and
 // plan's buffers empty.
+// `scratch`: bytes that the rows of one segment may take.
+constexpr uint64_t SUB_SCRATCH = 1ull << 30;
 int build_subband_plan(const std::vector<uint32_t> &tab, uint64_t nch, uint64_t n, double maxv,
                        const std::vector<uint64_t> &cstart, int G, SubbandPlan &plan,
-                       cudaStream_t st, bool once = false);
+                       cudaStream_t st, bool once = false, uint64_t scratch = SUB_SCRATCH);
 // With want_means = false (series only folded, not searched) the sums and
 // means are left unset.  With a subband plan (8-bit-storage samples), chunk
 // chunk_index of the plan runs the two-level kernels.

@@ -65,7 +65,7 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
   const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
   PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
-                             sbplan, st, once));
+                             sbplan, st, once, scratch));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&ev_fft[0], &ev_fft[1], &ev_sel[0], &ev_sel[1]})
     if (!*e) PSR_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));

@@ -16,6 +16,7 @@ struct SearchEngine {
   // (dedisp_subbands_default()).
   int subbands = -1;
   bool once = false;  // one pass only: a subband plan has to pay for itself
+  uint64_t scratch = SUB_SCRATCH;  // bytes that a subband plan's rows may take
   SubbandPlan sbplan;
   uint64_t ntrials = 0, n = 0, nch = 0, ldo = 0, ldp = 0, nparts = 0, nchunks = 0;
   // Outer chunk ci covers trials [cstart[ci], cstart[ci + 1]).  A search of

@@ -77,3 +77,31 @@ def test_plan_dropped(observation):
             b.set_chunking(0, 48, 48)
             assert memory()[0] - before == held[0]
         del b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("budget", [48 * MIB, 96 * MIB])
+def test_batch_budget(observation, budget):
+    """A batch's scratch takes an eighth of the budget at most, whatever the number
+    of observations, and lowers the trials per block for the rest."""
+    from pulsarsr_gb300 import batch, dedisperse, fbank, search
+    fb, trials = observation
+    h = fbank.HeaderInfo(64, 8, 64e-6, 1500.0, -4.0, 0)
+    obs = [dict(header=h, nsamples=60000, trials=trials, discovery=50000, config=config(),
+                rfi_block=0)] * 3
+    want = search.search_trials(fb, trials, 50000, config())
+    held, tables = {}, MIB  # (a plan's tables and the rounding of its rows)
+    for width in (0, 4):
+        dedisperse.set_subbands(width)
+        before = memory()[0]
+        b = batch.Batch(obs, budget)
+        held[width] = memory()[0] - before
+        for i in range(3):
+            b.load_fb(i, fb)
+        b.run()
+        b.sync()
+        for i in range(3):
+            counts, cands = b.candidates(i)
+            assert np.array_equal(counts, want[0]) and cands.tobytes() == want[1].tobytes()
+        del b
+    assert held[4] - held[0] <= budget // 8 + 3 * tables
