@@ -105,3 +105,30 @@ def test_batch_budget(observation, budget):
             assert np.array_equal(counts, want[0]) and cands.tobytes() == want[1].tobytes()
         del b
     assert held[4] - held[0] <= budget // 8 + 3 * tables
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nch,ntrials,length", [(2, 130, 300001), (1, 3, 17000001)])
+def test_series_block(gpu, nch, ntrials, length):
+    """Series with gaps between them are packed by blocks: no second copy of all
+    of them, and one by one where there is no room for a block."""
+    from pulsarsr_gb300 import dedisperse, synth
+    ns = length + 200
+    fb = synth.device(nch, 8, ns, 64e-6, 1500.0, -50.0, seed=5, noise_mean=100.0,
+                      noise_sigma=20.0)
+    trials = 0.1 * np.arange(ntrials)
+    dedisperse.set_subbands(0)
+    try:
+        even = length + 63 - (length - 1) % 64
+        want = dedisperse.apply_trials(fb, trials, even)[:, :length]
+        series = ntrials * even * 4
+        held = memory()[0]
+        got = dedisperse.apply_trials(fb, trials, length)
+        need = memory()[1] - held
+        assert need < series + 64 * MIB + 4 * MIB
+        assert np.array_equal(got, want)
+        memory(held + series + 4 * MIB)
+        assert np.array_equal(dedisperse.apply_trials(fb, trials, length), want)
+    finally:
+        memory(0)
+        dedisperse.set_subbands(-1)
