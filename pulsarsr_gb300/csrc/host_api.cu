@@ -1805,13 +1805,12 @@ int psr_batch_sync(psr_batch *b) {
   PSR_CUDA(cudaStreamSynchronize(b->main.s));
   bool regrown = false;
   for (auto &s : b->obs) {
-    // A raw-candidate overflow makes finish() regrow that session's buffers
-    // and redo the chunk; the captured graph would then hold stale pointers,
-    // so it is captured again on the next run.
-    const SpecWork &w = s->eng.sw;
-    const void *raw = w.raw.p, *gq = w.gq.p, *xq = w.xq.p;
+    // An overflow of a list makes finish() grow that session's buffers and redo
+    // the chunk; the captured graph would then hold stale pointers and
+    // capacities, so it is captured again on the next run.
+    const uint64_t grown = s->eng.sw.grown;
     PSR_TRY(psr_session_sync(s.get()));
-    regrown = regrown || w.raw.p != raw || w.gq.p != gq || w.xq.p != xq;
+    regrown = regrown || s->eng.sw.grown != grown;
   }
   if (regrown) b->drop_graph();
   return PSR_OK;

@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(HI_NT) k_harm_filter(HarmArgs a, GateArgs g) {
       at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1u));
       if (take) {
         if (at < g.xcap) xq[at] = entry[hi];
-        else atomicOr(a.overflow, OVERFLOW_QUEUE);
+        else atomicOr(a.overflow, OVERFLOW_EXACT);
       }
     }
   }
@@ -955,11 +955,15 @@ int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint
   PSR_TRY(w.floors.ensure(outer * 4));
   // Gated bins are ~2% of a noise spectrum; a quarter of the bins is ample
   // and an overflow (flagged) reruns the chunk with room for every bin.  Raw lists
-  // overflow on their own where a bright pulsar peaks in many bins.
-  w.qcap = w.queue_full ? plen : plen / 4 + 1024;
-  w.xcap = w.queue_full ? 6 * plen : w.qcap;  // every level of every bin at most
+  // overflow on their own where a bright pulsar peaks in many bins, exact lists
+  // where most bins pass the gates.
+  const uint64_t quarter = plen / 4 + 1024;
+  w.qcap = w.queue_full ? plen : quarter;
+  // every level of every bin at most
+  w.xcap = std::min(quarter * w.xgrow, (uint64_t)c.levels * plen);
+  w.xgroup = std::max<uint64_t>(1, outer * quarter / w.xcap);
   PSR_TRY(w.gq.ensure(2 * outer * w.qcap * 4));
-  PSR_TRY(w.xq.ensure(outer * w.xcap * 4));
+  PSR_TRY(w.xq.ensure(w.xgroup * w.xcap * 4));
   PSR_TRY(w.birdies.ensure(std::max<size_t>(c.birdies.size(), 2) * 8));
   if (!c.birdies.empty())
     PSR_CUDA(cudaMemcpyAsync(w.birdies.p, c.birdies.data(), c.birdies.size() * 8,
@@ -1055,16 +1059,25 @@ int spectrum_gate(const FftPlan &p, const SpecConfig &c, const float *d_power, u
   return PSR_OK;
 }
 
-// Exact evaluation of every queued bin of the outer chunk's `ntrials` spectra.
+// Exact evaluation of every queued bin of the outer chunk's `ntrials` spectra,
+// as many at a time as the exact lists hold.
 int spectrum_items(const FftPlan &p, const SpecConfig &c, const float *d_power, uint64_t ldp,
                    uint64_t ntrials, SpecWork &w, cudaStream_t st) {
   HarmArgs a = harm_args(p, c, d_power, ldp, w);
   if (a.end[0] == 0) return PSR_OK;
-  dim3 grid(HI_CTAS_PER_TRIAL, (unsigned)ntrials);
-  const GateArgs g = gate_args(w, 0);
-  if (c.levels == 6) k_harm_filter<6><<<grid, HI_NT, 0, st>>>(a, g);
-  else k_harm_filter<5><<<grid, HI_NT, 0, st>>>(a, g);
-  k_harm_exact<<<dim3(HX_CTAS_PER_TRIAL, (unsigned)ntrials), HX_NT, 0, st>>>(a, g);
+  for (uint64_t t = 0; t < ntrials; t += w.xgroup) {
+    const unsigned nt = (unsigned)std::min(w.xgroup, ntrials - t);
+    GateArgs g = gate_args(w, t);
+    g.xq = w.xq.as<uint32_t>();
+    const dim3 grid(HI_CTAS_PER_TRIAL, nt);
+    if (c.levels == 6) k_harm_filter<6><<<grid, HI_NT, 0, st>>>(a, g);
+    else k_harm_filter<5><<<grid, HI_NT, 0, st>>>(a, g);
+    k_harm_exact<<<dim3(HX_CTAS_PER_TRIAL, nt), HX_NT, 0, st>>>(a, g);
+    a.power += w.xgroup * ldp;
+    a.scale += w.xgroup * w.lds;
+    a.raw += w.xgroup * w.raw_cap;
+    a.raw_count += w.xgroup;
+  }
   PSR_CUDA(cudaGetLastError());
   return PSR_OK;
 }

@@ -255,13 +255,17 @@ struct SpecConfig {
   std::vector<double> birdies;  // pairs
   int levels = 5;               // harmonic sums h = 1 .. 2^(levels-1)
 };
-// Bits of the overflow word: raw candidate lists; gate queues or exact lists.
-constexpr unsigned OVERFLOW_RAW = 1, OVERFLOW_QUEUE = 2;
+// Bits of the overflow word: raw candidate lists; gate queues; exact lists.
+constexpr unsigned OVERFLOW_RAW = 1, OVERFLOW_QUEUE = 2, OVERFLOW_EXACT = 4;
 struct SpecWork {
   DevBuf scale, raw, counts, floors, birdies, gq, xq;
   uint64_t qcap = 0, xcap = 0;  // gate queue and exact list capacities per trial
   const unsigned *overflow() const { return counts.as<unsigned>(); }
   bool queue_full = false;    // size the gate queues for every bin
+  // Exact lists that overflow get 4 times as long and take as many fewer trials at
+  // a time (xgroup), in the same memory.
+  uint64_t xgrow = 1, xgroup = 0;
+  uint64_t grown = 0;         // times that any of them grew
   uint64_t outer_trials = 0;  // trials of the chunk being processed
   uint64_t raw_cap = 0;  // raw (pre-dedupe) candidates per trial
   uint64_t lds = 0;      // row stride of scale[]

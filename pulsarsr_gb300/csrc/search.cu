@@ -215,12 +215,14 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
     bool stands = ci + 2 >= nchunks;
     int guard = 0;
     while (ov[ci]) {
-      if (++guard > 9) {
+      if (++guard > 12) {  // (8 for the raw lists, 3 for the exact ones, 1)
         set_error("search: raw candidate storage overflow");
         return PSR_ECAPACITY;
       }
       if (ov[ci] & OVERFLOW_RAW) sw.raw_cap *= 4;
       if (ov[ci] & OVERFLOW_QUEUE) sw.queue_full = true;
+      if (ov[ci] & OVERFLOW_EXACT) sw.xgrow *= 4;
+      ++sw.grown;
       PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
       PSR_TRY(stands ? enqueue_spectrum(ci, st) : enqueue_chunk(o, ci, st));
       stands = true;

@@ -132,3 +132,24 @@ def test_series_block(gpu, nch, ntrials, length):
     finally:
         memory(0)
         dedisperse.set_subbands(-1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("harmonics", [16, 32])
+def test_exact_lists_of_most_bins(observation, harmonics):
+    """A threshold that half of the bins pass, with a birdie over the whole band (the
+    gates do not look at birdies, the scores do): gate queues grow to every bin, the
+    exact lists stay in their memory, taken by fewer trials at a time."""
+    from pulsarsr_gb300 import search
+    fb, trials = observation
+    n, bins = 12000, 16385
+    peak = {}
+    for threshold in (60.0, 0.2):
+        cfg = search.Config(min_hz=3.0, max_hz=7000.0, threshold=threshold,
+                            max_harmonics=harmonics, birdies=[(3900.0, 3905.0)])
+        held = memory()[0]
+        counts, _ = search.search_trials(fb, trials, n, cfg)
+        peak[threshold] = memory()[1] - held
+        assert not counts.any()
+    queues = 2 * len(trials) * (bins - bins // 4 - 1024) * 4
+    assert queues <= peak[0.2] - peak[60.0] <= queues + MIB
