@@ -208,22 +208,28 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
     return PSR_ETIMEOUT;
   }
   PSR_TRY(harvest());
-  // A chunk whose lists overflowed: grow what did and redo it.  The power
-  // spectra of the last two chunks still stand (those of others are made again), so
-  // the last come first.
+  // A chunk whose lists overflowed: grow what did and redo it, or redo it alone
+  // where an earlier one of these has grown them since it ran.  The power spectra
+  // of the last two chunks still stand (those of others are made again), so the
+  // last come first.
+  const uint64_t grown = sw.grown;
   for (uint64_t ci = nchunks; ci-- > 0;) {
     bool stands = ci + 2 >= nchunks;
+    uint64_t ran_at = grown;
     int guard = 0;
     while (ov[ci]) {
-      if (++guard > 12) {  // (8 for the raw lists, 3 for the exact ones, 1)
-        set_error("search: raw candidate storage overflow");
-        return PSR_ECAPACITY;
+      if (sw.grown == ran_at) {
+        if (++guard > 12) {  // (8 for the raw lists, 3 for the exact ones, 1)
+          set_error("search: raw candidate storage overflow");
+          return PSR_ECAPACITY;
+        }
+        if (ov[ci] & OVERFLOW_RAW) sw.raw_cap *= 4;
+        if (ov[ci] & OVERFLOW_QUEUE) sw.queue_full = true;
+        if (ov[ci] & OVERFLOW_EXACT) sw.xgrow *= 4;
+        ++sw.grown;
+        PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
       }
-      if (ov[ci] & OVERFLOW_RAW) sw.raw_cap *= 4;
-      if (ov[ci] & OVERFLOW_QUEUE) sw.queue_full = true;
-      if (ov[ci] & OVERFLOW_EXACT) sw.xgrow *= 4;
-      ++sw.grown;
-      PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
+      ran_at = sw.grown;
       PSR_TRY(stands ? enqueue_spectrum(ci, st) : enqueue_chunk(o, ci, st));
       stands = true;
       PSR_TRY(join(st));

@@ -153,3 +153,24 @@ def test_exact_lists_of_most_bins(observation, harmonics):
         assert not counts.any()
     queues = 2 * len(trials) * (bins - bins // 4 - 1024) * 4
     assert queues <= peak[0.2] - peak[60.0] <= queues + MIB
+
+
+@pytest.mark.gpu
+def test_lists_of_many_chunks(gpu):
+    """Raw lists that overflow in all of nine chunks grow for the first of them, not
+    again for each; lists are those of the trials alone."""
+    from pulsarsr_gb300 import dedisperse, search, synth
+    fb = synth.device(4, 8, 101000, 64e-6, 1500.0, -20.0, seed=9, noise_mean=100.0,
+                      noise_sigma=20.0)
+    trials, n, peak = 0.01 * np.arange(2304), 100000, {}
+    for threshold in (60.0, 2.5):
+        cfg = search.Config(min_hz=3.0, max_hz=7000.0, threshold=threshold, max_candidates=24)
+        held = memory()[0]
+        counts, cands = search.search_trials(fb, trials, n, cfg)
+        peak[threshold] = memory()[1] - held
+    assert peak[2.5] - peak[60.0] <= 256 * (16 - 1) * 2048 * 24 + MIB
+    at = np.concatenate([[0], np.cumsum(counts)]).astype(int)
+    for i in (0, 255, 256, 1000, 2015, 2016, 2303):
+        x = dedisperse.apply_trials(fb, trials[i:i + 1], n)[0]
+        alone = search.periodicity(x, 64e-6, float(trials[i]), cfg)
+        assert cands[at[i]:at[i + 1]].tobytes() == alone.tobytes(), i
