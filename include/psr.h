@@ -539,9 +539,12 @@ int psr_batch_load_fb(psr_batch *b, uint64_t i, const psr_fb *fb);
 /* Autotuner: per shape class (channels, bit depth, FFT size, trial count to
  * the nearest power of two), times whole searches of the class's first
  * loaded observation at each candidate tiling (DM block and half of it;
- * whole-block or 64-trial FFT launches; for 8-bit samples, channel-by-channel
- * or 8-channel subband dedispersion) and applies the fastest to the class.
- * chunk/inner/subbands (n entries each, may be NULL) receive the choices. */
+ * whole-block or 64-trial FFT launches; for samples stored in 8 bits, the
+ * dedispersion chosen from the plan as without tuning, channel by channel, and
+ * subbands of 4 and 8 channels) and applies the fastest to the class.
+ * chunk/inner/subbands (n entries each, may be NULL) receive the choices, the
+ * last as the width that each observation's plan then has (0: channel by
+ * channel). */
 int psr_batch_tune(psr_batch *b, uint64_t *chunk, uint64_t *inner, int *subbands);
 /* Pin observation i's dedispersion block (trials per outer chunk, >= 1) and
  * FFT launch size (trials per inner chunk; 0 = the whole block within a 4 GB

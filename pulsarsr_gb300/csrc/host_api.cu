@@ -1684,8 +1684,9 @@ int psr_batch_set_chunking(psr_batch *b, uint64_t i, uint64_t chunk, uint64_t in
 // class is searched whole at each candidate tiling, on its loaded data, and
 // the fastest is applied to the whole class.  Candidates: the budgeted DM
 // block and half of it (outer chunk), whole-block or 64-trial FFT launches
-// (inner chunk), and for 8-bit samples channel-by-channel or 8-channel
-// subband dedispersion.
+// (inner chunk), and for samples stored in 8 bits the dedispersion that the
+// plan chooses itself (first, so that a tie leaves it), then channel by channel
+// and subbands of 4 and of 8 channels where that was not its choice.
 int psr_batch_tune(psr_batch *b, uint64_t *chunk_out, uint64_t *inner_out, int *subbands_out) {
   if (!b) {
     set_error("batch: null handle");
@@ -1712,12 +1713,15 @@ int psr_batch_tune(psr_batch *b, uint64_t *chunk_out, uint64_t *inner_out, int *
       std::vector<Pick> cand;
       for (uint64_t c : {c0, std::max<uint64_t>(16, c0 / 2)})
         for (uint64_t inner : {(uint64_t)0, (uint64_t)64})
-          for (int g : {0, 8})
-            if (g == 0 || s->o.h.nbits == 8) cand.push_back(Pick{c, inner, g});
+          for (int g : {-1, 0, 4, 8})
+            if (g == -1 || s->o.kind == SAMPLE_U8) cand.push_back(Pick{c, inner, g});
       double best = 1e300;
       Pick pick = cand[0];
+      int chosen = 0;  // the width of the last candidate at -1
       for (const Pick &c : cand) {
+        if (c.subbands >= 0 && c.subbands == chosen) continue;
         if ((rc = reprepare(s, c.chunk, c.inner, c.subbands)) != PSR_OK) break;
+        if (c.subbands < 0) chosen = s->eng.sbplan.G;
         if ((rc = psr_session_run(s)) != PSR_OK || (rc = psr_session_sync(s)) != PSR_OK) break;
         if (cudaEventRecord(e0, s->stream.s) != cudaSuccess ||
             (rc = psr_session_run(s)) != PSR_OK ||
@@ -1745,7 +1749,7 @@ int psr_batch_tune(psr_batch *b, uint64_t *chunk_out, uint64_t *inner_out, int *
     b->inner[i] = p.inner;
     if (chunk_out) chunk_out[i] = p.chunk;
     if (inner_out) inner_out[i] = p.inner;
-    if (subbands_out) subbands_out[i] = p.subbands;
+    if (subbands_out) subbands_out[i] = s->eng.sbplan.G;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
