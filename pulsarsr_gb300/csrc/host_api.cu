@@ -1549,6 +1549,7 @@ int psr_session_analyze(psr_session *s, uint64_t limit, uint64_t bins, const psr
   psr_rules r;
   psr_rules_default(&r);
   std::unique_ptr<psr_outcome> o(new psr_outcome());
+  PoolScope scope(s->stream.s);  // (the session's own buffers stand already)
   PSR_TRY(analyze_obs(s->o, s->trials.data(), s->trials.size(), all.data(), all.size(), limit,
                       bins, rules ? *rules : r, o->o, s->stream.s));
   *out = o.release();

@@ -174,3 +174,23 @@ def test_lists_of_many_chunks(gpu):
         x = dedisperse.apply_trials(fb, trials[i:i + 1], n)[0]
         alone = search.periodicity(x, 64e-6, float(trials[i]), cfg)
         assert cands[at[i]:at[i + 1]].tobytes() == alone.tobytes(), i
+
+
+@pytest.mark.gpu
+def test_confirmation_of_a_session(observation):
+    """A session's confirmation takes its temporary buffers from the pool, as a
+    filterbank's does, and says the same."""
+    from pulsarsr_gb300 import confirmation, fbank, search, session
+    fb, trials = observation
+    h = fbank.HeaderInfo(64, 8, 64e-6, 1500.0, -4.0, 0)
+    s = session.SearchSession(h, 60000, trials, 50000, config(), 0, 8.0)
+    s.load(np.rint(fb.data.T).astype(np.uint8).tobytes())
+    s.run()
+    s.sync()
+    _, cands = s.candidates()
+    memory()
+    of_fb = confirmation.analyze(fb, trials, cands)
+    calls = memory()[2]
+    of_session = confirmation.analyze_session(s)
+    assert memory()[2] <= calls
+    assert len(of_fb.data) and of_fb.json() == of_session.json()
