@@ -319,6 +319,12 @@ int psr_measure(const float *x, uint64_t n, uint64_t offset, double tsamp,
                 double period, uint64_t start_bin, uint64_t width_bins,
                 uint64_t bins, psr_measurement *out);
 
+/* Test hook, no reference counterpart; needs no device: a fold's phase per sample
+ * in fixed point, tsamp / period modulo 1 in 2^-128 (out[0] its high 64 bits, out[1]
+ * the low) for samples up to `last`, and out[2] the margin in 2^-32 bins within which
+ * a bin comes from the f64 operations (2^31: always). */
+int psr_test_fold_phase(double tsamp, double period, uint64_t last, uint64_t bins, uint64_t *out);
+
 /* ------------------------------------------------ gradient refinement */
 /* Refinement of (P, Pdot, DM) by gradient ascent on a differentiable fold
  * objective.  No counterpart in the reference, whose refinement is the grid of

@@ -54,7 +54,7 @@ unsigned __int128 fixed128(double x) {
 FoldPhase fold_phase(double tsamp, double period, uint64_t last, uint64_t bins) {
   const double r = tsamp / period, d = std::fma(-r, period, tsamp) / period;
   unsigned __int128 f = 0;
-  if (std::isfinite(r) && std::isfinite(d)) {
+  if (r >= 0.0 && std::isfinite(r) && std::isfinite(d)) {
     f = fixed128(r);
     if (d >= 0.0) f += fixed128(d);
     else f -= fixed128(-d);
@@ -64,10 +64,11 @@ FoldPhase fold_phase(double tsamp, double period, uint64_t last, uint64_t bins) 
   p.rlo = (unsigned long long)f;
   p.period = period;
   p.tsamp = tsamp;
-  // bins (cycles 2^-51 + 2^-32 + 2^-52) in units of 2^-32 bins, and 2
+  // bins (cycles 2^-51 + 2^-32 + 2^-52) in units of 2^-32 bins, and 2; a negative
+  // ratio leaves every sample to the f64 operations
   const double cycles = (double)last * r;
   const double m = (double)bins * (cycles * 0x1p-19 + 1.0 + 0x1p-20) + 2.0;
-  p.margin = m < 2147483648.0 ? (uint32_t)std::ceil(m) : 0x80000000u;
+  p.margin = r >= 0.0 && m < 2147483648.0 ? (uint32_t)std::ceil(m) : 0x80000000u;
   return p;
 }
 
@@ -864,3 +865,16 @@ int dm_response(const std::vector<float> &chp, const std::vector<double> &chmean
 }
 
 }  // namespace psr
+
+extern "C" int psr_test_fold_phase(double tsamp, double period, uint64_t last, uint64_t bins,
+                                   uint64_t *out) {
+  if (!out) {
+    psr::set_error("test_fold_phase: null argument");
+    return PSR_EINVAL;
+  }
+  const psr::FoldPhase p = psr::fold_phase(tsamp, period, last, bins);
+  out[0] = p.rhi;
+  out[1] = p.rlo;
+  out[2] = p.margin;
+  return PSR_OK;
+}
