@@ -50,3 +50,66 @@ def test_more_tiles_than_a_grid(gpu):
     finally:
         dedisperse.set_subbands(-1)
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+def delay_table(nch, trials, fch1=1500.0, bw=300.0, tsamp=64e-6):
+    f = fch1 - np.arange(nch) * (bw / nch)
+    x = 4148.808 * np.asarray(trials)[:, None] * (1 / f ** 2 - 1 / f[0] ** 2) / tsamp
+    return np.floor(x + 0.5).astype(np.uint32)
+
+
+@pytest.mark.parametrize("nbits,nch", [(1, 9), (2, 64), (4, 97), (4, 8), (8, 5), (8, 256),
+                                       (8, 261), (8, 1030)])
+def test_widths_are_taken(nbits, nch):
+    """The plans of tests/test_dedisperse_two_level.py are there at the widths it asks
+    for, with flushes past 65,535; its long case takes several segments."""
+    step = 1.0 / (4148.808 * (1 / 1200.0 ** 2 - 1 / 1500.0 ** 2) / 64e-6)
+    maxv = 2.0 ** nbits - 1
+    for order in (np.arange(37), np.arange(40, 0, -1) * 0.5, np.repeat(np.arange(9), 3)):
+        for width in (4, 8):
+            w, flush, _, nseg, _ = plan(delay_table(nch, step * order), 9000, maxv, width,
+                                        chunk=len(order), once=True)
+            assert (w, flush, nseg) == (width, int(nch * maxv > 65535), 1)
+    if nch == 1030:
+        t = delay_table(1024, 400 * step + step * np.arange(100))
+        w, _, _, nseg, _ = plan(t, 399491, 255.0, 8, chunk=100, once=True)
+        assert w == 8 and nseg > 1
+
+
+# a search that the plan's own choice takes in two levels, in five blocks of trials
+AUTO = dict(nch=96, ntrials=300, chunk=64, n=100000)
+
+
+def test_own_choice():
+    step = 1.0 / (4148.808 * (1 / 1200.0 ** 2 - 1 / 1500.0 ** 2) / 64e-6)
+    t = delay_table(AUTO["nch"], step * np.arange(AUTO["ntrials"]))
+    assert plan(t, AUTO["n"], 255.0, -1, chunk=AUTO["chunk"])[0] in (4, 8)
+    assert plan(t, 1000, 255.0, -1, once=True)[0] == 0  # (does not pay for one short pass)
+
+
+@pytest.mark.gpu
+def test_own_choice_over_blocks(gpu):
+    """The chosen plan (whose middle block reuses the patterns it was chosen by)
+    against channel by channel, over blocks with a short last one."""
+    from pulsarsr_gb300 import batch, dedisperse, fbank, search, synth
+    nch, n = AUTO["nch"], AUTO["n"]
+    fb = synth.device(nch, 8, n + 500, 64e-6, 1500.0, -300.0 / nch, seed=2, noise_mean=100.0,
+                      noise_sigma=20.0, pulsars=[synth.Pulsar(0.02, 2.0, 0.1, 1.0)])
+    step = dedisperse.dm_step(fb.header.frequencies(), 64e-6)
+    cfg = search.Config(min_hz=2.0, max_hz=3000.0, threshold=4.0)
+    b = batch.Batch([dict(header=fbank.HeaderInfo(nch, 8, 64e-6, 1500.0, -300.0 / nch, 0),
+                          nsamples=n + 500, trials=step * np.arange(AUTO["ntrials"]),
+                          discovery=n, config=cfg, rfi_block=0)])
+    b.load_fb(0, fb)
+    got = {}
+    try:
+        for width in (0, -1):
+            dedisperse.set_subbands(width)
+            b.set_chunking(0, AUTO["chunk"], 0)
+            b.run()
+            b.sync()
+            got[width] = b.candidates(0)
+    finally:
+        dedisperse.set_subbands(-1)
+    assert got[0][0].sum() > 0 and np.array_equal(got[0][0], got[-1][0])
+    assert got[0][1].tobytes() == got[-1][1].tobytes()
