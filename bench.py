@@ -332,10 +332,14 @@ def run_ours(args):
     fft_kernels = 2 if N // 2 > 4096 else 1
     # unpack + 13 RFI kernels (8-bit storage: sums, guesses, two passes of maps
     # and scans, block sums, median histograms + pick, channel and block
-    # decisions, block means, fill); per outer chunk dedispersion (one kernel more
-    # where it takes two levels) + part reduction + harmonic filter + exact scores
-    # + selection; per inner chunk the FFT pass(es), the floors and the gates
-    launches = 1 + 13 + D * 5 + F * (fft_kernels + 2)
+    # decisions, block means, fill); per outer chunk the dedispersion's (two per
+    # segment where it takes two levels, else one per group of channels whose sums
+    # fit 16 bits) + part reduction + harmonic filter + exact scores + selection; per
+    # inner chunk the FFT pass(es), the floors and the gates
+    width, segments = s.dedispersion()
+    groups = -(-obs.nchans // (65535 // (2 ** obs.nbits - 1))) if obs.nbits <= 8 else 1
+    dedisp_kernels = 2 * segments if width else groups
+    launches = 1 + 13 + D * (dedisp_kernels + 4) + F * (fft_kernels + 2)
     if rank != 0:
         if dist:
             dist.destroy_process_group()

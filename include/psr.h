@@ -511,6 +511,10 @@ int psr_session_mask(psr_session *s, uint64_t *channels, uint64_t *nchannels_bad
  * reset. */
 int psr_session_set_profiling(psr_session *s, int enable);
 int psr_session_stage_times(psr_session *s, double *ms, uint64_t *launches, int reset);
+/* The dedispersion that the session's plan takes: the subband width (0: channel by
+ * channel) and, at a width, the segments that each block of trials is made in (two
+ * kernels each).  Either pointer may be NULL. */
+int psr_session_dedispersion(const psr_session *s, int *subbands, uint64_t *segments);
 /* confirmation::analyze over the last run's candidates (the psr search
  * command, cli/src/main.rs:474-478), on the session's masked observation. */
 int psr_session_analyze(psr_session *s, uint64_t limit, uint64_t bins,

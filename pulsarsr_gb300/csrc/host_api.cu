@@ -1496,6 +1496,17 @@ int psr_session_stage_times(psr_session *s, double *ms, uint64_t *launches, int 
   return PSR_OK;
 }
 
+int psr_session_dedispersion(const psr_session *s, int *subbands, uint64_t *segments) {
+  if (!s) {
+    set_error("session_dedispersion: null handle");
+    return PSR_EINVAL;
+  }
+  const SubbandPlan &p = s->eng.sbplan;
+  if (subbands) *subbands = p.G;
+  if (segments) *segments = p.G ? (s->eng.n + p.seg - 1) / p.seg : 0;
+  return PSR_OK;
+}
+
 int psr_session_candidates(psr_session *s, uint64_t *counts, psr_candidate *out, uint64_t cap,
                            uint64_t *n_total) {
   if (!s || !n_total) {

@@ -89,6 +89,13 @@ class SearchSession:
                                             C.c_int(1 if reset else 0)))
         return {k: (float(ms[i]), int(n[i])) for i, k in enumerate(self.STAGES)}
 
+    def dedispersion(self) -> tuple[int, int]:
+        """(subband width, segments per block of trials) of the session's plan;
+        width 0: channel by channel (psr_session_dedispersion)."""
+        g, n = C.c_int(), C.c_uint64()
+        check(lib().psr_session_dedispersion(self._s, C.byref(g), C.byref(n)))
+        return g.value, n.value
+
     def close(self) -> None:
         if self._s:
             lib().psr_session_free(self._s)
