@@ -915,7 +915,7 @@ int psr_dedisperse_trials(const psr_fb *fb, const double *trials, uint64_t ntria
   PSR_CUDA(cudaMemsetAsync(err.p, 0, 8, st));
   SubbandPlan sbp;
   PSR_TRY(build_subband_plan(tab, o.nch, length, o.kind == SAMPLE_U8 ? o.max_value() : 0.0,
-                             {0, ntrials}, dedisp_subbands_default(o), sbp, st, true));
+                             {0, ntrials}, dedisp_subbands_default(), sbp, st, true));
   PSR_TRY(launch_dedisperse_ex(o, dd.as<uint32_t>(), ntrials, length, ser.as<float>(), ldo,
                                parts.as<double>(), sums.as<double>(), means.as<float>(), spread,
                                err.as<unsigned>(), st, 0, 0, sums_out != nullptr, &sbp, 0));

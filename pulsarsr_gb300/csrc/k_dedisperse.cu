@@ -1390,8 +1390,7 @@ double two_level_cost(const ChunkPatterns &cp, uint64_t nt, int G, double maxv) 
 }
 }  // namespace
 
-int dedisp_subbands_default(const DeviceObs &o) {
-  (void)o;
+int dedisp_subbands_default() {
   return g_subbands.load();
 }
 
@@ -1579,7 +1578,8 @@ void choose_subband_tables(const std::vector<uint32_t> &tab, uint64_t nch, uint6
   // A plan for one pass has to save more than it takes to make: 25 ns per
   // channel and trial, 150 us for its buffers and copies (299 channels, 59 trials
   // of 131,000 to 400,000 samples: 0.3 to 0.5 ms, the kernels saved 0.1).  Seconds
-  // per unit of the costs below: 512 samples, four issue slots a clock of 152 SMs.
+  // per unit of the costs below, which are fitted to a GB300: 512 samples, four
+  // issue slots a clock of 152 SMs at 1.9 GHz.
   const double unit = (double)n / 512.0 / 1.155e12;
   const uint64_t total = cstart.back() - cstart.front();
   const double making = once ? 150e-6 + 25e-9 * (double)(nch * total) : 0.0;

@@ -409,53 +409,53 @@ __global__ void __launch_bounds__(SC_NT)
       }
     }
     if (!found) {
-    // Rank-bound skips: with p_d elements of chunk d already known to lie
-    // below the target and rr = r - sum(p_d), let y = min_d A_d[p_d + rr/5].
-    // Each chunk has at most rr/5 unskipped elements below y, so at most rr
-    // elements below y remain and the rank-r element is >= y: skip them.
-    // Every round shrinks rr geometrically; a short merge walk finishes.
-    for (int round = 0; round < 6; ++round) {
-      const int q = rr / 5;
-      if (q < 3) break;  // (a walk over up to 14 is cheaper than another round)
-      uint32_t y = 0xffffffffu;
+      // Rank-bound skips: with p_d elements of chunk d already known to lie
+      // below the target and rr = r - sum(p_d), let y = min_d A_d[p_d + rr/5].
+      // Each chunk has at most rr/5 unskipped elements below y, so at most rr
+      // elements below y remain and the rank-r element is >= y: skip them.
+      // Every round shrinks rr geometrically; a short merge walk finishes.
+      for (int round = 0; round < 6; ++round) {
+        const int q = rr / 5;
+        if (q < 3) break;  // (a walk over up to 14 is cheaper than another round)
+        uint32_t y = 0xffffffffu;
 #pragma unroll
-      for (int d = 0; d < 5; ++d)
-        if (p[d] + q < 64) y = min(y, w[d * SC_STRIDE + p[d] + q]);
-      if (y == 0u) break;
-      int adv = 0;
+        for (int d = 0; d < 5; ++d)
+          if (p[d] + q < 64) y = min(y, w[d * SC_STRIDE + p[d] + q]);
+        if (y == 0u) break;
+        int adv = 0;
 #pragma unroll
-      for (int d = 0; d < 5; ++d) {
-        const int np = count_le64(w + d * SC_STRIDE, y - 1u);  // elements < y
-        adv += np - p[d];
-        p[d] = np;
+        for (int d = 0; d < 5; ++d) {
+          const int np = count_le64(w + d * SC_STRIDE, y - 1u);  // elements < y
+          adv += np - p[d];
+          p[d] = np;
+        }
+        rr -= adv;
+        if (adv == 0) break;
       }
-      rr -= adv;
-      if (adv == 0) break;
-    }
-    // 5-way merge walk over the rest: advance the smallest head rr times; the
-    // smallest head is then the rank-r element.
-    uint32_t hd[5];
+      // 5-way merge walk over the rest: advance the smallest head rr times; the
+      // smallest head is then the rank-r element.
+      uint32_t hd[5];
 #pragma unroll
-    for (int d = 0; d < 5; ++d) hd[d] = p[d] < 64 ? w[d * SC_STRIDE + p[d]] : 0xffffffffu;
-    for (int step = 0; step < rr; ++step) {
-      uint32_t m = hd[0];
-      int am = 0;
+      for (int d = 0; d < 5; ++d) hd[d] = p[d] < 64 ? w[d * SC_STRIDE + p[d]] : 0xffffffffu;
+      for (int step = 0; step < rr; ++step) {
+        uint32_t m = hd[0];
+        int am = 0;
 #pragma unroll
-      for (int d = 1; d < 5; ++d)
-        if (hd[d] < m) {
-          m = hd[d];
-          am = d;
-        }
+        for (int d = 1; d < 5; ++d)
+          if (hd[d] < m) {
+            m = hd[d];
+            am = d;
+          }
 #pragma unroll
-      for (int d = 0; d < 5; ++d)
-        if (d == am) {
-          ++p[d];
-          hd[d] = p[d] < 64 ? w[d * SC_STRIDE + p[d]] : 0xffffffffu;
-        }
-    }
-    med_k = hd[0];
+        for (int d = 0; d < 5; ++d)
+          if (d == am) {
+            ++p[d];
+            hd[d] = p[d] < 64 ? w[d * SC_STRIDE + p[d]] : 0xffffffffu;
+          }
+      }
+      med_k = hd[0];
 #pragma unroll
-    for (int d = 1; d < 5; ++d) med_k = min(med_k, hd[d]);
+      for (int d = 1; d < 5; ++d) med_k = min(med_k, hd[d]);
     }
     const float sc = fmaxf(fmaxf(__fdiv_rn(__uint_as_float(med_k), LN2F), floor_s), 1e-20f);
     inv_s[threadIdx.x] = __frcp_rn(sc);
@@ -553,7 +553,8 @@ __global__ void __launch_bounds__(SC_NT)
     base2 = atomicAdd(&g.n2[trial], (unsigned)m2);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && (base1 + m1 > g.qcap || base2 + m2 > g.qcap)) atomicOr(a.overflow, OVERFLOW_QUEUE);
+  if (threadIdx.x == 0 && (base1 + m1 > g.qcap || base2 + m2 > g.qcap))
+    atomicOr(a.overflow, OVERFLOW_QUEUE);
   for (int i = threadIdx.x; i < m1 && base1 + i < g.qcap; i += SC_NT)
     gq1[base1 + i] = (uint32_t)(kb0 + lq1[i]);
   for (int i = threadIdx.x; i < m2 && base2 + i < g.qcap; i += SC_NT)
@@ -936,10 +937,10 @@ __global__ void __launch_bounds__(SEL_NT) k_select(SelArgs a) {
 
 }  // namespace
 
-// Buffers for up to `outer` trials of raw candidates and `inner` trials of
-// normalisation scales; uploads the birdie list.
-int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint64_t inner,
-                     SpecWork &w, cudaStream_t st) {
+// Buffers for up to `outer` trials' scales, queues and raw candidates; uploads the
+// birdie list.
+int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, SpecWork &w,
+                     cudaStream_t st) {
   if (c.max_candidates > 64 || c.max_candidates < 1) {
     set_error("search: 1..64 candidates per trial are supported");
     return PSR_EINVAL;
@@ -949,7 +950,6 @@ int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint
   w.lds = ((nblocks + 63) / 64) * 64;
   if (w.raw_cap == 0) w.raw_cap = 2048;
   PSR_TRY(w.scale.ensure(outer * w.lds * 4));
-  (void)inner;
   PSR_TRY(w.raw.ensure(outer * w.raw_cap * sizeof(RawCand)));
   PSR_TRY(w.counts.ensure((4 * outer + 4) * 4));
   PSR_TRY(w.floors.ensure(outer * 4));

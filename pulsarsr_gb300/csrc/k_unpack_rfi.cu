@@ -346,8 +346,8 @@ __global__ void __launch_bounds__(MH_NT)
   if (total) atomicAdd(&hist[(uint64_t)blockIdx.y * 256 + tid], total);
 }
 
-// Element of rank ns / 2 from each row's histogram (one thread per row).
-// One warp per channel: 8 bins per lane, a prefix over the lanes.
+// Element of rank ns / 2 from each row's histogram: one warp per channel, 8 bins
+// per lane, a prefix over the lanes.
 __global__ void __launch_bounds__(128)
     k_hist_median(const unsigned *__restrict__ hist, uint64_t nch, uint64_t ns,
                   float *__restrict__ med) {

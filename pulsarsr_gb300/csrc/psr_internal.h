@@ -270,8 +270,8 @@ struct SpecWork {
   uint64_t raw_cap = 0;  // raw (pre-dedupe) candidates per trial
   uint64_t lds = 0;      // row stride of scale[]
 };
-int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, uint64_t inner,
-                     SpecWork &w, cudaStream_t st);
+int spectrum_prepare(const FftPlan &p, const SpecConfig &c, uint64_t outer, SpecWork &w,
+                     cudaStream_t st);
 int spectrum_reset(SpecWork &w, uint64_t outer_trials, cudaStream_t st);
 int spectrum_gate(const FftPlan &p, const SpecConfig &c, const float *d_power, uint64_t ldp,
                   const double *d_psum, uint32_t npsum, uint64_t ntrials, uint64_t slot0,
@@ -320,7 +320,7 @@ struct SubbandPlan : SubbandShape {
 };
 // The subband width searches use when not told otherwise: the process-wide
 // setting of psr_set_dedisp_subbands (-1: chosen from the delay table).
-int dedisp_subbands_default(const DeviceObs &o);
+int dedisp_subbands_default();
 // n: series length; maxv: largest sample (0: no plan); G: 4, 8, 0 (no plan)
 // or -1 (the cheapest; with `once`, counting what the plan takes to make).  A plan
 // that does not fit, or for which there is no device memory, leaves plan.G = 0 and

@@ -51,7 +51,7 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   PSR_TRY(work.ensure(fft.m > 12 ? inner * fft.M * 8 : 16));
   PSR_TRY(power.ensure(2 * chunk * ldp * 4));
   PSR_TRY(psum.ensure(2 * chunk * npsum * 8));
-  PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
+  PSR_TRY(spectrum_prepare(fft, spec, chunk, sw, st));
   PSR_TRY(kept.ensure(list_bytes() + ntrials * 4));
   const uint64_t tail = chunk >= 16 && ntrials > chunk ? chunk / 8 : 0;
   cstart.clear();
@@ -63,7 +63,7 @@ int SearchEngine::prepare(const DeviceObs &o, const double *trials, uint64_t ntr
   nchunks = cstart.size() - 1;
   PSR_TRY(status.ensure(nchunks * 4 + 16));
   PSR_CUDA(cudaMemsetAsync(err(), 0, 4, st));
-  const int G = subbands >= 0 ? subbands : dedisp_subbands_default(o);
+  const int G = subbands >= 0 ? subbands : dedisp_subbands_default();
   PSR_TRY(build_subband_plan(tab, o.nch, n, o.kind == SAMPLE_U8 ? o.max_value() : 0.0, cstart, G,
                              sbplan, st, once, scratch));
   if (!aux) PSR_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
@@ -227,7 +227,7 @@ int SearchEngine::finish(const DeviceObs &o, cudaStream_t st) {
         if (ov[ci] & OVERFLOW_QUEUE) sw.queue_full = true;
         if (ov[ci] & OVERFLOW_EXACT) sw.xgrow *= 4;
         ++sw.grown;
-        PSR_TRY(spectrum_prepare(fft, spec, chunk, inner, sw, st));
+        PSR_TRY(spectrum_prepare(fft, spec, chunk, sw, st));
       }
       ran_at = sw.grown;
       PSR_TRY(stands ? enqueue_spectrum(ci, st) : enqueue_chunk(o, ci, st));
