@@ -29,7 +29,7 @@
 // Bound: instruction issue (about 2.5 M warp instructions per 2^20-point
 // trial) at half occupancy (64 registers, 2 CTAs of 512 threads per SM).
 // Measured on a GB300, 2^20 points, 700 trials: pass 1 1.68 -> 1.55 ms, pass 2
-// 1.67 -> 1.34 ms against stages that all went through shared memory.
+// 1.67 -> 1.37 ms against stages that all went through shared memory.
 #include <cuda_runtime.h>
 
 #include <type_traits>

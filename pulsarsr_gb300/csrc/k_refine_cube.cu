@@ -622,7 +622,8 @@ __device__ __forceinline__ float sample_float(unsigned v) {
 // warps' sums go into their own tiles' memory, so that three CTAs fit an SM.
 // Bound: issue; conversions and ceilings, on the quarter-rate pipe, are done by
 // sums at 2^23.  Measured on a GB300, 256 channels of 1,048,576 f32 samples, 0.3
-// bins per sample: 1.05 ms before, 0.50 now (0.16 for the bytes).
+// bins per sample: 1.05 ms before, 0.57 now (0.16 for the bytes; 0.50 with channel
+// sums in f32 pairs, which are fewer bits than f64).
 constexpr int CB_TL = 2048;
 constexpr int CB_BO_MAXB = 256;
 constexpr int CB_BO_NB = CB_BO_MAXB / 32;
