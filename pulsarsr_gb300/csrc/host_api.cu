@@ -104,7 +104,9 @@ cudaError_t alloc_raw(void **p, size_t n, cudaStream_t &st, bool &pooled) {
 }  // namespace
 
 cudaError_t device_alloc(void **p, size_t n, cudaStream_t &st, bool &pooled) {
-  if ((int64_t)n > t_mem.limit - t_mem.held) return cudaErrorMemoryAllocation;
+  // (held is below 0 on a thread that frees what others made)
+  if (t_mem.limit != INT64_MAX && t_mem.held > t_mem.limit - (int64_t)n)
+    return cudaErrorMemoryAllocation;
   const cudaError_t e = alloc_raw(p, n, st, pooled);
   if (e == cudaSuccess) {
     t_mem.held += (int64_t)n;

@@ -194,3 +194,26 @@ def test_confirmation_of_a_session(observation):
     of_session = confirmation.analyze_session(s)
     assert memory()[2] <= calls
     assert len(of_fb.data) and of_fb.json() == of_session.json()
+
+
+@pytest.mark.gpu
+def test_freed_by_another_thread(gpu):
+    """A handle made on one thread and closed on another, which goes on allocating."""
+    import threading
+
+    from pulsarsr_gb300 import synth
+
+    def make():
+        return synth.device(4, 8, 60000, 64e-6, 1500.0, -4.0, seed=3, noise_mean=100.0,
+                            noise_sigma=20.0)
+
+    fb, seen = make(), []
+
+    def work():
+        fb.close()
+        seen.append(make().data.shape)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert seen == [(4, 60000)]
